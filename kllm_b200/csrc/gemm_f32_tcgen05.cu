@@ -1,0 +1,490 @@
+// y = x . W^T of float32 matrices on the fifth-generation tensor cores, at float32 accuracy.
+//
+//   x [M, K] float32 (K contiguous), W [N, K] float32 (a projection's weight as the checkpoint
+//   stores it), y float32: stored, added into, or silu(x Wg^T) * (x Wu^T).
+//
+// The reference runs these products through cublasSgemm (backend/model.cu:496-503); on the
+// CUDA cores they are bound by the FMA rate (the library reached 50 TFLOP/s at 1003 rows of
+// TinyLlama's sizes).  Here every float32 number is the sum of three bfloat16 numbers,
+//     v = v0 + v1 + v2,  v0 = bf16(v), v1 = bf16(v - v0), v2 = bf16(v - v0 - v1)
+// (8 + 8 + 8 bits of mantissa: exact unless v2 is below the smallest bfloat16), and
+//     x w = x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0) + terms below 2^-24 |x w|,
+// six tcgen05 products with float32 accumulators.  An accumulator only ever holds one k block
+// (32 values of k, the small terms first): it is then added, by the rounding add of the CUDA
+// cores, to a sum in registers, so that the tensor core's own accumulation, which cuts digits
+// off, cannot drift over a long K.
+//
+// Two kernels.  `split_kernel` writes the three parts of a matrix as three bfloat16 planes;
+// `gemm_f32_tc5_kernel` multiplies planes.  W is taken in pieces of rows whose planes (6 bytes a
+// number) stay in L2 between the two (PLANE_LIMIT).  A kernel that split inside the product, in
+// registers, was measured at 392 us for 1003 x 11264 x 2048 (the splitting warps' loads were
+// exposed, and every tile of x split the same weights again).
+//
+// The product: one persistent CTA per SM, tiles of 128 rows x 256 columns (gated: 128 gate rows
+// of W and the 128 up rows beside them), ten warps:
+//   warp 0     one lane loads the planes of a k block by TMA (64-byte rows, 64-byte swizzle; 72 KB
+//              a stage, three stages),
+//   warp 1     one lane issues the 12 tcgen05.mma (2 k steps x 6 terms) of a block into one of two
+//              accumulators,
+//   warps 2-9  fetch each finished accumulator (tcgen05.ld) and add it to their sums: a thread
+//              owns one row of half of the tile's columns, and stores it at the end of the tile.
+// Where the tiles leave SMs idle (few rows, narrow matrices) the k range is cut into splits
+// of whole blocks, each a unit of work of its own that leaves its sums in a workspace;
+// a third kernel adds them in split order.
+//
+// A row of x or W that holds an infinity or a NaN gives NaN (the parts of an infinity are
+// an infinity and NaN); finite numbers of any size are split exactly.
+#include "common.cuh"
+
+KLLM_EXPORT_LAST_ERROR(gemm_f32_tcgen05)
+
+#include "tc5_common.cuh"
+
+namespace {
+
+constexpr int BM = 128, BN = 256;
+constexpr int BK = 32;                          // a row of a plane is 64 bytes
+constexpr int THREADS = 320;
+constexpr int FETCHERS = 256;
+constexpr int STAGES = 3;
+constexpr int A_PLANE = BM * 64, B_PLANE = BN * 64;
+constexpr int STAGE_BYTES = 3 * (A_PLANE + B_PLANE);
+constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES;
+constexpr int TMEM_COLS = 512;
+// Bytes of the planes of one piece of W: with x's planes and the result they stay in the 126 MB of L2.
+constexpr long long PLANE_LIMIT = 72LL << 20;
+
+enum Epilogue { EPI_STORE = 0, EPI_ADD = 1, EPI_SWIGLU = 2, EPI_PARTIAL = 3 };
+
+// K-major operand in the 64-byte swizzled layout: 8-row groups 512 bytes apart, layout type 4
+__device__ __forceinline__ uint64_t make_desc64(unsigned addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
+// two numbers into their three bfloat16 parts.  The first part is taken of the number clamped
+// to the largest bfloat16, so that a finite number never becomes an infinity.
+__device__ __forceinline__ void split2(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
+    constexpr float TOP = 3.3895313892515355e38f;
+    p0 = pack_bf16(fminf(fmaxf(a, -TOP), TOP), fminf(fmaxf(b, -TOP), TOP));
+    const float ra = a - __uint_as_float(p0 << 16), rb = b - __uint_as_float(p0 & 0xffff0000u);
+    p1 = pack_bf16(ra, rb);
+    p2 = pack_bf16(ra - __uint_as_float(p1 << 16), rb - __uint_as_float(p1 & 0xffff0000u));
+}
+
+// planes [3][plane_rows][kp] of the rows of src [rows, K] at ld, from plane row `row0` on; a second matrix (src2) may
+// follow after the first one's rows.  Memory bound: 4 bytes read and 6 written a number.
+__global__ void split_kernel(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld, int rows, int K,
+                             bf16* __restrict__ planes, int64_t plane_rows, int kp) {
+    griddep_launch();
+    griddep_wait();
+    const int pieces = kp / 8;
+    const int64_t plane = plane_rows * kp, total = (int64_t)rows * (src2 ? 2 : 1) * pieces;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / pieces;
+        const int k = (int)(i - r * pieces) * 8;
+        const float* p = (r < rows ? src + r * ld : src2 + (r - rows) * ld) + k;
+        const float4 u = __ldg(reinterpret_cast<const float4*>(p));                     // K is a multiple of 4
+        const float4 v = k + 4 < K ? __ldg(reinterpret_cast<const float4*>(p + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint4 q0, q1, q2;
+        split2(u.x, u.y, q0.x, q1.x, q2.x);
+        split2(u.z, u.w, q0.y, q1.y, q2.y);
+        split2(v.x, v.y, q0.z, q1.z, q2.z);
+        split2(v.z, v.w, q0.w, q1.w, q2.w);
+        bf16* o = planes + r * kp + k;
+        *reinterpret_cast<uint4*>(o) = q0;
+        *reinterpret_cast<uint4*>(o + plane) = q1;
+        *reinterpret_cast<uint4*>(o + 2 * plane) = q2;
+    }
+}
+
+struct Args {
+    float* y;
+    int64_t ldy, split_stride;              // split_stride: elements between the workspace's splits
+    int M, N, K, splits, blocks_per_split;
+    int a_rows, b_rows;                     // rows of a plane of x and of W (gated: gate rows, then up rows)
+    int* status;
+};
+
+template <int EPI>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Args a) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
+    __shared__ unsigned s_tmem;
+    __shared__ int s_abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    constexpr int NOUT = EPI == EPI_SWIGLU ? BN / 2 : BN;
+    const int m_tiles = (a.M + BM - 1) / BM, n_tiles = (a.N + NOUT - 1) / NOUT;
+    const int units = m_tiles * n_tiles * a.splits;
+    const int kblocks = (a.K + BK - 1) / BK;
+    volatile int* abort_flag = &s_abort;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], FETCHERS); }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = s_tmem;
+    griddep_launch();
+    griddep_wait();
+
+    if (warp == 0) {
+        // ---- producer ----
+        int s = 0, issued = 0;
+        unsigned ph = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+            const int split = unit / (m_tiles * n_tiles), tile = unit - split * (m_tiles * n_tiles);
+            const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * NOUT;
+            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = mbar_wait(&bar_empty[s], ph ^ 1u, abort_flag, a.status, 1);
+                if (!ok) break;
+                if (lane == 0) {
+                    const unsigned pa = base + (unsigned)(s * STAGE_BYTES), pb = pa + 3 * A_PLANE;
+                    mbar_expect_tx(&bar_full[s], (unsigned)STAGE_BYTES);
+#pragma unroll
+                    for (int p = 0; p < 3; p++) {
+                        tma_load_2d(pa + p * A_PLANE, &map_a, kb * BK, p * a.a_rows + m0, &bar_full[s]);
+                        if (EPI == EPI_SWIGLU) {
+                            tma_load_2d(pb + p * B_PLANE, &map_b, kb * BK, p * a.b_rows + n0, &bar_full[s]);
+                            tma_load_2d(pb + p * B_PLANE + B_PLANE / 2, &map_b, kb * BK, p * a.b_rows + a.N + n0, &bar_full[s]);
+                        } else {
+                            tma_load_2d(pb + p * B_PLANE, &map_b, kb * BK, p * a.b_rows + n0, &bar_full[s]);
+                        }
+                    }
+                }
+                __syncwarp();
+                issued++;
+                if (++s == STAGES) { s = 0; ph ^= 1u; }
+            }
+        }
+        if (!ok || *abort_flag) {
+            // copies still in flight must land before the shared memory goes away
+            const int back = issued < STAGES ? issued : STAGES;
+            for (int j = 0; j < back; j++) {
+                int sj = s - 1 - j;
+                unsigned pj = ph;
+                if (sj < 0) { sj += STAGES; pj ^= 1u; }
+                const long long t0 = clock64();
+                while (!mbar_try_wait(&bar_full[sj], pj) && clock64() - t0 < kCycleLimit) {}
+            }
+        }
+    } else if (warp == 1) {
+        // ---- tensor-core issuer ----
+        const uint32_t idesc = make_idesc(BM, BN);
+        int s = 0, acc = 0;
+        unsigned ph = 0, acc_ph = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+            const int split = unit / (m_tiles * n_tiles);
+            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = mbar_wait(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, a.status, 2) &&
+                     mbar_wait(&bar_full[s], ph, abort_flag, a.status, 3);
+                if (!ok) break;
+                tc_fence_after();
+                if (lane == 0) {
+                    const unsigned d = tmem + (unsigned)(acc * BN);
+                    const unsigned pa = base + (unsigned)(s * STAGE_BYTES), pb = pa + 3 * A_PLANE;
+                    constexpr int TA[6] = {0, 2, 1, 0, 1, 0}, TB[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+                    for (int t = 0; t < 6; t++)
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; kk++)
+                            umma(d, make_desc64(pa + TA[t] * A_PLANE + kk * 32), make_desc64(pb + TB[t] * B_PLANE + kk * 32),
+                                 idesc, kk > 0 || t > 0);
+                    umma_commit(&bar_empty[s]);
+                    umma_commit(&bar_acc_full[acc]);
+                }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ph ^= 1u; }
+                acc ^= 1;
+                if (acc == 0) acc_ph ^= 1u;
+            }
+        }
+    } else {
+        // ---- sums and epilogue ----
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const unsigned lane_base = (unsigned)(quarter * 32) << 16;
+        int acc = 0;
+        unsigned acc_ph = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
+            const int split = unit / (m_tiles * n_tiles), tile = unit - split * (m_tiles * n_tiles);
+            const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * NOUT;
+            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+            float sum[4][32];
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+#pragma unroll
+                for (int j = 0; j < 32; j++) sum[c][j] = 0.f;
+            for (int kb = kb0; kb < kb1; kb++) {
+                ok = mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, a.status, 4);
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned t = tmem + lane_base + (unsigned)(acc * BN);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    float v[32];
+                    // gated: two pieces of gate columns, then the two of the same up columns
+                    tmem_ld32(t + (EPI == EPI_SWIGLU ? (c >> 1) * 128 + half * 64 + (c & 1) * 32 : half * 128 + c * 32), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) sum[c][j] += v[j];
+                }
+                tc_fence_before();
+                mbar_arrive(&bar_acc_empty[acc]);
+                acc ^= 1;
+                if (acc == 0) acc_ph ^= 1u;
+            }
+            if (!ok) break;
+            const int r = m0 + quarter * 32 + lane;
+            if (r < a.M) {
+                float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (int64_t)r * a.ldy;
+                constexpr int CH = EPI == EPI_SWIGLU ? 2 : 4;
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        if (col + 4 * q < a.N) {                    // N is a multiple of 4
+                            float4 o;
+                            if constexpr (EPI == EPI_SWIGLU) {
+                                o.x = silu_mul(sum[c][4 * q], sum[c + 2][4 * q]);
+                                o.y = silu_mul(sum[c][4 * q + 1], sum[c + 2][4 * q + 1]);
+                                o.z = silu_mul(sum[c][4 * q + 2], sum[c + 2][4 * q + 2]);
+                                o.w = silu_mul(sum[c][4 * q + 3], sum[c + 2][4 * q + 3]);
+                            } else {
+                                o = make_float4(sum[c][4 * q], sum[c][4 * q + 1], sum[c][4 * q + 2], sum[c][4 * q + 3]);
+                            }
+                            float4* p = reinterpret_cast<float4*>(y + col + 4 * q);
+                            if (EPI == EPI_ADD) {
+                                const float4 h = *p;
+                                o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
+                            }
+                            *p = o;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+}
+
+// The splits' sums, in split order, into the result: stored, added, or (gated: [M, 2 N] sums, the up columns behind the
+// gate columns) silu(gate) * up.  Bound by the workspace's bytes, which lie in L2.
+template <int EPI>
+__global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const float* __restrict__ ws, int64_t split_stride,
+                                     int M, int N, int splits) {
+    griddep_launch();
+    griddep_wait();
+    const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? 2 * N : N;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)M * n4; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t r = i / n4;
+        const int c = (int)(i - r * n4) * 4;
+        auto sum = [&](const float* p) {
+            float4 v = *reinterpret_cast<const float4*>(p);
+            for (int s = 1; s < splits; s++) {
+                const float4 u = *reinterpret_cast<const float4*>(p + s * split_stride);
+                v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+            }
+            return v;
+        };
+        float4 v = sum(ws + r * ldw + c);
+        float4* o = reinterpret_cast<float4*>(y + r * ldy + c);
+        if (EPI == EPI_ADD) {
+            const float4 h = *o;
+            v.x += h.x; v.y += h.y; v.z += h.z; v.w += h.w;
+        } else if (EPI == EPI_SWIGLU) {
+            const float4 u = sum(ws + r * ldw + N + c);
+            v.x = silu_mul(v.x, u.x); v.y = silu_mul(v.y, u.y); v.z = silu_mul(v.z, u.z); v.w = silu_mul(v.w, u.w);
+        }
+        *o = v;
+    }
+}
+
+// ---- host side -----------------------------------------------------------------
+
+int planes_map(CUtensorMap* out, const bf16* planes, int64_t rows, int K, int kp, int box_rows) {
+    EncodeTiledFn fn = encoder();
+    if (!fn) KLLM_FAIL("gemm float32 (tcgen05): the driver does not offer cuTensorMapEncodeTiled");
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)kp * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)planes, dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) KLLM_FAIL("gemm float32 (tcgen05): tensor map for %lld x %d planes refused: %d", (long long)rows, K, (int)r);
+    return 0;
+}
+
+template <int EPI>
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Args& a, cudaStream_t s) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e != cudaSuccess) {
+            snprintf(g_kllm_err, sizeof(g_kllm_err), "gemm float32 (tcgen05): %d bytes of shared memory refused: %s", SMEM_BYTES,
+                     cudaGetErrorString(e));
+            return (int)e;
+        }
+        attr_set = true;
+    }
+    const int nout = EPI == EPI_SWIGLU ? BN / 2 : BN;
+    const long long units = (long long)((a.M + BM - 1) / BM) * ((a.N + nout - 1) / nout) * a.splits;
+    const int grid = (int)(units < sm_count() ? units : sm_count());
+    kllm_launch((gemm_f32_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, s, ma, mb, a);
+    KLLM_LAUNCH_STATUS();
+}
+
+int launch_split(const float* src, const float* src2, int64_t ld, int rows, int K, bf16* planes, int64_t plane_rows, int kp,
+                 cudaStream_t s) {
+    const int64_t work = (int64_t)rows * (src2 ? 2 : 1) * (kp / 8);
+    const int64_t blocks = (work + 255) / 256, most = 8LL * sm_count();
+    kllm_launch((split_kernel), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, src, src2, ld, rows, K, planes,
+                plane_rows, kp);
+    KLLM_LAUNCH_STATUS();
+}
+
+template <int EPI>
+int launch_reduce(float* y, int64_t ldy, const float* ws, int64_t split_stride, int M, int N, int splits, cudaStream_t s) {
+    const int64_t blocks = ((int64_t)M * (N / 4) + 255) / 256, most = 8LL * sm_count();
+    kllm_launch((reduce_splits_kernel<EPI>), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, y, ldy, ws, split_stride,
+                M, N, splits);
+    KLLM_LAUNCH_STATUS();
+}
+
+// How a product is cut: W in pieces of `piece` output columns (whole tiles, the last piece takes the rest), a piece's K
+// in `splits` ranges.  The cost that is made least, in k blocks of one CTA (0.8 us): a unit costs its blocks and about 3
+// for filling the pipeline and storing; a launch about 3; split sums are written and read at about 4 MB a block's time.
+struct Plan {
+    int piece, splits, kp;
+    int64_t a_bytes, b_bytes, ws_bytes;
+};
+int64_t up256(int64_t b) { return (b + 255) / 256 * 256; }
+
+Plan make_plan(int M, int N, int K, int epilogue) {
+    Plan p;
+    const bool gated = epilogue == EPI_SWIGLU;
+    const int nout = gated ? BN / 2 : BN, sms = sm_count(), kblocks = (K + BK - 1) / BK;
+    p.kp = (K + 7) / 8 * 8;
+    const long long m_tiles = (M + BM - 1) / BM, n_tiles = (N + nout - 1) / nout;
+    long long most = PLANE_LIMIT / (6LL * p.kp * BN);
+    if (most < 1) most = 1;
+    if (most > n_tiles) most = n_tiles;
+    double best = -1;
+    p.piece = N;
+    p.splits = 1;
+    for (long long c = most; c >= 1; c--) {
+        const long long full = n_tiles / c, rest = n_tiles - full * c;
+        for (int s = 1; s <= 16; s++) {
+            const int per = (kblocks + s - 1) / s;
+            if (s > 1 && (per < 6 || (kblocks + per - 1) / per != s)) continue;
+            auto cost = [&](long long tiles) {
+                const double sums = s > 1 ? 3.0 + 8.0 * s * (double)M * tiles * BN / 4e6 : 0.0;
+                return (double)((m_tiles * tiles * s + sms - 1) / sms) * (per + 3) + 3.0 + sums;
+            };
+            const double all = full * cost(c) + (rest ? cost(rest) : 0.0);
+            if (best < 0 || all < best) { best = all; p.piece = c == n_tiles ? N : (int)c * nout; p.splits = s; }
+        }
+    }
+    const int64_t cols = (int64_t)p.piece * (gated ? 2 : 1);
+    p.a_bytes = up256(6LL * M * p.kp);
+    p.b_bytes = up256(6LL * cols * p.kp);
+    p.ws_bytes = p.splits > 1 ? up256(4LL * p.splits * M * cols) : 0;
+    return p;
+}
+
+}  // namespace
+
+// Bytes of workspace that the product of these sizes wants (256-byte aligned, its own until it has run).
+extern "C" int kllm_gemm_f32_tcgen05_workspace(int M, int N, int K, int epilogue, int64_t* bytes) {
+    if (M <= 0 || N <= 0 || K <= 0) { *bytes = 0; return 0; }
+    const Plan p = make_plan(M, N, K, epilogue);
+    *bytes = p.a_bytes + p.b_bytes + p.ws_bytes;
+    return 0;
+}
+
+// 1 if the kernel takes these sizes and addresses, else 0.
+extern "C" int kllm_gemm_f32_tcgen05_fits(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* w_up, int M,
+                                          int N, int K, const void* y, int64_t ldy, int epilogue) {
+    if (M <= 0 || N <= 0 || K <= 0 || epilogue < 0 || epilogue > 2) return 0;
+    if ((K & 3) || (N & 3) || (ldx & 3) || (ldw & 3) || (ldy & 3)) return 0;           // 16-byte loads and stores
+    if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)w_up & 15) || ((uintptr_t)y & 15)) return 0;
+    if (ldx < K || ldw < K || ldy < N) return 0;
+    if (epilogue == EPI_SWIGLU && !w_up) return 0;
+    if (M > (1 << 28) || N > (1 << 28)) return 0;                                       // plane rows are 32-bit coordinates
+    const long long tiles = ((long long)(M + BM - 1) / BM) * ((N + BN / 2 - 1) / (BN / 2));
+    return tiles * 16 < (1LL << 31) ? 1 : 0;
+}
+
+// epilogue 0: y = x W^T, 1: y += x W^T, 2: y = silu(x W^T) * (x W_up^T).  ws: kllm_gemm_f32_tcgen05_workspace bytes.
+// status: device int that a wait which ran out sets (1: stage free, 2: accumulator free, 3: stage full, 4: accumulator full).
+extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* w_up, int M, int N,
+                                     int K, void* y, int64_t ldy, int epilogue, void* ws, int* status, void* stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (!kllm_gemm_f32_tcgen05_fits(x, ldx, w, ldw, w_up, M, N, K, y, ldy, epilogue) || ((uintptr_t)ws & 255) || !ws)
+        KLLM_FAIL("gemm float32 (tcgen05): sizes %d x %d x %d, strides %lld/%lld/%lld or an address not taken (sizes and "
+                  "strides multiples of 4, 16-byte aligned addresses)", M, N, K, (long long)ldx, (long long)ldw, (long long)ldy);
+    const Plan p = make_plan(M, N, K, epilogue);
+    const bool gated = epilogue == EPI_SWIGLU;
+    const int kblocks = (K + BK - 1) / BK;
+    bf16* pa = (bf16*)ws;
+    bf16* pb = (bf16*)((char*)ws + p.a_bytes);
+    float* part = (float*)((char*)ws + p.a_bytes + p.b_bytes);
+    cudaStream_t s = (cudaStream_t)stream;
+    int r = launch_split((const float*)x, nullptr, ldx, M, K, pa, M, p.kp, s);
+    if (r) return r;
+    CUtensorMap ma, mb;
+    r = planes_map(&ma, pa, 3LL * M, K, p.kp, BM);
+    if (r) return r;
+    Args a;
+    a.M = M; a.K = K; a.splits = p.splits; a.blocks_per_split = (kblocks + p.splits - 1) / p.splits; a.status = status;
+    a.a_rows = M;
+    for (int n0 = 0; n0 < N; n0 += p.piece) {
+        const int cols = N - n0 < p.piece ? N - n0 : p.piece;
+        float* yp = (float*)y + n0;
+        a.b_rows = cols * (gated ? 2 : 1);
+        r = launch_split((const float*)w + n0 * ldw, gated ? (const float*)w_up + n0 * ldw : nullptr, ldw, cols, K, pb, a.b_rows, p.kp, s);
+        if (r) return r;
+        // with splits a gated piece is a plain product with the gate and up columns beside each other
+        const bool pairs = gated && p.splits == 1;
+        r = planes_map(&mb, pb, 3LL * a.b_rows, K, p.kp, pairs ? BN / 2 : BN);
+        if (r) return r;
+        if (p.splits == 1) {
+            a.N = cols; a.y = yp; a.ldy = ldy; a.split_stride = 0;
+            r = epilogue == EPI_STORE ? launch<EPI_STORE>(ma, mb, a, s) : epilogue == EPI_ADD ? launch<EPI_ADD>(ma, mb, a, s)
+                                                                                             : launch<EPI_SWIGLU>(ma, mb, a, s);
+        } else {
+            a.N = a.b_rows; a.y = part; a.ldy = a.b_rows; a.split_stride = (int64_t)M * a.b_rows;
+            r = launch<EPI_PARTIAL>(ma, mb, a, s);
+            if (r) return r;
+            r = epilogue == EPI_STORE ? launch_reduce<EPI_STORE>(yp, ldy, part, a.split_stride, M, cols, p.splits, s)
+                : epilogue == EPI_ADD ? launch_reduce<EPI_ADD>(yp, ldy, part, a.split_stride, M, cols, p.splits, s)
+                                      : launch_reduce<EPI_SWIGLU>(yp, ldy, part, a.split_stride, M, cols, p.splits, s);
+        }
+        if (r) return r;
+    }
+    return 0;
+}

@@ -1255,7 +1255,7 @@ def _skinny_gemm_f32(weight, x, x_f32, gain, eps, rows, n_rows, weight_up, epilo
 
 
 def linear_add(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> None:
-    """acc += x @ weight^T through the vendor GEMM library, acc float32 (the residual
+    """acc += x @ weight^T through the vendor GEMM library (large float32 products: ``gemm_f32``), acc float32 (the residual
     stream), the sum formed in float32 inside the product's epilogue: what the reference
     does in a kernel of its own after cublasSgemm (backend/model.cu:97-110)."""
     _cuda(acc, x, weight)
@@ -1263,7 +1263,9 @@ def linear_add(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> None
         raise KernelError("TF32 matmul mode is on; the float32 path must stay true 32-bit")
     if acc.dtype != torch.float32 or not acc.is_contiguous():
         raise KernelError("linear_add: the matrix added into must be contiguous float32")
-    if x.dtype == torch.float32:
+    if x.dtype == torch.float32 and gemm_f32_fits(x, weight, acc):
+        gemm_f32(x, weight, epilogue="add", out=acc)
+    elif x.dtype == torch.float32:
         torch.addmm(acc, x, weight.t(), out=acc)
     else:
         torch.addmm(acc, x, weight.t(), out_dtype=torch.float32, out=acc)
@@ -1351,6 +1353,72 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "bf16", out: 
     return out
 
 
+# From these sizes on a float32 product runs on the tensor cores (csrc/gemm_f32_tcgen05.cu), below them through the
+# library, both timed over 9 to 2048 rows.  The weights' three parts are written and read back by every call: at 16 rows
+# that costs what the tensor cores save (the four products of a TinyLlama layer: 204 us against 218), at 33 rows 216 us
+# against 322.  A matrix whose parts are larger than L2 goes through HBM again: 32000 x 2048 takes 271 us against the
+# library's 178 at 64 rows and 302 against 313 at 128.  Small matrices are latency: 1024 x 512 at 1003 rows 31.8 against 30.8.
+GEMM_F32_LEAST_ROWS = 33
+GEMM_F32_LEAST_WEIGHTS = 1 << 20
+GEMM_F32_L2_WEIGHTS = 25 << 20          # 150 MB of parts: about what L2 and the write-back in flight hide
+GEMM_F32_ROWS_BEYOND_L2 = 128
+
+
+def gemm_f32_fits(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, epilogue: str = "f32",
+                  weight_up: Optional[torch.Tensor] = None) -> bool:
+    """Whether ``gemm_f32`` takes these operands and is the faster route (float32, dense rows, sizes and row strides
+    multiples of 4, 16-byte aligned addresses)."""
+    if not USE_TCGEN05 or x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or weight.dim() != 2:
+        return False
+    n, K = x.shape
+    N = weight.shape[0]
+    if n < (GEMM_F32_LEAST_ROWS if N * K <= GEMM_F32_L2_WEIGHTS else GEMM_F32_ROWS_BEYOND_L2):
+        return False
+    if weight.shape[1] != K or N * K < GEMM_F32_LEAST_WEIGHTS or (N | K) & 3:
+        return False
+    for t in (x, weight, weight_up, out):
+        if t is not None and (t.dtype != torch.float32 or t.stride(1) != 1 or t.stride(0) & 3 or t.data_ptr() & 15
+                              or t.stride(0) < t.shape[1]):
+            return False
+    return weight_up is None or (weight_up.shape == weight.shape and weight_up.stride() == weight.stride())
+
+
+def gemm_f32(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "f32", out: Optional[torch.Tensor] = None,
+             weight_up: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """y = x @ weight^T of float32 matrices at float32 accuracy on the tcgen05 tensor cores (csrc/gemm_f32_tcgen05.cu:
+    every number as three bfloat16 parts, six products).
+
+    ``epilogue``: "f32" stores y [n, N]; "add" adds it into ``out``; "swiglu" takes ``weight`` as gate and ``weight_up``
+    as up matrix and stores silu(gate) * up."""
+    _cuda(x, weight, weight_up, out)
+    n, N = x.shape[0], weight.shape[0]
+    if out is None:
+        if epilogue == "add":
+            raise KernelError("gemm_f32: 'add' needs the matrix to add into")
+        out = torch.empty((n, N), dtype=torch.float32, device=x.device)
+    if out.dtype != torch.float32 or tuple(out.shape) != (n, N):
+        raise KernelError("gemm_f32: out has the wrong dtype or shape")
+    if epilogue == "swiglu" and weight_up is None:
+        raise KernelError("gemm_f32: swiglu needs an up matrix like the gate matrix")
+    lib = load_library("gemm_f32_tcgen05")
+    epi = {"f32": 0, "add": 1, "swiglu": 2}[epilogue]
+    dense = all(t is None or (t.dtype == torch.float32 and t.dim() == 2 and t.stride(1) == 1) for t in (x, weight, weight_up, out))
+    if not dense or x.shape[1] != weight.shape[1] or (weight_up is not None and (
+            weight_up.shape != weight.shape or weight_up.stride() != weight.stride())) \
+            or not lib.kllm_gemm_f32_tcgen05_fits(_p(x), ctypes.c_int64(x.stride(0)), _p(weight), ctypes.c_int64(weight.stride(0)),
+                                                  _p(weight_up), n, N, x.shape[1], _p(out), ctypes.c_int64(out.stride(0)), epi):
+        raise KernelError(f"gemm_f32: operands {tuple(x.shape)} x {tuple(weight.shape)} (strides {x.stride()}, "
+                          f"{weight.stride()}, out {out.stride()}) are not supported")
+    size = ctypes.c_int64(0)
+    lib.kllm_gemm_f32_tcgen05_workspace(n, N, x.shape[1], epi, ctypes.byref(size))
+    ws = torch.empty(size.value, dtype=torch.uint8, device=x.device)
+    rc = lib.kllm_gemm_f32_tcgen05(_p(x), ctypes.c_int64(x.stride(0)), _p(weight), ctypes.c_int64(weight.stride(0)),
+                                   _p(weight_up), n, N, x.shape[1], _p(out), ctypes.c_int64(out.stride(0)), epi,
+                                   _p(ws), _p(status_word(x.device)), _stream())
+    _check(lib, "gemm_f32_tcgen05", rc)
+    return out
+
+
 _bmm_takes_out_dtype = None
 
 
@@ -1434,8 +1502,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
     """y = x @ weight^T through the vendor GEMM library (cuBLAS, via torch.mm), as
     the reference does for every projection (backend/model.cu:496-503).
 
-    float32 operands run as true float32 (the reduced-precision TF32 mode stays
-    off); bfloat16 operands accumulate in float32.  ``small_ok`` with a float32 result: a step
+    float32 operands run at float32 accuracy, large ones on this repository's tensor-core kernel (``gemm_f32``), the
+    others as true float32 (the reduced-precision TF32 mode stays off); bfloat16 operands accumulate in float32.  ``small_ok`` with a float32 result: a step
     of a few rows (``skinny_fits``) takes this repository's weight-streaming product instead,
     which reads the matrix once at the speed of HBM; which of the two runs depends on the row
     count alone.
@@ -1450,6 +1518,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = 
         raise KernelError("TF32 matmul mode is on; the float32 path must stay true 32-bit")
     if out_dtype is not None and out_dtype != x.dtype:
         return torch.mm(x, weight.t(), out_dtype=out_dtype)
+    if x.dtype == torch.float32 and gemm_f32_fits(x, weight, out):
+        return gemm_f32(x, weight, out=out)
     if out is not None:
         return torch.mm(x, weight.t(), out=out)
     return torch.mm(x, weight.t())

@@ -95,6 +95,8 @@ class GatedMLP:
                 and kernels.gemm_fits(xn, w_gate, act, epilogue, w_up)):
             # large portions: both products and the activation in one tcgen05 kernel
             kernels.gemm(xn, w_gate, weight_up=w_up, epilogue=epilogue, out=act, limit=self.limit, alpha=self.alpha)
+        elif epilogue == "swiglu" and kernels.gemm_f32_fits(xn, w_gate, act, epilogue, w_up):
+            kernels.gemm_f32(xn, w_gate, weight_up=w_up, epilogue=epilogue, out=act)
         else:
             gu = kernels.linear(xn, self.w_gate_up, out_dtype=torch.float32)
             if self.activation == "clamped":

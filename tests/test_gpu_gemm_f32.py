@@ -1,0 +1,80 @@
+"""The float32 product on the tensor cores (csrc/gemm_f32_tcgen05.cu) against float64, at the edges of its tiles (128
+rows, 256 columns, k blocks of 32), with and without splits of K, in one piece of W and in several."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [  # rows, columns, k
+    (1, 4, 4), (33, 256, 32), (127, 252, 36), (128, 260, 60), (129, 512, 100), (300, 1028, 2052), (33, 2560, 2048),
+    (257, 4100, 160),
+    (131, 11264, 1100),       # W in pieces: its parts are larger than what stays in L2
+]
+
+
+def _bound(K):
+    # An element's error over sqrt(mean square of the results): the dropped terms are below 2^-24 of every product, an
+    # accumulator of 12 products cuts less than 12 x 2^-23 of what it holds, and K / 32 rounded adds follow: a random walk
+    # of sqrt(K / 32) x 2^-24 times the sums' size.  Five standard deviations and more for the largest of the results.
+    return 5 * 2.0 ** -23 * (12.0 ** 0.5 + (K / 32.0) ** 0.5)
+
+
+@pytest.mark.parametrize("epilogue", ["f32", "add", "swiglu"])
+@pytest.mark.parametrize("rows,cols,k", SIZES)
+def test_float32_product(rows, cols, k, epilogue):
+    from kllm_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + cols + k)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    wide = rnd(rows, k + 8)
+    x, w = wide[:, 4:4 + k], rnd(cols, k) * 0.05                 # a view: rows at a stride, 16 bytes off
+    want = x.double() @ w.double().T
+    scale = want.square().mean().sqrt()
+    if epilogue == "swiglu":
+        up = rnd(cols, k) * 0.05
+        y = kernels.gemm_f32(x, w, weight_up=up, epilogue="swiglu")
+        u = x.double() @ up.double().T
+        # an error e in gate or up moves the result by at most 1.1 |u| e and |silu(g)| e; expf adds a few ulp of it
+        slack = _bound(k) * scale * (1.1 * u.abs() + want.abs() + 1e-30) + 8 * 2.0 ** -24 * (want * u).abs()
+        want = torch.nn.functional.silu(want) * u
+    elif epilogue == "add":
+        y = rnd(rows, cols)
+        want = want + y.double()
+        kernels.gemm_f32(x, w, epilogue="add", out=y)
+        slack = _bound(k) * scale + 2.0 ** -23 * want.abs()
+    else:
+        y = kernels.gemm_f32(x, w)
+        slack = torch.full_like(want, float(_bound(k) * scale))
+    bad = (y.double() - want).abs() - slack
+    assert bad.max() <= 0, f"{int((bad > 0).sum())} of {bad.numel()} beyond the bound, worst by {float(bad.max())}"
+    assert int(kernels.status_word(y.device).item()) == 0
+
+
+def test_large_and_non_finite_numbers():
+    """Finite numbers up to the largest float32 are exact; an infinity or NaN makes its row NaN and no other."""
+    from kllm_b200 import kernels
+    x = torch.zeros(40, 64, device="cuda")
+    x[0], x[1], x[2, 5], x[3, 6] = 3.4028234e38, -3.4e38, float("inf"), float("nan")
+    x[4], x[5] = 1.1754944e-38, 1.0 + 2.0 ** -23
+    y = kernels.gemm_f32(x, torch.eye(64, device="cuda"))
+    assert torch.isnan(y[2]).all() and torch.isnan(y[3]).all()
+    keep = [0, 1, 4, 5] + list(range(6, 40))
+    assert torch.equal(y[keep], x[keep])
+
+
+def test_route():
+    """Which float32 products run here, and that the general product takes the route and agrees with float64."""
+    from kllm_b200 import kernels
+    w = torch.randn(2048, 1024, device="cuda")
+    for rows, taken in ((32, False), (33, True), (200, True)):
+        x = torch.randn(rows, 1024, device="cuda")
+        assert kernels.gemm_f32_fits(x, w) is taken
+        y = kernels.linear(x, w)
+        want = x.double() @ w.double().T
+        assert (y.double() - want).norm() <= 2e-6 * want.norm()
+    x = torch.randn(64, 1024, device="cuda")
+    assert not kernels.gemm_f32_fits(x[:, 1:1001], w[:, 1:1001])        # not 16-byte aligned
+    assert not kernels.gemm_f32_fits(x.t().contiguous().t(), w)         # k not contiguous
+    assert not kernels.gemm_f32_fits(x[:, :1022], w[:, :1022])
+    assert not kernels.gemm_f32_fits(x, w[:512])                        # too small to pay
+    assert not kernels.gemm_f32_fits(torch.empty(0, 1024, device="cuda"), w)
