@@ -1106,6 +1106,15 @@ extern "C" int kllm_attention_decode(void* out, void* part_o, void* part_ml, con
 
 #if KLLM_VD == KLLM_HD
 
+// How much of the matrix to prefetch the decode kernel's CTAs ask for: at most 96 KB each, about what a CTA of the
+// weight-streaming products asks for.  A batch of one or two has a dozen CTAs; asking for 24 MB through them took longer
+// than all the rest of the layer (decode step of TinyLlama's sizes at 100 tokens of context, batch 1: 1.05 ms without the
+// limit, 0.70 with it; batch 2: 0.88 and 0.71; from 8 on the limit is not reached; 32 to 160 KB measured alike).
+static long long prefetch_limit(long long bytes, long long ctas) {
+    const long long most = ctas * (96LL << 10);
+    return bytes < most ? bytes : most;
+}
+
 // Decode form with the step's rotary encoding, cache write and split merge inside
 // (one token per request).  q [n, n_heads*HD], k_new and v_new [n, n_kv*HD] are this
 // step's projections, unrotated; cos_sin [max_position, HD] (cos | sin); counters
@@ -1134,7 +1143,7 @@ extern "C" int kllm_attention_decode_fused(void* out, void* part_o, void* part_m
     if ((rc = set_attributes())) return rc;
     const float sl2e = scale * 1.4426950408889634f;
     DecodeFusion fu{(const bf16*)k_new, k_stride, (const bf16*)v_new, v_stride, cos_sin, (unsigned int*)counters, TL_SLOT(),
-                    prefetch, prefetch ? (long long)prefetch_bytes : 0LL, nullptr, 0.f, 0};
+                    prefetch, prefetch ? prefetch_limit(prefetch_bytes, (long long)n_tokens * n_kv * num_splits) : 0LL, nullptr, 0.f, 0};
     dim3 grid(num_splits, n_kv, n_tokens);
     const bool deep = (int64_t)num_splits * n_kv * n_tokens <= 2 * 148;
     auto go = [&](auto kernel, size_t smem) {
