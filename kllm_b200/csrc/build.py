@@ -160,8 +160,21 @@ def compile_library(name: str, verbose: bool = True, defines=None) -> str:
     return out
 
 
-def entry_arity(name: str) -> Dict[str, int]:
-    """Number of parameters of every ``extern "C"`` function that ``<name>.cu`` defines,
+def _ctype(param: str):
+    """The ctypes type of a parameter of an ``extern "C"`` function, as its declaration reads."""
+    if "*" in param:
+        return ctypes.c_void_p
+    words = param.split()[:-1]
+    if "int64_t" in words or words.count("long") == 2:
+        return ctypes.c_int64
+    for word, ctype in (("double", ctypes.c_double), ("float", ctypes.c_float), ("unsigned", ctypes.c_uint), ("int", ctypes.c_int)):
+        if word in words:
+            return ctype
+    raise KernelBuildError(f"a kernel entry point has a parameter of unknown type: {param!r}")
+
+
+def entry_params(name: str) -> Dict[str, list]:
+    """The ctypes types of the parameters of every ``extern "C"`` function that ``<name>.cu`` defines,
     read from the source text."""
     import re
     with open(os.path.join(CSRC, name + ".cu")) as fh:
@@ -169,23 +182,30 @@ def entry_arity(name: str) -> Dict[str, int]:
     out = {}
     for m in re.finditer(r'extern\s+"C"\s+[\w\s\*]+?\b(kllm_\w+)\s*\(([^)]*)\)\s*\{', text):
         params = m.group(2).strip()
-        out[m.group(1)] = 0 if params in ("", "void") else params.count(",") + 1
+        out[m.group(1)] = [] if params in ("", "void") else [_ctype(p.strip()) for p in params.split(",")]
     return out
 
 
 class CheckedLibrary:
     """A loaded kernel library whose entry points refuse a call with another number
     of arguments than the C source declares: ctypes itself would pass whatever it is
-    given, and the launcher would read the rest from wherever."""
+    given, and the launcher would read the rest from wherever.  The parameters' types are the
+    source's too, so that addresses and 64-bit numbers are passed as Python ints."""
 
-    def __init__(self, cdll: ctypes.CDLL, arity: Dict[str, int], path: str):
-        self._cdll, self._arity, self.path = cdll, arity, path
+    def __init__(self, cdll: ctypes.CDLL, params: Dict[str, list], path: str):
+        self._cdll, self._params, self.path = cdll, params, path
+
+    def address(self, fname: str) -> int:
+        """The address of an entry point, for native code that calls it."""
+        return ctypes.cast(getattr(self._cdll, fname), ctypes.c_void_p).value
 
     def __getattr__(self, fname):
         fn = getattr(self._cdll, fname)
-        want = self._arity.get(fname)
-        if want is None:
+        params = self._params.get(fname)
+        if params is None:
             return fn
+        fn.argtypes = params
+        want = len(params)
 
         def call(*args):
             if len(args) != want:
@@ -208,7 +228,7 @@ def load_library(name: str, defines=None) -> "CheckedLibrary":
         if lib is None:
             path = compile_library(name, defines=defines)
             try:
-                lib = CheckedLibrary(ctypes.CDLL(path), entry_arity(name), path)
+                lib = CheckedLibrary(ctypes.CDLL(path), entry_params(name), path)
             except OSError as e:
                 raise KernelBuildError(f"cannot load {path}: {e}") from None
             _loaded[key] = lib

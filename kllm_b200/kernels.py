@@ -15,9 +15,21 @@ from typing import Optional
 
 import torch
 
-from .csrc.build import load_library
+from .csrc import build as _build
 
 launches = 0
+
+# A prompt's step is a few hundred launches, and each passes through the functions below: they do little.
+_libraries = {}
+
+
+def load_library(name: str, defines=None):
+    """``csrc.build.load_library``, remembered by name and definitions."""
+    key = name if defines is None else (name, *defines.items())
+    lib = _libraries.get(key)
+    if lib is None:
+        lib = _libraries[key] = _build.load_library(name, defines)
+    return lib
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 
@@ -33,12 +45,13 @@ def dtype_code(dtype: torch.dtype) -> int:
         raise KernelError(f"kernels take float32 or bfloat16, not {dtype}") from None
 
 
-def _stream() -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """The current stream of the current device, as the launchers take it."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _p(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _p(t: Optional[torch.Tensor]) -> Optional[int]:
+    return None if t is None else t.data_ptr()
 
 
 def _cuda(*tensors):
@@ -79,7 +92,7 @@ def embed(out_x: torch.Tensor, table: torch.Tensor, ids: torch.Tensor,
     if table.shape[1] != d or ids.numel() != n:
         raise KernelError("embed: shapes do not agree")
     lib = load_library("embedding")
-    rc = lib.kllm_embed(_p(out_x), _p(table), _p(ids), _p(last_token), n, d, table.shape[0], ctypes.c_float(scale),
+    rc = lib.kllm_embed(_p(out_x), _p(table), _p(ids), _p(last_token), n, d, table.shape[0], scale,
                         dtype_code(table.dtype), _stream())
     _check(lib, "embedding", rc)
 
@@ -92,7 +105,7 @@ def gather_rows(out: torch.Tensor, src: torch.Tensor, rows: torch.Tensor) -> Non
         raise KernelError("gather_rows: operands do not agree")
     lib = load_library("embedding")
     rc = lib.kllm_gather_rows(_p(out), _p(src), _p(rows), rows.numel(),
-                              ctypes.c_int64(src.shape[1] * src.element_size()), _stream())
+                              src.shape[1] * src.element_size(), _stream())
     _check(lib, "embedding", rc)
 
 
@@ -109,7 +122,7 @@ def gated_slice(gate: torch.Tensor, table: torch.Tensor, offset: int, ids: torch
         raise KernelError("gated_slice: gate float32 [n, P] with dense rows, table contiguous with columns offset .. offset + P")
     out = torch.empty((n, P), dtype=table.dtype, device=gate.device)
     lib = load_library("embedding")
-    rc = lib.kllm_gated_slice(_p(out), _p(gate), ctypes.c_int64(gate.stride(0)), _p(table), ctypes.c_int64(table.shape[1]),
+    rc = lib.kllm_gated_slice(_p(out), _p(gate), gate.stride(0), _p(table), table.shape[1],
                               int(offset), P, _p(ids), _p(last_token), n, table.shape[0], dtype_code(table.dtype), _stream())
     _check(lib, "embedding", rc)
     return out
@@ -138,7 +151,7 @@ def add_rmsnorm(x: torch.Tensor, res: Optional[torch.Tensor], out: torch.Tensor,
         raise KernelError("add_rmsnorm: rows and out do not agree")
     lib = load_library("norm")
     rc = lib.kllm_add_rmsnorm(_p(x), _p(res), _p(out), _p(gain), _p(rows), n_rows, d,
-                              ctypes.c_float(eps), dtype_code(out.dtype),
+                              eps, dtype_code(out.dtype),
                               dtype_code(res.dtype if res is not None else out.dtype), _stream())
     _check(lib, "norm", rc)
 
@@ -161,7 +174,7 @@ def add_layernorm(x: torch.Tensor, res: Optional[torch.Tensor], out: torch.Tenso
     if (rows is None and n_rows != x.shape[0]) or (rows is not None and rows.numel() != n_rows):
         raise KernelError("add_layernorm: row counts do not agree")
     lib = load_library("norm")
-    rc = lib.kllm_add_layernorm(_p(x), _p(res), _p(out), _p(gain), _p(bias), _p(rows), n_rows, d, ctypes.c_float(eps),
+    rc = lib.kllm_add_layernorm(_p(x), _p(res), _p(out), _p(gain), _p(bias), _p(rows), n_rows, d, eps,
                                 dtype_code(out.dtype), dtype_code(res.dtype if res is not None else out.dtype), _stream())
     _check(lib, "norm", rc)
 
@@ -179,7 +192,7 @@ def layernorm_add(x: torch.Tensor, y: torch.Tensor, gain: torch.Tensor, bias: Op
     if out is not None and (not out.is_contiguous() or out.shape != x.shape):
         raise KernelError("layernorm_add: out contiguous like x")
     lib = load_library("norm")
-    rc = lib.kllm_layernorm_add(_p(x), _p(y), _p(gain), _p(bias), ctypes.c_float(eps), _p(out), x.shape[0], d,
+    rc = lib.kllm_layernorm_add(_p(x), _p(y), _p(gain), _p(bias), eps, _p(out), x.shape[0], d,
                                 dtype_code(out.dtype if out is not None else torch.float32), _stream())
     _check(lib, "norm", rc)
 
@@ -196,8 +209,8 @@ def embed_layernorm(out_x: torch.Tensor, table: torch.Tensor, ids: torch.Tensor,
         raise KernelError("embed_layernorm: contiguous operands, x float32 [n, d], table [vocab, d], one id per row")
     _bias(gain, d, "embed_layernorm"); _bias(bias, d, "embed_layernorm")
     lib = load_library("norm")
-    rc = lib.kllm_embed_layernorm(_p(out_x), _p(table), _p(ids), _p(last_token), table.shape[0], ctypes.c_float(scale), _p(gain),
-                                  _p(bias), ctypes.c_float(eps), _p(rows), n, d, dtype_code(table.dtype),
+    rc = lib.kllm_embed_layernorm(_p(out_x), _p(table), _p(ids), _p(last_token), table.shape[0], scale, _p(gain),
+                                  _p(bias), eps, _p(rows), n, d, dtype_code(table.dtype),
                                   dtype_code(rows.dtype if rows is not None else torch.float32), _stream())
     _check(lib, "norm", rc)
 
@@ -220,7 +233,7 @@ def rmsnorm_add(x: torch.Tensor, y: torch.Tensor, gain: torch.Tensor, eps: float
             gain2 is not None and (gain2.dtype != torch.float32 or gain2.numel() != d))):
         raise KernelError("rmsnorm_add: out contiguous like x, a second norm's gain float32 [d]")
     lib = load_library("norm")
-    rc = lib.kllm_rmsnorm_add(_p(x), _p(y), _p(gain), ctypes.c_float(eps), _p(out), _p(gain2), ctypes.c_float(eps2),
+    rc = lib.kllm_rmsnorm_add(_p(x), _p(y), _p(gain), eps, _p(out), _p(gain2), eps2,
                               x.shape[0], d, dtype_code(out.dtype if out is not None else torch.float32), _stream())
     _check(lib, "norm", rc)
 
@@ -259,8 +272,8 @@ def qknorm_append(q_out: torch.Tensor, qkv: torch.Tensor, q_gain: torch.Tensor, 
                 or tuple(vcache.shape[1:]) != (n_kv, page_size, v_head_dim) or vcache.shape[0] != kcache.shape[0]):
             raise KernelError("qknorm_append: caches must be [pages, kv heads, page_size, size] in q_out's dtype")
     lib = load_library("qknorm_append")
-    rc = lib.kllm_qknorm_append(_p(q_out), _p(qkv), ctypes.c_int64(qkv.stride(0)), _p(q_gain), _p(k_gain),
-                                ctypes.c_float(eps), ctypes.c_float(temp_coef), int(temp_every or 1), _p(positions),
+    rc = lib.kllm_qknorm_append(_p(q_out), _p(qkv), qkv.stride(0), _p(q_gain), _p(k_gain),
+                                eps, temp_coef, int(temp_every or 1), _p(positions),
                                 _p(token_req), _p(block_table), max_blocks, _p(kcache), _p(vcache), n, n_heads, n_kv,
                                 head_dim, v_head_dim, page_size, int(rot or 0), _p(freq if rot else None),
                                 dtype_code(q_out.dtype), _stream())
@@ -289,8 +302,8 @@ def latent_norm_append(q_out: torch.Tensor, proj: torch.Tensor, q_gain: torch.Te
     if not q_out.is_contiguous() or q_gain.dtype != torch.float32 or q_gain.numel() != Rq or not q_gain.is_contiguous():
         raise KernelError("latent_norm_append: q_out contiguous [n, Rq], the query gain float32 [Rq]")
     lib = load_library("latent")
-    rc = lib.kllm_latent_norm_append(_p(q_out), _p(proj), ctypes.c_int64(proj.stride(0)), _p(q_gain), _p(kv_gain),
-                                     ctypes.c_float(eps), _p(positions), _p(token_req), _p(block_table), max_blocks,
+    rc = lib.kllm_latent_norm_append(_p(q_out), _p(proj), proj.stride(0), _p(q_gain), _p(kv_gain),
+                                     eps, _p(positions), _p(token_req), _p(block_table), max_blocks,
                                      _p(cache), n, Rq, R, page_size, dtype_code(q_out.dtype), _stream())
     _check(lib, "latent", rc)
 
@@ -327,8 +340,8 @@ def latent_rope_append(q_plain: torch.Tensor, q_full: torch.Tensor, proj: torch.
         if kv_gain is None or kv_gain.dtype != torch.float32 or kv_gain.numel() != rank or not kv_gain.is_contiguous():
             raise KernelError("latent_rope_append: the latent's gain must be float32 [R]")
     lib = load_library("latent")
-    rc = lib.kllm_latent_rope_append(_p(q_plain), _p(q_full), _p(proj), ctypes.c_int64(proj.stride(0)), _p(kv_gain),
-                                     ctypes.c_float(eps), _p(freq), ctypes.c_float(amplitude), _p(positions),
+    rc = lib.kllm_latent_rope_append(_p(q_plain), _p(q_full), _p(proj), proj.stride(0), _p(kv_gain),
+                                     eps, _p(freq), amplitude, _p(positions),
                                      _p(token_req), _p(block_table), max_blocks, _p(cache), n, n_heads, dk, dr, rank,
                                      page_size, dtype_code(q_plain.dtype), _stream())
     _check(lib, "latent", rc)
@@ -370,8 +383,8 @@ def headnorm_rope_append(q_out: torch.Tensor, qkv: torch.Tensor, bias: Optional[
                 or tuple(vcache.shape[1:]) != (v_heads, page_size, dv) or vcache.shape[0] != kcache.shape[0]):
             raise KernelError("headnorm_rope_append: caches must be [pages, heads, page_size, size] in q_out's dtype")
     lib = load_library("qk_headnorm")
-    rc = lib.kllm_headnorm_rope_append(_p(q_out), _p(qkv), ctypes.c_int64(qkv.stride(0)), _p(bias), _p(q_gain), _p(k_gain),
-                                       ctypes.c_float(eps), _p(freq), ctypes.c_float(amplitude), int(rot), int(interleaved),
+    rc = lib.kllm_headnorm_rope_append(_p(q_out), _p(qkv), qkv.stride(0), _p(bias), _p(q_gain), _p(k_gain),
+                                       eps, _p(freq), amplitude, int(rot), int(interleaved),
                                        _p(positions), _p(token_req), _p(block_table), max_blocks, _p(kcache), _p(vcache), n,
                                        q_heads, k_heads, v_heads, dk, dv, page_size, dtype_code(q_out.dtype), _stream())
     _check(lib, "qk_headnorm", rc)
@@ -388,8 +401,8 @@ def maps_combine(out: torch.Tensor, a: torch.Tensor, kv_heads: int, group: int, 
     if tuple(out.shape) != (n, kv_heads * group * dv) or not out.is_contiguous():
         raise KernelError("maps_combine: out must be contiguous [n, G * gs * dv]")
     lib = load_library("qk_headnorm")
-    rc = lib.kllm_maps_combine(_p(out), _p(a), n, kv_heads, group, dv, ctypes.c_float(lam), ctypes.c_float(eps),
-                               ctypes.c_float(post), dtype_code(out.dtype), _stream())
+    rc = lib.kllm_maps_combine(_p(out), _p(a), n, kv_heads, group, dv, lam, eps,
+                               post, dtype_code(out.dtype), _stream())
     _check(lib, "qk_headnorm", rc)
 
 
@@ -405,8 +418,8 @@ def sigmoid_gate(out: torch.Tensor, a: torch.Tensor, gate: torch.Tensor, factor:
             raise KernelError("sigmoid_gate: operands must have dense rows")
     n, f = out.shape
     lib = load_library("activation")
-    rc = lib.kllm_sigmoid_gate(_p(out), ctypes.c_int64(out.stride(0)), _p(a), ctypes.c_int64(a.stride(0)), _p(gate),
-                               ctypes.c_int64(gate.stride(0)), n, f, ctypes.c_float(factor), dtype_code(out.dtype),
+    rc = lib.kllm_sigmoid_gate(_p(out), out.stride(0), _p(a), a.stride(0), _p(gate),
+                               gate.stride(0), n, f, factor, dtype_code(out.dtype),
                                dtype_code(a.dtype), _stream())
     _check(lib, "activation", rc)
 
@@ -433,8 +446,8 @@ def streams_step(streams: torch.Tensor, *, init: Optional[torch.Tensor] = None, 
     if (y is not None and (mix is None or out_w is None)) or (in_w is not None and (gain is None or normed is None)):
         raise KernelError("streams_step: a write needs mix and out_w, a read needs gain and normed")
     lib = load_library("streams")
-    rc = lib.kllm_streams_step(_p(streams), ctypes.c_int64(n * d), _p(init), _p(y), _p(mix), _p(out_w), _p(in_w),
-                               _p(gain), ctypes.c_float(eps), _p(normed), _p(total), n, d, S,
+    rc = lib.kllm_streams_step(_p(streams), n * d, _p(init), _p(y), _p(mix), _p(out_w), _p(in_w),
+                               _p(gain), eps, _p(normed), _p(total), n, d, S,
                                dtype_code(normed.dtype if normed is not None else torch.float32), _stream())
     _check(lib, "streams", rc)
 
@@ -466,8 +479,8 @@ def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos_sin: Opti
     else:
         page_size, max_blocks = 1, 0
     lib = load_library("rope")
-    rc = lib.kllm_rope_append(_p(q), ctypes.c_int64(q.stride(0)), _p(k), ctypes.c_int64(k.stride(0)),
-                              _p(v), ctypes.c_int64(v.stride(0)), _p(cos_sin), _p(positions),
+    rc = lib.kllm_rope_append(_p(q), q.stride(0), _p(k), k.stride(0),
+                              _p(v), v.stride(0), _p(cos_sin), _p(positions),
                               _p(token_req), _p(block_table), max_blocks, _p(kcache), _p(vcache),
                               n, n_heads, n_kv, head_dim, rot, page_size, dtype_code(q.dtype), _stream())
     _check(lib, "rope", rc)
@@ -495,10 +508,10 @@ def attention_generic(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, 
         raise KernelError("attention: cache layout must be [pages, n_kv, page_size, head_dim]")
     n = q.shape[0]
     lib = load_library("attention_generic")
-    rc = lib.kllm_attention_generic(_p(out), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache),
+    rc = lib.kllm_attention_generic(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache),
                                     _p(positions), _p(token_req), _p(block_table), block_table.shape[1],
                                     n, n_heads, n_kv, head_dim, vd, kcache.shape[2], int(window or 0),
-                                    ctypes.c_float(scale), _slopes_arg(score_slopes, n_heads),
+                                    scale, _slopes_arg(score_slopes, n_heads),
                                     _slopes_arg(sinks, n_heads, "sinks"), int(segment or 0), v_heads, v_row,
                                     int(out.dtype == torch.float32 and q.dtype != torch.float32), int(keep or 0),
                                     dtype_code(q.dtype), _stream())
@@ -577,13 +590,13 @@ def attention_simt(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vca
     if segment:
         bound = min(bound, segment)
     splits = max(1, -(-bound // SIMT_CHUNK))
-    common = (n_heads, n_kv, head_dim, vd, kcache.shape[2], int(window or 0), ctypes.c_float(scale))
+    common = (n_heads, n_kv, head_dim, vd, kcache.shape[2], int(window or 0), scale)
     first = 0
     global launches
     if singles and splits > 1:
         part_o = torch.empty((singles * n_heads, splits, vd), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((singles * n_heads, splits, 2), dtype=torch.float32, device=q.device)
-        rc = lib.kllm_attention_simt(_p(out), _p(part_o), _p(part_ml), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache),
+        rc = lib.kllm_attention_simt(_p(out), _p(part_o), _p(part_ml), _p(q), q.stride(0), _p(kcache),
                                      _p(vcache), _p(ctx.q_start), _p(ctx.start_pos), _p(block_table),
                                      block_table.shape[1], singles, singles, *common, 1, SIMT_CHUNK, splits,
                                      _p(score_slopes), _p(sinks), segment, v_heads, v_row, out_f32, int(keep or 0),
@@ -597,7 +610,7 @@ def attention_simt(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vca
     if first < n_req:
         qt = max(1, 64 // group)
         rest = n_tokens - first
-        rc = lib.kllm_attention_simt(_p(out), None, None, _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache),
+        rc = lib.kllm_attention_simt(_p(out), None, None, _p(q), q.stride(0), _p(kcache), _p(vcache),
                                      _p(ctx.q_start[first:]), _p(ctx.start_pos[first:]), _p(block_table[first:]),
                                      block_table.shape[1], n_req - first, rest // qt + (n_req - first), *common, qt, 0, 1,
                                      _p(score_slopes), _p(sinks), segment, v_heads, v_row, out_f32, int(keep or 0),
@@ -813,10 +826,10 @@ def attention_decode(out, q, kcache, vcache, positions, token_req, block_table, 
         part_o = torch.empty((n, n_heads, num_splits, vd), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n, n_heads, num_splits, 2), dtype=torch.float32, device=q.device)
     lib = load_library("attention_tc", {"KLLM_HD": head_dim} if vd == head_dim else {"KLLM_HD": head_dim, "KLLM_VD": vd})
-    rc = lib.kllm_attention_decode(_p(out), _p(part_o), _p(part_ml), _p(q), ctypes.c_int64(q.stride(0)),
+    rc = lib.kllm_attention_decode(_p(out), _p(part_o), _p(part_ml), _p(q), q.stride(0),
                                    _p(kcache), _p(vcache), _p(positions), _p(token_req), _p(block_table),
                                    block_table.shape[1], n, n_heads, n_kv, head_dim, kcache.shape[2],
-                                   int(window or 0), ctypes.c_float(scale), int(num_splits), _slopes_arg(slopes, n_heads),
+                                   int(window or 0), scale, int(num_splits), _slopes_arg(slopes, n_heads),
                                    int(bool(split_weights)), _slopes_arg(sinks, n_heads, "sinks"), int(keep or 0), _stream())
     _check(lib, "attention_tc", rc)
     global launches
@@ -850,10 +863,10 @@ def attention_decode_fused(out, q, k_new, v_new, cos_sin, kcache, vcache, positi
         part_ml = torch.empty((n, n_heads, num_splits, 2), dtype=torch.float32, device=q.device)
     lib = load_library("attention_tc", {"KLLM_HD": head_dim})
     rc = lib.kllm_attention_decode_fused(
-        _p(out), _p(part_o), _p(part_ml), _p(counters), _p(q), ctypes.c_int64(q.stride(0)), _p(k_new),
-        ctypes.c_int64(k_new.stride(0)), _p(v_new), ctypes.c_int64(v_new.stride(0)), _p(cos_sin), _p(kcache),
+        _p(out), _p(part_o), _p(part_ml), _p(counters), _p(q), q.stride(0), _p(k_new),
+        k_new.stride(0), _p(v_new), v_new.stride(0), _p(cos_sin), _p(kcache),
         _p(vcache), _p(positions), _p(token_req), _p(block_table), block_table.shape[1], n, n_heads, n_kv,
-        head_dim, kcache.shape[2], int(window or 0), ctypes.c_float(scale), int(num_splits),
+        head_dim, kcache.shape[2], int(window or 0), scale, int(num_splits),
         *_prefetch_args(prefetch), _stream())
     _check(lib, "attention_tc", rc)
 
@@ -879,10 +892,10 @@ def attention_prefill(out, q, kcache, vcache, q_start, start_pos, block_table, n
     _i32(block_table, "block_table")
     _i32(q_start, "q_start"); _i32(start_pos, "start_pos")
     lib = load_library("attention_tc", {"KLLM_HD": head_dim} if vd == head_dim else {"KLLM_HD": head_dim, "KLLM_VD": vd})
-    rc = lib.kllm_attention_prefill(_p(out), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache),
+    rc = lib.kllm_attention_prefill(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache),
                                     _p(q_start), _p(start_pos), _p(block_table), block_table.shape[1],
                                     q.shape[0], int(n_requests), n_heads, n_kv, head_dim, kcache.shape[2],
-                                    int(window or 0), ctypes.c_float(scale), _slopes_arg(slopes, n_heads),
+                                    int(window or 0), scale, _slopes_arg(slopes, n_heads),
                                     int(bool(split_weights)), _slopes_arg(sinks, n_heads, "sinks"), vd,
                                     int(segment or 0), v_heads, v_row, int(out.dtype == torch.float32), int(keep or 0), _stream())
     _check(lib, "attention_tc", rc)
@@ -922,9 +935,9 @@ def attention_prefill_tcgen05(out, q, kcache, vcache, q_start, start_pos, block_
     name = "attention_tcgen05" + ("_ptmem" if probabilities == "tmem" else "")
     lib = load_library(name, {"KLLM_HD": head_dim})
     fn = lib.kllm_attention_prefill_tcgen05_ptmem if probabilities == "tmem" else lib.kllm_attention_prefill_tcgen05
-    rc = fn(_p(out), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache), _p(q_start), _p(start_pos),
+    rc = fn(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache), _p(q_start), _p(start_pos),
             _p(block_table), block_table.shape[1], q.shape[0], int(n_requests), n_heads, n_kv, head_dim,
-            kcache.shape[2], int(window or 0), ctypes.c_float(scale), _p(status_word(q.device)), _stream())
+            kcache.shape[2], int(window or 0), scale, _p(status_word(q.device)), _stream())
     _check(lib, name, rc)
 
 
@@ -995,8 +1008,8 @@ def silu_mul(out: torch.Tensor, gate: torch.Tensor, up: torch.Tensor) -> None:
         raise KernelError("silu_mul: gate and up must share a dtype, float32 or out's")
     n, f = out.shape
     lib = load_library("activation")
-    rc = lib.kllm_silu_mul(_p(out), ctypes.c_int64(out.stride(0)), _p(gate), ctypes.c_int64(gate.stride(0)),
-                           _p(up), ctypes.c_int64(up.stride(0)), n, f, dtype_code(out.dtype),
+    rc = lib.kllm_silu_mul(_p(out), out.stride(0), _p(gate), gate.stride(0),
+                           _p(up), up.stride(0), n, f, dtype_code(out.dtype),
                            dtype_code(gate.dtype), _stream())
     _check(lib, "activation", rc)
 
@@ -1012,8 +1025,8 @@ def clamped_glu(out: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, limit: 
         raise KernelError("clamped_glu: gate and up must be float32 of out's shape")
     n, f = out.shape
     lib = load_library("activation")
-    rc = lib.kllm_clamped_glu(_p(out), ctypes.c_int64(out.stride(0)), _p(gate), ctypes.c_int64(gate.stride(0)),
-                              _p(up), ctypes.c_int64(up.stride(0)), n, f, ctypes.c_float(limit), ctypes.c_float(alpha),
+    rc = lib.kllm_clamped_glu(_p(out), out.stride(0), _p(gate), gate.stride(0),
+                              _p(up), up.stride(0), n, f, limit, alpha,
                               dtype_code(out.dtype), _stream())
     _check(lib, "activation", rc)
 
@@ -1031,8 +1044,8 @@ def biased_glu(out: torch.Tensor, gate: torch.Tensor, up: torch.Tensor, bias_gat
         raise KernelError("biased_glu: gate and up must be float32, the activation silu or gelu_tanh")
     _bias(bias_gate, f, "biased_glu"); _bias(bias_up, f, "biased_glu")
     lib = load_library("activation")
-    rc = lib.kllm_biased_glu(_p(out), ctypes.c_int64(out.stride(0)), _p(gate), ctypes.c_int64(gate.stride(0)), _p(up),
-                             ctypes.c_int64(up.stride(0)), _p(bias_gate), _p(bias_up), n, f, int(activation == "gelu_tanh"),
+    rc = lib.kllm_biased_glu(_p(out), out.stride(0), _p(gate), gate.stride(0), _p(up),
+                             up.stride(0), _p(bias_gate), _p(bias_up), n, f, int(activation == "gelu_tanh"),
                              dtype_code(out.dtype), _stream())
     _check(lib, "activation", rc)
 
@@ -1070,7 +1083,7 @@ def sample(out: torch.Tensor, logits: torch.Tensor, temperature: Optional[torch.
         if t is not None and (t.dtype != torch.float32 or not t.is_contiguous() or t.numel() != logits.shape[0]):
             raise KernelError("sample: temperature and uniform must be float32 [rows]")
     lib = load_library("sampling")
-    rc = lib.kllm_sample(_p(out), _p(logits), ctypes.c_int64(logits.stride(0)), logits.shape[0],
+    rc = lib.kllm_sample(_p(out), _p(logits), logits.stride(0), logits.shape[0],
                          logits.shape[1], _p(temperature), _p(uniform), _p(last_token), _p(slots), _p(host_out), _stream())
     _check(lib, "sampling", rc)
 
@@ -1112,10 +1125,10 @@ def _skinny_max_width(n: int) -> int:
 
 def _prefetch_args(t: Optional[torch.Tensor]):
     if t is None or not PREFETCH_L2:
-        return None, ctypes.c_int64(0)
+        return None, 0
     if not t.is_contiguous():
         raise KernelError("prefetch: the tensor to bring into L2 must be contiguous")
-    return _p(t), ctypes.c_int64(min(t.numel() * t.element_size(), PREFETCH_L2_BYTES) // 16 * 16)
+    return _p(t), min(t.numel() * t.element_size(), PREFETCH_L2_BYTES) // 16 * 16
 
 
 def skinny_gemm(weight: torch.Tensor, *, x: Optional[torch.Tensor] = None, x_f32: Optional[torch.Tensor] = None,
@@ -1196,10 +1209,10 @@ def skinny_gemm(weight: torch.Tensor, *, x: Optional[torch.Tensor] = None, x_f32
     lib = load_library("skinny_gemm", _bias_form(bias, bias_up, activation))
     y16 = out if want == torch.bfloat16 else None
     y32 = out if want == torch.float32 else None
-    rc = lib.kllm_skinny_gemm(_p(weight), _p(weight_up), ctypes.c_int64(weight.stride(0)), N, K, n, _p(x),
-                              ctypes.c_int64(x.stride(0) if x is not None else 0), _p(x_f32), _p(gain), _p(rows),
-                              ctypes.c_float(eps), _p(y16), _p(y32), ctypes.c_int64(out.stride(0)), pro, epi,
-                              _p(bias), _p(bias_up), _SKINNY_ACT[activation], ctypes.c_float(limit), ctypes.c_float(alpha),
+    rc = lib.kllm_skinny_gemm(_p(weight), _p(weight_up), weight.stride(0), N, K, n, _p(x),
+                              (x.stride(0) if x is not None else 0), _p(x_f32), _p(gain), _p(rows),
+                              eps, _p(y16), _p(y32), out.stride(0), pro, epi,
+                              _p(bias), _p(bias_up), _SKINNY_ACT[activation], limit, alpha,
                               *_prefetch_args(prefetch), _stream())
     _check(lib, "skinny_gemm", rc)
     return out
@@ -1245,13 +1258,97 @@ def _skinny_gemm_f32(weight, x, x_f32, gain, eps, rows, n_rows, weight_up, epilo
     if out.dtype != torch.float32 or out.stride(1) != 1 or out.shape[0] < n or out.shape[1] != N:
         raise KernelError("skinny_gemm: out has the wrong dtype or shape")
     lib = load_library("skinny_gemm_f32", _bias_form(bias, bias_up, activation))
-    rc = lib.kllm_skinny_gemm_f32(_p(weight), _p(weight_up), ctypes.c_int64(weight.stride(0)), N, K, n, _p(src),
-                                  ctypes.c_int64(stride), _p(gain), _p(rows), ctypes.c_float(eps), _p(out),
-                                  ctypes.c_int64(out.stride(0)), pro, {"f32": 0, "add": 1, "swiglu": 2}[epilogue],
-                                  _p(bias), _p(bias_up), _SKINNY_ACT[activation], ctypes.c_float(limit), ctypes.c_float(alpha),
+    rc = lib.kllm_skinny_gemm_f32(_p(weight), _p(weight_up), weight.stride(0), N, K, n, _p(src),
+                                  stride, _p(gain), _p(rows), eps, _p(out),
+                                  out.stride(0), pro, {"f32": 0, "add": 1, "swiglu": 2}[epilogue],
+                                  _p(bias), _p(bias_up), _SKINNY_ACT[activation], limit, alpha,
                                   _stream())
     _check(lib, "skinny_gemm_f32", rc)
     return out
+
+
+def prompt_layers_ready() -> bool:
+    """Whether ``prompt_layers`` can run in this process (it calls the product library that torch has loaded)."""
+    return bool(load_library("prompt_layers").kllm_prompt_layers_ready())
+
+
+def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,
+                  head_dim: int, inter: int, eps: float, scale: float) -> None:
+    """The layers of a step with portions, launched from one call (csrc/prompt_layers.cu): x [n, d] float32 is the
+    residual stream, updated in place; ``layers`` holds (w_qkv, w_o, w_gate_up, w_down, gain1, gain2, k pages, v pages)
+    per layer, in bfloat16 with float32 gains.  The same kernels as ``attention``, ``add_rmsnorm``, ``linear`` and so on
+    launch for this step, with the routes that they choose."""
+    global launches
+    n, d = x.shape
+    positions, token_req, q_start, start_pos = ctx.positions, ctx.token_req, ctx.q_start, ctx.start_pos
+    _cuda(x, cos_sin, positions, token_req, q_start, start_pos, block_table)
+    for t, what in ((positions, "positions"), (token_req, "token_req"), (q_start, "q_start"), (start_pos, "start_pos"),
+                    (block_table, "block_table")):
+        _i32(t, what)
+    if x.dtype != torch.float32 or not x.is_contiguous() or positions.numel() != n or token_req.numel() != n:
+        raise KernelError("prompt_layers: x must be contiguous float32 [n, d], with one position and one request a token")
+    if cos_sin.dtype != torch.float32 or not cos_sin.is_contiguous() or cos_sin.shape[1] != head_dim:
+        raise KernelError("prompt_layers: the cos/sin table must be float32 [positions, head_dim]")
+    page_size, q_dim = layers[0][6].shape[2], n_heads * head_dim
+    wide = q_dim + 2 * n_kv * head_dim
+    want = ((wide, d), (d, q_dim), (2 * inter, d), (d, inter), (d,), (d,))
+    ptrs = []
+    for layer in layers:
+        for i, t in enumerate(layer):
+            ok = t.is_cuda and t.is_contiguous() and t.dtype == (torch.float32 if i in (4, 5) else torch.bfloat16)
+            if not ok or (t.shape != want[i] if i < 6 else t.shape[1:] != (n_kv, page_size, head_dim)):
+                raise KernelError(f"prompt_layers: operand {i} of a layer ({t.dtype}, {tuple(t.shape)}) does not fit the sizes")
+            ptrs.append(t.data_ptr())
+    singles = 0
+    while singles < ctx.n_requests and ctx.host_n_new[singles] == 1:
+        singles += 1
+    if singles == ctx.n_requests:
+        raise KernelError("prompt_layers: a step without a portion")
+    new = lambda *shape, dtype=torch.bfloat16: torch.empty(shape, dtype=dtype, device=x.device)
+    splits, part_o, part_ml = 1, None, None
+    if singles:
+        group = n_heads // n_kv
+        groups = n_kv * next((s for s in range(1, group + 1) if group % s == 0 and group // s <= 16), 1)
+        splits = decode_splits(singles, groups, ctx.max_ctx)
+        if splits > 1:
+            part_o = new(singles, n_heads, splits, head_dim, dtype=torch.float32)
+            part_ml = new(singles, n_heads, splits, 2, dtype=torch.float32)
+    form = tcgen05_form(head_dim, n_heads // n_kv, n_kv, n - singles, ctx.n_requests - singles, ctx.max_ctx)
+    xn, qkv, attn, act = new(n, d), new(n, wide), new(n, q_dim), new(n, inter)
+    gate_up = None
+    if not (gemm_pays(n, inter, "swiglu") and all(gemm_fits(xn, layer[2][:inter], act, "swiglu", layer[2][inter:]) for layer in layers)):
+        gate_up = new(n, 2 * inter, dtype=torch.float32)
+    name = "attention_tcgen05" + ("_ptmem" if form == "tmem" else "")
+    used = [("norm", None, "kllm_add_rmsnorm"), ("rope", None, "kllm_rope_append"),
+            ("attention_tc", {"KLLM_HD": head_dim}, "kllm_attention_decode"),
+            (name, {"KLLM_HD": head_dim}, "kllm_attention_prefill_tcgen05" + ("_ptmem" if form == "tmem" else "")),
+            ("activation", None, "kllm_silu_mul")]
+    entries = (ctypes.c_void_p * len(used))(*(load_library(lib, defs).address(fn) for lib, defs, fn in used))
+    table = (ctypes.c_void_p * len(ptrs))(*ptrs)
+    failed = ctypes.c_int(-1)
+    lib = load_library("prompt_layers")
+    args = (ctypes.addressof(table), len(layers), ctypes.addressof(entries), torch.cuda.current_blas_handle(), n, d, n_heads, n_kv,
+            head_dim, inter, eps, scale, _p(x), _p(cos_sin), _p(positions), _p(token_req), _p(block_table), block_table.shape[1],
+            ctx.n_requests, _p(q_start), _p(start_pos), singles, splits, page_size, _p(xn), _p(qkv), _p(attn), _p(part_o),
+            _p(part_ml), _p(act), _p(gate_up), _p(status_word(x.device)), ctypes.addressof(failed), _stream())
+
+    def halves(first, last):
+        rc = lib.kllm_prompt_layers(first, last, *args)
+        if rc != 0 and 0 <= failed.value < len(used):
+            _check(load_library(*used[failed.value][:2]), used[failed.value][0], rc)
+        if rc != 0 and failed.value == len(used):
+            raise KernelError("prompt_layers: the library product failed")
+        _check(lib, "prompt_layers", rc)
+    before = launches
+    if gate_up is not None:
+        halves(0, 2 * len(layers))
+    else:
+        # gate, up and activation as one kernel, between the halves of every layer
+        for i, layer in enumerate(layers):
+            halves(max(0, 2 * i - 1), 2 * i + 1)
+            gemm(xn, layer[2][:inter], weight_up=layer[2][inter:], epilogue="swiglu", out=act)
+        halves(2 * len(layers) - 1, 2 * len(layers))
+    launches = before + len(layers) * (5 + (1 if singles else 0) + (1 if splits > 1 else 0))
 
 
 def linear_add(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> None:
@@ -1288,8 +1385,8 @@ def linear_into(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor, bias: 
 
 
 def _gemm_args(x, weight, weight_up, out, epilogue):
-    return (_p(x), ctypes.c_int64(x.stride(0)), _p(weight), ctypes.c_int64(weight.stride(0)), _p(weight_up),
-            x.shape[0], weight.shape[0], x.shape[1], _p(out), ctypes.c_int64(out.stride(0)), _GEMM_EPI[epilogue])
+    return (_p(x), x.stride(0), _p(weight), weight.stride(0), _p(weight_up),
+            x.shape[0], weight.shape[0], x.shape[1], _p(out), out.stride(0), _GEMM_EPI[epilogue])
 
 
 def gemm_fits(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: str = "bf16",
@@ -1347,8 +1444,8 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "bf16", out: 
         raise KernelError(f"gemm: operands {tuple(x.shape)} x {tuple(weight.shape)} (strides {x.stride()}, "
                           f"{weight.stride()}, out {out.stride()}) are not supported")
     lib = load_library("gemm_tcgen05")
-    rc = lib.kllm_gemm_tcgen05(*_gemm_args(x, weight, weight_up, out, epilogue), int(bn), ctypes.c_float(limit),
-                               ctypes.c_float(alpha), _p(status_word(x.device)), _stream())
+    rc = lib.kllm_gemm_tcgen05(*_gemm_args(x, weight, weight_up, out, epilogue), int(bn), limit,
+                               alpha, _p(status_word(x.device)), _stream())
     _check(lib, "gemm_tcgen05", rc)
     return out
 
@@ -1405,15 +1502,15 @@ def gemm_f32(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "f32", ou
     dense = all(t is None or (t.dtype == torch.float32 and t.dim() == 2 and t.stride(1) == 1) for t in (x, weight, weight_up, out))
     if not dense or x.shape[1] != weight.shape[1] or (weight_up is not None and (
             weight_up.shape != weight.shape or weight_up.stride() != weight.stride())) \
-            or not lib.kllm_gemm_f32_tcgen05_fits(_p(x), ctypes.c_int64(x.stride(0)), _p(weight), ctypes.c_int64(weight.stride(0)),
-                                                  _p(weight_up), n, N, x.shape[1], _p(out), ctypes.c_int64(out.stride(0)), epi):
+            or not lib.kllm_gemm_f32_tcgen05_fits(_p(x), x.stride(0), _p(weight), weight.stride(0),
+                                                  _p(weight_up), n, N, x.shape[1], _p(out), out.stride(0), epi):
         raise KernelError(f"gemm_f32: operands {tuple(x.shape)} x {tuple(weight.shape)} (strides {x.stride()}, "
                           f"{weight.stride()}, out {out.stride()}) are not supported")
     size = ctypes.c_int64(0)
     lib.kllm_gemm_f32_tcgen05_workspace(n, N, x.shape[1], epi, ctypes.byref(size))
     ws = torch.empty(size.value, dtype=torch.uint8, device=x.device)
-    rc = lib.kllm_gemm_f32_tcgen05(_p(x), ctypes.c_int64(x.stride(0)), _p(weight), ctypes.c_int64(weight.stride(0)),
-                                   _p(weight_up), n, N, x.shape[1], _p(out), ctypes.c_int64(out.stride(0)), epi,
+    rc = lib.kllm_gemm_f32_tcgen05(_p(x), x.stride(0), _p(weight), weight.stride(0),
+                                   _p(weight_up), n, N, x.shape[1], _p(out), out.stride(0), epi,
                                    _p(ws), _p(status_word(x.device)), _stream())
     _check(lib, "gemm_f32_tcgen05", rc)
     return out
@@ -1540,8 +1637,8 @@ def wkv_shift_mix(h: torch.Tensor, mu: torch.Tensor, state: torch.Tensor, prev_o
         raise KernelError("wkv_shift_mix: the state must be float32 [slots, size] with room for a row at prev_off")
     out = torch.empty((mu.shape[0], n, d), dtype=h.dtype, device=h.device)
     lib = load_library("wkv")
-    rc = lib.kllm_wkv_shift_mix(_p(out), _p(h), _p(mu), _p(state), ctypes.c_int64(state.stride(0)),
-                                ctypes.c_int64(prev_off), _p(ctx.q_start), _p(ctx.token_req), _p(ctx.state_slots), n, d,
+    rc = lib.kllm_wkv_shift_mix(_p(out), _p(h), _p(mu), _p(state), state.stride(0),
+                                prev_off, _p(ctx.q_start), _p(ctx.token_req), _p(ctx.state_slots), n, d,
                                 mu.shape[0], dtype_code(h.dtype), _stream())
     _check(lib, "wkv", rc)
     return out
@@ -1568,9 +1665,9 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, z: torch.Tensor,
         raise KernelError("wkv_scan: the state must be float32 [slots, >= heads * size * size]")
     o = torch.empty((r.shape[0], A), dtype=torch.float32, device=r.device)
     lib = load_library("wkv")
-    rc = lib.kllm_wkv_scan(_p(o), ctypes.c_int64(o.stride(0)), _p(r), ctypes.c_int64(r.stride(0)), _p(k),
-                           ctypes.c_int64(k.stride(0)), _p(v), ctypes.c_int64(v.stride(0)), _p(z),
-                           ctypes.c_int64(z.stride(0)), _p(w0), _p(u), _p(state), ctypes.c_int64(state.stride(0)),
+    rc = lib.kllm_wkv_scan(_p(o), o.stride(0), _p(r), r.stride(0), _p(k),
+                           k.stride(0), _p(v), v.stride(0), _p(z),
+                           z.stride(0), _p(w0), _p(u), _p(state), state.stride(0),
                            _p(ctx.q_start), _p(ctx.state_slots), r.shape[0], ctx.n_requests, heads, size, _stream())
     _check(lib, "wkv", rc)
     return o
@@ -1585,7 +1682,7 @@ def wkv_decay_outer(low: torch.Tensor, w2: torch.Tensor) -> torch.Tensor:
         raise KernelError("wkv_decay_outer: low float32 [n, R] with dense rows, w2 contiguous [A, R]")
     z = torch.empty((n, w2.shape[0]), dtype=torch.float32, device=low.device)
     lib = load_library("wkv")
-    rc = lib.kllm_wkv_decay_outer(_p(z), _p(low), ctypes.c_int64(low.stride(0)), _p(w2), n, w2.shape[0], R,
+    rc = lib.kllm_wkv_decay_outer(_p(z), _p(low), low.stride(0), _p(w2), n, w2.shape[0], R,
                                   dtype_code(w2.dtype), _stream())
     _check(lib, "wkv", rc)
     return z
@@ -1601,8 +1698,8 @@ def wkv_gate_norm(o: torch.Tensor, g: torch.Tensor, gain: torch.Tensor, eps: flo
         raise KernelError("wkv_gate_norm: gain must be contiguous float32 [heads * size]")
     y = torch.empty((o.shape[0], A), dtype=dtype, device=o.device)
     lib = load_library("wkv")
-    rc = lib.kllm_wkv_gate_norm(_p(y), _p(o), ctypes.c_int64(o.stride(0)), _p(g), ctypes.c_int64(g.stride(0)), _p(gain),
-                                o.shape[0], heads, size, ctypes.c_float(eps), dtype_code(dtype), _stream())
+    rc = lib.kllm_wkv_gate_norm(_p(y), _p(o), o.stride(0), _p(g), g.stride(0), _p(gain),
+                                o.shape[0], heads, size, eps, dtype_code(dtype), _stream())
     _check(lib, "wkv", rc)
     return y
 
@@ -1623,8 +1720,8 @@ def unary(x: torch.Tensor, op: str, dtype: torch.dtype, arg: float = 0.0, out: O
     elif out.dtype != dtype or out.shape != x.shape or out.stride(1) != 1:
         raise KernelError("unary: out must have x's shape, dense rows and the named dtype")
     lib = load_library("activation")
-    rc = lib.kllm_unary(_p(out), ctypes.c_int64(out.stride(0)), _p(x), ctypes.c_int64(x.stride(0)), x.shape[0],
-                        x.shape[1], _UNARY[op], ctypes.c_float(arg), dtype_code(dtype), _stream())
+    rc = lib.kllm_unary(_p(out), out.stride(0), _p(x), x.stride(0), x.shape[0],
+                        x.shape[1], _UNARY[op], arg, dtype_code(dtype), _stream())
     _check(lib, "activation", rc)
     return out
 
@@ -1651,9 +1748,9 @@ def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
         # portions: the chunks' own sums in parallel, then the state's walk (two kernels; see csrc/lightning.cu)
         n = q.shape[0]
         work = torch.empty((3, n, heads * max(dk, dv)), dtype=torch.float32, device=q.device)
-        rc = lib.kllm_lightning_scan_portions(_p(o), ctypes.c_int64(o.stride(0)), _p(q), ctypes.c_int64(q.stride(0)), _p(k),
-                                              ctypes.c_int64(k.stride(0)), _p(v), ctypes.c_int64(v.stride(0)), _p(decay),
-                                              _p(state), ctypes.c_int64(state.stride(0)), _p(ctx.q_start),
+        rc = lib.kllm_lightning_scan_portions(_p(o), o.stride(0), _p(q), q.stride(0), _p(k),
+                                              k.stride(0), _p(v), v.stride(0), _p(decay),
+                                              _p(state), state.stride(0), _p(ctx.q_start),
                                               _p(ctx.state_slots), n, ctx.n_requests, n // 32 + ctx.n_requests, heads, dk,
                                               dv, _p(work[0]), _p(work[1]), _p(work[2]), _stream())
         if rc != -3:
@@ -1661,9 +1758,9 @@ def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
             global launches
             launches += 1
             return o
-    rc = lib.kllm_lightning_scan(_p(o), ctypes.c_int64(o.stride(0)), _p(q), ctypes.c_int64(q.stride(0)), _p(k),
-                                 ctypes.c_int64(k.stride(0)), _p(v), ctypes.c_int64(v.stride(0)), _p(decay), _p(state),
-                                 ctypes.c_int64(state.stride(0)), _p(ctx.q_start), _p(ctx.state_slots), q.shape[0],
+    rc = lib.kllm_lightning_scan(_p(o), o.stride(0), _p(q), q.stride(0), _p(k),
+                                 k.stride(0), _p(v), v.stride(0), _p(decay), _p(state),
+                                 state.stride(0), _p(ctx.q_start), _p(ctx.state_slots), q.shape[0],
                                  ctx.n_requests, heads, dk, dv, _stream())
     _check(lib, "lightning", rc)
     return o
@@ -1678,8 +1775,8 @@ def lightning_gate_norm(o: torch.Tensor, g: torch.Tensor, gain: torch.Tensor, ep
         raise KernelError("lightning_gate_norm: gain must be contiguous float32 [width], g as many rows as o")
     y = torch.empty((o.shape[0], width), dtype=dtype, device=o.device)
     lib = load_library("lightning")
-    rc = lib.kllm_lightning_gate_norm(_p(y), _p(o), ctypes.c_int64(o.stride(0)), _p(g), ctypes.c_int64(g.stride(0)),
-                                      _p(gain), o.shape[0], width, ctypes.c_float(eps), dtype_code(dtype), _stream())
+    rc = lib.kllm_lightning_gate_norm(_p(y), _p(o), o.stride(0), _p(g), g.stride(0),
+                                      _p(gain), o.shape[0], width, eps, dtype_code(dtype), _stream())
     _check(lib, "lightning", rc)
     return y
 
@@ -1735,11 +1832,11 @@ def gla(y: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: t
         a_last, s_in = torch.empty((bound, heads * dk), **f32), torch.empty((bound, heads, dk, dv), **f32)
         w = torch.empty((bound, heads, C, C), **f32)
         o = torch.empty((n, heads * dv), **f32) if dv > 256 else None
-    rc = lib.kllm_gla(_p(y), ctypes.c_int64(y.stride(0)), _p(q), _p(k), _p(v), _p(g), ctypes.c_int64(q.stride(0)), _p(low),
-                      _p(w2), _p(w2_bias), R, ctypes.c_float(1.0 / tau), _p(decay), _p(freq),
-                      2 * freq.numel() if freq is not None else 0, ctypes.c_float(amplitude), ctypes.c_float(q_scale),
-                      ctypes.c_float(k_scale), _p(ctx.positions), _p(ctx.q_start), _p(ctx.start_pos), _p(ctx.state_slots),
-                      _p(state), ctypes.c_int64(state.stride(0)), _p(gain), ctypes.c_float(eps), n, ctx.n_requests, heads,
+    rc = lib.kllm_gla(_p(y), y.stride(0), _p(q), _p(k), _p(v), _p(g), q.stride(0), _p(low),
+                      _p(w2), _p(w2_bias), R, 1.0 / tau, _p(decay), _p(freq),
+                      2 * freq.numel() if freq is not None else 0, amplitude, q_scale,
+                      k_scale, _p(ctx.positions), _p(ctx.q_start), _p(ctx.start_pos), _p(ctx.state_slots),
+                      _p(state), state.stride(0), _p(gain), eps, n, ctx.n_requests, heads,
                       dk, dv, int(ctx.all_single), int(early), bound, _p(o), _p(qa), _p(kd), _p(a_last),
                       _p(w), _p(s_in), dtype_code(y.dtype), _stream())
     _check(lib, "gla", rc)
@@ -1793,9 +1890,9 @@ def ssd(proj: torch.Tensor, conv: torch.Tensor, conv_bias: torch.Tensor, dt_bias
             s_split = torch.empty((2, bound, heads, N, dv), dtype=torch.bfloat16, device=proj.device)
         else:
             xc, pairs = torch.empty((n, row), **f32), torch.empty((bound, groups, C, C), **f32)
-    rc = lib.kllm_ssd(_p(y), _p(proj), ctypes.c_int64(proj.stride(0)), _p(conv), _p(conv_bias), _p(dt_bias), _p(a_log), _p(d),
-                      _p(ctx.q_start), _p(ctx.start_pos), _p(ctx.state_slots), _p(state), ctypes.c_int64(state.stride(0)),
-                      _p(ring), ctypes.c_int64(ring.stride(0)), n, ctx.n_requests, heads, groups, N, dv, taps,
+    rc = lib.kllm_ssd(_p(y), _p(proj), proj.stride(0), _p(conv), _p(conv_bias), _p(dt_bias), _p(a_log), _p(d),
+                      _p(ctx.q_start), _p(ctx.start_pos), _p(ctx.state_slots), _p(state), state.stride(0),
+                      _p(ring), ring.stride(0), n, ctx.n_requests, heads, groups, N, dv, taps,
                       int(ctx.all_single), int(early), bound, _p(xc), _p(dt), _p(cum), _p(pairs), _p(s_in), _p(s_split),
                       dtype_code(dtype), _stream())
     _check(lib, "ssd", rc)
@@ -1814,8 +1911,8 @@ def part_norm(out: torch.Tensor, y: torch.Tensor, gain: torch.Tensor, parts: int
         raise KernelError("part_norm: y contiguous float32 [n, width], out alike with dense rows, the parts dividing the width")
     _bias(gain, width, "part_norm")
     lib = load_library("ssd")
-    rc = lib.kllm_part_norm(_p(out), ctypes.c_int64(out.stride(0)), _p(y), _p(gain), n, int(parts), width // parts,
-                            ctypes.c_float(eps), dtype_code(out.dtype), _stream())
+    rc = lib.kllm_part_norm(_p(out), out.stride(0), _p(y), _p(gain), n, int(parts), width // parts,
+                            eps, dtype_code(out.dtype), _stream())
     _check(lib, "ssd", rc)
 
 
@@ -1835,8 +1932,8 @@ def norm_shift(x: torch.Tensor, gain: torch.Tensor, eps: float, mu: torch.Tensor
         raise KernelError("norm_shift: the state must be float32 [slots, >= d]")
     h, hs = (torch.empty((n, d), dtype=dtype, device=x.device) for _ in range(2))
     lib = load_library("shift_norm")
-    rc = lib.kllm_norm_shift(_p(h), _p(hs), _p(x), _p(gain), _p(mu), ctypes.c_float(eps), _p(state),
-                             ctypes.c_int64(state.stride(0)), _p(ctx.q_start), _p(ctx.token_req), _p(ctx.state_slots), n, d,
+    rc = lib.kllm_norm_shift(_p(h), _p(hs), _p(x), _p(gain), _p(mu), eps, _p(state),
+                             state.stride(0), _p(ctx.q_start), _p(ctx.token_req), _p(ctx.state_slots), n, d,
                              dtype_code(dtype), _stream())
     _check(lib, "shift_norm", rc)
     return h, hs
@@ -1891,9 +1988,9 @@ def attention_mixed(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vc
     key = (n_heads, n_kv, head_dim, v_head_dim)
     if (MIXED_MMA and q.dtype == torch.bfloat16 and not ctx.all_single and q.data_ptr() % 16 == 0 and q.stride(0) % 8 == 0):
         tiles = ctx.n_tokens // 16 + ctx.n_requests
-        args = (_p(out), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache), _p(mix), _p(sinks), _p(ctx.q_start),
+        args = (_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache), _p(mix), _p(sinks), _p(ctx.q_start),
                 _p(ctx.start_pos), _p(block_table), block_table.shape[1], ctx.n_requests, int(tiles), n_heads, n_kv, head_dim,
-                v_head_dim, page_size, int(window or 0), ctypes.c_float(scale), _stream())
+                v_head_dim, page_size, int(window or 0), scale, _stream())
         # first the form in which the blocks of heads of a tile share their raw scores across a cluster of CTAs
         if MIXED_CLUSTER and lib.kllm_attention_mixed_cluster_fits(*key):
             rc = lib.kllm_attention_mixed_cluster(*args)
@@ -1924,10 +2021,10 @@ def attention_mixed(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vc
         if splits > 1:
             part_o = torch.empty((n, splits, n_heads * v_head_dim), dtype=torch.float32, device=q.device)
             part_ml = torch.empty((n, splits, n_heads, 2), dtype=torch.float32, device=q.device)
-    rc = lib.kllm_attention_mixed(_p(out), _p(q), ctypes.c_int64(q.stride(0)), _p(kcache), _p(vcache), _p(mix), _p(sinks),
+    rc = lib.kllm_attention_mixed(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache), _p(mix), _p(sinks),
                                   _p(ctx.q_start), _p(ctx.start_pos), _p(block_table), block_table.shape[1],
                                   ctx.n_requests, int(tiles), int(rows), n_heads, n_kv, head_dim, v_head_dim, page_size,
-                                  int(window or 0), ctypes.c_float(scale), int(splits), _p(part_o), _p(part_ml),
+                                  int(window or 0), scale, int(splits), _p(part_o), _p(part_ml),
                                   dtype_code(q.dtype), _stream())
     _check(lib, "attention_mixed", rc)
     if splits > 1:
@@ -1965,7 +2062,7 @@ def moe_route(h: torch.Tensor, router: torch.Tensor, top: int, score: str = "sig
     lib = load_library("moe")
     rc = lib.kllm_moe_route(_p(idx), _p(wt), _p(h), _p(router), n, d, router.shape[0], int(top),
                             int(score == "softmax"), int(bool(renormalize)), int(groups or 1), int(keep or 1),
-                            _p(correction), ctypes.c_float(sum_eps), dtype_code(h.dtype), _stream())
+                            _p(correction), sum_eps, dtype_code(h.dtype), _stream())
     _check(lib, "moe", rc)
     return idx, wt
 
@@ -2012,9 +2109,9 @@ def moe_gemm(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, perm: torc
         raise KernelError("moe_gemm: one float32 weight per (token, choice)")
     c = torch.empty((rows, N), dtype=a.dtype if gated else torch.float32, device=a.device)
     lib = load_library("moe")
-    rc = lib.kllm_moe_gemm(_p(c), _p(a), ctypes.c_int64(a.stride(0)), _p(w), _p(offsets), _p(perm), _p(wt), rows, E,
+    rc = lib.kllm_moe_gemm(_p(c), _p(a), a.stride(0), _p(w), _p(offsets), _p(perm), _p(wt), rows, E,
                            int(top), N, K, form, int(scale_in), int(scale_out), _GATED_ACT.get(activation, 0),
-                           ctypes.c_float(limit), ctypes.c_float(alpha), dtype_code(a.dtype), _stream())
+                           limit, alpha, dtype_code(a.dtype), _stream())
     _check(lib, "moe", rc)
     return c
 
@@ -2059,7 +2156,7 @@ def moe_gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, pe
     lib = load_library("moe_gemm_tcgen05")
     if gated:
         xs = torch.empty((rows, K), dtype=a.dtype, device=a.device)
-        rc = lib.kllm_moe_gather_sorted(_p(xs), _p(a), ctypes.c_int64(a.stride(0)), _p(perm), rows, int(top), K,
+        rc = lib.kllm_moe_gather_sorted(_p(xs), _p(a), a.stride(0), _p(perm), rows, int(top), K,
                                         _p(offsets[E:]), _stream())
         _check(lib, "moe_gemm_tcgen05", rc)
         a = xs
@@ -2067,7 +2164,7 @@ def moe_gemm_tcgen05(a: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, pe
         raise KernelError("moe_gemm_tcgen05: the sorted rows must be contiguous")
     c = torch.empty((rows, N), dtype=a.dtype if gated else torch.float32, device=a.device)
     rc = lib.kllm_moe_gemm_tcgen05(_p(c), _p(a), _p(w), _p(offsets), _p(perm), _p(wt), rows, E, N, K, form,
-                                   int(scale_out), _GATED_ACT.get(activation, 0), ctypes.c_float(limit), ctypes.c_float(alpha),
+                                   int(scale_out), _GATED_ACT.get(activation, 0), limit, alpha,
                                    _p(status_word(a.device)), _stream())
     _check(lib, "moe_gemm_tcgen05", rc)
     return c
@@ -2104,7 +2201,7 @@ def moe_combine(parts: torch.Tensor, top: int, shared: Optional[torch.Tensor] = 
     y = into if into is not None else torch.empty((n, d), dtype=torch.float32, device=parts.device)
     lib = load_library("moe")
     rc = lib.kllm_moe_combine(_p(y), _p(parts), n, d, int(top), _p(shared), _p(gate),
-                              ctypes.c_int64(gate.stride(0) if gate is not None else 0), ctypes.c_float(scale),
+                              (gate.stride(0) if gate is not None else 0), scale,
                               int(into is not None), _p(h), _p(idx), _p(wt), int(experts),
                               dtype_code(h.dtype if h is not None else torch.float32), _stream())
     _check(lib, "moe", rc)
@@ -2123,6 +2220,6 @@ def moe_table_route(token_ids: torch.Tensor, table: torch.Tensor, experts: int, 
     wt = torch.empty((n, top), dtype=torch.float32, device=table.device)
     lib = load_library("moe")
     rc = lib.kllm_moe_table_route(_p(idx), _p(wt), _p(token_ids), _p(last_token), _p(table), n, vocab, int(experts),
-                                  top, ctypes.c_float(weight), _stream())
+                                  top, weight, _stream())
     _check(lib, "moe", rc)
     return idx, wt

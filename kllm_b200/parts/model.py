@@ -17,6 +17,7 @@ import torch
 from . import (attention, block, embedding, gla, latent_attention, lightning, mlp, moe, norm, qk_norm, rotary,  # noqa: F401
                side_by_side, side_input, ssd, stream_entry, streams, wkv)
 from .context import LayerCache, StepContext
+from .prompt_layers import PromptLayers
 from .spec import BuildEnv, ModelSpec, PagedKVNeed, StateNeed, TensorSpec, part_factory
 
 
@@ -36,6 +37,7 @@ class DecoderModel:
         self.schedule = list(spec.schedule)
         self.tap = None         # debugging: tap(i, x) is called with the residual stream after schedule entry i
         self._check_schedule()
+        self.prompt_layers = None   # the layers of a step with portions from one native call, where the model allows it
 
     def _check_schedule(self):
         writers: Dict[int, int] = {}
@@ -89,6 +91,7 @@ class DecoderModel:
             if tell is not None and call.block not in told:
                 told.add(call.block)
                 tell(self.blocks[nxt.block])
+        self.prompt_layers = PromptLayers.of(self)
 
     # ---- cache -----------------------------------------------------------
     def cache_needs(self):
@@ -114,7 +117,11 @@ class DecoderModel:
             x = self.embedding.forward(ctx.token_ids, ctx.last_token)
         held = [e.begin(x, bool(self.schedule) and self.schedule[0].entry is not None
                         and self.schedule[0].entry[0] == j) for j, e in enumerate(self.entries)]
-        for i, call in enumerate(self.schedule):
+        schedule = self.schedule
+        if self.prompt_layers is not None and self.tap is None and self.prompt_layers.takes(ctx, caches):
+            self.prompt_layers.run(x, ctx, caches)
+            schedule = []
+        for i, call in enumerate(schedule):
             cache = caches[call.cache]
             if cache.writes != call.writes_cache:
                 cache = LayerCache(cache.k, cache.v, cache.block_table, cache.state,

@@ -1,0 +1,79 @@
+"""All layers of a prompt's step, launched from one native call (csrc/prompt_layers.cu).
+
+``PromptLayers.of(model)`` is None unless every layer of the model is a pre-norm block of
+rotary attention over its own cache and a gated silu feed-forward with plain RMS norms, all
+of one size, in bfloat16 (the Llama layer).  ``takes(ctx, caches)`` says whether a step goes
+that way: more tokens than the weight-streaming products take, portions among them, a head
+size of the tcgen05 attention.  The kernels, their arguments and their order are those of the
+blocks' own forward; weights and cache pages are named at every call.
+"""
+from __future__ import annotations
+
+from .. import kernels
+from .attention import PagedAttention
+from .block import PreNormBlock
+from .mlp import GatedMLP
+from .norm import RMSNorm
+
+import torch
+
+
+def _plain_attention(m) -> bool:
+    return (type(m) is PagedAttention and not m.window and m.qk_transform is None and m.score_slopes is None
+            and m.v_head_dim == m.head_dim and not m.exact_weights and not m.segment and not m.keep_first
+            and m.maps == 1 and not m.gate_name and m.out_factor == 1.0 and m.sinks is None and not m.has_bias
+            and m.mix_name is None and m.position is not None
+            and getattr(m.position, "full_rotary_table", lambda: None)() is not None)
+
+
+class PromptLayers:
+    def __init__(self, model):
+        self.blocks = [model.blocks[call.block] for call in model.schedule]
+        self.slots = [call.cache for call in model.schedule]
+        m, f = self.blocks[0].mixer, self.blocks[0].feed_forward
+        self.d, self.heads, self.kv, self.head_dim, self.inter = m.hidden, m.n_heads, m.n_kv, m.head_dim, f.inter
+        self.eps, self.scale = self.blocks[0].mixer_norm.eps, m.scale
+        self.table = m.position.full_rotary_table()
+
+    @staticmethod
+    def of(model):
+        if model.dtype != torch.bfloat16 or model.device.type != "cuda" or not model.schedule or model.entries:
+            return None
+        first = None
+        for call in model.schedule:
+            b = model.blocks[call.block]
+            if type(b) is not PreNormBlock or not call.writes_cache or call.entry is not None:
+                return None
+            m, f = b.mixer, b.feed_forward
+            if not _plain_attention(m) or type(f) is not GatedMLP or not f.plain:
+                return None
+            if type(b.mixer_norm) is not RMSNorm or type(b.ff_norm) is not RMSNorm:
+                return None
+            if not all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (
+                    m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain)):
+                return None
+            key = (m.hidden, m.n_heads, m.n_kv, m.head_dim, m.scale, f.hidden, f.inter, b.mixer_norm.eps, b.ff_norm.eps)
+            if m.hidden != f.hidden or b.mixer_norm.eps != b.ff_norm.eps or (first is not None and key != first[0]):
+                return None
+            table = m.position.full_rotary_table()
+            if first is not None and not (table is first[1] or torch.equal(table, first[1])):
+                return None
+            first = first or (key, table)
+        return PromptLayers(model)
+
+    def takes(self, ctx, caches) -> bool:
+        group = self.heads // self.kv
+        if (ctx.all_single or not ctx.host_n_new or ctx.n_tokens <= kernels.SKINNY_MAX_ROWS or group > 64
+                or not kernels.USE_TCGEN05 or self.head_dim not in kernels.TCGEN05_HEAD_DIMS):
+            return False
+        c = caches[self.slots[0]]
+        return kernels.prompt_layers_ready() and all(
+            caches[i].block_table is c.block_table and caches[i].k.shape[2] == c.page_size for i in self.slots)
+
+    def run(self, x, ctx, caches) -> None:
+        layers = []
+        for b, i in zip(self.blocks, self.slots):
+            m, f, c = b.mixer, b.feed_forward, caches[i]
+            layers.append((m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain, c.k, c.v))
+        kernels.prompt_layers(x, layers, self.table, ctx, caches[self.slots[0]].block_table, self.heads, self.kv, self.head_dim,
+                              self.inter, self.eps, self.scale)

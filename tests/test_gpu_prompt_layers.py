@@ -1,0 +1,101 @@
+"""A step with portions launched from one native call (csrc/prompt_layers.cu) against the same step launched part by
+part: the same kernels in the same order, so the caches and logits agree to the bit where the library picks the same
+product kernel, and within two ways of summing in any case."""
+import random
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+CONFIGS = {  # hidden, heads, kv heads, head size, feed-forward
+    "d64": (256, 8, 2, 64, 704), "d128": (512, 4, 4, 128, 1024), "wide group": (640, 20, 1, 64, 192),
+}
+# requests' tokens in the step: single tokens first, then portions; the first portion continues a prompt
+STEPS = [[17], [1, 16], [1, 1, 1, 40, 9, 1], [200, 3], [1] * 6 + [130]]
+
+
+def _config(name):
+    d, h, g, hd, f = CONFIGS[name]
+    return {"architectures": ["LlamaForCausalLM"], "num_hidden_layers": 3, "hidden_size": d, "num_attention_heads": h,
+            "num_key_value_heads": g, "head_dim": hd, "intermediate_size": f, "vocab_size": 512, "rope_theta": 10000.0,
+            "rms_norm_eps": 1e-5, "max_position_embeddings": 1024}
+
+
+def _run(name, step, native):
+    from kllm_b200 import Engine, Options, StepEntry
+    rng = random.Random(len(step))
+    engine = Engine(None, Options(max_seq=512, block_size=16, num_blocks=300, max_batch=8, max_step_tokens=512, dtype="bfloat16"),
+                    config=_config(name), random_seed=3)
+    assert engine.model.prompt_layers is not None
+    runs = []
+    if native:
+        inner = engine.model.prompt_layers
+        inner_run = inner.run
+        inner.run = lambda *a: (runs.append(1), inner_run(*a))
+    else:
+        engine.model.prompt_layers = None
+    requests = [engine.cache.open() for _ in step]
+    for i, r in enumerate(requests):
+        engine.step([StepEntry(r, [rng.randrange(512) for _ in range(5 + 37 * i % 90)])])
+    del runs[:]
+    tokens = [[rng.randrange(512) for _ in range(n)] for n in step]
+    logits = engine.step([StepEntry(r, t, [len(t) - 1]) for r, t in zip(requests, tokens)]).clone()
+    keys = [k.clone() for k in engine.cache.groups[0].k_store + engine.cache.groups[0].v_store]
+    engine.close()
+    assert len(runs) == (1 if native else 0)
+    return logits, keys
+
+
+@pytest.mark.parametrize("step", STEPS, ids=lambda s: "+".join(map(str, s)))
+@pytest.mark.parametrize("name", list(CONFIGS))
+def test_native_launches_agree(name, step):
+    a, ka = _run(name, step, False)
+    b, kb = _run(name, step, True)
+    # two orders of summing the same bfloat16 products differ by 7e-3 of the largest logit at most (tests/test_gpu_replay.py)
+    assert (a - b).abs().max() <= 1e-2 * a.abs().max()
+    for x, y in zip(ka, kb):
+        assert (x.float() - y.float()).abs().max() <= 2.0 ** -6 * x.float().abs().max()
+
+
+def test_steps_that_stay_with_the_parts():
+    """Decode steps and steps of few tokens do not go that way, nor a step that is watched layer by layer."""
+    from kllm_b200 import Engine, Options, StepEntry
+    engine = Engine(None, Options(max_seq=128, block_size=16, num_blocks=80, max_batch=4, dtype="bfloat16", max_step_tokens=128),
+                    config=_config("d64"), random_seed=1)
+    taken = []
+    inner = engine.model.prompt_layers.run
+    engine.model.prompt_layers.run = lambda *a: (taken.append(1), inner(*a))
+    r = [engine.cache.open() for _ in range(3)]
+    engine.step([StepEntry(r[0], [1] * 16, [15])])
+    engine.step([StepEntry(x, [2], [0]) for x in r])
+    engine.model.tap = lambda i, x: None
+    engine.step([StepEntry(r[1], [1] * 30, [29])])
+    engine.model.tap = None
+    assert not taken
+    engine.step([StepEntry(r[2], [1] * 30, [29])])
+    assert taken
+    engine.close()
+
+
+def test_wide_step_takes_the_gated_product():
+    """Where gate, up and activation are one kernel it runs between the halves of every layer."""
+    from kllm_b200 import Engine, Options, StepEntry, kernels
+    cfg = dict(_config("d64"), intermediate_size=9472, max_position_embeddings=4096)
+    assert kernels.gemm_pays(512, 9472, "swiglu")
+    out = []
+    for native in (False, True):
+        engine = Engine(None, Options(max_seq=600, block_size=16, num_blocks=160, max_batch=3, max_step_tokens=600, dtype="bfloat16"),
+                        config=cfg, random_seed=5)
+        if not native:
+            engine.model.prompt_layers = None
+        r = [engine.cache.open() for _ in range(2)]
+        engine.step([StepEntry(r[0], [3] * 20)])
+        before = kernels.launches
+        out.append((engine.step([StepEntry(r[0], [7], [0]), StepEntry(r[1], [i % 512 for i in range(511)], [100, 510])]).clone(),
+                    kernels.launches - before))
+        engine.close()
+    (a, la), (b, lb) = out
+    assert (a - b).abs().max() <= 1e-2 * a.abs().max()
+    assert la == lb                                   # the same kernels
