@@ -653,19 +653,27 @@ def sm_count() -> int:
     return _sm_count[dev]
 
 
-def decode_splits(n_tokens: int, n_kv: int, ctx_bound: int) -> int:
+def decode_splits(n_tokens: int, n_kv: int, ctx_bound: int, head_dim: int = 128) -> int:
     """Into how many key ranges the decode kernel cuts a token's context.
 
-    A CTA takes one (token, kv head, range); two CTAs fit an SM.  The ranges are
-    whole 64-key tiles, as many as fill the SMs in ONE wave (a second wave of short
-    CTAs would double the kernel's time), at most 16, all the same length.  When one
-    range per token would be long, two are used even if that spills into a second
-    wave: long CTAs hide it."""
+    A CTA takes one (token, kv head, range) and walks it in tiles of 64 keys.  Cutting costs about
+    2.3 us (partial results out and in again, the merge), a tile 0.35 us in a CTA whose tiles are all
+    requested at once.  So, measured (us, by ranges):
+      - up to 8 tiles are not cut: 24 x 4 (tokens x kv heads) of size 64 at 200 keys 1: 4.9, 2: 7.2;
+        4 x 32 of size 128 at 300 keys 1: 7.4, 2: 8.9; at 10 tiles it makes no difference (9.8, 9.9);
+      - fewer (token, kv head) pairs than slots (two CTAs an SM): as many ranges as fill the SMs in ONE wave,
+        at most 16 (a second wave of short CTAs would double the time);
+      - more pairs are CTAs enough: 64 x 8 of size 128 at 1280 keys 1: 57.4, 2: 69.9; 32 x 8 at 2000 keys 1: 48.1,
+        2: 50.0; 24 x 32 at 1500 keys 1: 94.3, 2: 106.9.  Only at small head sizes, where a tile is half the bytes and
+        two CTAs do not keep an SM's share of the memory busy, a long context is cut in two while the CTAs still fit at
+        once: 64 x 4 of size 64 at 2000 keys 1: 32.3, 2: 27.5."""
     slots = 2 * sm_count()
     tiles = max(1, -(-ctx_bound // 64))
     base = max(1, n_tokens * n_kv)
+    if tiles <= 8:
+        return 1
     splits = max(1, min(slots // base, tiles, 16))
-    if splits == 1 and tiles >= 16:
+    if splits == 1 and tiles >= 16 and head_dim <= 64 and base <= slots:
         splits = 2
     per = -(-tiles // splits)
     return -(-tiles // per)
@@ -726,7 +734,7 @@ def attention(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcache: 
         # token t of the first `singles` is request t: no token-to-request table needed
         attention_decode(out[:singles], q[:singles], kcache, vcache, ctx.positions[:singles], None, block_table[:singles],
                          n_heads, n_kv, head_dim, window, scale,
-                         decode_splits(singles, groups, min(bound, seen)), slopes=score_slopes,
+                         decode_splits(singles, groups, min(bound, seen), head_dim), slopes=score_slopes,
                          split_weights=exact_weights, sinks=sinks, v_head_dim=vd, keep=keep)
     if wide and not short and (ctx.all_single or not ctx.host_n_new):
         if wide_decode and ctx.all_single:
@@ -761,7 +769,7 @@ def attention(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcache: 
     if tc and ctx.all_single and group <= 64:
         return attention_decode(out, q, kcache, vcache, ctx.positions, ctx.token_req, block_table, n_heads,
                                 n_kv, head_dim, window, scale,
-                                decode_splits(ctx.n_tokens, groups, min(ctx.split_bound or ctx.max_ctx, seen)),
+                                decode_splits(ctx.n_tokens, groups, min(ctx.split_bound or ctx.max_ctx, seen), head_dim),
                                 slopes=score_slopes, split_weights=exact_weights, sinks=sinks, keep=keep)
     singles = 0
     if tc and group <= 64 and ctx.host_n_new:
@@ -1309,7 +1317,7 @@ def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_tab
     if singles:
         group = n_heads // n_kv
         groups = n_kv * next((s for s in range(1, group + 1) if group % s == 0 and group // s <= 16), 1)
-        splits = decode_splits(singles, groups, ctx.max_ctx)
+        splits = decode_splits(singles, groups, ctx.max_ctx, head_dim)
         if splits > 1:
             part_o = new(singles, n_heads, splits, head_dim, dtype=torch.float32)
             part_ml = new(singles, n_heads, splits, 2, dtype=torch.float32)

@@ -282,7 +282,7 @@ class PagedAttention:
             kernels.attention_decode_fused(
                 attn, q, k, v, table, cache.k, cache.v, ctx.positions, None, cache.block_table,   # token t is request t
                 self._counters, self.n_heads, self.n_kv, self.head_dim, self.window or 0, self.scale,
-                kernels.decode_splits(n, self.n_kv, ctx.split_bound or ctx.max_ctx), prefetch=prefetch)
+                kernels.decode_splits(n, self.n_kv, ctx.split_bound or ctx.max_ctx, self.head_dim), prefetch=prefetch)
             return attn
         if self.position is not None:
             self.position.apply(q, k, v, ctx, cache, self.n_heads, self.n_kv)
