@@ -4,8 +4,9 @@
 rotary attention over its own cache and a gated silu feed-forward with plain RMS norms, all
 of one size, in bfloat16 (the Llama layer).  ``takes(ctx, caches)`` says whether a step goes
 that way: more tokens than the weight-streaming products take, portions among them, a head
-size of the tcgen05 attention.  The kernels, their arguments and their order are those of the
-blocks' own forward; weights and cache pages are named at every call.
+size of the tcgen05 attention, and so little work that the host's launches would be the longer
+part.  The kernels, their arguments and their order are those of the blocks' own forward;
+weights and cache pages are named at every call.
 """
 from __future__ import annotations
 
@@ -16,6 +17,11 @@ from .mlp import GatedMLP
 from .norm import RMSNorm
 
 import torch
+
+# Steps of up to so many operations in a layer's products go this way.  The parts' own launches take 0.21 ms a layer on the
+# host: at 0.74e11 (841 tokens of TinyLlama's sizes, 0.13 ms of GPU work a layer) that is the step's time, 4.6 ms against
+# 2.9 from here; at 1.8e11 (2048 tokens) the GPU is the slower of the two and the parts' launches were measured 0.5 % faster.
+MOST_WORK = 1.5e11
 
 
 def _plain_attention(m) -> bool:
@@ -34,6 +40,7 @@ class PromptLayers:
         self.d, self.heads, self.kv, self.head_dim, self.inter = m.hidden, m.n_heads, m.n_kv, m.head_dim, f.inter
         self.eps, self.scale = self.blocks[0].mixer_norm.eps, m.scale
         self.table = m.position.full_rotary_table()
+        self.weights = m.w_qkv.numel() + m.w_o.numel() + f.w_gate_up.numel() + f.w_down.numel()      # of one layer
 
     @staticmethod
     def of(model):
@@ -63,6 +70,8 @@ class PromptLayers:
 
     def takes(self, ctx, caches) -> bool:
         group = self.heads // self.kv
+        if 2.0 * ctx.n_tokens * self.weights > MOST_WORK:
+            return False
         if (ctx.all_single or not ctx.host_n_new or ctx.n_tokens <= kernels.SKINNY_MAX_ROWS or group > 64
                 or not kernels.USE_TCGEN05 or self.head_dim not in kernels.TCGEN05_HEAD_DIMS):
             return False
