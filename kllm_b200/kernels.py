@@ -911,14 +911,17 @@ def attention_prefill(out, q, kcache, vcache, q_start, start_pos, block_table, n
 
 def tcgen05_form(head_dim: int, group: int, n_kv: int, n_tokens: int, n_requests: int, max_ctx: int) -> str:
     """Which of the two tcgen05 attention kernels a step of portions takes ("smem" / "tmem",
-    see ``attention_prefill_tcgen05``), from measurements (profiles/attn_prefill_tc5_forms.md):
-    head size 128 always keeps its probabilities in tensor memory.  At head size 64 that form
-    (four CTAs per SM) wins when the step is many short chains of tiles or several waves of
-    CTAs, and loses to the other (two CTAs per SM, two score buffers) when one long prompt's
-    longest chain is the whole kernel: all CTAs resident at once and more than 16 key tiles."""
-    if head_dim != 64:
-        return "tmem"
+    see ``attention_prefill_tcgen05``), from measurements.
+
+    Head size 128 keeps its probabilities in tensor memory (two CTAs an SM) unless the step is about one CTA an
+    SM, where the other form's double-buffered scores win (8 kv heads, 700 tokens: smem 25.2 us, tmem 29.8; 32 kv heads,
+    300 tokens: 15.8, 19.7; 700 + 350 tokens: 70.7, 56.4; 8192: 1299, 843).  At head size 64 the tmem form has two
+    score buffers in small launches and four CTAs an SM in large ones (1000 tokens: smem 23.8, tmem 25.7; 8 x 150
+    tokens: 17.3, 16.8; 8192: 494, 480) and loses to the other when one long prompt's longest chain is the whole
+    kernel: all CTAs resident at once and more than 16 key tiles (2048 tokens: 45.6, 51.6)."""
     ctas = (n_tokens // max(1, 128 // group) + n_requests) * n_kv
+    if head_dim != 64:
+        return "smem" if ctas <= sm_count() * 6 // 5 else "tmem"
     tiles = -(-max_ctx // 64)
     return "tmem" if tiles <= 16 or ctas >= 6 * sm_count() else "smem"
 
@@ -931,8 +934,8 @@ def attention_prefill_tcgen05(out, q, kcache, vcache, q_start, start_pos, block_
     (csrc/attention_tcgen05.cu: two score buffers in tensor memory, P through shared
     memory, two CTAs of head size 64 per SM) or ``"tmem"`` (csrc/attention_tcgen05_ptmem.cu:
     P written over the scores in tensor memory and read from there, half the tensor memory
-    and shared memory per CTA, four / two CTAs per SM).  Default (no step shape known): tmem
-    for head size 128 (1.3 to 1.6 times faster), smem for head size 64; ``attention`` picks
+    and shared memory per CTA, up to four / two CTAs per SM).  Default (no step shape known): tmem
+    for head size 128, smem for head size 64; ``attention`` picks
     by the step's shape (``tcgen05_form``)."""
     _cuda(out, q, kcache, vcache, q_start, start_pos, block_table)
     _check_attention(out, q, kcache, vcache, block_table, n_kv, head_dim)
