@@ -15,6 +15,7 @@ from .attention import PagedAttention
 from .block import PreNormBlock
 from .mlp import GatedMLP
 from .norm import RMSNorm
+from .rotary import RotaryEmbedding
 
 import torch
 
@@ -30,6 +31,15 @@ def _plain_attention(m) -> bool:
             and m.maps == 1 and not m.gate_name and m.out_factor == 1.0 and m.sinks is None and not m.has_bias
             and m.mix_name is None and m.position is not None
             and getattr(m.position, "full_rotary_table", lambda: None)() is not None)
+
+
+def _same_rotation(p, q) -> bool:
+    """Whether two position parts have one table of angles (built-in ones by their parameters: comparing 22 tables on the
+    device took 10 ms of an engine's start)."""
+    a, b = p.full_rotary_table(), q.full_rotary_table()
+    if type(p) is RotaryEmbedding and type(q) is RotaryEmbedding:
+        return (p.theta, p.rotary_dim, a.shape) == (q.theta, q.rotary_dim, b.shape)
+    return a is b or torch.equal(a, b)
 
 
 class PromptLayers:
@@ -62,10 +72,9 @@ class PromptLayers:
             key = (m.hidden, m.n_heads, m.n_kv, m.head_dim, m.scale, f.hidden, f.inter, b.mixer_norm.eps, b.ff_norm.eps)
             if m.hidden != f.hidden or b.mixer_norm.eps != b.ff_norm.eps or (first is not None and key != first[0]):
                 return None
-            table = m.position.full_rotary_table()
-            if first is not None and not (table is first[1] or torch.equal(table, first[1])):
+            if first is not None and not _same_rotation(m.position, first[1]):
                 return None
-            first = first or (key, table)
+            first = first or (key, m.position)
         return PromptLayers(model)
 
     def takes(self, ctx, caches) -> bool:
