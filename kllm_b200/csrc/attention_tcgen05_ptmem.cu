@@ -89,6 +89,14 @@ struct Form {
     static constexpr int REGS_SOFTMAX = CTAS_PER_SM == 4 ? 88 : 184, REGS_OTHERS = CTAS_PER_SM == 4 ? 40 : 64;
     // setmaxnreg moves registers inside the CTA's own allocation (threads x registers at launch)
     static_assert(SOFTMAX_THREADS * (REGS_SOFTMAX + REGS_OTHERS) <= THREADS * ((65536 / (THREADS * CTAS_PER_SM)) / 8 * 8), "setmaxnreg budget");
+
+    // The products into the output that a barrier phase of their own announces (bar_o_full), and the phase that the
+    // last one's is.  A wait by parity is only sound for the phase behind the one waited for last: with two score buffers
+    // the softmax waits for every product, with one for the last alone (those before it are ordered by the scores that
+    // come behind them), so that the barrier completes only once.
+    __host__ __device__ static constexpr bool announces_product(int j, int ntiles) { return SBUF > 1 || j == ntiles - 1; }
+    __host__ __device__ static constexpr bool awaits_before_rescale(int j) { return SBUF > 1 && j > 0; }      // the product of tile j - 1
+    __host__ __device__ static constexpr int last_phase(int ntiles) { return SBUF > 1 ? ntiles - 1 : 0; }
 };
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const void* gmem, bool valid) {
@@ -326,7 +334,7 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
                 for (int kk = 0; kk < TILE / 16; kk++)
                     umma_tmem_a_words(t_o, t_s + (unsigned)(b * TILE + kk * 8), v_lo + (uint32_t)(kk * (2048 >> 4)), IDESC_O, j > 0 || kk > 0);
                 umma_commit(&bar_v_empty[s]);
-                umma_commit(&bar_o_full);
+                if (Form<SBUF>::announces_product(j, ntiles)) umma_commit(&bar_o_full);
             }
             __syncwarp();
             if (j + SBUF < ntiles) {
@@ -431,10 +439,9 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
                 tmem_st16(t_s + c * 16, pk);
             }
             l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            if (SBUF > 1 && j > 0) {
+            if (Form<SBUF>::awaits_before_rescale(j)) {
                 // The product of tile j - 1 must be over before the accumulator is rescaled (with one buffer it is: the
-                // scores of tile j came behind it).  Every tile waits, also where nothing is rescaled: a wait by parity
-                // is only sound for the phase that follows the one waited for last.
+                // scores of tile j came behind it).  Every tile waits, also where nothing is rescaled (see Form).
                 ok = mbar_wait(&bar_o_full, (unsigned)(j - 1) & 1u, abort_flag, status, 10);
                 if (!ok) break;
                 tc_fence_after();
@@ -458,7 +465,7 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
             tc_fence_before();
             mbar_arrive(&bar_p_full[b]);       // P of tile j is in tensor memory, the accumulator is rescaled
         }
-        if (ok) ok = mbar_wait(&bar_o_full, (unsigned)(ntiles - 1) & 1u, abort_flag, status, 9);
+        if (ok) ok = mbar_wait(&bar_o_full, (unsigned)Form<SBUF>::last_phase(ntiles) & 1u, abort_flag, status, 9);
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / l_run;
@@ -493,6 +500,24 @@ bool g_attr_set[2] = {false, false};
 }  // namespace
 
 extern "C" int kllm_attention_tcgen05_ptmem_head_dim() { return HD; }
+
+// For a chain of ntiles tiles with 1 or 2 score buffers: announced[j] is whether tile j's product completes a phase of the
+// output's barrier; awaited[0 .. n - 1] are the phases that the softmax waits for, in its order.  Returns n (0: no such form).
+extern "C" int kllm_attention_tcgen05_ptmem_output_phases(int score_buffers, int ntiles, int* announced, int* awaited) {
+    auto list = [&](auto form) {
+        int n = 0;
+        for (int j = 0; j < ntiles; j++) {
+            announced[j] = form.announces_product(j, ntiles);
+            if (form.awaits_before_rescale(j)) awaited[n++] = j - 1;
+        }
+        awaited[n++] = form.last_phase(ntiles);
+        return n;
+    };
+#if KLLM_HD == 64
+    if (score_buffers == 2) return list(Form<2>());
+#endif
+    return score_buffers == 1 ? list(Form<1>()) : 0;
+}
 
 // Same contract as the mma.sync prefill kernel: requests' portions
 // q_start[s]..q_start[s+1] start at cache position start_pos[s]; out [n, n_heads*HD].
