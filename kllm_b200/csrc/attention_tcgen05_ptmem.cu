@@ -7,7 +7,7 @@
 // shared memory; the Python face picks between them by head size from measurements.
 //
 // A CTA takes 128 rows = (tokens of one request's portion) x (heads of one kv group) and
-// walks that portion's keys in tiles of 64 (head size 64) or 128 (128).  Its warps have three roles that meet only at
+// walks that portion's keys in tiles of 64.  Its warps have three roles that meet only at
 // mbarriers:
 //
 //   warp 5   loader: K and V tiles by cp.async into a ring of stages, written directly in
@@ -16,17 +16,17 @@
 //            XORed with the row index modulo 8; head sizes above 64 as panels of 64
 //            dims); the copies' completion arrives on the stage's mbarrier;
 //   warp 4   one lane issues every tcgen05.mma of the CTA, in the order in which they must
-//            run: Q.K^T of the first tile (two tiles with two score buffers), then for every
-//            tile P.V of that tile followed by Q.K^T of the tile that takes its buffer (M=128, N = the tile or the head size, K=16 per instruction);
-//   warps 0-3  softmax: every thread owns one row (one TMEM lane), reads its scores from
+//            run: Q.K^T of tile 0, then for every tile P.V of that tile followed by Q.K^T
+//            of the next (M=128, N=64 or the head size, K=16 per instruction);
+//   warps 0-3  softmax: every thread owns one row (one TMEM lane), reads its 64 scores from
 //            TMEM (tcgen05.ld 32x32b), applies the mask and the online-softmax recurrence
 //            without any cross-thread traffic, and writes its probabilities as bfloat16
 //            back into tensor memory (tcgen05.st), over the scores they came from.
 //
 // The probabilities never pass through shared memory: the second product takes its A
-// operand from tensor memory.  Scores and probabilities share their columns, the output has
-// columns of its own, so a CTA holds 128 or 256 columns and four or two CTAs
-// fit an SM (see Form).  A CTA's tiles form a chain (scores -> softmax -> product -> next scores); the
+// operand from tensor memory.  Scores and probabilities share 64 columns, the output has
+// columns of its own, so a CTA holds 128 (head size 64) or 256 columns and four (two) CTAs
+// fit an SM.  A CTA's tiles form a chain (scores -> softmax -> product -> next scores); the
 // CTAs of an SM interleave their chains on the tensor core and on the special-function
 // units, which is what keeps both busy.  The softmax warps are one warp group, the others
 // a second one that hands most of its registers to the first (setmaxnreg).
@@ -60,44 +60,27 @@ constexpr int HD = KLLM_HD;
 static_assert(HD == 64 || HD == 128, "head size 64 or 128");
 constexpr int PANELS = HD / 64;            // 64-dim panels of a row
 constexpr int ROWS = 128;                  // query rows per CTA = TMEM lanes
-// Keys per tile.  An instruction with both operands in shared memory takes 103 cycles whatever its N up to 128 (measured;
-// with A in tensor memory N / 2 cycles, at least 59), so at head size 128, where the scores are eight of them, a tile has
-// 128 keys: 824 + 522 cycles of tensor core for 128 keys against 2 x (824 + 261), and half the handshakes
-// (8192 tokens, 32 heads over 8: 914 us with tiles of 64 and held scores, 840 with 128).
-constexpr int TILE = HD == 128 ? 128 : 64;
+constexpr int TILE = 64;                   // keys per tile
 constexpr int THREADS = 256;               // 4 softmax warps; the issuing warp, the loader warp, two idle ones
 constexpr int SOFTMAX_THREADS = 128;
+constexpr int CTAS_PER_SM = HD == 64 ? 4 : 2;
 constexpr int Q_BYTES = PANELS * ROWS * 128;          // [panel][128 rows][64 dims]
-constexpr int KV_BYTES = PANELS * TILE * 128;         // [panel][TILE keys][64 dims]
-constexpr int STAGES = HD == 128 ? 1 : 2;             // of keys and of values, each with barriers of its own
+constexpr int KV_BYTES = PANELS * TILE * 128;         // [panel][64 keys][64 dims]
+constexpr int STAGES = 2;
 constexpr int SMEM_BYTES = 1024 + Q_BYTES + STAGES * 2 * KV_BYTES;
 constexpr float kRescaleAt = 8.f;                     // move a row's reference when its maximum grew by 2^8
-constexpr unsigned COL_S = 0;
+constexpr int TMEM_COLS = HD == 64 ? 128 : 256;       // scores / probabilities (64) + output (HD): a power of two
+constexpr unsigned COL_S = 0, COL_O = 64;
+// registers after setmaxnreg: all of a CTA's threads together stay inside its share of the SM's 64 K
+constexpr int REGS_SOFTMAX = CTAS_PER_SM == 4 ? 88 : 184, REGS_OTHERS = CTAS_PER_SM == 4 ? 40 : 64;
+// setmaxnreg moves registers inside the CTA's own allocation (threads x registers at launch)
+static_assert(SOFTMAX_THREADS * (REGS_SOFTMAX + REGS_OTHERS) <= THREADS * ((65536 / (THREADS * CTAS_PER_SM)) / 8 * 8), "setmaxnreg budget");
 
-// SBUF score buffers.  One: the scores of a tile are made when its predecessor's product has been issued; at head size 64
-// four such CTAs fit an SM and hide one another's chains.  Two (head size 64): a tile's scores are ready when the softmax
-// of the tile before ends, two CTAs an SM with the registers to hold a row's scores; the form for launches that are not
-// four CTAs an SM deep (1000 tokens x 32 heads: 35.7 -> 25.7 us; 333 + 278 + 222 tokens 22.3 -> 16.8; 8192 tokens 480
-// with one buffer, 624 with two).
-template <int SBUF>
-struct Form {
-    static constexpr int CTAS_PER_SM = SBUF * TILE + HD <= 128 ? 4 : 2;
-    static constexpr int TMEM_COLS = SBUF * TILE + HD <= 128 ? 128 : 256;      // scores / probabilities + output (HD): a power of two
-    static_assert(SBUF * TILE + HD <= TMEM_COLS, "columns");
-    static constexpr unsigned COL_O = SBUF * TILE;
-    // registers after setmaxnreg: all of a CTA's threads together stay inside its share of the SM's 64 K
-    static constexpr int REGS_SOFTMAX = CTAS_PER_SM == 4 ? 88 : 184, REGS_OTHERS = CTAS_PER_SM == 4 ? 40 : 64;
-    // setmaxnreg moves registers inside the CTA's own allocation (threads x registers at launch)
-    static_assert(SOFTMAX_THREADS * (REGS_SOFTMAX + REGS_OTHERS) <= THREADS * ((65536 / (THREADS * CTAS_PER_SM)) / 8 * 8), "setmaxnreg budget");
-
-    // The products into the output that a barrier phase of their own announces (bar_o_full), and the phase that the
-    // last one's is.  A wait by parity is only sound for the phase behind the one waited for last: with two score buffers
-    // the softmax waits for every product, with one for the last alone (those before it are ordered by the scores that
-    // come behind them), so that the barrier completes only once.
-    __host__ __device__ static constexpr bool announces_product(int j, int ntiles) { return SBUF > 1 || j == ntiles - 1; }
-    __host__ __device__ static constexpr bool awaits_before_rescale(int j) { return SBUF > 1 && j > 0; }      // the product of tile j - 1
-    __host__ __device__ static constexpr int last_phase(int ntiles) { return SBUF > 1 ? ntiles - 1 : 0; }
-};
+// The product into the output that completes a phase of bar_o_full, and the phase that is waited for.  A wait by parity is
+// only sound for the phase behind the one waited for last: the softmax waits once, so the barrier completes once, for the
+// last tile (the products before it are ordered by the scores that come behind them).
+__host__ __device__ constexpr bool announces_product(int j, int ntiles) { return j == ntiles - 1; }
+constexpr int OUTPUT_PHASE = 0;
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const void* gmem, bool valid) {
     const int bytes = valid ? 16 : 0;
@@ -150,12 +133,6 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const uint32_t (&r)[32
                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st16(unsigned taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 // byte offset of 16-byte piece `ch` (0..7) of row `r` inside a swizzled panel of 128-byte rows
@@ -173,58 +150,56 @@ __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// keys (or values) key0 .. key0 + TILE - 1 of kv head g into a buffer [panel][TILE][64 dims], by the 32 lanes of the loader
-// warp, 64 rows at a time.  A lane keeps its 16-byte piece of the row and walks the rows.
-__device__ __forceinline__ void load_rows(unsigned dst0, const bf16* __restrict__ cache, const int* __restrict__ table, int key0,
-                                          int hi, int g, int n_kv, int page_size, int lane) {
+// keys key0 .. key0+63 of kv head g into a stage (K panels, then V panels), by the 32
+// lanes of the loader warp.  A lane keeps its 16-byte piece of the row and walks the rows.
+__device__ __forceinline__ void load_kv(unsigned stage, const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
+                                        const int* __restrict__ table, int key0, int hi, int g, int n_kv, int page_size,
+                                        int lane) {
     constexpr int PIECES = HD / 8;                        // 16-byte pieces of a row
     constexpr int ROWS_PER_PASS = 32 / PIECES;            // 4 (HD 64) or 2 (HD 128)
     const int piece = lane % PIECES, r0 = lane / PIECES;
     const unsigned col = (unsigned)((piece >> 3) * (TILE * 128));
     const int64_t head_off = (int64_t)g * page_size * HD + piece * 8;
     const int64_t page_elems = (int64_t)n_kv * page_size * HD;
-#pragma unroll 1
-    for (int sub = 0; sub < TILE; sub += 64) {
-        const int first = key0 + sub;
-        const int lp0 = first / page_size, in_page = first - lp0 * page_size;
-        if (first < hi && in_page + 64 <= page_size) {
-            // the 64 rows lie in one page: one look-up, the rows follow one another
-            const int64_t base = (int64_t)table[lp0] * page_elems + head_off + (int64_t)in_page * HD;
-#pragma unroll 8
-            for (int j = 0; j < 64 / ROWS_PER_PASS; j++) {
-                const int row = r0 + j * ROWS_PER_PASS;
-                const bool valid = first + row < hi;
-                cp_async16(dst0 + col + swz(sub + row, piece & 7), cache + (valid ? base + row * HD : 0), valid);
-            }
-            continue;
-        }
-#pragma unroll 2
-        for (int j = 0; j < 64 / ROWS_PER_PASS; j++) {
+    const int lp0 = key0 / page_size, in_page = key0 - lp0 * page_size;
+    if (in_page + TILE <= page_size) {
+        // the whole tile lies in one page: one look-up, the rows follow one another
+        const int64_t base = (int64_t)table[lp0] * page_elems + head_off + (int64_t)in_page * HD;
+#pragma unroll 4
+        for (int j = 0; j < TILE / ROWS_PER_PASS; j++) {
             const int row = r0 + j * ROWS_PER_PASS;
-            const int key = first + row;
-            const bool valid = key < hi;
-            int64_t off = 0;
-            if (valid) {
-                const int lp = key / page_size;
-                off = (int64_t)table[lp] * page_elems + head_off + (int64_t)(key - lp * page_size) * HD;
-            }
-            cp_async16(dst0 + col + swz(sub + row, piece & 7), cache + off, valid);
+            const bool valid = key0 + row < hi;
+            const int64_t off = valid ? base + row * HD : 0;
+            const unsigned dst = col + swz(row, piece & 7);
+            cp_async16(stage + dst, kcache + off, valid);
+            cp_async16(stage + KV_BYTES + dst, vcache + off, valid);
         }
+        return;
+    }
+#pragma unroll 2
+    for (int j = 0; j < TILE / ROWS_PER_PASS; j++) {
+        const int row = r0 + j * ROWS_PER_PASS;
+        const int key = key0 + row;
+        const bool valid = key < hi;
+        int64_t off = 0;
+        if (valid) {
+            const int lp = key / page_size;
+            off = (int64_t)table[lp] * page_elems + head_off + (int64_t)(key - lp * page_size) * HD;
+        }
+        const unsigned dst = col + swz(row, piece & 7);
+        cp_async16(stage + dst, kcache + off, valid);
+        cp_async16(stage + KV_BYTES + dst, vcache + off, valid);
     }
 }
 
-template <int SBUF>
-__global__ void __launch_bounds__(THREADS, Form<SBUF>::CTAS_PER_SM)
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
 attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, int64_t q_stride,
                         const bf16* __restrict__ kcache, const bf16* __restrict__ vcache,
                         const int* __restrict__ q_start, const int* __restrict__ start_pos,
                         const int* __restrict__ block_table, int max_blocks, int n_requests, int n_heads,
                         int n_kv, int page_size, int window, float scale_log2e, int tokens_per_tile, int* status) {
-    constexpr int CTAS_PER_SM = Form<SBUF>::CTAS_PER_SM, TMEM_COLS = Form<SBUF>::TMEM_COLS;
-    constexpr unsigned COL_O = Form<SBUF>::COL_O;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bar_k_full[STAGES], bar_k_empty[STAGES], bar_v_full[STAGES], bar_v_empty[STAGES],
-        bar_q_full, bar_s_full[SBUF], bar_p_full[SBUF], bar_o_full;
+    __shared__ __align__(8) uint64_t bar_kv_full[STAGES], bar_kv_empty[STAGES], bar_q_full, bar_s_full, bar_p_full, bar_o_full;
     __shared__ unsigned s_tmem;
     __shared__ int s_req, s_tok0, s_abort;
     const int g = blockIdx.x % n_kv;          // CTAs start in the order of blockIdx.x: all kv heads' longest tiles first
@@ -239,12 +214,10 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
             tile -= nt;
         }
         s_req = req; s_tok0 = tok0; s_abort = 0;
-        for (int s = 0; s < STAGES; s++) {
-            mbar_init(&bar_k_full[s], 32); mbar_init(&bar_k_empty[s], 1);
-            mbar_init(&bar_v_full[s], 32); mbar_init(&bar_v_empty[s], 1);
-        }
+        for (int s = 0; s < STAGES; s++) { mbar_init(&bar_kv_full[s], 32); mbar_init(&bar_kv_empty[s], 1); }
         mbar_init(&bar_q_full, 32);
-        for (int b = 0; b < SBUF; b++) { mbar_init(&bar_s_full[b], 1); mbar_init(&bar_p_full[b], SOFTMAX_THREADS); }
+        mbar_init(&bar_s_full, 1);
+        mbar_init(&bar_p_full, SOFTMAX_THREADS);
         mbar_init(&bar_o_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
@@ -274,7 +247,7 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
     const unsigned sQ = base, sKV = base + Q_BYTES;
 
     if (warp >= 4) {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Form<SBUF>::REGS_OTHERS));
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(REGS_OTHERS));
       if (warp == 5) {
         // ---- loader ----------------------------------------------------------------
         for (int c = lane; c < ROWS * (HD / 8); c += 32) {     // Q tile: each row's HD dims, zero for unused rows
@@ -287,70 +260,62 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
         cp_async_arrive(&bar_q_full);
         for (int j = 0; j < ntiles; j++) {
             const int s = j % STAGES;
-            const unsigned free = (((unsigned)(j / STAGES)) & 1u) ^ 1u;
-            if (!mbar_wait(&bar_k_empty[s], free, abort_flag, status, 1)) break;      // the scores of tile j - STAGES are done
-            load_rows(sKV + (unsigned)s * 2u * KV_BYTES, kcache, table, lo + j * TILE, hi, g, n_kv, page_size, lane);
-            cp_async_arrive(&bar_k_full[s]);
-            if (!mbar_wait(&bar_v_empty[s], free, abort_flag, status, 7)) break;
-            load_rows(sKV + (unsigned)s * 2u * KV_BYTES + KV_BYTES, vcache, table, lo + j * TILE, hi, g, n_kv, page_size, lane);
-            cp_async_arrive(&bar_v_full[s]);
+            if (!mbar_wait(&bar_kv_empty[s], (((unsigned)(j / STAGES)) & 1u) ^ 1u, abort_flag, status, 1)) break;
+            load_kv(sKV + (unsigned)s * 2u * KV_BYTES, kcache, vcache, table, lo + j * TILE, hi, g, n_kv, page_size, lane);
+            cp_async_arrive(&bar_kv_full[s]);
         }
         cp_async_wait<0>();                    // nothing of this warp is in flight when the CTA ends
       } else if (warp == 4) {
-        // ---- the issuer: S(0) .. S(SBUF - 1), then per tile P.V(j) and S(j + SBUF), in this order ------------
+        // ---- the issuer: S(0), then per tile P.V(j) and S(j + 1), in this order ------------
         constexpr uint32_t IDESC_S = make_idesc(ROWS, TILE, false);
         constexpr uint32_t IDESC_O = make_idesc(ROWS, HD, true);
         const uint32_t q_lo = desc_lo(sQ, 16), k_lo0 = desc_lo(sKV, 16), v_lo0 = desc_lo(sKV + KV_BYTES, TILE * 128);
         const unsigned t_s = tmem + COL_S, t_o = tmem + COL_O;
-        auto issue_scores = [&](int s, int b) {
+        auto issue_scores = [&](int s) {
             const uint32_t k_lo = k_lo0 + (uint32_t)s * (2u * KV_BYTES >> 4);
 #pragma unroll
             for (int kk = 0; kk < HD / 16; kk++)
-                umma_words(t_s + (unsigned)(b * TILE), q_lo + (uint32_t)(((kk >> 2) * (ROWS * 128) + (kk & 3) * 32) >> 4),
+                umma_words(t_s, q_lo + (uint32_t)(((kk >> 2) * (ROWS * 128) + (kk & 3) * 32) >> 4),
                            k_lo + (uint32_t)(((kk >> 2) * (TILE * 128) + (kk & 3) * 32) >> 4), IDESC_S, kk > 0);
-            umma_commit(&bar_s_full[b]);
-            umma_commit(&bar_k_empty[s]);
+            umma_commit(&bar_s_full);
         };
-        bool ok = mbar_wait(&bar_q_full, 0, abort_flag, status, 2);
-        for (int j = 0; ok && j < SBUF && j < ntiles; j++) {
-            ok = mbar_wait(&bar_k_full[j % STAGES], (unsigned)(j / STAGES) & 1u, abort_flag, status, 3);
-            if (!ok) break;
+        bool ok = mbar_wait(&bar_q_full, 0, abort_flag, status, 2) &&
+                  mbar_wait(&bar_kv_full[0], 0, abort_flag, status, 3);
+        if (ok) {
             fence_async_smem();                // the copies landed through the generic proxy
             tc_fence_after();
-            if (lane == 0) issue_scores(j % STAGES, j);
+            if (lane == 0) issue_scores(0);
             __syncwarp();
         }
         for (int j = 0; ok && j < ntiles; j++) {
-            const int s = j % STAGES, b = j % SBUF;
+            const int s = j % STAGES;
             // the probabilities of tile j are in tensor memory and the output is rescaled
-            ok = mbar_wait(&bar_v_full[s], ((unsigned)(j / STAGES)) & 1u, abort_flag, status, 8) &&
-                 mbar_wait(&bar_p_full[b], (unsigned)(j / SBUF) & 1u, abort_flag, status, 4);
+            ok = mbar_wait(&bar_p_full, (unsigned)j & 1u, abort_flag, status, 4);
             if (!ok) break;
-            fence_async_smem();
             tc_fence_after();
             if (lane == 0) {                   // output += P . V
                 const uint32_t v_lo = v_lo0 + (uint32_t)s * (2u * KV_BYTES >> 4);
 #pragma unroll
                 for (int kk = 0; kk < TILE / 16; kk++)
-                    umma_tmem_a_words(t_o, t_s + (unsigned)(b * TILE + kk * 8), v_lo + (uint32_t)(kk * (2048 >> 4)), IDESC_O, j > 0 || kk > 0);
-                umma_commit(&bar_v_empty[s]);
-                if (Form<SBUF>::announces_product(j, ntiles)) umma_commit(&bar_o_full);
+                    umma_tmem_a_words(t_o, t_s + (unsigned)(kk * 8), v_lo + (uint32_t)(kk * (2048 >> 4)), IDESC_O, j > 0 || kk > 0);
+                umma_commit(&bar_kv_empty[s]);             // this stage's K was read by the scores before
+                if (announces_product(j, ntiles)) umma_commit(&bar_o_full);
             }
             __syncwarp();
-            if (j + SBUF < ntiles) {
-                const int s2 = (j + SBUF) % STAGES;
-                ok = mbar_wait(&bar_k_full[s2], ((unsigned)((j + SBUF) / STAGES)) & 1u, abort_flag, status, 5);
+            if (j + 1 < ntiles) {
+                const int s2 = (j + 1) % STAGES;
+                ok = mbar_wait(&bar_kv_full[s2], ((unsigned)((j + 1) / STAGES)) & 1u, abort_flag, status, 5);
                 if (!ok) break;
                 fence_async_smem();
                 tc_fence_after();
                 // in issue order behind P.V(j), which reads the columns that these scores overwrite
-                if (lane == 0) issue_scores(s2, b);
+                if (lane == 0) issue_scores(s2);
                 __syncwarp();
             }
         }
       }                                        // warps 6 and 7 only fill the warp group
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(Form<SBUF>::REGS_SOFTMAX));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(REGS_SOFTMAX));
         // ---- softmax: this thread's row is (token, head of the group) ---------------
         const int row = threadIdx.x;
         const int tt = row / gs, hh = row - tt * gs;
@@ -358,54 +323,35 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
         const int p_row = valid_row ? pos0 + tt : -1;                       // -1: sees no key
         const int w_row = (window > 0) ? p_row + 1 - window : 0;
         const unsigned lane_base = (unsigned)(warp * 32) << 16;
-        const unsigned t_o = tmem + lane_base + COL_O;
+        const unsigned t_s = tmem + lane_base + COL_S, t_o = tmem + lane_base + COL_O;
         float m_ref = -INFINITY, l_run = 0.f;          // the row's reference maximum; its sum relative to it
         bool ok = true;
         for (int j = 0; j < ntiles; j++) {
-            // scores of tile j are complete; so is every product issued before them (P.V of tile j - SBUF)
-            const int b = j % SBUF;
-            const unsigned t_s = tmem + lane_base + COL_S + (unsigned)(b * TILE);
-            ok = mbar_wait(&bar_s_full[b], (unsigned)(j / SBUF) & 1u, abort_flag, status, 6);
+            // scores of tile j are complete; so is every product issued before them (P.V of tile j - 1)
+            ok = mbar_wait(&bar_s_full, (unsigned)j & 1u, abort_flag, status, 6);
             if (!ok) break;
             tc_fence_after();
             const int key0 = lo + j * TILE;
             // the mask matters only where the tile crosses this row's diagonal or window edge
             const bool masked = key0 + TILE - 1 > p_row || key0 < w_row;
-            constexpr int PIECES = TILE / 32;
-            // With registers for it (two CTAs an SM) the row's scores are read once and stay: no second round through
-            // tensor memory, and the exponentials of one piece overlap the sums of another.
-            constexpr bool HELD = CTAS_PER_SM == 2;
-            float s[HELD ? PIECES : 1][32];
-            auto mask = [&](int c, float (&v)[32]) {
-                if (masked) {
-#pragma unroll
-                    for (int jj = 0; jj < 32; jj++) {
-                        const int key = key0 + c * 32 + jj;
-                        if (key > p_row || key < w_row) v[jj] = -INFINITY;
-                    }
-                }
-            };
-            if (HELD) {
-#pragma unroll
-                for (int c = 0; c < PIECES; c++) tmem_ld32(t_s + c * 32, s[HELD ? c : 0]);
-                tmem_ld_wait();
-#pragma unroll
-                for (int c = 0; c < PIECES; c++) mask(c, s[HELD ? c : 0]);
-            }
-            // the row's maximum
+            // first pass over the scores: the row's maximum
             float mx;
             {
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-                for (int c = 0; c < PIECES; c++) {
-                    float (&v)[32] = s[HELD ? c : 0];
-                    if (!HELD) {
-                        tmem_ld32(t_s + c * 32, v);
-                        tmem_ld_wait();
-                        mask(c, v);
+                for (int half = 0; half < 2; half++) {
+                    float s[32];
+                    tmem_ld32(t_s + half * 32, s);
+                    tmem_ld_wait();
+                    if (masked) {
+#pragma unroll
+                        for (int jj = 0; jj < 32; jj++) {
+                            const int key = key0 + half * 32 + jj;
+                            if (key > p_row || key < w_row) s[jj] = -INFINITY;
+                        }
                     }
 #pragma unroll
-                    for (int jj = 0; jj < 32; jj++) mx4[jj & 3] = fmaxf(mx4[jj & 3], v[jj]);
+                    for (int jj = 0; jj < 32; jj++) mx4[jj & 3] = fmaxf(mx4[jj & 3], s[jj]);
                 }
                 mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             }
@@ -417,39 +363,34 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
                 m_ref = mx;
             }
             const float neg = (m_ref == -INFINITY) ? 0.f : -m_ref * scale_log2e;   // p = 2^(s * scale - m * scale): one FMA each
-            // the probabilities, two per column as the tensor core reads its A operand.  Piece c becomes the
-            // columns 16 c .. 16 c + 15, which pieces up to c have held: they have been read.
+            // second pass: the probabilities, two per column as the tensor core reads its A operand
+            uint32_t pk[32];
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int c = 0; c < PIECES; c++) {
-                float (&v)[32] = s[HELD ? c : 0];
-                if (!HELD) {
-                    tmem_ld32(t_s + c * 32, v);
-                    tmem_ld_wait();
-                    mask(c, v);
+            for (int half = 0; half < 2; half++) {
+                float s[32];
+                tmem_ld32(t_s + half * 32, s);
+                tmem_ld_wait();
+                if (masked) {
+#pragma unroll
+                    for (int jj = 0; jj < 32; jj++) {
+                        const int key = key0 + half * 32 + jj;
+                        if (key > p_row || key < w_row) s[jj] = -INFINITY;
+                    }
                 }
 #pragma unroll
                 for (int jj = 0; jj < 32; jj++) {
-                    v[jj] = fast_exp2(fmaf(v[jj], scale_log2e, neg));
-                    sum4[jj & 3] += v[jj];
+                    s[jj] = fast_exp2(fmaf(s[jj], scale_log2e, neg));
+                    sum4[jj & 3] += s[jj];
                 }
-                uint32_t pk[16];
 #pragma unroll
-                for (int i = 0; i < 16; i++) pk[i] = pack_bf16(v[2 * i], v[2 * i + 1]);
-                tmem_st16(t_s + c * 16, pk);
+                for (int c = 0; c < 16; c++) pk[half * 16 + c] = pack_bf16(s[2 * c], s[2 * c + 1]);
             }
             l_run = l_run * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            if (Form<SBUF>::awaits_before_rescale(j)) {
-                // The product of tile j - 1 must be over before the accumulator is rescaled (with one buffer it is: the
-                // scores of tile j came behind it).  Every tile waits, also where nothing is rescaled (see Form).
-                ok = mbar_wait(&bar_o_full, (unsigned)(j - 1) & 1u, abort_flag, status, 10);
-                if (!ok) break;
-                tc_fence_after();
-            }
             if (j > 0 && __any_sync(0xffffffffu, move)) {
                 // rows of this warp rescale what the products so far have added up (rows that
-                // did not move multiply by one); the product of tile j - 1 is over, the one of tile j
-                // waits for this thread's probabilities
+                // did not move multiply by one); the product of tile j - 1 is over (see above),
+                // the one of tile j waits for this thread's probabilities
 #pragma unroll
                 for (int cb = 0; cb < HD / 32; cb++) {
                     float t[32];
@@ -461,11 +402,13 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
                     tmem_st32(t_o + cb * 32, u);
                 }
             }
+            // the first 32 columns of the scores become the 64 probabilities
+            tmem_st32(t_s, pk);
             tmem_st_wait();
             tc_fence_before();
-            mbar_arrive(&bar_p_full[b]);       // P of tile j is in tensor memory, the accumulator is rescaled
+            mbar_arrive(&bar_p_full);          // P of tile j is in tensor memory, the accumulator is rescaled
         }
-        if (ok) ok = mbar_wait(&bar_o_full, (unsigned)Form<SBUF>::last_phase(ntiles) & 1u, abort_flag, status, 9);
+        if (ok) ok = mbar_wait(&bar_o_full, OUTPUT_PHASE, abort_flag, status, 9);
         if (ok) {
             tc_fence_after();
             const float inv = 1.f / l_run;
@@ -495,34 +438,24 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-bool g_attr_set[2] = {false, false};
+bool g_attr_set = false;
 
 }  // namespace
 
 extern "C" int kllm_attention_tcgen05_ptmem_head_dim() { return HD; }
 
-// For a chain of ntiles tiles with 1 or 2 score buffers: announced[j] is whether tile j's product completes a phase of the
-// output's barrier; awaited[0 .. n - 1] are the phases that the softmax waits for, in its order.  Returns n (0: no such form).
-extern "C" int kllm_attention_tcgen05_ptmem_output_phases(int score_buffers, int ntiles, int* announced, int* awaited) {
-    auto list = [&](auto form) {
-        int n = 0;
-        for (int j = 0; j < ntiles; j++) {
-            announced[j] = form.announces_product(j, ntiles);
-            if (form.awaits_before_rescale(j)) awaited[n++] = j - 1;
-        }
-        awaited[n++] = form.last_phase(ntiles);
-        return n;
-    };
-#if KLLM_HD == 64
-    if (score_buffers == 2) return list(Form<2>());
-#endif
-    return score_buffers == 1 ? list(Form<1>()) : 0;
+// For a chain of ntiles tiles: announced[j] is whether tile j's product completes a phase of the output's barrier;
+// awaited[0 .. n - 1] are the phases that the softmax waits for, in its order.  Returns n.
+extern "C" int kllm_attention_tcgen05_ptmem_output_phases(int ntiles, int* announced, int* awaited) {
+    for (int j = 0; j < ntiles; j++) announced[j] = announces_product(j, ntiles);
+    awaited[0] = OUTPUT_PHASE;
+    return 1;
 }
 
 // Same contract as the mma.sync prefill kernel: requests' portions
 // q_start[s]..q_start[s+1] start at cache position start_pos[s]; out [n, n_heads*HD].
-// status: device int that a bounded wait which ran out sets (1 and 7: loader, 2-5 and 8: tensor-core
-// issuer, 6, 9 and 10: softmax).
+// status: device int that a bounded wait which ran out sets (1: loader, 2-5: tensor-core
+// issuer, 6 and 9: softmax).
 extern "C" int kllm_attention_prefill_tcgen05_ptmem(void* out, const void* q, int64_t q_stride, const void* kcache,
                                               const void* vcache, const int* q_start, const int* start_pos,
                                               const int* block_table, int max_blocks, int n_tokens,
@@ -536,27 +469,20 @@ extern "C" int kllm_attention_prefill_tcgen05_ptmem(void* out, const void* q, in
     if (page_size <= 0) KLLM_FAIL("attention: page size %d", page_size);
     if (((uintptr_t)q & 15) || (q_stride & 7) || ((uintptr_t)out & 15) || ((uintptr_t)kcache & 15) || ((uintptr_t)vcache & 15))
         KLLM_FAIL("attention (tcgen05, P in TMEM): q, out and the caches must be 16-byte aligned, q's row stride a multiple of 8");
+    if (!g_attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_ptmem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e != cudaSuccess) {
+            snprintf(g_kllm_err, sizeof(g_kllm_err), "attention (tcgen05, P in TMEM): %d bytes of shared memory refused: %s",
+                     SMEM_BYTES, cudaGetErrorString(e));
+            return (int)e;
+        }
+        g_attr_set = true;
+    }
     const int tpt = ROWS / gs;
     const int max_tiles = n_tokens / tpt + n_requests;
     const float sl2e = scale * 1.4426950408889634f;
-    const int ctas = max_tiles * n_kv;
-    auto launch = [&](auto kernel, bool& attr_set) -> int {
-        if (!attr_set) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-            if (e != cudaSuccess) {
-                snprintf(g_kllm_err, sizeof(g_kllm_err), "attention (tcgen05, P in TMEM): %d bytes of shared memory refused: %s",
-                         SMEM_BYTES, cudaGetErrorString(e));
-                return (int)e;
-            }
-            attr_set = true;
-        }
-        kllm_launch(kernel, dim3(ctas), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
-                    (bf16*)out, (const bf16*)q, q_stride, (const bf16*)kcache, (const bf16*)vcache, q_start, start_pos,
-                    block_table, max_blocks, n_requests, n_heads, n_kv, page_size, window, sl2e, tpt, status);
-        KLLM_LAUNCH_STATUS();
-    };
-#if KLLM_HD == 64
-    if (ctas <= 4 * sm_count()) return launch(attn_prefill_tc5_ptmem_kernel<2>, g_attr_set[1]);     // up to two waves (see Form)
-#endif
-    return launch(attn_prefill_tc5_ptmem_kernel<1>, g_attr_set[0]);
+    kllm_launch((attn_prefill_tc5_ptmem_kernel), dim3(max_tiles * n_kv), dim3(THREADS), SMEM_BYTES, (cudaStream_t)stream,
+                (bf16*)out, (const bf16*)q, q_stride, (const bf16*)kcache, (const bf16*)vcache, q_start, start_pos,
+                block_table, max_blocks, n_requests, n_heads, n_kv, page_size, window, sl2e, tpt, status);
+    KLLM_LAUNCH_STATUS();
 }

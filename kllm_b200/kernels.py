@@ -783,8 +783,8 @@ def attention(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcache: 
     if tc and USE_TCGEN05 and head_dim in TCGEN05_HEAD_DIMS and group <= 128 and not special:
         return attention_prefill_tcgen05(out, q, kcache, vcache, q_start, start_pos, table,
                                          n_req, n_heads, n_kv, head_dim, window, scale,
-                                         probabilities=tcgen05_form(head_dim, group, n_kv, ctx.n_tokens - singles,
-                                                                    n_req, ctx.max_ctx))
+                                         probabilities=tcgen05_choice(head_dim, group, n_kv, ctx.n_tokens - singles,
+                                                                      n_req, ctx.max_ctx))
     if tc and group <= 64:
         return attention_prefill(out, q, kcache, vcache, q_start, start_pos, table,
                                  n_req, n_heads, n_kv, head_dim, window, scale, slopes=score_slopes,
@@ -910,20 +910,36 @@ def attention_prefill(out, q, kcache, vcache, q_start, start_pos, block_table, n
 
 
 def tcgen05_form(head_dim: int, group: int, n_kv: int, n_tokens: int, n_requests: int, max_ctx: int) -> str:
-    """Which of the two tcgen05 attention kernels a step of portions takes ("smem" / "tmem",
-    see ``attention_prefill_tcgen05``), from measurements.
+    """Which of the two tcgen05 attention kernels ("smem" / "tmem", see ``attention_prefill_tcgen05``) suits a step of
+    portions whose CTAs do not all run at once, from measurements (us, each call alone with a cold L2).
 
-    Head size 128 keeps its probabilities in tensor memory (two CTAs an SM) unless the step is about one CTA an
-    SM, where the other form's double-buffered scores win (8 kv heads, 700 tokens: smem 25.2 us, tmem 29.8; 32 kv heads,
-    300 tokens: 15.8, 19.7; 700 + 350 tokens: 70.7, 56.4; 8192: 1299, 843).  At head size 64 the tmem form has two
-    score buffers in small launches and four CTAs an SM in large ones (1000 tokens: smem 23.8, tmem 25.7; 8 x 150
-    tokens: 17.3, 16.8; 8192: 494, 480) and loses to the other when one long prompt's longest chain is the whole
-    kernel: all CTAs resident at once and more than 16 key tiles (2048 tokens: 45.6, 51.6)."""
+    Head size 128: "tmem" fits two CTAs an SM, "smem" one, but with double-buffered scores.  Launches of at most one CTA an
+    SM take "smem" (32 heads over 8, 300 tokens: smem 22.5, tmem 24.6; 300 behind 8000: 222, 280; 64 behind 8000: 199, 193),
+    as do those a little above it while the chains are short, so that the last CTAs are the shortest (700 tokens: 30.7,
+    34.8; but 600 behind 2000: 111, 86); the others "tmem" (1150 tokens: 51, 49; 8192: 1313, 790).
+
+    Head size 64: four CTAs an SM with "tmem", two with "smem".  Many short chains want "tmem" (8 x 150 tokens: smem 24.6,
+    tmem 21.5; 24 x 100: 37.7, 29.6; 8 x 300: 35.7, 29.7), as does a launch of several waves (8 x 500: 56.3, 54.1; 8192:
+    502, 467); "smem" is faster where one long prompt's longest chain is the whole kernel (2048: 53, 58)."""
+    sms = sm_count()
     ctas = (n_tokens // max(1, 128 // group) + n_requests) * n_kv
     if head_dim != 64:
-        return "smem" if ctas <= sm_count() * 6 // 5 else "tmem"
+        return "smem" if ctas <= sms or (ctas <= sms * 6 // 5 and max_ctx <= 1024) else "tmem"
     tiles = -(-max_ctx // 64)
-    return "tmem" if tiles <= 16 or ctas >= 6 * sm_count() else "smem"
+    return "tmem" if tiles <= 16 or ctas >= 6 * sms else "smem"
+
+
+def tcgen05_choice(head_dim: int, group: int, n_kv: int, n_tokens: int, n_requests: int, max_ctx: int) -> str:
+    """The form that a step takes.  ``tcgen05_form``, except at head size 64 where the launch is one wave of the two
+    CTAs an SM of "smem", which is then faster however short the chains (32 heads over 4, 300 tokens: smem 16.4, tmem
+    20.5; 700: 22.7, 30.7; 333 + 278 + 222: 19.4, 23.4), and where chains of more than 8 tiles are not several waves
+    (2 x 1000 tokens: 37.9, 49.2; 16 x 17 behind 900, 32 kv heads: 69.6, 80.8; 4 x 400 behind 500: 46.0, 43.0, and
+    49.2, 53.2 over 8 kv heads)."""
+    sms = sm_count()
+    ctas = (n_tokens // max(1, 128 // group) + n_requests) * n_kv
+    if head_dim == 64 and (ctas <= 2 * sms or (max_ctx > 512 and ctas < 6 * sms)):
+        return "smem"
+    return tcgen05_form(head_dim, group, n_kv, n_tokens, n_requests, max_ctx)
 
 
 def attention_prefill_tcgen05(out, q, kcache, vcache, q_start, start_pos, block_table, n_requests, n_heads, n_kv,
@@ -934,9 +950,9 @@ def attention_prefill_tcgen05(out, q, kcache, vcache, q_start, start_pos, block_
     (csrc/attention_tcgen05.cu: two score buffers in tensor memory, P through shared
     memory, two CTAs of head size 64 per SM) or ``"tmem"`` (csrc/attention_tcgen05_ptmem.cu:
     P written over the scores in tensor memory and read from there, half the tensor memory
-    and shared memory per CTA, up to four / two CTAs per SM).  Default (no step shape known): tmem
+    and shared memory per CTA, four / two CTAs per SM).  Default (no step shape known): tmem
     for head size 128, smem for head size 64; ``attention`` picks
-    by the step's shape (``tcgen05_form``)."""
+    by the step's shape (``tcgen05_choice``)."""
     _cuda(out, q, kcache, vcache, q_start, start_pos, block_table)
     _check_attention(out, q, kcache, vcache, block_table, n_kv, head_dim)
     _i32(q_start, "q_start"); _i32(start_pos, "start_pos")
@@ -1324,7 +1340,7 @@ def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_tab
         if splits > 1:
             part_o = new(singles, n_heads, splits, head_dim, dtype=torch.float32)
             part_ml = new(singles, n_heads, splits, 2, dtype=torch.float32)
-    form = tcgen05_form(head_dim, n_heads // n_kv, n_kv, n - singles, ctx.n_requests - singles, ctx.max_ctx)
+    form = tcgen05_choice(head_dim, n_heads // n_kv, n_kv, n - singles, ctx.n_requests - singles, ctx.max_ctx)
     xn, qkv, attn, act = new(n, d), new(n, wide), new(n, q_dim), new(n, inter)
     gate_up = None
     if not (gemm_pays(n, inter, "swiglu") and all(gemm_fits(xn, layer[2][:inter], act, "swiglu", layer[2][inter:]) for layer in layers)):

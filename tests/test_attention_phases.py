@@ -7,14 +7,26 @@ import ctypes
 import pytest
 
 
-@pytest.mark.parametrize("hd,buffers", [(64, 1), (64, 2), (128, 1)])
+@pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("ntiles", [1, 2, 3, 4, 33])
-def test_every_phase_is_awaited_in_turn(hd, buffers, ntiles):
+def test_every_phase_is_awaited_in_turn(hd, ntiles):
     from kllm_b200.csrc.build import load_library
     lib = load_library("attention_tcgen05_ptmem", {"KLLM_HD": hd})
     announced, awaited = (ctypes.c_int * ntiles)(), (ctypes.c_int * (ntiles + 1))()
-    n = lib.kllm_attention_tcgen05_ptmem_output_phases(buffers, ntiles, ctypes.addressof(announced), ctypes.addressof(awaited))
+    n = lib.kllm_attention_tcgen05_ptmem_output_phases( ntiles, ctypes.addressof(announced), ctypes.addressof(awaited))
     phases = [j for j in range(ntiles) if announced[j]]         # phase p is the product of tile phases[p]
     assert list(awaited[:n]) == list(range(len(phases)))
     assert phases[awaited[n - 1]] == ntiles - 1                 # the last wait is for the last product
 
+
+
+def test_which_form_a_step_takes(monkeypatch):
+    """Long chains and a second wave do not go to the form of one CTA an SM at head size 128, and one wave goes to the form
+    with two score buffers at 64, also where the chains are short."""
+    from kllm_b200 import kernels
+    monkeypatch.setattr(kernels, "sm_count", lambda: 148)
+    form = kernels.tcgen05_choice
+    assert form(128, 4, 8, 600, 1, 2600) == "tmem" and form(128, 4, 8, 600, 1, 600) == "smem"
+    assert form(128, 4, 8, 300, 1, 8300) == "smem" and form(128, 4, 8, 850, 1, 850) == "tmem"
+    assert form(64, 8, 4, 700, 1, 700) == "smem" and form(64, 8, 4, 2048, 1, 2048) == "smem"
+    assert form(64, 8, 4, 2400, 24, 100) == "tmem" and form(64, 8, 4, 8192, 1, 8192) == "tmem"

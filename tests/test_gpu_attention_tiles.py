@@ -1,5 +1,5 @@
-"""The tcgen05 attention that keeps its probabilities in tensor memory at the edges of its tiles (64 keys at head size 64,
-128 at 128), with one and two score buffers, windows, pages that split a tile, and many tiles of one chain."""
+"""The tcgen05 attention that keeps its probabilities in tensor memory at the edges of its tiles (64 keys; cases at the
+edges of 128 too), with windows, pages that split a tile, and many tiles of one chain."""
 import pytest
 
 from test_gpu_kernels import attention_case, close
@@ -22,9 +22,8 @@ def test_tile_edges(hd, H, G, window, start, new):
 
 @pytest.mark.parametrize("hd,H,G,tokens", [(64, 32, 4, 700), (64, 32, 32, 2600), (128, 32, 8, 900)])
 def test_long_chains_agree_with_the_other_form(hd, H, G, tokens):
-    """Launches of one and of several waves (head size 64: the form with two score buffers, and the one with four CTAs an
-    SM) against the form that passes the probabilities through shared memory.  At head size 64 both sum in the same order;
-    at 128 the tile differs: two bfloat16 roundings of an output apart and a little more."""
+    """Launches of one and of several waves against the form that passes the probabilities through shared memory.  At head
+    size 64 both sum in the same order; at 128 the bound leaves two bfloat16 roundings of an output and a little more."""
     import torch
     from kllm_b200 import kernels
     g = torch.Generator(device="cuda").manual_seed(tokens)
