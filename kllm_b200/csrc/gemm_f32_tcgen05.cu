@@ -32,8 +32,9 @@
 // of whole blocks, each a unit of work of its own that leaves its sums in a workspace;
 // a third kernel adds them in split order.
 //
-// A row of x or W that holds an infinity or a NaN gives NaN (the parts of an infinity are
-// an infinity and NaN); finite numbers of any size are split exactly.
+// The parts of an infinity are infinities and NaN, and a product of parts may overflow where the numbers' own does not cancel:
+// a sum that is not finite is taken again, as plain float32 multiply-adds of the operands (plain_dot), so that
+// infinities come out where arithmetic gives them.  Finite numbers of any size are split exactly.
 #include "common.cuh"
 
 KLLM_EXPORT_LAST_ERROR(gemm_f32_tcgen05)
@@ -103,7 +104,21 @@ __global__ void split_kernel(const float* __restrict__ src, const float* __restr
     }
 }
 
+// x . w as float32 multiply-adds in the order of k, for the few elements whose six products did not add up to a number
+// (an operand that is not finite, an overflow).  Ends at a NaN, which stays one.
+__device__ __noinline__ float plain_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {
+    float s = 0.f;
+    for (int k = 0; k < K && s == s; k += 4) {                                          // K is a multiple of 4
+        const float4 u = *reinterpret_cast<const float4*>(x + k), v = *reinterpret_cast<const float4*>(w + k);
+        s = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, s))));
+    }
+    return s;
+}
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
 struct Args {
+    const float *x, *w, *w_up;              // the operands themselves (w: of the piece)
+    int64_t ldx, ldw;
     float* y;
     int64_t ldy, split_stride;              // split_stride: elements between the workspace's splits
     int M, N, K, splits, blocks_per_split;
@@ -258,6 +273,19 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (r < a.M) {
                 float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (int64_t)r * a.ldy;
                 constexpr int CH = EPI == EPI_SWIGLU ? 2 : 4;
+                unsigned odd[CH];                                   // columns whose sum is not finite: taken again below
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    odd[c] = 0;
+                    if constexpr (EPI != EPI_PARTIAL) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) {
+                            const bool ok_sum = finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]));
+                            odd[c] |= (unsigned)!ok_sum << j;
+                            if (EPI == EPI_ADD && !ok_sum) sum[c][j] = 0.f;
+                        }
+                    }
+                }
 #pragma unroll
                 for (int c = 0; c < CH; c++) {
                     const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
@@ -282,6 +310,20 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         }
                     }
                 }
+                if constexpr (EPI != EPI_PARTIAL) {
+#pragma unroll
+                    for (int c = 0; c < CH; c++) {
+                        const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
+                        for (unsigned left = odd[c]; left != 0; left &= left - 1) {
+                            const int j = col + __ffs(left) - 1;
+                            if (j >= a.N) break;                    // the tile's columns beyond the matrix
+                            const float* xr = a.x + r * a.ldx;
+                            const float v = plain_dot(xr, a.w + j * a.ldw, a.K);
+                            if (EPI == EPI_SWIGLU) y[j] = silu_mul(v, plain_dot(xr, a.w_up + j * a.ldw, a.K));
+                            else y[j] = EPI == EPI_ADD ? y[j] + v : v;
+                        }
+                    }
+                }
             }
         }
     }
@@ -295,7 +337,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // gate columns) silu(gate) * up.  Bound by the workspace's bytes, which lie in L2.
 template <int EPI>
 __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const float* __restrict__ ws, int64_t split_stride,
-                                     int M, int N, int splits) {
+                                     int M, int N, int splits, const Args a) {
     griddep_launch();
     griddep_wait();
     const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? 2 * N : N;
@@ -310,13 +352,21 @@ __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const f
             }
             return v;
         };
+        auto again = [&](float4& v, const float* w) {                    // the sums that are not finite, from the operands
+            float* e = &v.x;
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (!finite(e[j])) e[j] = plain_dot(a.x + r * a.ldx, w + (c + j) * a.ldw, a.K);
+        };
         float4 v = sum(ws + r * ldw + c);
+        again(v, a.w);
         float4* o = reinterpret_cast<float4*>(y + r * ldy + c);
         if (EPI == EPI_ADD) {
             const float4 h = *o;
             v.x += h.x; v.y += h.y; v.z += h.z; v.w += h.w;
         } else if (EPI == EPI_SWIGLU) {
-            const float4 u = sum(ws + r * ldw + N + c);
+            float4 u = sum(ws + r * ldw + N + c);
+            again(u, a.w_up);
             v.x = silu_mul(v.x, u.x); v.y = silu_mul(v.y, u.y); v.z = silu_mul(v.z, u.z); v.w = silu_mul(v.w, u.w);
         }
         *o = v;
@@ -368,10 +418,10 @@ int launch_split(const float* src, const float* src2, int64_t ld, int rows, int 
 }
 
 template <int EPI>
-int launch_reduce(float* y, int64_t ldy, const float* ws, int64_t split_stride, int M, int N, int splits, cudaStream_t s) {
+int launch_reduce(float* y, int64_t ldy, const float* ws, int64_t split_stride, int M, int N, int splits, const Args& a, cudaStream_t s) {
     const int64_t blocks = ((int64_t)M * (N / 4) + 255) / 256, most = 8LL * sm_count();
     kllm_launch((reduce_splits_kernel<EPI>), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, y, ldy, ws, split_stride,
-                M, N, splits);
+                M, N, splits, a);
     KLLM_LAUNCH_STATUS();
 }
 
@@ -461,12 +511,13 @@ extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, 
     if (r) return r;
     Args a;
     a.M = M; a.K = K; a.splits = p.splits; a.blocks_per_split = (kblocks + p.splits - 1) / p.splits; a.status = status;
-    a.a_rows = M;
+    a.a_rows = M; a.x = (const float*)x; a.ldx = ldx; a.ldw = ldw;
     for (int n0 = 0; n0 < N; n0 += p.piece) {
         const int cols = N - n0 < p.piece ? N - n0 : p.piece;
         float* yp = (float*)y + n0;
         a.b_rows = cols * (gated ? 2 : 1);
-        r = launch_split((const float*)w + n0 * ldw, gated ? (const float*)w_up + n0 * ldw : nullptr, ldw, cols, K, pb, a.b_rows, p.kp, s);
+        a.w = (const float*)w + n0 * ldw; a.w_up = gated ? (const float*)w_up + n0 * ldw : nullptr;
+        r = launch_split(a.w, a.w_up, ldw, cols, K, pb, a.b_rows, p.kp, s);
         if (r) return r;
         // with splits a gated piece is a plain product with the gate and up columns beside each other
         const bool pairs = gated && p.splits == 1;
@@ -480,9 +531,9 @@ extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, 
             a.N = a.b_rows; a.y = part; a.ldy = a.b_rows; a.split_stride = (int64_t)M * a.b_rows;
             r = launch<EPI_PARTIAL>(ma, mb, a, s);
             if (r) return r;
-            r = epilogue == EPI_STORE ? launch_reduce<EPI_STORE>(yp, ldy, part, a.split_stride, M, cols, p.splits, s)
-                : epilogue == EPI_ADD ? launch_reduce<EPI_ADD>(yp, ldy, part, a.split_stride, M, cols, p.splits, s)
-                                      : launch_reduce<EPI_SWIGLU>(yp, ldy, part, a.split_stride, M, cols, p.splits, s);
+            r = epilogue == EPI_STORE ? launch_reduce<EPI_STORE>(yp, ldy, part, a.split_stride, M, cols, p.splits, a, s)
+                : epilogue == EPI_ADD ? launch_reduce<EPI_ADD>(yp, ldy, part, a.split_stride, M, cols, p.splits, a, s)
+                                      : launch_reduce<EPI_SWIGLU>(yp, ldy, part, a.split_stride, M, cols, p.splits, a, s);
         }
         if (r) return r;
     }

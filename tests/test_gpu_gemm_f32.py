@@ -51,15 +51,54 @@ def test_float32_product(rows, cols, k, epilogue):
 
 
 def test_large_and_non_finite_numbers():
-    """Finite numbers up to the largest float32 are exact; an infinity or NaN makes its row NaN and no other."""
+    """Finite numbers up to the largest float32 are exact; an infinity or NaN leaves the other rows alone, and the infinity
+    stays one where it meets a number that is not zero."""
     from kllm_b200 import kernels
     x = torch.zeros(40, 64, device="cuda")
     x[0], x[1], x[2, 5], x[3, 6] = 3.4028234e38, -3.4e38, float("inf"), float("nan")
     x[4], x[5] = 1.1754944e-38, 1.0 + 2.0 ** -23
     y = kernels.gemm_f32(x, torch.eye(64, device="cuda"))
-    assert torch.isnan(y[2]).all() and torch.isnan(y[3]).all()
+    assert y[2, 5] == float("inf") and torch.isnan(y[2, :5]).all() and torch.isnan(y[2, 6:]).all() and torch.isnan(y[3]).all()
     keep = [0, 1, 4, 5] + list(range(6, 40))
     assert torch.equal(y[keep], x[keep])
+
+
+@pytest.mark.parametrize("epilogue", ["f32", "add", "swiglu"])
+@pytest.mark.parametrize("rows,cols,k", [(40, 260, 64), (64, 2560, 2048), (300, 1028, 52)])
+def test_infinities(rows, cols, k, epilogue):
+    """Operands with infinities and products that overflow against float64 rounded to float32, and every other row and
+    column the same bits as without them.  64 x 2560 x 2048 sums in several ranges of k, the others in one."""
+    from kllm_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, up, h = rnd(rows, k), rnd(cols, k), rnd(cols, k), rnd(rows, cols)
+    call = lambda x, w, up: (kernels.gemm_f32(x, w, weight_up=up, epilogue="swiglu") if epilogue == "swiglu" else
+                             kernels.gemm_f32(x, w, epilogue="add", out=h.clone()) if epilogue == "add" else kernels.gemm_f32(x, w))
+    plain = call(x, w, up)
+    inf = float("inf")
+    xi, wi, ui = x.clone(), w.clone(), up.clone()
+    xi[3, 7], xi[5, 0], xi[5, k - 1], xi[rows - 1, 30] = inf, -inf, inf, -inf
+    xi[9] = 0.0
+    xi[9, 11] = 1.2345678e30
+    wi[4, 9], wi[cols - 1, 2], ui[6, 3] = inf, -inf, inf
+    wi[17, 11], ui[17, 11] = -1.2345678e30, 1.7654321e30
+    got = call(xi, wi, ui)
+    wide = xi.double() @ wi.double().T
+    if epilogue == "swiglu":
+        # the activation in float32, as the kernels take it: exp(-g) overflows from g = -88.7 on, and 0 times an infinite
+        # up is NaN where float64 still has a tiny number
+        gate = wide.float()
+        wide = (gate / (1 + torch.exp(-gate))) * (xi.double() @ ui.double().T).float()
+    elif epilogue == "add":
+        wide = wide + h.double()
+    want = wide.float()
+    hit_r, hit_c = [3, 5, 9, rows - 1], [4, 6, 17, cols - 1]
+    touched = torch.zeros(rows, cols, dtype=torch.bool, device="cuda")
+    touched[hit_r] = True
+    touched[:, hit_c] = True
+    assert torch.equal(got[~touched], plain[~touched])
+    for kind in (torch.isnan, torch.isposinf, torch.isneginf):
+        assert torch.equal(kind(got), kind(want)), kind.__name__
 
 
 def test_route():
