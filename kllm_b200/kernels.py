@@ -1491,7 +1491,7 @@ GEMM_F32_ROWS_BEYOND_L2 = 128
 def gemm_f32_fits(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor] = None, epilogue: str = "f32",
                   weight_up: Optional[torch.Tensor] = None) -> bool:
     """Whether ``gemm_f32`` takes these operands and is the faster route (float32, dense rows, sizes and row strides
-    multiples of 4, 16-byte aligned addresses)."""
+    multiples of 4, 16-byte aligned addresses, an ``out`` of the result's shape, no gradient wanted)."""
     if not USE_TCGEN05 or x.dtype != torch.float32 or weight.dtype != torch.float32 or x.dim() != 2 or weight.dim() != 2:
         return False
     n, K = x.shape
@@ -1499,6 +1499,10 @@ def gemm_f32_fits(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Ten
     if n < (GEMM_F32_LEAST_ROWS if N * K <= GEMM_F32_L2_WEIGHTS else GEMM_F32_ROWS_BEYOND_L2):
         return False
     if weight.shape[1] != K or N * K < GEMM_F32_LEAST_WEIGHTS or (N | K) & 3:
+        return False
+    if out is not None and tuple(out.shape) != (n, N):        # the library's product resizes it, or refuses
+        return False
+    if (x.requires_grad or weight.requires_grad) and torch.is_grad_enabled():
         return False
     for t in (x, weight, weight_up, out):
         if t is not None and (t.dtype != torch.float32 or t.stride(1) != 1 or t.stride(0) & 3 or t.data_ptr() & 15

@@ -117,3 +117,21 @@ def test_route():
     assert not kernels.gemm_f32_fits(x[:, :1022], w[:, :1022])
     assert not kernels.gemm_f32_fits(x, w[:512])                        # too small to pay
     assert not kernels.gemm_f32_fits(torch.empty(0, 1024, device="cuda"), w)
+
+
+def test_what_the_library_does_stays_with_it():
+    """An ``out`` of another shape is resized, as below the route's sizes; a product whose gradient is wanted has one."""
+    from kllm_b200 import kernels
+    x, w = torch.randn(64, 1024, device="cuda"), torch.randn(2048, 1024, device="cuda")
+    want = x.double() @ w.double().T
+    for shape in ((0,), (3, 3)):
+        out = torch.empty(shape, device="cuda")
+        y = kernels.linear(x, w, out=out)
+        assert y is out and y.shape == (64, 2048) and (y.double() - want).norm() <= 2e-6 * want.norm()
+    v = w.clone().requires_grad_()
+    y = kernels.linear(x, v)
+    assert y.requires_grad
+    y.sum().backward()
+    assert (v.grad - x.sum(dim=0)).abs().max() <= 1e-4 * x.sum(dim=0).abs().max()
+    with torch.no_grad():
+        assert kernels.gemm_f32_fits(x, v) and not kernels.linear(x, v).requires_grad
