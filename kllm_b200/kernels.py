@@ -1294,9 +1294,17 @@ def _skinny_gemm_f32(weight, x, x_f32, gain, eps, rows, n_rows, weight_up, epilo
     return out
 
 
+_DIRECT_BLAS = (torch._C._BlasBackend.Cublas, torch._C._BlasBackend.Default)
+
+
 def prompt_layers_ready() -> bool:
-    """Whether ``prompt_layers`` can run in this process (it calls the product library that torch has loaded)."""
-    return bool(load_library("prompt_layers").kllm_prompt_layers_ready())
+    """Whether ``prompt_layers`` can run in this process (it calls the product library that torch has loaded) and would
+    do what ``linear`` does: torch's settings of its products, which the direct calls know nothing of, are as they are by
+    default (1 us).  With others the parts go through torch, which obeys them, or ``linear`` refuses."""
+    m = torch.backends.cuda.matmul
+    return (not m.allow_tf32 and m.allow_bf16_reduced_precision_reduction and not torch.are_deterministic_algorithms_enabled()
+            and torch.backends.cuda.preferred_blas_library() in _DIRECT_BLAS and not torch.cuda.tunable.is_enabled()
+            and bool(load_library("prompt_layers").kllm_prompt_layers_ready()))
 
 
 def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,

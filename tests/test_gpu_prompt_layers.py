@@ -99,3 +99,40 @@ def test_wide_step_takes_the_gated_product():
     (a, la), (b, lb) = out
     assert (a - b).abs().max() <= 1e-2 * a.abs().max()
     assert la == lb                                   # the same kernels
+
+
+def test_settings_of_the_products_are_obeyed(monkeypatch):
+    """The direct calls of the library know nothing of torch's settings: with any that is not the default the parts run."""
+    from kllm_b200 import Engine, Options, StepEntry, kernels
+    engine = Engine(None, Options(max_seq=128, block_size=16, num_blocks=80, max_batch=8, dtype="bfloat16", max_step_tokens=128),
+                    config=_config("d64"), random_seed=1)
+    taken = []
+    inner = engine.model.prompt_layers.run
+    engine.model.prompt_layers.run = lambda *a: (taken.append(1), inner(*a))
+
+    def step():
+        del taken[:]
+        r = engine.cache.open()
+        logits = engine.step([StepEntry(r, list(range(30)), [29])]).clone()
+        engine.cache.close(r)
+        return logits, bool(taken)
+    want, native = step()
+    assert native
+    m = torch.backends.cuda.matmul
+    with monkeypatch.context() as mp:
+        mp.setattr(m, "allow_bf16_reduced_precision_reduction", False)
+        got, native = step()
+        assert not native and (got - want).abs().max() <= 1e-2 * want.abs().max()
+    before = torch.backends.cuda.preferred_blas_library()
+    try:
+        torch.backends.cuda.preferred_blas_library("cublaslt")
+        got, native = step()
+        assert not native and (got - want).abs().max() <= 1e-2 * want.abs().max()
+    finally:
+        torch.backends.cuda.preferred_blas_library(before)
+    with monkeypatch.context() as mp:
+        mp.setattr(m, "allow_tf32", True)
+        with pytest.raises(kernels.KernelError, match="TF32"):
+            step()
+    assert step()[1]
+    engine.close()
