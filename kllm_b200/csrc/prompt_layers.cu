@@ -52,8 +52,8 @@ bool product(cublasHandle_t blas, const void* w, int N, int K, const void* x, in
 // 1 if the library product can be called from here.
 extern "C" int kllm_prompt_layers_ready() { return library_product() != nullptr ? 1 : 0; }
 
-// layers: host array of n_layers x 8 addresses (w_qkv [(H + 2G) hd, d], w_o [d, H hd], w_gate_up [2F, d], w_down [d, F],
-// gain1, gain2 float32 [d], key pages, value pages).  entries: the addresses of `Entries`.  blas: a handle of the library
+// layers: host array of n_layers x 9 addresses (w_qkv [(H + 2G) hd, d], w_o [d, H hd], w_gate_up [2F, d], w_down [d, F],
+// gain1, gain2 float32 [d], key pages, value pages, cos / sin table float32 [positions, hd]).  entries: the addresses of `Entries`.  blas: a handle of the library
 // product that is set to the stream.  A layer has two halves, the first up to the norm in front of the feed-forward (left
 // in xn), the second the down product (from act): the halves first .. last - 1 of the layers' 2 n_layers are run.  x [n, d] float32; positions, token_req [n]; table [requests, max_blocks]; the first
 // `singles` requests bring one token each and run as decoding tokens in num_splits ranges (part_o, part_ml: their
@@ -62,7 +62,7 @@ extern "C" int kllm_prompt_layers_ready() { return library_product() != nullptr 
 // makes act from xn between two calls.  failed: the number of the entry that refused (5: the library product), whose
 // library holds the message.
 extern "C" int kllm_prompt_layers(int first, int last, const void* layers, int n_layers, const void* entries, void* blas, int n, int d, int H, int G,
-                                  int hd, int F, float eps, float scale, float* x, const float* cos_sin, const int* positions,
+                                  int hd, int F, float eps, float scale, float* x, const int* positions,
                                   const int* token_req, const int* table, int max_blocks, int n_requests, const int* q_start,
                                   const int* start_pos, int singles, int num_splits, int page_size, void* xn, void* qkv,
                                   void* attn, void* part_o, void* part_ml, void* act, void* gate_up, int* status, int* failed,
@@ -78,14 +78,14 @@ extern "C" int kllm_prompt_layers(int first, int last, const void* layers, int n
     auto refuse = [&](int which, int rc) { *failed = which; return rc; };
     int rc;
     for (int half = first; half < last; half++) {
-        void* const* p = (void* const*)layers + 8 * (half / 2);
+        void* const* p = (void* const*)layers + 9 * (half / 2);
         if (half & 1) {
             if (!product(b, p[3], d, F, act, n, x, CUDA_R_32F, true)) return refuse(5, -1);
             continue;
         }
         if ((rc = e.norm(x, nullptr, xn, p[4], nullptr, n, d, eps, KLLM_BF16, KLLM_BF16, stream))) return refuse(0, rc);
         if (!product(b, p[0], w, d, xn, n, q, CUDA_R_16BF, false)) return refuse(5, -1);
-        if ((rc = e.rope(q, w, q + qd, w, q + qd + kd, w, cos_sin, positions, token_req, table, max_blocks, p[6], p[7], n, H, G, hd, hd,
+        if ((rc = e.rope(q, w, q + qd, w, q + qd + kd, w, (const float*)p[8], positions, token_req, table, max_blocks, p[6], p[7], n, H, G, hd, hd,
                          page_size, KLLM_BF16, stream)))
             return refuse(1, rc);
         if (singles > 0 && (rc = e.decode(attn, part_o, part_ml, q, w, p[6], p[7], positions, nullptr, table, max_blocks, singles, H, G,

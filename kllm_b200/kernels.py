@@ -1307,33 +1307,35 @@ def prompt_layers_ready() -> bool:
             and bool(load_library("prompt_layers").kllm_prompt_layers_ready()))
 
 
-def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,
-                  head_dim: int, inter: int, eps: float, scale: float) -> None:
+def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,
+                  head_dim: int, inter: int, eps: float, scale: float) -> bool:
     """The layers of a step with portions, launched from one call (csrc/prompt_layers.cu): x [n, d] float32 is the
-    residual stream, updated in place; ``layers`` holds (w_qkv, w_o, w_gate_up, w_down, gain1, gain2, k pages, v pages)
-    per layer, in bfloat16 with float32 gains.  The same kernels as ``attention``, ``add_rmsnorm``, ``linear`` and so on
+    residual stream, updated in place; ``layers`` holds (w_qkv, w_o, w_gate_up, w_down, gain1, gain2, k pages, v pages,
+    cos / sin table) per layer, in bfloat16 with float32 gains and tables.  False, and nothing done, where one of them does not
+    fit (sizes, types, dense rows, 16-byte alignment).  The same kernels as ``attention``, ``add_rmsnorm``, ``linear`` and so on
     launch for this step, with the routes that they choose."""
     global launches
     n, d = x.shape
     positions, token_req, q_start, start_pos = ctx.positions, ctx.token_req, ctx.q_start, ctx.start_pos
-    _cuda(x, cos_sin, positions, token_req, q_start, start_pos, block_table)
+    _cuda(x, positions, token_req, q_start, start_pos, block_table)
     for t, what in ((positions, "positions"), (token_req, "token_req"), (q_start, "q_start"), (start_pos, "start_pos"),
                     (block_table, "block_table")):
         _i32(t, what)
     if x.dtype != torch.float32 or not x.is_contiguous() or positions.numel() != n or token_req.numel() != n:
         raise KernelError("prompt_layers: x must be contiguous float32 [n, d], with one position and one request a token")
-    if cos_sin.dtype != torch.float32 or not cos_sin.is_contiguous() or cos_sin.shape[1] != head_dim:
-        raise KernelError("prompt_layers: the cos/sin table must be float32 [positions, head_dim]")
     page_size, q_dim = layers[0][6].shape[2], n_heads * head_dim
     wide = q_dim + 2 * n_kv * head_dim
-    want = ((wide, d), (d, q_dim), (2 * inter, d), (d, inter), (d,), (d,))
+    pages, want = (n_kv, page_size, head_dim), ((wide, d), (d, q_dim), (2 * inter, d), (d, inter), (d,), (d,))
     ptrs = []
     for layer in layers:
         for i, t in enumerate(layer):
-            ok = t.is_cuda and t.is_contiguous() and t.dtype == (torch.float32 if i in (4, 5) else torch.bfloat16)
-            if not ok or (t.shape != want[i] if i < 6 else t.shape[1:] != (n_kv, page_size, head_dim)):
-                raise KernelError(f"prompt_layers: operand {i} of a layer ({t.dtype}, {tuple(t.shape)}) does not fit the sizes")
-            ptrs.append(t.data_ptr())
+            if (t is None or not t.is_cuda or not t.is_contiguous() or t.dtype != (torch.float32 if i in (4, 5, 8) else torch.bfloat16)
+                    or (t.shape != want[i] if i < 6 else t.shape[1:] != (pages if i < 8 else (head_dim,)))):
+                return False
+            ptr = t.data_ptr()
+            if ptr & 15:
+                return False
+            ptrs.append(ptr)
     singles = 0
     while singles < ctx.n_requests and ctx.host_n_new[singles] == 1:
         singles += 1
@@ -1363,7 +1365,7 @@ def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_tab
     failed = ctypes.c_int(-1)
     lib = load_library("prompt_layers")
     args = (ctypes.addressof(table), len(layers), ctypes.addressof(entries), torch.cuda.current_blas_handle(), n, d, n_heads, n_kv,
-            head_dim, inter, eps, scale, _p(x), _p(cos_sin), _p(positions), _p(token_req), _p(block_table), block_table.shape[1],
+            head_dim, inter, eps, scale, _p(x), _p(positions), _p(token_req), _p(block_table), block_table.shape[1],
             ctx.n_requests, _p(q_start), _p(start_pos), singles, splits, page_size, _p(xn), _p(qkv), _p(attn), _p(part_o),
             _p(part_ml), _p(act), _p(gate_up), _p(status_word(x.device)), ctypes.addressof(failed), _stream())
 
@@ -1384,6 +1386,7 @@ def prompt_layers(x: torch.Tensor, layers, cos_sin: torch.Tensor, ctx, block_tab
             gemm(xn, layer[2][:inter], weight_up=layer[2][inter:], epilogue="swiglu", out=act)
         halves(2 * len(layers) - 1, 2 * len(layers))
     launches = before + len(layers) * (5 + (1 if singles else 0) + (1 if splits > 1 else 0))
+    return True
 
 
 def linear_add(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> None:

@@ -6,7 +6,7 @@ of one size, in bfloat16 (the Llama layer).  ``takes(ctx, caches)`` says whether
 that way: more tokens than the weight-streaming products take, portions among them, a head
 size of the tcgen05 attention, and so little work that the host's launches would be the longer
 part.  The kernels, their arguments and their order are those of the blocks' own forward;
-weights and cache pages are named at every call.
+weights, tables of angles and cache pages are named at every call, and where one does not fit the parts run.
 """
 from __future__ import annotations
 
@@ -15,7 +15,6 @@ from .attention import PagedAttention
 from .block import PreNormBlock
 from .mlp import GatedMLP
 from .norm import RMSNorm
-from .rotary import RotaryEmbedding
 
 import torch
 
@@ -33,15 +32,6 @@ def _plain_attention(m) -> bool:
             and getattr(m.position, "full_rotary_table", lambda: None)() is not None)
 
 
-def _same_rotation(p, q) -> bool:
-    """Whether two position parts have one table of angles (built-in ones by their parameters: comparing 22 tables on the
-    device took 10 ms of an engine's start)."""
-    a, b = p.full_rotary_table(), q.full_rotary_table()
-    if type(p) is RotaryEmbedding and type(q) is RotaryEmbedding:
-        return (p.theta, p.rotary_dim, a.shape) == (q.theta, q.rotary_dim, b.shape)
-    return a is b or torch.equal(a, b)
-
-
 class PromptLayers:
     def __init__(self, model):
         self.blocks = [model.blocks[call.block] for call in model.schedule]
@@ -49,7 +39,6 @@ class PromptLayers:
         m, f = self.blocks[0].mixer, self.blocks[0].feed_forward
         self.d, self.heads, self.kv, self.head_dim, self.inter = m.hidden, m.n_heads, m.n_kv, m.head_dim, f.inter
         self.eps, self.scale = self.blocks[0].mixer_norm.eps, m.scale
-        self.table = m.position.full_rotary_table()
         self.weights = m.w_qkv.numel() + m.w_o.numel() + f.w_gate_up.numel() + f.w_down.numel()      # of one layer
 
     @staticmethod
@@ -70,11 +59,9 @@ class PromptLayers:
                     m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain)):
                 return None
             key = (m.hidden, m.n_heads, m.n_kv, m.head_dim, m.scale, f.hidden, f.inter, b.mixer_norm.eps, b.ff_norm.eps)
-            if m.hidden != f.hidden or b.mixer_norm.eps != b.ff_norm.eps or (first is not None and key != first[0]):
+            if m.hidden != f.hidden or b.mixer_norm.eps != b.ff_norm.eps or (first is not None and key != first):
                 return None
-            if first is not None and not _same_rotation(m.position, first[1]):
-                return None
-            first = first or (key, m.position)
+            first = first or key
         return PromptLayers(model)
 
     def takes(self, ctx, caches) -> bool:
@@ -88,10 +75,11 @@ class PromptLayers:
         return kernels.prompt_layers_ready() and all(
             caches[i].block_table is c.block_table and caches[i].k.shape[2] == c.page_size for i in self.slots)
 
-    def run(self, x, ctx, caches) -> None:
+    def run(self, x, ctx, caches) -> bool:
         layers = []
         for b, i in zip(self.blocks, self.slots):
             m, f, c = b.mixer, b.feed_forward, caches[i]
-            layers.append((m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain, c.k, c.v))
-        kernels.prompt_layers(x, layers, self.table, ctx, caches[self.slots[0]].block_table, self.heads, self.kv, self.head_dim,
-                              self.inter, self.eps, self.scale)
+            layers.append((m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain, c.k, c.v,
+                           m.position.full_rotary_table()))
+        return kernels.prompt_layers(x, layers, ctx, caches[self.slots[0]].block_table, self.heads, self.kv, self.head_dim,
+                                     self.inter, self.eps, self.scale)
