@@ -654,27 +654,43 @@ def sm_count() -> int:
 
 
 def decode_splits(n_tokens: int, n_kv: int, ctx_bound: int, head_dim: int = 128) -> int:
-    """Into how many key ranges the decode kernel cuts a token's context.
+    """Into how many key ranges the decode kernel cuts a token's context of up to ``ctx_bound`` places (in a replayed step
+    the bound that the graph was captured with, the engine's longest sequence).
 
-    A CTA takes one (token, kv head, range) and walks it in tiles of 64 keys.  Cutting costs about
-    2.3 us (partial results out and in again, the merge), a tile 0.35 us in a CTA whose tiles are all
-    requested at once.  So, measured (us, by ranges):
-      - up to 8 tiles are not cut: 24 x 4 (tokens x kv heads) of size 64 at 200 keys 1: 4.9, 2: 7.2;
-        4 x 32 of size 128 at 300 keys 1: 7.4, 2: 8.9; at 10 tiles it makes no difference (9.8, 9.9);
-      - fewer (token, kv head) pairs than slots (two CTAs an SM): as many ranges as fill the SMs in ONE wave,
-        at most 16 (a second wave of short CTAs would double the time);
-      - more pairs are CTAs enough: 64 x 8 of size 128 at 1280 keys 1: 57.4, 2: 69.9; 32 x 8 at 2000 keys 1: 48.1,
-        2: 50.0; 24 x 32 at 1500 keys 1: 94.3, 2: 106.9.  Only at small head sizes, where a tile is half the bytes and
-        two CTAs do not keep an SM's share of the memory busy, a long context is cut in two while the CTAs still fit at
-        once: 64 x 4 of size 64 at 2000 keys 1: 32.3, 2: 27.5."""
-    slots = 2 * sm_count()
+    A CTA takes one (token, kv head, range) and walks it in tiles of 64 keys, of which it has the first two to four in
+    flight at once.  Cutting costs 2.2 to 5 us (partial results out and in again, the merge; the more CTAs the more), a tile
+    0.4 to 0.8 us at head size 64, 0.95 at 128, 1.5 at 256.  Measured (us, by ranges; tokens x kv heads of a size at keys):
+
+      - short contexts are not cut.  Few pairs: 1 x 4 of size 64 at 200 1: 4.6, 4: 5.9, at 512 1: 7.6, 8: 6.1; 1 x 8 of size
+        128 at 200 1: 6.1, 4: 6.3, at 300 1: 7.1, 5: 6.5, at 512 1: 9.9, 8: 6.4; 1 x 8 of size 256 at 100 1: 6.4, 2: 8.1, at
+        200 1: 9.2, 4: 8.4.  More pairs: 16 x 4 of size 64 at 300 1: 5.5, 3: 7.1; 8 x 8 of 128 at 300 1: 7.3, 3: 8.2, at 512
+        1: 10.4, 4: 9.4; 24 x 4 of 64 at 512 1: 8.3, 3: 8.7; 16 x 8 of 128 at 512 1: 11.7, 2: 13.2.  At size 64 and up to 64
+        pairs the line is drawn by whole decode steps, in which the ranges' CTAs also ask for the next matrix
+        (22 layers, 8 x 4 at 300 1: 773, 5: 732; 16 x 4 at 400 1: 999, 4: 947; 8 x 4 under a bound of 256, at 60 1: 698,
+        4: 730, at 200 1: 749, 4: 732);
+      - fewer pairs than slots (two CTAs an SM): as many ranges as fill the SMs in ONE wave, at most 16 (a second wave
+        of short CTAs would double the time);
+      - more pairs are CTAs enough, unless one range each leaves the last wave nearly empty and two fill it better: 64 x 8
+        of size 128 at 1280 1: 68, 2: 79; 16 x 32 of size 64 at 2000 1: 49, 2: 56; but 24 x 32 at 2000 1: 84, 2: 79 (1.3
+        waves of four CTAs an SM), 64 x 4 of size 64 at 2000 1: 35, 2: 30 (a wave that half of the slots would
+        take), 24 x 8 of size 256 at 2000 1: 103, 2: 88."""
+    sms = sm_count()
     tiles = max(1, -(-ctx_bound // 64))
     base = max(1, n_tokens * n_kv)
-    if tiles <= 8:
+    if head_dim < 128:
+        uncut = 4 if base <= 32 else 5
+    elif head_dim == 128:
+        uncut = 4 if base <= 16 else 5
+    else:
+        uncut = 3 if base <= 16 else 8
+    if tiles <= (uncut if base <= 64 else 8):
         return 1
-    splits = max(1, min(slots // base, tiles, 16))
-    if splits == 1 and tiles >= 16 and head_dim <= 64 and base <= slots:
-        splits = 2
+    splits = max(1, min(2 * sms // base, tiles, 16))
+    if splits == 1 and tiles >= 16:
+        slots = sms * max(1, min(4, 256 // head_dim))
+        # waves x a CTA's time, in tiles; starting and merging take about as long as six tiles
+        if -(-2 * base // slots) * (-(-tiles // 2) + 6) < -(-base // slots) * (tiles + 6):
+            splits = 2
     per = -(-tiles // splits)
     return -(-tiles // per)
 

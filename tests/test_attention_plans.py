@@ -1,4 +1,4 @@
-"""The barrier on which the tensor-memory attention kernel announces its products into the output, by its own account of
+"""How the attention kernels are cut and chosen, and the barrier on which the tensor-memory attention kernel announces its products into the output, by its own account of
 which products complete a phase and which phases are waited for (csrc/attention_tcgen05_ptmem.cu).  A wait by parity
 passes at once while the phase before it is open, so it is sound only for the phase behind the one waited for
 last; no order between arrivals on different barriers is taken for granted here."""
@@ -30,3 +30,21 @@ def test_which_form_a_step_takes(monkeypatch):
     assert form(128, 4, 8, 300, 1, 8300) == "smem" and form(128, 4, 8, 850, 1, 850) == "tmem"
     assert form(64, 8, 4, 700, 1, 700) == "smem" and form(64, 8, 4, 2048, 1, 2048) == "smem"
     assert form(64, 8, 4, 2400, 24, 100) == "tmem" and form(64, 8, 4, 8192, 1, 8192) == "tmem"
+
+
+# tokens, kv heads, context, head size: ranges.  Times of the ranges beside it, in kernels.decode_splits.
+SPLITS = [
+    (1, 4, 256, 64, 1), (1, 4, 512, 64, 8), (8, 4, 300, 64, 5), (16, 4, 300, 64, 1), (16, 4, 400, 64, 4), (24, 4, 512, 64, 1),
+    (1, 8, 200, 128, 1), (1, 8, 300, 128, 5), (8, 8, 300, 128, 1), (8, 8, 512, 128, 4), (16, 8, 512, 128, 1),
+    (1, 8, 100, 256, 1), (1, 8, 200, 256, 4), (8, 8, 512, 256, 1),
+    (64, 8, 1280, 128, 1), (24, 32, 1500, 128, 1), (64, 4, 2000, 64, 2), (16, 32, 2000, 64, 1), (24, 32, 2000, 64, 2),
+    (24, 8, 2000, 256, 2), (32, 8, 2000, 256, 1), (8, 4, 2048, 64, 8), (1, 8, 8000, 128, 16),
+]
+
+
+@pytest.mark.parametrize("n,kv,ctx,hd,ranges", SPLITS)
+def test_ranges_of_a_context(monkeypatch, n, kv, ctx, hd, ranges):
+    """Few pairs cut contexts that outlast the merge, many do not; long contexts are cut where that fills the last wave."""
+    from kllm_b200 import kernels
+    monkeypatch.setattr(kernels, "sm_count", lambda: 148)
+    assert kernels.decode_splits(n, kv, ctx, hd) == ranges
