@@ -1323,13 +1323,16 @@ def prompt_layers_ready() -> bool:
             and bool(load_library("prompt_layers").kllm_prompt_layers_ready()))
 
 
-def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,
-                  head_dim: int, inter: int, eps: float, scale: float) -> bool:
-    """The layers of a step with portions, launched from one call (csrc/prompt_layers.cu): x [n, d] float32 is the
-    residual stream, updated in place; ``layers`` holds (w_qkv, w_o, w_gate_up, w_down, gain1, gain2, k pages, v pages,
-    cos / sin table) per layer, in bfloat16 with float32 gains and tables.  False, and nothing done, where one of them does not
-    fit (sizes, types, dense rows, 16-byte alignment).  The same kernels as ``attention``, ``add_rmsnorm``, ``linear`` and so on
-    launch for this step, with the routes that they choose."""
+def prompt_layers(x: torch.Tensor, layers, n_layers: int, ctx, block_table: torch.Tensor, n_heads: int, n_kv: int,
+                  head_dim: int, inter: int, eps: float, scale: float) -> int:
+    """The layers of a step with portions, launched from native code (csrc/prompt_layers.cu): x [n, d] float32 is the
+    residual stream, updated in place; ``layers`` gives (w_qkv, w_o, w_gate_up, w_down, gain1, gain2, k pages, v pages,
+    cos / sin table) layer by layer, in bfloat16 with float32 gains and tables.  Returns how many layers were launched: those
+    up to the first with an operand that does not fit (sizes, types, dense rows, 16-byte alignment).  The same kernels as
+    ``attention``, ``add_rmsnorm``, ``linear`` and so on launch for this step, with the routes that they choose.
+
+    The first layer is launched before the others are looked at: reading and checking the operands of 22 layers takes
+    0.2 ms, which a step that finds the GPU idle would wait for."""
     global launches
     n, d = x.shape
     positions, token_req, q_start, start_pos = ctx.positions, ctx.token_req, ctx.q_start, ctx.start_pos
@@ -1339,11 +1342,14 @@ def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_hea
         _i32(t, what)
     if x.dtype != torch.float32 or not x.is_contiguous() or positions.numel() != n or token_req.numel() != n:
         raise KernelError("prompt_layers: x must be contiguous float32 [n, d], with one position and one request a token")
-    page_size, q_dim = layers[0][6].shape[2], n_heads * head_dim
+    layers = iter(layers)
+    first = next(layers)
+    page_size, q_dim = first[6].shape[2], n_heads * head_dim
     wide = q_dim + 2 * n_kv * head_dim
     pages, want = (n_kv, page_size, head_dim), ((wide, d), (d, q_dim), (2 * inter, d), (d, inter), (d,), (d,))
-    ptrs = []
-    for layer in layers:
+    table = (ctypes.c_void_p * (9 * n_layers))()
+
+    def fits(j, layer):
         for i, t in enumerate(layer):
             if (t is None or not t.is_cuda or not t.is_contiguous() or t.dtype != (torch.float32 if i in (4, 5, 8) else torch.bfloat16)
                     or (t.shape != want[i] if i < 6 else t.shape[1:] != (pages if i < 8 else (head_dim,)))):
@@ -1351,7 +1357,10 @@ def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_hea
             ptr = t.data_ptr()
             if ptr & 15:
                 return False
-            ptrs.append(ptr)
+            table[9 * j + i] = ptr
+        return True
+    if not fits(0, first):
+        return 0
     singles = 0
     while singles < ctx.n_requests and ctx.host_n_new[singles] == 1:
         singles += 1
@@ -1369,7 +1378,7 @@ def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_hea
     form = tcgen05_choice(head_dim, n_heads // n_kv, n_kv, n - singles, ctx.n_requests - singles, ctx.max_ctx)
     xn, qkv, attn, act = new(n, d), new(n, wide), new(n, q_dim), new(n, inter)
     gate_up = None
-    if not (gemm_pays(n, inter, "swiglu") and all(gemm_fits(xn, layer[2][:inter], act, "swiglu", layer[2][inter:]) for layer in layers)):
+    if not (gemm_pays(n, inter, "swiglu") and gemm_fits(xn, first[2][:inter], act, "swiglu", first[2][inter:])):
         gate_up = new(n, 2 * inter, dtype=torch.float32)
     name = "attention_tcgen05" + ("_ptmem" if form == "tmem" else "")
     used = [("norm", None, "kllm_add_rmsnorm"), ("rope", None, "kllm_rope_append"),
@@ -1377,10 +1386,9 @@ def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_hea
             (name, {"KLLM_HD": head_dim}, "kllm_attention_prefill_tcgen05" + ("_ptmem" if form == "tmem" else "")),
             ("activation", None, "kllm_silu_mul")]
     entries = (ctypes.c_void_p * len(used))(*(load_library(lib, defs).address(fn) for lib, defs, fn in used))
-    table = (ctypes.c_void_p * len(ptrs))(*ptrs)
     failed = ctypes.c_int(-1)
     lib = load_library("prompt_layers")
-    args = (ctypes.addressof(table), len(layers), ctypes.addressof(entries), torch.cuda.current_blas_handle(), n, d, n_heads, n_kv,
+    args = (ctypes.addressof(table), n_layers, ctypes.addressof(entries), torch.cuda.current_blas_handle(), n, d, n_heads, n_kv,
             head_dim, inter, eps, scale, _p(x), _p(positions), _p(token_req), _p(block_table), block_table.shape[1],
             ctx.n_requests, _p(q_start), _p(start_pos), singles, splits, page_size, _p(xn), _p(qkv), _p(attn), _p(part_o),
             _p(part_ml), _p(act), _p(gate_up), _p(status_word(x.device)), ctypes.addressof(failed), _stream())
@@ -1392,17 +1400,28 @@ def prompt_layers(x: torch.Tensor, layers, ctx, block_table: torch.Tensor, n_hea
         if rc != 0 and failed.value == len(used):
             raise KernelError("prompt_layers: the library product failed")
         _check(lib, "prompt_layers", rc)
-    before = launches
+    before, done = launches, 1
     if gate_up is not None:
-        halves(0, 2 * len(layers))
+        halves(0, 2)
+        for layer in layers:
+            if not fits(done, layer):
+                break
+            done += 1
+        if done > 1:
+            halves(2, 2 * done)
     else:
         # gate, up and activation as one kernel, between the halves of every layer
-        for i, layer in enumerate(layers):
-            halves(max(0, 2 * i - 1), 2 * i + 1)
+        halves(0, 1)
+        gemm(xn, first[2][:inter], weight_up=first[2][inter:], epilogue="swiglu", out=act)
+        for layer in layers:
+            if not fits(done, layer):
+                break
+            halves(2 * done - 1, 2 * done + 1)
             gemm(xn, layer[2][:inter], weight_up=layer[2][inter:], epilogue="swiglu", out=act)
-        halves(2 * len(layers) - 1, 2 * len(layers))
-    launches = before + len(layers) * (5 + (1 if singles else 0) + (1 if splits > 1 else 0))
-    return True
+            done += 1
+        halves(2 * done - 1, 2 * done)
+    launches = before + done * (5 + (1 if singles else 0) + (1 if splits > 1 else 0))
+    return done
 
 
 def linear_add(acc: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> None:

@@ -118,8 +118,8 @@ class DecoderModel:
         held = [e.begin(x, bool(self.schedule) and self.schedule[0].entry is not None
                         and self.schedule[0].entry[0] == j) for j, e in enumerate(self.entries)]
         schedule = self.schedule
-        if self.prompt_layers is not None and self.tap is None and self.prompt_layers.takes(ctx, caches) \
-                and self.prompt_layers.run(x, ctx, caches):
+        if self.prompt_layers is not None and self.tap is None and self.prompt_layers.takes(ctx, caches):
+            self.prompt_layers.run(x, ctx, caches)
             schedule = []
         for i, call in enumerate(schedule):
             cache = caches[call.cache]

@@ -6,7 +6,8 @@ of one size, in bfloat16 (the Llama layer).  ``takes(ctx, caches)`` says whether
 that way: more tokens than the weight-streaming products take, portions among them, a head
 size of the tcgen05 attention, and so little work that the host's launches would be the longer
 part.  The kernels, their arguments and their order are those of the blocks' own forward;
-weights, tables of angles and cache pages are named at every call, and where one does not fit the parts run.
+weights, tables of angles and cache pages are named at every call, and from a layer on where one does not fit the
+blocks' own forward runs.
 """
 from __future__ import annotations
 
@@ -18,9 +19,12 @@ from .norm import RMSNorm
 
 import torch
 
-# Steps of up to so many operations in a layer's products go this way.  The parts' own launches take 0.21 ms a layer on the
-# host: at 0.74e11 (841 tokens of TinyLlama's sizes, 0.13 ms of GPU work a layer) that is the step's time, 4.6 ms against
-# 2.9 from here; at 1.8e11 (2048 tokens) the GPU is the slower of the two and the parts' launches were measured 0.5 % faster.
+# Steps of up to so many operations in a layer's products go this way.  The parts' own launches take 0.16 ms a layer on the
+# host; where a layer is less GPU work than that they are the step's time, above it the two are level and the parts run.
+# Passes that find the GPU idle, in turn (us, median [quartiles] of 20, this way / parts): TinyLlama's sizes, 300 tokens
+# (0.26e11) 2166 [2155 2179] / 3635 [3613 3660], 1200 (1.06e11) 3607 [3594 3633] / 3664 [3639 3705], 1704 (1.5e11) 4949
+# [4892 5005] / 4985 [4901 5082] and 4871 [4837 4935] / 4828 [4802 4932], 2048 (1.8e11) 5479 [5436 5518] / 5449
+# [5424 5471]; eight Llama-2-7B layers, 24 tokens and 450 of prompts (2.2e11) 3634 [3595 3675] / 3582 [3542 3632].
 MOST_WORK = 1.5e11
 
 
@@ -75,11 +79,13 @@ class PromptLayers:
         return kernels.prompt_layers_ready() and all(
             caches[i].block_table is c.block_table and caches[i].k.shape[2] == c.page_size for i in self.slots)
 
-    def run(self, x, ctx, caches) -> bool:
-        layers = []
-        for b, i in zip(self.blocks, self.slots):
-            m, f, c = b.mixer, b.feed_forward, caches[i]
-            layers.append((m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain, c.k, c.v,
-                           m.position.full_rotary_table()))
-        return kernels.prompt_layers(x, layers, ctx, caches[self.slots[0]].block_table, self.heads, self.kv, self.head_dim,
-                                     self.inter, self.eps, self.scale)
+    def run(self, x, ctx, caches) -> None:
+        def operands():
+            for b, i in zip(self.blocks, self.slots):
+                m, f, c = b.mixer, b.feed_forward, caches[i]
+                yield (m.w_qkv, m.w_o, f.w_gate_up, f.w_down, b.mixer_norm.gain, b.ff_norm.gain, c.k, c.v,
+                       m.position.full_rotary_table())
+        done = kernels.prompt_layers(x, operands(), len(self.blocks), ctx, caches[self.slots[0]].block_table, self.heads, self.kv,
+                                     self.head_dim, self.inter, self.eps, self.scale)
+        for b, i in zip(self.blocks[done:], self.slots[done:]):      # from an operand that does not fit on: the parts
+            b.forward(x, None, ctx, caches[i])

@@ -138,16 +138,16 @@ def test_settings_of_the_products_are_obeyed(monkeypatch):
     engine.close()
 
 
-def test_tables_and_weights_are_those_of_the_call():
+def test_tables_and_weights_are_those_of_the_call(monkeypatch):
     """What the parts hold when the step runs counts, not what they held when the model was bound: a layer's own table of
-    angles is used, and a weight that the native launches do not take (rows at a stride) sends the step to the parts."""
-    from kllm_b200 import Engine, Options, StepEntry
+    angles is used, and from a weight on that the native launches do not take (rows at a stride) the parts run."""
+    from kllm_b200 import Engine, Options, StepEntry, kernels
     engine = Engine(None, Options(max_seq=128, block_size=16, num_blocks=80, max_batch=8, dtype="bfloat16", max_step_tokens=128),
                     config=_config("d64"), random_seed=1)
     layers, model = engine.model.prompt_layers, engine.model
-    took = []
-    inner = layers.run
-    layers.run = lambda *a: (took.append(inner(*a)), took[-1])[1]
+    took = []                                                    # layers launched natively, of three
+    inner = kernels.prompt_layers
+    monkeypatch.setattr(kernels, "prompt_layers", lambda *a: (took.append(inner(*a)), took[-1])[1])
 
     def step(native):
         model.prompt_layers = layers if native else None
@@ -159,10 +159,12 @@ def test_tables_and_weights_are_those_of_the_call():
     position = model.blocks[1].mixer.position
     position.cos_sin = position.cos_sin.roll(7, dims=0)          # another rotation in one layer
     a, b = step(True), step(False)
-    assert torch.equal(a, b) and not torch.equal(a, before) and took == [True, True]
-    mlp = model.blocks[2].feed_forward
-    wide = torch.zeros(mlp.w_down.shape[0], mlp.w_down.shape[1] + 8, dtype=mlp.w_down.dtype, device="cuda")
-    wide[:, :mlp.w_down.shape[1]] = mlp.w_down
-    mlp.w_down = wide[:, :mlp.w_down.shape[1]]
-    assert torch.equal(step(True), step(False)) and took == [True, True, False]
+    assert torch.equal(a, b) and not torch.equal(a, before) and took == [3, 3]
+    for i in (2, 1, 0):
+        del took[:]
+        mlp = model.blocks[i].feed_forward
+        wide = torch.zeros(mlp.w_down.shape[0], mlp.w_down.shape[1] + 8, dtype=mlp.w_down.dtype, device="cuda")
+        wide[:, :mlp.w_down.shape[1]] = mlp.w_down
+        mlp.w_down = wide[:, :mlp.w_down.shape[1]]
+        assert torch.equal(step(True), step(False)) and took == [i]
     engine.close()
