@@ -7,7 +7,7 @@
 // CUDA cores they are bound by the FMA rate (the library reached 50 TFLOP/s at 1003 rows of
 // TinyLlama's sizes).  Here every float32 number is the sum of three bfloat16 numbers,
 //     v = v0 + v1 + v2,  v0 = bf16(v), v1 = bf16(v - v0), v2 = bf16(v - v0 - v1)
-// (8 + 8 + 8 bits of mantissa: exact unless v2 is below the smallest bfloat16), and
+// (8 + 8 + 8 bits of mantissa), and
 //     x w = x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0) + terms below 2^-24 |x w|,
 // six tcgen05 products with float32 accumulators.  An accumulator only ever holds one k block
 // (32 values of k, the small terms first): it is then added, by the rounding add of the CUDA
@@ -32,9 +32,11 @@
 // of whole blocks, each a unit of work of its own that leaves its sums in a workspace;
 // a third kernel adds them in split order.
 //
-// The parts of an infinity are infinities and NaN, and a product of parts may overflow where the numbers' own does not cancel:
-// a sum that is not finite is taken again, as plain float32 multiply-adds of the operands (plain_dot), so that
-// infinities come out where arithmetic gives them.  Finite numbers of any size are split exactly.
+// The numbers are split after a multiplication by 2^24, an accumulator is multiplied by 2^-48 where it is added to the sum: bfloat16 ends at 2^-133 as float32 does
+// at 2^-149, so that without it numbers below 2^-110 would lose digits.  With it every float32 below 2^104 is split exactly.
+// Larger ones, accumulators above 2^80 and infinities do not give a number this way (an infinity's parts are infinities and
+// NaN): a sum that is not finite is taken again, as plain float32 multiply-adds of the operands (plain_dot), so that
+// large numbers keep their value and infinities come out where arithmetic gives them.
 #include "common.cuh"
 
 KLLM_EXPORT_LAST_ERROR(gemm_f32_tcgen05)
@@ -68,11 +70,13 @@ __device__ __forceinline__ uint64_t make_desc64(unsigned addr) {
     return d;
 }
 
-// two numbers into their three bfloat16 parts.  The first part is taken of the number clamped
-// to the largest bfloat16, so that a finite number never becomes an infinity.
+constexpr float SCALE = 16777216.f, UNSCALE = 1.f / (SCALE * SCALE);       // 2^24, 2^-48: multiplied exactly
+
+// two numbers, scaled, into their three bfloat16 parts
 __device__ __forceinline__ void split2(float a, float b, uint32_t& p0, uint32_t& p1, uint32_t& p2) {
-    constexpr float TOP = 3.3895313892515355e38f;
-    p0 = pack_bf16(fminf(fmaxf(a, -TOP), TOP), fminf(fmaxf(b, -TOP), TOP));
+    a *= SCALE;
+    b *= SCALE;
+    p0 = pack_bf16(a, b);
     const float ra = a - __uint_as_float(p0 << 16), rb = b - __uint_as_float(p0 & 0xffff0000u);
     p1 = pack_bf16(ra, rb);
     p2 = pack_bf16(ra - __uint_as_float(p1 << 16), rb - __uint_as_float(p1 & 0xffff0000u));
@@ -104,17 +108,32 @@ __global__ void split_kernel(const float* __restrict__ src, const float* __restr
     }
 }
 
-// x . w as float32 multiply-adds in the order of k, for the few elements whose six products did not add up to a number
-// (an operand that is not finite, an overflow).  Ends at a NaN, which stays one.
+__device__ __forceinline__ bool is_nan(float v) { return v != v; }
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// x . w as float32 multiply-adds by the 32 lanes of a warp (the same arguments in all of them), for the few elements whose
+// six products did not add up to a number (an operand that is not finite or too large, an overflow).  Ends at a NaN,
+// which stays one.  A row of 2560 sums over 2048 of k takes 0.3 ms this way; a lane that sums alone took 4.
 __device__ __noinline__ float plain_dot(const float* __restrict__ x, const float* __restrict__ w, int K) {
+    const int lane = threadIdx.x & 31;
     float s = 0.f;
-    for (int k = 0; k < K && s == s; k += 4) {                                          // K is a multiple of 4
-        const float4 u = *reinterpret_cast<const float4*>(x + k), v = *reinterpret_cast<const float4*>(w + k);
-        s = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, s))));
+    for (int k0 = 4 * lane; k0 - 4 * lane < K; k0 += 512) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = k0 + 128 * q;
+            if (k < K) {                                                                // K is a multiple of 4
+                const float4 u = *reinterpret_cast<const float4*>(x + k), v = *reinterpret_cast<const float4*>(w + k);
+                t = fmaf(u.w, v.w, fmaf(u.z, v.z, fmaf(u.y, v.y, fmaf(u.x, v.x, t))));
+            }
+        }
+        s += t;
+        if (__any_sync(0xffffffffu, is_nan(s))) break;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
 }
-__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
 
 struct Args {
     const float *x, *w, *w_up;              // the operands themselves (w: of the piece)
@@ -261,28 +280,38 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tmem_ld32(t + (EPI == EPI_SWIGLU ? (c >> 1) * 128 + half * 64 + (c & 1) * 32 : half * 128 + c * 32), v);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; j++) sum[c][j] += v[j];
+                    for (int j = 0; j < 32; j++) sum[c][j] = fmaf(v[j], UNSCALE, sum[c][j]);      // one rounding, as the add
                 }
                 tc_fence_before();
                 mbar_arrive(&bar_acc_empty[acc]);
                 acc ^= 1;
                 if (acc == 0) acc_ph ^= 1u;
             }
+            ok = __all_sync(0xffffffffu, ok);                       // the warp leaves together or stays for its votes below
             if (!ok) break;
             const int r = m0 + quarter * 32 + lane;
+            constexpr int CH = EPI == EPI_SWIGLU ? 2 : 4;
+            unsigned odd[CH] = {};                                  // columns whose sum is not finite: taken again below
             if (r < a.M) {
                 float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (int64_t)r * a.ldy;
-                constexpr int CH = EPI == EPI_SWIGLU ? 2 : 4;
-                unsigned odd[CH];                                   // columns whose sum is not finite: taken again below
+                if constexpr (EPI != EPI_PARTIAL) {
+                    unsigned any = 0;
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    odd[c] = 0;
-                    if constexpr (EPI != EPI_PARTIAL) {
+                    for (int c = 0; c < CH; c++) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) {
-                            const bool ok_sum = finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]));
-                            odd[c] |= (unsigned)!ok_sum << j;
-                            if (EPI == EPI_ADD && !ok_sum) sum[c][j] = 0.f;
+                        for (int j = 0; j < 32; j++)
+                            odd[c] |= (unsigned)!(finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]))) << j;
+                        any |= odd[c];
+                    }
+                    if (any != 0) {
+                        const bool stays = is_nan(a.x[r * a.ldx]);              // a row of NaN, the common case, needs no second look
+#pragma unroll
+                        for (int c = 0; c < CH; c++) {
+                            if (stays) odd[c] = 0;
+                            if (EPI == EPI_ADD)
+#pragma unroll
+                                for (int j = 0; j < 32; j++)
+                                    if (odd[c] >> j & 1) sum[c][j] = 0.f;
                         }
                     }
                 }
@@ -310,17 +339,22 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                         }
                     }
                 }
-                if constexpr (EPI != EPI_PARTIAL) {
+            }
+            if constexpr (EPI != EPI_PARTIAL) {
+                __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < CH; c++) {
-                        const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
-                        for (unsigned left = odd[c]; left != 0; left &= left - 1) {
+                for (int c = 0; c < CH; c++) {
+                    const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
+                    for (unsigned rows = __ballot_sync(0xffffffffu, odd[c] != 0); rows != 0; rows &= rows - 1) {
+                        const int of = __ffs(rows) - 1, row = m0 + quarter * 32 + of;
+                        const float* xr = a.x + row * a.ldx;
+                        for (unsigned left = __shfl_sync(0xffffffffu, odd[c], of); left != 0; left &= left - 1) {
                             const int j = col + __ffs(left) - 1;
                             if (j >= a.N) break;                    // the tile's columns beyond the matrix
-                            const float* xr = a.x + r * a.ldx;
-                            const float v = plain_dot(xr, a.w + j * a.ldw, a.K);
-                            if (EPI == EPI_SWIGLU) y[j] = silu_mul(v, plain_dot(xr, a.w_up + j * a.ldw, a.K));
-                            else y[j] = EPI == EPI_ADD ? y[j] + v : v;
+                            float v = plain_dot(xr, a.w + j * a.ldw, a.K);
+                            if (EPI == EPI_SWIGLU) v = silu_mul(v, plain_dot(xr, a.w_up + j * a.ldw, a.K));
+                            float* e = a.y + row * a.ldy + j;
+                            if (lane == of) *e = EPI == EPI_ADD ? *e + v : v;
                         }
                     }
                 }
@@ -340,10 +374,13 @@ __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const f
                                      int M, int N, int splits, const Args a) {
     griddep_launch();
     griddep_wait();
-    const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? 2 * N : N;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)M * n4; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / n4;
+    const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? 2 * N : N, lane = threadIdx.x & 31;
+    const int64_t total = (int64_t)M * n4;
+    // whole warps walk the elements: a sum that is not finite is taken again by all lanes
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < total; i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + lane, r = i / n4;
         const int c = (int)(i - r * n4) * 4;
+        const bool mine = i < total;
         auto sum = [&](const float* p) {
             float4 v = *reinterpret_cast<const float4*>(p);
             for (int s = 1; s < splits; s++) {
@@ -352,21 +389,31 @@ __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const f
             }
             return v;
         };
-        auto again = [&](float4& v, const float* w) {                    // the sums that are not finite, from the operands
+        auto again = [&](float4& v, const float* w) {
             float* e = &v.x;
+            const bool look = mine && !(finite(v.x) && finite(v.y) && finite(v.z) && finite(v.w)) && !is_nan(a.x[r * a.ldx]);
 #pragma unroll
             for (int j = 0; j < 4; j++)
-                if (!finite(e[j])) e[j] = plain_dot(a.x + r * a.ldx, w + (c + j) * a.ldw, a.K);
+                for (unsigned odd = __ballot_sync(0xffffffffu, look && !finite(e[j])); odd != 0; odd &= odd - 1) {
+                    const int of = __ffs(odd) - 1;
+                    const float d = plain_dot(a.x + __shfl_sync(0xffffffffu, r, of) * a.ldx,
+                                                    w + (__shfl_sync(0xffffffffu, c, of) + j) * a.ldw, a.K);
+                    if (lane == of) e[j] = d;
+                }
         };
-        float4 v = sum(ws + r * ldw + c);
+        float4 v = mine ? sum(ws + r * ldw + c) : make_float4(0.f, 0.f, 0.f, 0.f);
         again(v, a.w);
+        float4 u = v;
+        if (EPI == EPI_SWIGLU) {
+            if (mine) u = sum(ws + r * ldw + N + c);
+            again(u, a.w_up);
+        }
+        if (!mine) continue;
         float4* o = reinterpret_cast<float4*>(y + r * ldy + c);
         if (EPI == EPI_ADD) {
             const float4 h = *o;
             v.x += h.x; v.y += h.y; v.z += h.z; v.w += h.w;
         } else if (EPI == EPI_SWIGLU) {
-            float4 u = sum(ws + r * ldw + N + c);
-            again(u, a.w_up);
             v.x = silu_mul(v.x, u.x); v.y = silu_mul(v.y, u.y); v.z = silu_mul(v.z, u.z); v.w = silu_mul(v.w, u.w);
         }
         *o = v;

@@ -63,6 +63,22 @@ def test_large_and_non_finite_numbers():
     assert torch.equal(y[keep], x[keep])
 
 
+@pytest.mark.parametrize("rows,cols,k", [(40, 260, 64), (64, 2560, 2048)])
+@pytest.mark.parametrize("scale", [2.0 ** -125, 2.0 ** -113, 2.0 ** -107, 2.0 ** 70, 2.0 ** 98])
+def test_full_mantissas_of_any_size(rows, cols, k, scale):
+    """Operands of every size with full mantissas, their partners such that the results are of ordinary size."""
+    from kllm_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(int(k + cols))
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").clamp(-8, 8)
+    x, w = rnd(rows, k) * scale, rnd(cols, k)
+    partner = min(1.0 / scale, 2.0 ** 100)                    # below 2^104, where numbers are split
+    for a, b in ((x, w), (x, w * partner), (rnd(rows, k) * partner, rnd(cols, k) * scale)):
+        want = a.double() @ b.double().T
+        rms = want.square().mean().sqrt()
+        # results that are subnormal are rounded to multiples of 2^-149 (the sums of several ranges of k one by one)
+        assert ((kernels.gemm_f32(a, b).double() - want).abs().max() - 16 * 2.0 ** -149) <= _bound(k) * rms
+
+
 @pytest.mark.parametrize("epilogue", ["f32", "add", "swiglu"])
 @pytest.mark.parametrize("rows,cols,k", [(40, 260, 64), (64, 2560, 2048), (300, 1028, 52)])
 def test_infinities(rows, cols, k, epilogue):
