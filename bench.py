@@ -434,7 +434,7 @@ def main():
                "frac": round(flops / (ms * 1e-3) / (pk["bf16_tflops"] * 1e12), 4),
                "spread_ms": [round(min(times), 3), round(max(times), 3)]}
         if eng.dtype != torch.bfloat16:
-            out["frac_of"] = "bf16 tensor peak (the float32 path does not use tensor cores)"
+            out["frac_of"] = "bf16 tensor peak (a float32 product on the tensor cores is six bf16 products)"
         return out
 
     def roofline(eng, run, batch):

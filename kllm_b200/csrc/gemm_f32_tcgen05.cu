@@ -523,6 +523,15 @@ extern "C" int kllm_gemm_f32_tcgen05_workspace(int M, int N, int K, int epilogue
     return 0;
 }
 
+// How the product of these sizes is cut: output columns of a piece of W (the last piece takes the rest), ranges of k.
+extern "C" int kllm_gemm_f32_tcgen05_plan(int M, int N, int K, int epilogue, int* piece, int* splits) {
+    if (M <= 0 || N <= 0 || K <= 0) { *piece = *splits = 0; return 0; }
+    const Plan p = make_plan(M, N, K, epilogue);
+    *piece = p.piece;
+    *splits = p.splits;
+    return 0;
+}
+
 // 1 if the kernel takes these sizes and addresses, else 0.
 extern "C" int kllm_gemm_f32_tcgen05_fits(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* w_up, int M,
                                           int N, int K, const void* y, int64_t ldy, int epilogue) {

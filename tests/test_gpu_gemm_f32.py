@@ -1,5 +1,7 @@
 """The float32 product on the tensor cores (csrc/gemm_f32_tcgen05.cu) against float64, at the edges of its tiles (128
 rows, 256 columns, k blocks of 32), with and without splits of K, in one piece of W and in several."""
+import ctypes
+
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -9,7 +11,15 @@ pytestmark = pytest.mark.gpu
 SIZES = [  # rows, columns, k
     (1, 4, 4), (33, 256, 32), (127, 252, 36), (128, 260, 60), (129, 512, 100), (300, 1028, 2052), (33, 2560, 2048),
     (257, 4100, 160),
-    (131, 11264, 1100),       # W in pieces: its parts are larger than what stays in L2
+    (131, 11264, 1100),
+]
+
+# rows, columns, k, epilogue: columns of a piece of W whose parts stay in L2, and ranges of k.  A shorter last piece, pieces
+# with ranges of k, and the columns' offset in the result of each epilogue.
+CUTS = [
+    (131, 11264, 1100, "swiglu", 5632, 1), (1003, 5632, 2048, "swiglu", 2304, 1), (64, 5632, 2048, "swiglu", 3072, 6),
+    (128, 32000, 2048, "f32", 5632, 6), (128, 32000, 2048, "add", 5632, 6), (700, 12004, 2048, "f32", 6144, 1),
+    (700, 12004, 2048, "add", 6144, 1),
 ]
 
 
@@ -20,9 +30,7 @@ def _bound(K):
     return 5 * 2.0 ** -23 * (12.0 ** 0.5 + (K / 32.0) ** 0.5)
 
 
-@pytest.mark.parametrize("epilogue", ["f32", "add", "swiglu"])
-@pytest.mark.parametrize("rows,cols,k", SIZES)
-def test_float32_product(rows, cols, k, epilogue):
+def _product(rows, cols, k, epilogue):
     from kllm_b200 import kernels
     g = torch.Generator(device="cuda").manual_seed(rows * 7 + cols + k)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
@@ -48,6 +56,33 @@ def test_float32_product(rows, cols, k, epilogue):
     bad = (y.double() - want).abs() - slack
     assert bad.max() <= 0, f"{int((bad > 0).sum())} of {bad.numel()} beyond the bound, worst by {float(bad.max())}"
     assert int(kernels.status_word(y.device).item()) == 0
+
+
+@pytest.mark.parametrize("epilogue", ["f32", "add", "swiglu"])
+@pytest.mark.parametrize("rows,cols,k", SIZES)
+def test_float32_product(rows, cols, k, epilogue):
+    _product(rows, cols, k, epilogue)
+
+
+@pytest.mark.parametrize("rows,cols,k,epilogue,piece,splits", CUTS)
+def test_float32_product_in_pieces(rows, cols, k, epilogue, piece, splits):
+    from kllm_b200.csrc.build import load_library
+    cut = (ctypes.c_int * 2)()
+    load_library("gemm_f32_tcgen05").kllm_gemm_f32_tcgen05_plan(rows, cols, k, ("f32", "add", "swiglu").index(epilogue),
+                                                                ctypes.addressof(cut), ctypes.addressof(cut) + 4)
+    assert tuple(cut) == (piece, splits)
+    _product(rows, cols, k, epilogue)
+
+
+def test_sums_of_one_sign_do_not_drift():
+    """Every product positive and a long k: what the tensor core's accumulation cuts off stays within one block of k."""
+    from kllm_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(11)
+    x, w = (torch.rand(n, 16384, generator=g, device="cuda") for n in (64, 256))
+    want = x.double() @ w.double().T
+    # every block of 32 is short by less than 12 x 2^-23 of itself; the 512 rounded adds are a walk of 0.29 x 2^-23 a step
+    # at the sum's full size, sqrt(512 / 3) steps' worth over a growing sum: five deviations are 19 x 2^-23
+    assert ((kernels.gemm_f32(x, w).double() - want).abs() / want).max() <= (12 + 19) * 2.0 ** -23
 
 
 def test_large_and_non_finite_numbers():

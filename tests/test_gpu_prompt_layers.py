@@ -1,6 +1,6 @@
-"""A step with portions launched from one native call (csrc/prompt_layers.cu) against the same step launched part by
-part: the same kernels in the same order, so the caches and logits agree to the bit where the library picks the same
-product kernel, and within two ways of summing in any case."""
+"""A step with portions launched from native code (csrc/prompt_layers.cu) against the same step launched part by
+part: the same kernels and library products with the same arguments in the same order, so the caches and logits agree to
+the bit."""
 import random
 
 import pytest
@@ -53,10 +53,36 @@ def _run(name, step, native):
 def test_native_launches_agree(name, step):
     a, ka = _run(name, step, False)
     b, kb = _run(name, step, True)
-    # two orders of summing the same bfloat16 products differ by 7e-3 of the largest logit at most (tests/test_gpu_replay.py)
-    assert (a - b).abs().max() <= 1e-2 * a.abs().max()
+    assert torch.equal(a, b)
     for x, y in zip(ka, kb):
-        assert (x.float() - y.float()).abs().max() <= 2.0 ** -6 * x.float().abs().max()
+        assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["d64", "d128"])
+def test_native_launches_agree_behind_long_contexts(name, monkeypatch):
+    """Single tokens whose contexts are cut into ranges (the scratch of partial results and their merge), and a portion
+    behind a context of its own."""
+    from kllm_b200 import Engine, Options, StepEntry, kernels
+    cuts = []
+    rule = kernels.decode_splits
+    monkeypatch.setattr(kernels, "decode_splits", lambda *a: (cuts.append(rule(*a)), cuts[-1])[1])
+    out = []
+    for native in (False, True):
+        engine = Engine(None, Options(max_seq=1600, block_size=64, num_blocks=120, max_batch=4, max_step_tokens=1500, dtype="bfloat16"),
+                        config=dict(_config(name), max_position_embeddings=2048), random_seed=3)
+        if not native:
+            engine.model.prompt_layers = None
+        rng = random.Random(7)
+        requests = [engine.cache.open() for _ in range(3)]
+        for r, n in zip(requests, (1400, 700, 900)):
+            engine.step([StepEntry(r, [rng.randrange(512) for _ in range(n)])])
+        del cuts[:]
+        logits = engine.step([StepEntry(r, [rng.randrange(512) for _ in range(n)], [n - 1]) for r, n in zip(requests, (1, 1, 40))])
+        out.append([logits.clone()] + [t.clone() for t in engine.cache.groups[0].k_store + engine.cache.groups[0].v_store])
+        assert cuts and min(cuts) > 1
+        engine.close()
+    for x, y in zip(*out):
+        assert torch.equal(x, y)
 
 
 def test_steps_that_stay_with_the_parts():
@@ -97,7 +123,7 @@ def test_wide_step_takes_the_gated_product():
                     kernels.launches - before))
         engine.close()
     (a, la), (b, lb) = out
-    assert (a - b).abs().max() <= 1e-2 * a.abs().max()
+    assert torch.equal(a, b)
     assert la == lb                                   # the same kernels
 
 
