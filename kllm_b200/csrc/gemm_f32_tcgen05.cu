@@ -295,24 +295,21 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (r < a.M) {
                 float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (int64_t)r * a.ldy;
                 if constexpr (EPI != EPI_PARTIAL) {
-                    unsigned any = 0;
+                    float zero[4] = {};                             // 0 times every sum: NaN where one is not finite
 #pragma unroll
-                    for (int c = 0; c < CH; c++) {
+                    for (int c = 0; c < 4; c++)
 #pragma unroll
-                        for (int j = 0; j < 32; j++)
-                            odd[c] |= (unsigned)!(finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]))) << j;
-                        any |= odd[c];
-                    }
-                    if (any != 0) {
-                        const bool stays = is_nan(a.x[r * a.ldx]);              // a row of NaN, the common case, needs no second look
+                        for (int j = 0; j < 32; j++) zero[j & 3] = fmaf(sum[c][j], 0.f, zero[j & 3]);
+                    // a row of NaN, the common case, needs no second look
+                    if (is_nan((zero[0] + zero[1]) + (zero[2] + zero[3])) && !is_nan(a.x[r * a.ldx])) {
 #pragma unroll
-                        for (int c = 0; c < CH; c++) {
-                            if (stays) odd[c] = 0;
-                            if (EPI == EPI_ADD)
+                        for (int c = 0; c < CH; c++)
 #pragma unroll
-                                for (int j = 0; j < 32; j++)
-                                    if (odd[c] >> j & 1) sum[c][j] = 0.f;
-                        }
+                            for (int j = 0; j < 32; j++) {
+                                const bool good = finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]));
+                                odd[c] |= (unsigned)!good << j;
+                                if (EPI == EPI_ADD && !good) sum[c][j] = 0.f;
+                            }
                     }
                 }
 #pragma unroll
