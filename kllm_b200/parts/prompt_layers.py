@@ -24,7 +24,7 @@ import torch
 # Passes that find the GPU idle, in turn (us, median [quartiles] of 20, this way / parts): TinyLlama's sizes, 300 tokens
 # (0.26e11) 2166 [2155 2179] / 3635 [3613 3660], 1200 (1.06e11) 3607 [3594 3633] / 3664 [3639 3705], 1704 (1.5e11) 4949
 # [4892 5005] / 4985 [4901 5082] and 4871 [4837 4935] / 4828 [4802 4932], 2048 (1.8e11) 5479 [5436 5518] / 5449
-# [5424 5471]; eight Llama-2-7B layers, 24 tokens and 450 of prompts (2.2e11) 3634 [3595 3675] / 3582 [3542 3632].
+# [5424 5471]; eight Llama-2-7B layers, 24 tokens and 525 of prompts (2.2e11) 3634 [3595 3675] / 3582 [3542 3632].
 MOST_WORK = 1.5e11
 
 
