@@ -389,6 +389,7 @@ __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const f
         auto again = [&](float4& v, const float* w) {
             float* e = &v.x;
             const bool look = mine && !(finite(v.x) && finite(v.y) && finite(v.z) && finite(v.w)) && !is_nan(a.x[r * a.ldx]);
+            if (!__any_sync(0xffffffffu, look)) return;
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 for (unsigned odd = __ballot_sync(0xffffffffu, look && !finite(e[j])); odd != 0; odd &= odd - 1) {
