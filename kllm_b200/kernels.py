@@ -663,7 +663,7 @@ def decode_splits(n_tokens: int, n_kv: int, ctx_bound: int, head_dim: int = 128)
 
       - short contexts are not cut.  Few pairs: 1 x 4 of size 64 at 200 1: 4.6, 4: 5.9, at 512 1: 7.6, 8: 6.1; 1 x 8 of size
         128 at 200 1: 6.1, 4: 6.3, at 300 1: 7.1, 5: 6.5, at 512 1: 9.9, 8: 6.4; 1 x 8 of size 256 at 100 1: 6.4, 2: 8.1, at
-        200 1: 9.2, 4: 8.4.  More pairs: 16 x 4 of size 64 at 300 1: 5.5, 3: 7.1; 8 x 8 of 128 at 300 1: 7.3, 3: 8.2, at 512
+        200 1: 9.2, 4: 8.4, at 300 1: 10.9, 5: 10.3 (the bound is seldom reached: the line stays at 4 tiles).  More pairs: 16 x 4 of size 64 at 300 1: 5.5, 3: 7.1; 8 x 8 of 128 at 300 1: 7.3, 3: 8.2, at 512
         1: 10.4, 4: 9.4; 24 x 4 of 64 at 512 1: 8.3, 3: 8.7; 16 x 8 of 128 at 512 1: 11.7, 2: 13.2.  At size 64 and up to 64
         pairs the line is drawn by whole decode steps, in which the ranges' CTAs also ask for the next matrix
         (22 layers, 8 x 4 at 300 1: 773, 5: 732; 16 x 4 at 400 1: 999, 4: 947; 8 x 4 under a bound of 256, at 60 1: 698,
@@ -682,7 +682,7 @@ def decode_splits(n_tokens: int, n_kv: int, ctx_bound: int, head_dim: int = 128)
     elif head_dim == 128:
         uncut = 4 if base <= 16 else 5
     else:
-        uncut = 3 if base <= 16 else 8
+        uncut = 4 if base <= 16 else 8
     if tiles <= (uncut if base <= 64 else 8):
         return 1
     splits = max(1, min(2 * sms // base, tiles, 16))

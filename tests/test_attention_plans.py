@@ -36,7 +36,7 @@ def test_which_form_a_step_takes(monkeypatch):
 SPLITS = [
     (1, 4, 256, 64, 1), (1, 4, 512, 64, 8), (8, 4, 300, 64, 5), (16, 4, 300, 64, 1), (16, 4, 400, 64, 4), (24, 4, 512, 64, 1),
     (1, 8, 200, 128, 1), (1, 8, 300, 128, 5), (8, 8, 300, 128, 1), (8, 8, 512, 128, 4), (16, 8, 512, 128, 1),
-    (1, 8, 100, 256, 1), (1, 8, 200, 256, 4), (8, 8, 512, 256, 1),
+    (1, 8, 100, 256, 1), (1, 8, 256, 256, 1), (1, 8, 300, 256, 5), (8, 8, 512, 256, 1),
     (64, 8, 1280, 128, 1), (24, 32, 1500, 128, 1), (64, 4, 2000, 64, 2), (16, 32, 2000, 64, 1), (24, 32, 2000, 64, 2),
     (24, 8, 2000, 256, 2), (32, 8, 2000, 256, 1), (8, 4, 2048, 64, 8), (1, 8, 8000, 128, 16),
 ]
