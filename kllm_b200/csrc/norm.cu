@@ -10,6 +10,8 @@
 // Formula: reference backend/model.cu:101-122 (norm) and :144-165 (sum + norm).
 #include "common.cuh"
 
+#include <type_traits>
+
 KLLM_EXPORT_LAST_ERROR(norm)
 
 namespace {
@@ -52,113 +54,78 @@ add_rmsnorm_kernel(float* __restrict__ x, const R* __restrict__ res, T* __restri
     }
 }
 
-// The common case of a step's rows (every row, float32 residual or none, bfloat16 out,
-// width a multiple of 4 up to kThreads * 4 * kVec) in one pass: a thread keeps its
-// elements in registers between the sum of squares and the scaling, 16-byte accesses.
-// Same sums in the same order as the kernel above: thread k adds its elements i = k,
-// k + kThreads, ... in that order (here four neighbours at a time, whose squares are
-// added first; a rounding may differ from the scalar kernel's).
-constexpr int kVec = 8;
-
-__global__ void __launch_bounds__(kThreads)
-add_rmsnorm_vec4_kernel(float* __restrict__ x, const float* __restrict__ res, bf16* __restrict__ out,
-                        const float* __restrict__ gain, int d, float eps) {
-    __shared__ float red[32];
-    griddep_wait();
-    griddep_launch();
-    const int r = blockIdx.x;
-    float4* xr = reinterpret_cast<float4*>(x + (int64_t)r * d);
-    const float4* rr = res ? reinterpret_cast<const float4*>(res + (int64_t)r * d) : nullptr;
-    const float4* g4 = reinterpret_cast<const float4*>(gain);
-    const int n4 = d >> 2;
-    float4 v[kVec];
-    float ss = 0.f;
-#pragma unroll
-    for (int k = 0; k < kVec; k++) {
-        const int i = threadIdx.x + k * kThreads;
-        if (i < n4) {
-            v[k] = xr[i];
-            if (rr) {
-                const float4 a = rr[i];
-                v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
-                xr[i] = v[k];
-            }
-            ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-        }
-    }
-    ss = block_sum(ss, red);
-    const float scale = rsqrtf(ss / (float)d + eps);
-    uint2* orow = reinterpret_cast<uint2*>(out + (int64_t)r * d);
-#pragma unroll
-    for (int k = 0; k < kVec; k++) {
-        const int i = threadIdx.x + k * kThreads;
-        if (i < n4) {
-            const float4 g = g4[i];
-            __nv_bfloat162 lo = __floats2bfloat162_rn(v[k].x * scale * g.x, v[k].y * scale * g.y);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(v[k].z * scale * g.z, v[k].w * scale * g.w);
-            uint2 pk;
-            pk.x = *reinterpret_cast<uint32_t*>(&lo);
-            pk.y = *reinterpret_cast<uint32_t*>(&hi);
-            orow[i] = pk;
-        }
-    }
+// four neighbouring elements of a row, stored at once
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    uint2 pk;
+    pk.x = *reinterpret_cast<uint32_t*>(&lo);
+    pk.y = *reinterpret_cast<uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(p) = pk;
+}
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 
-// One warp per row, the row in registers, no block-wide synchronisation; 8 rows per CTA.
-// Width a multiple of 4 up to 32 * 4 * kWarpVec.  Lane l adds the squares of its float4 l,
-// l + 32, ... in that order, then the lanes are added in a fixed tree.  Which of the two
-// vectorised kernels runs is decided by the width alone, never by the number of rows, so
-// a row is summed in the same order whatever else the step holds.
-constexpr int kWarpVec = 16;
+// The widths that are multiples of 4 up to kThreads * 4 * kVec, 16-byte rows: a thread keeps its V float4 of the row in
+// registers between the sum of squares and the scaling.  One CTA per row and as many threads as the row has float4, up to
+// kThreads, so that all of a row's loads are in flight at once: a row's latency is what a step of few rows waits for, and a
+// step of many is bound by its bytes either way.  In a decode step of 64 rows of 2048 a warp per row took 4.2 us, this takes
+// 2.4; the gains do not depend on the kernel before and are fetched while it ends.  V and the block's size follow from the
+// width alone, so a row is summed in the same order whatever else the step holds.
+constexpr int kVec = 8;
 
-__global__ void __launch_bounds__(256)
-add_rmsnorm_warp_kernel(float* __restrict__ x, const float* __restrict__ res, bf16* __restrict__ out,
-                        const float* __restrict__ gain, int n_rows, int d, float eps) {
+__host__ __device__ constexpr int row_threads(int d) { return d / 4 >= kThreads ? kThreads : (d / 4 + 31) / 32 * 32; }
+
+template <typename T, int V>
+__global__ void __launch_bounds__(kThreads)
+add_rmsnorm_row_kernel(float* __restrict__ x, const float* __restrict__ res, T* __restrict__ out,
+                       const float* __restrict__ gain, const int* __restrict__ rows, int d, float eps) {
+    __shared__ float red[32];
+    const int n4 = d >> 2;
+    float4 g[V], v[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) g[k] = load4(gain + 4 * i);
+    }
     griddep_wait();
     griddep_launch();
-    const int lane = threadIdx.x & 31;
-    const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (r >= n_rows) return;
-    float4* xr = reinterpret_cast<float4*>(x + (int64_t)r * d);
-    const float4* rr = res ? reinterpret_cast<const float4*>(res + (int64_t)r * d) : nullptr;
-    const float4* g4 = reinterpret_cast<const float4*>(gain);
-    const int n4 = d >> 2;
-    float4 v[kWarpVec];
+    const int64_t src = rows ? rows[blockIdx.x] : (int)blockIdx.x;
+    float* xr = x + src * d;
+    float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < kWarpVec; k++) {
-        const int i = lane + k * 32;
-        if (i < n4) v[k] = xr[i];
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) v[k] = load4(xr + 4 * i);
     }
-    if (rr) {
+    if (res) {
+        const float* rr = res + src * d;
 #pragma unroll
-        for (int k = 0; k < kWarpVec; k++) {
-            const int i = lane + k * 32;
+        for (int k = 0; k < V; k++) {
+            const int i = threadIdx.x + k * blockDim.x;
             if (i < n4) {
-                const float4 a = rr[i];
+                const float4 a = load4(rr + 4 * i);
                 v[k].x += a.x; v[k].y += a.y; v[k].z += a.z; v[k].w += a.w;
-                xr[i] = v[k];
+                if (!rows) store4(xr + 4 * i, v[k]);
             }
         }
     }
-    float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < kWarpVec; k++)
-        if (lane + k * 32 < n4) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-    ss = warp_sum(ss);
-    const float scale = rsqrtf(ss / (float)d + eps);
-    uint2* orow = reinterpret_cast<uint2*>(out + (int64_t)r * d);
+    for (int k = 0; k < V; k++)
+        if (threadIdx.x + k * blockDim.x < n4) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    const float scale = rsqrtf(block_sum(ss, red) / (float)d + eps);
+    T* orow = out + (int64_t)blockIdx.x * d;
 #pragma unroll
-    for (int k = 0; k < kWarpVec; k++) {
-        const int i = lane + k * 32;
-        if (i < n4) {
-            const float4 g = g4[i];
-            __nv_bfloat162 lo = __floats2bfloat162_rn(v[k].x * scale * g.x, v[k].y * scale * g.y);
-            __nv_bfloat162 hi = __floats2bfloat162_rn(v[k].z * scale * g.z, v[k].w * scale * g.w);
-            uint2 pk;
-            pk.x = *reinterpret_cast<uint32_t*>(&lo);
-            pk.y = *reinterpret_cast<uint32_t*>(&hi);
-            orow[i] = pk;
-        }
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4)
+            store4(orow + 4 * i, make_float4(v[k].x * scale * g[k].x, v[k].y * scale * g[k].y, v[k].z * scale * g[k].z,
+                                             v[k].w * scale * g[k].w));
     }
 }
 
@@ -197,6 +164,64 @@ rmsnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
     s2 = block_sum(s2, red);
     const float scale2 = rsqrtf(s2 / (float)d + eps2);
     for (int i = threadIdx.x; i < d; i += blockDim.x) orow[i] = from_f32<T>(xr[i] * scale2 * gain2[i]);
+}
+
+// The same with the row in registers (V float4 a thread; widths, threads and order as in add_rmsnorm_row_kernel).  Two rows
+// of 2048 in a decode step, beside the end of the product before: 9.8 us more with one element a load and three passes
+// through memory, 1.8 this way; 2017 rows 17 us and 8.2.
+template <typename T, int V>
+__global__ void __launch_bounds__(kThreads)
+rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ gain, float eps,
+                       T* __restrict__ out, const float* __restrict__ gain2, float eps2, int d) {
+    __shared__ float red[32];
+    const int n4 = d >> 2;
+    float4 g[V], v[V], h[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) g[k] = load4(gain + 4 * i);
+    }
+    griddep_wait();
+    griddep_launch();
+    float* xr = x + (int64_t)blockIdx.x * d;
+    const float* yr = y + (int64_t)blockIdx.x * d;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) {
+            v[k] = load4(yr + 4 * i);
+            h[k] = load4(xr + 4 * i);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < V; k++)
+        if (threadIdx.x + k * blockDim.x < n4) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    const float scale = rsqrtf(block_sum(ss, red) / (float)d + eps);
+    T* orow = out ? out + (int64_t)blockIdx.x * d : nullptr;
+    float s2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) {
+            h[k].x += v[k].x * scale * g[k].x; h[k].y += v[k].y * scale * g[k].y;
+            h[k].z += v[k].z * scale * g[k].z; h[k].w += v[k].w * scale * g[k].w;
+            store4(xr + 4 * i, h[k]);
+            if (orow && !gain2) store4(orow + 4 * i, h[k]);
+            s2 += (h[k].x * h[k].x + h[k].y * h[k].y) + (h[k].z * h[k].z + h[k].w * h[k].w);
+        }
+    }
+    if (!orow || !gain2) return;
+    const float scale2 = rsqrtf(block_sum(s2, red) / (float)d + eps2);
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) {
+            const float4 b = load4(gain2 + 4 * i);
+            store4(orow + 4 * i, make_float4(h[k].x * scale2 * b.x, h[k].y * scale2 * b.y, h[k].z * scale2 * b.z,
+                                             h[k].w * scale2 * b.w));
+        }
+    }
 }
 
 // Layer norm with gain and an optional bias, the residual sum folded in as in add_rmsnorm_kernel:
@@ -311,23 +336,6 @@ add_layernorm_vec4_kernel(float* __restrict__ x, const float* __restrict__ res, 
             }
         }
     }
-}
-
-// four neighbouring elements of a row, stored at once
-__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-__device__ __forceinline__ void store4(bf16* p, float4 v) {
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 pk;
-    pk.x = *reinterpret_cast<uint32_t*>(&lo);
-    pk.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(p) = pk;
-}
-__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-    return make_float4(a.x, a.y, b.x, b.y);
 }
 
 // Layer norm of a row y whose result joins or becomes the residual stream, one CTA per row:
@@ -466,6 +474,24 @@ extern "C" int kllm_embed_layernorm(float* x, const void* table, const int* ids,
     KLLM_FAIL("embed_layernorm: unknown element type %d", table_dtype);
 }
 
+namespace {
+// Widths and addresses (NULL counts as aligned) that the kernels with the row in registers take.
+template <typename... P>
+bool rows_fit(int d, P... p) {
+    const uintptr_t addr = ((uintptr_t)p | ...);
+    return (d & 3) == 0 && d <= kThreads * 4 * kVec && !(addr & 15);
+}
+// go(integral_constant<int, V>) with the V of a width: 1, 2, 4 or 8 float4 a thread
+template <typename F>
+void by_width(int d, F go) {
+    const int need = (d / 4 + row_threads(d) - 1) / row_threads(d);
+    if (need <= 1) go(std::integral_constant<int, 1>());
+    else if (need <= 2) go(std::integral_constant<int, 2>());
+    else if (need <= 4) go(std::integral_constant<int, 4>());
+    else go(std::integral_constant<int, 8>());
+}
+}  // namespace
+
 // x float32 [n][d] (updated), y float32 [n][d], gain float32 [d]; out (optional, element type
 // `dtype`) [n][d] with gain2 [d]; gain2 NULL: out gets the updated rows as they are, in its element type.
 extern "C" int kllm_rmsnorm_add(void* x, const void* y, const void* gain, float eps, void* out, const void* gain2,
@@ -473,15 +499,24 @@ extern "C" int kllm_rmsnorm_add(void* x, const void* y, const void* gain, float 
     if (n_rows <= 0) return 0;
     if (d <= 0) KLLM_FAIL("rmsnorm_add: width %d must be positive", d);
     cudaStream_t s = (cudaStream_t)stream;
+    if (dtype != KLLM_F32 && dtype != KLLM_BF16) KLLM_FAIL("rmsnorm_add: unknown element type %d", dtype);
+    if (rows_fit(d, x, y, gain, out, gain2)) {
+        auto go = [&](auto element, auto size) {
+            using T = decltype(element);
+            kllm_launch((rmsnorm_add_row_kernel<T, decltype(size)::value>), dim3(n_rows), dim3(row_threads(d)), 0, s, (float*)x,
+                        (const float*)y, (const float*)gain, eps, (T*)out, (const float*)gain2, eps2, d);
+        };
+        if (dtype == KLLM_F32) by_width(d, [&](auto size) { go(float(), size); });
+        else by_width(d, [&](auto size) { go(bf16(), size); });
+        KLLM_LAUNCH_STATUS();
+    }
     const int threads = d <= 512 ? 64 : (d <= 2048 ? 128 : kThreads);
     if (dtype == KLLM_F32)
         kllm_launch((rmsnorm_add_kernel<float>), dim3(n_rows), dim3(threads), 0, s, (float*)x, (const float*)y,
                     (const float*)gain, eps, (float*)out, (const float*)gain2, eps2, d);
-    else if (dtype == KLLM_BF16)
+    else
         kllm_launch((rmsnorm_add_kernel<bf16>), dim3(n_rows), dim3(threads), 0, s, (float*)x, (const float*)y,
                     (const float*)gain, eps, (bf16*)out, (const float*)gain2, eps2, d);
-    else
-        KLLM_FAIL("rmsnorm_add: unknown element type %d", dtype);
     KLLM_LAUNCH_STATUS();
 }
 
@@ -492,16 +527,14 @@ extern "C" int kllm_add_rmsnorm(void* x, const void* res, void* out, const void*
     if (n_rows <= 0) return 0;
     if (d <= 0) KLLM_FAIL("rmsnorm: width %d must be positive", d);
     cudaStream_t s = (cudaStream_t)stream;
-    auto aligned = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    if (dtype == KLLM_BF16 && (res == nullptr || res_dtype == KLLM_F32) && rows == nullptr && (d & 3) == 0 &&
-        d <= kThreads * 4 * kVec && aligned(x) && aligned(res) && aligned(gain) && ((uintptr_t)out & 7) == 0) {
-        if (d <= 32 * 4 * kWarpVec) {
-            kllm_launch((add_rmsnorm_warp_kernel), dim3((n_rows + 7) / 8), dim3(256), 0, s, (float*)x, (const float*)res,
-                        (bf16*)out, (const float*)gain, n_rows, d, eps);
-            KLLM_LAUNCH_STATUS();
-        }
-        kllm_launch((add_rmsnorm_vec4_kernel), dim3(n_rows), dim3(kThreads), 0, s, (float*)x, (const float*)res, (bf16*)out,
-                    (const float*)gain, d, eps);
+    if ((dtype == KLLM_F32 || dtype == KLLM_BF16) && (res == nullptr || res_dtype == KLLM_F32) && rows_fit(d, x, res, gain, out)) {
+        auto go = [&](auto element, auto size) {
+            using T = decltype(element);
+            kllm_launch((add_rmsnorm_row_kernel<T, decltype(size)::value>), dim3(n_rows), dim3(row_threads(d)), 0, s, (float*)x,
+                        (const float*)res, (T*)out, (const float*)gain, rows, d, eps);
+        };
+        if (dtype == KLLM_F32) by_width(d, [&](auto size) { go(float(), size); });
+        else by_width(d, [&](auto size) { go(bf16(), size); });
         KLLM_LAUNCH_STATUS();
     }
     if (res == nullptr) res_dtype = dtype;

@@ -60,7 +60,7 @@ def test_embed_and_gather(dtype):
 
 @pytest.mark.parametrize("d", [2048, 200, 2052])
 def test_add_rmsnorm_of_many_rows(d):
-    """600 rows: widths up to 2048 take the kernel with a warp per row, wider ones the block per row."""
+    """600 rows, one CTA each."""
     from kllm_b200 import kernels
     rng = np.random.default_rng(d)
     n, eps = 600, 1e-5
@@ -73,6 +73,33 @@ def test_add_rmsnorm_of_many_rows(d):
     close(out, plain.rmsnorm(x0.astype(np.float64) + res, gain, eps), "bfloat16", "norm after the sum")
     kernels.add_rmsnorm(x, None, out, dev(gain), eps)
     close(out, plain.rmsnorm(x0.astype(np.float64) + res, gain, eps), "bfloat16", "norm alone")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("d", [4, 132, 1024, 1028, 2052, 4100, 8192, 8196])
+def test_norms_with_the_row_in_registers(dtype, d):
+    """Widths around every number of float4 a thread holds (1, 2, 4, 8), the smallest and largest of the kernels that keep
+    the row in registers, and the first one beyond: all rows, chosen rows, and the norm of a sublayer's output with what
+    follows it."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(d)
+    n, eps = 5, 1e-5
+    x0, y = ((rng.standard_normal((n, d)) * s).astype(np.float32) for s in (2, 1))
+    g1, g2 = ((1 + 0.2 * rng.standard_normal(d)).astype(np.float32) for _ in range(2))
+    x, out = dev(x0), torch.empty((n, d), dtype=DT[dtype], device="cuda")
+    kernels.add_rmsnorm(x, dev(y), out, dev(g1), eps)
+    close(x, x0.astype(np.float64) + y, "float32", "residual sum")
+    close(out, plain.rmsnorm(x0.astype(np.float64) + y, g1, eps), dtype, "norm after the sum")
+    x, rows = dev(x0), np.array([4, 0, 4], dtype=np.int32)
+    kernels.add_rmsnorm(x, dev(y), out[:3], dev(g1), eps, rows=dev(rows))
+    assert np.array_equal(x.cpu().numpy(), x0)
+    close(out[:3], plain.rmsnorm((x0.astype(np.float64) + y)[rows], g1, eps), dtype, "norm of chosen rows")
+    want = x0 + plain.rmsnorm(y.astype(np.float64), g1, eps)
+    for gain2 in (None, g2):
+        x = dev(x0)
+        kernels.rmsnorm_add(x, dev(y), dev(g1), eps, out=out, gain2=None if gain2 is None else dev(gain2), eps2=3e-4)
+        close(x, want, "float32", "the output's norm in the stream")
+        close(out, want if gain2 is None else plain.rmsnorm(want, gain2, 3e-4), dtype, "what the next sublayer reads")
 
 
 @pytest.mark.parametrize("d", [2048, 4096, 200])
