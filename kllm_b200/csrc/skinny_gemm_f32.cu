@@ -16,24 +16,30 @@
 //                         silu(gate row) * (up row) as float32 [n, F]
 //                         (backend/model.cu:477-483, :1112-1114)
 //
-// Layout of the work: a CTA of 16 warps, one per SM, keeps X in shared memory.  A tile is
-// eight weight rows (SWIGLU: four gate rows and their four up rows).  The warps of a CTA
-// are two row groups (four rows each) times eight k slices: a warp takes the k steps of
-// 128 elements of its slice, its lanes split a step in float4 pieces, so a lane's X values
-// (8 rows x float4, read once per k step) serve its four weight rows from registers.  Two
-// register buffers take turns, so the next step's (or the next tile's) weights are in
-// flight while this one's are multiplied.  The lanes' partial sums meet in a butterfly of
-// shuffles, the eight slices' sums in shared memory, added in slice order: every order is
-// fixed by K alone.
+// Layout of the work: a CTA of 16 warps, one per SM, walks tiles of eight weight rows (SWIGLU: four gate rows and their
+// four up rows).  A warp owns a contiguous sixteenth of K for every tile of its CTA: it brings that part of X (8 rows) into
+// shared memory for itself, and nothing waits for another warp until the CTA's tiles are through.  The norm's scale is a
+// factor of a whole row, so it multiplies the finished sums; the sums of squares are taken beside the products.  Within
+// a warp eight lanes share a weight row (128 bytes a load) and a lane has two of the tile's rows, so a batch of four steps
+// of 32 elements is eight 16-byte loads a lane; two register buffers take turns, 64 KB an SM in flight in each.  The products
+// are two-wide (fma.rn.f32x2 on neighbouring k: weights and X both lie in memory as such pairs).  A tile ends in three
+// exchanges between the eight lanes (14 shuffles) and a store of the warp's 64 partial sums; they are added in warp order,
+// for up to MAX_SLOTS tiles at a time.  Every order is fixed by K alone.
+//
+// Measured in a decode step of 8 rows of TinyLlama's sizes (B200; us beside what the kernel before hides): gate and up 23.4
+// (32.0 in the form that met in shared memory at every tile, with eight parts of K and four rows a warp), down 15.5, O 7.2
+// (22.7 together), QKV 12.6 (13.8).
 #include "common.cuh"
 
 KLLM_EXPORT_LAST_ERROR(skinny_gemm_f32)
 
 namespace {
 
-constexpr int THREADS = 512, WARPS = 16, ROWS = 8, WR = 4;      // X rows; weight rows per warp
-constexpr int KSLICES = 8, GROUPS = 2;                          // the 16 warps: k slices x row groups
-constexpr int UNROLL = 2;                                       // k steps of 128 per register buffer
+constexpr int THREADS = 512, WARPS = 16, ROWS = 8;              // ROWS: rows of X
+constexpr int TILE = 8, PARTS = TILE * ROWS;                    // weight rows of a tile; partial sums a warp leaves of one
+constexpr int STEP = 32, UNROLL = 4;                            // elements of k a step takes, steps a register buffer holds
+constexpr int MAX_SLOTS = 16;                                   // tiles whose partial sums are kept until they are added up
+constexpr size_t SMEM_MOST = 227 * 1024;
 enum { X_PLAIN = 0, X_NORM = 1 };
 enum { STORE = 0, ADD = 1, SWIGLU = 2 };
 
@@ -57,172 +63,211 @@ struct Args {
 #endif
 };
 
-__device__ __forceinline__ float4 ldg_stream(const float* p) {
-    float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];\n"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+// four neighbouring weights as two pairs
+__device__ __forceinline__ ulonglong2 ldg_stream(const float* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u64 {%0,%1}, [%2];\n" : "=l"(v.x), "=l"(v.y) : "l"(p));
     return v;
 }
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum2(unsigned long long v) {
+    return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
 
-template <int PRO, int EPI>
+// EXACT: every warp's part of K is a whole number of batches.
+template <int PRO, int EPI, bool EXACT>
 __global__ void __launch_bounds__(THREADS, 1)
-skinny_f32_kernel(const Args a) {
-    extern __shared__ __align__(16) float xs[];            // [ROWS][K]
-    __shared__ float ss_part[ROWS][2];
-    __shared__ float red[KSLICES * GROUPS * 32];           // per warp: its 4 rows x 8 tokens
+skinny_f32_kernel(const Args a, const int slots) {
+    extern __shared__ __align__(16) float xs[];            // [ROWS][K], then the partial sums [slots][WARPS][TILE][ROWS]
+    __shared__ float ss_part[WARPS][ROWS];
     const int K = a.K, N = a.N, n = a.n;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = warp & 1, ks = warp >> 1;
-    constexpr int OUT_PER_TILE = EPI == SWIGLU ? WR : GROUPS * WR;   // output columns of a tile
+    float* red = xs + (size_t)ROWS * K;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane >> 3, kl = lane & 7;
+    constexpr int OUT_PER_TILE = EPI == SWIGLU ? TILE / 2 : TILE;    // output columns of a tile
     const int n_tiles = (N + OUT_PER_TILE - 1) / OUT_PER_TILE;
-    const int steps = K / 128;
-    const int my_steps = steps > ks ? (steps - ks + KSLICES - 1) / KSLICES : 0;
-    const int nb = max(1, ((steps + KSLICES - 1) / KSLICES + UNROLL - 1) / UNROLL);   // batches per tile, same for all warps
+    const int steps = K / STEP, per_warp = (steps + WARPS - 1) / WARPS;
+    const int my_steps = max(0, min(per_warp, steps - warp * per_warp));
+    const int nb = (per_warp + UNROLL - 1) / UNROLL;                 // batches per tile, the same for all warps
+    const int k0 = warp * per_warp * STEP;                           // this warp's part of K: k0 .. k0 + my_steps * STEP
 
-    // this warp's four weight rows of a tile (rows past the end repeat the last one; their sums are not stored)
-    auto row_ptr = [&](int tile, int r) -> const float* {
-        if (EPI == SWIGLU) return (grp == 0 ? a.w : a.w_up) + (int64_t)min(tile * WR + r, N - 1) * a.w_stride + 4 * lane;
-        return a.w + (int64_t)min(tile * GROUPS * WR + grp * WR + r, N - 1) * a.w_stride + 4 * lane;
-    };
-    float4 buf0[UNROLL][WR], buf1[UNROLL][WR];
-    auto load_batch = [&](float4 (&buf)[UNROLL][WR], int tile, int b) {
-#pragma unroll
-        for (int u = 0; u < UNROLL; u++) {
-            const int i = b * UNROLL + u;
-            if (i < my_steps) {
-                const int off = (ks + i * KSLICES) * 128;
-#pragma unroll
-                for (int r = 0; r < WR; r++) buf[u][r] = ldg_stream(row_ptr(tile, r) + off);
-            }
+    // two register buffers: [step][0] a row of the tile's first four, [step][1] of its other four (SWIGLU: the up row)
+    ulonglong2 buf0[UNROLL][2], buf1[UNROLL][2];
+    auto load_batch = [&](ulonglong2 (&buf)[UNROLL][2], int tile, int b) {
+        const float *p0, *p1;                                        // rows past the end repeat the last one
+        if (EPI == SWIGLU) {
+            const int64_t r = min(tile * 4 + sub, N - 1);
+            p0 = a.w + r * a.w_stride;
+            p1 = a.w_up + r * a.w_stride;
+        } else {
+            p0 = a.w + (int64_t)min(tile * 8 + sub, N - 1) * a.w_stride;
+            p1 = a.w + (int64_t)min(tile * 8 + 4 + sub, N - 1) * a.w_stride;
         }
+        const int off = k0 + b * UNROLL * STEP + 4 * kl;
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++)
+            if (EXACT || b * UNROLL + u < my_steps) {
+                buf[u][0] = ldg_stream(p0 + off + u * STEP);
+                buf[u][1] = ldg_stream(p1 + off + u * STEP);
+            }
     };
-    int cur_tile = blockIdx.x, cur_b = 0;          // the batch that sits in the buffer used next
-    if (cur_tile < n_tiles) load_batch(buf0, cur_tile, 0);     // weights do not depend on X: on their way first
+    int cur_tile = blockIdx.x, cur_b = 0, slot = 0;        // the batch that sits in the buffer used next
+    load_batch(buf0, cur_tile, 0);                         // weights do not depend on X: on their way first
     griddep_wait();
     griddep_launch();
 
-    // ---- X into shared memory as float32, rows past n are zero ----
+    // ---- this warp's part of X into shared memory, rows past n are zero ----
     {
-        const int r = warp >> 1, half = warp & 1;                  // two warps share a row
-        const int span = K / 2, lo_k = half * span;                // K % 128 == 0: a multiple of 4
-        const bool live = r < n;
-        const float* src = live ? a.x + (int64_t)((PRO == X_NORM && a.rows) ? a.rows[r] : r) * a.x_stride : nullptr;
-        float* dst = xs + (size_t)r * K;
+        const int len = my_steps * STEP;
         if (PRO == X_NORM) {
-            float ss = 0.f;
-            if (live)
-                for (int k = lo_k + lane * 4; k < lo_k + span; k += 128) {
-                    const float4 v = __ldcg(reinterpret_cast<const float4*>(src + k));
-                    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            float ss[ROWS];
+#pragma unroll
+            for (int c = 0; c < ROWS; c++) ss[c] = 0.f;
+            for (int i = 4 * lane; i < len; i += 128) {
+                float4 v[ROWS];
+#pragma unroll
+                for (int c = 0; c < ROWS; c++)
+                    v[c] = c < n ? __ldcg(reinterpret_cast<const float4*>(a.x + (int64_t)(a.rows ? a.rows[c] : c) * a.x_stride + k0 + i))
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 g = __ldg(reinterpret_cast<const float4*>(a.gain + k0 + i));
+#pragma unroll
+                for (int c = 0; c < ROWS; c++) {
+                    ss[c] += (v[c].x * v[c].x + v[c].y * v[c].y) + (v[c].z * v[c].z + v[c].w * v[c].w);
+                    *reinterpret_cast<float4*>(xs + (size_t)c * K + k0 + i) =
+                        make_float4(v[c].x * g.x, v[c].y * g.y, v[c].z * g.z, v[c].w * g.w);
                 }
-            ss = warp_sum(ss);
-            if (lane == 0) ss_part[r][half] = ss;
-            __syncthreads();
-            const float scale = rsqrtf((ss_part[r][0] + ss_part[r][1]) / (float)K + a.eps);
-            for (int k = lo_k + lane * 4; k < lo_k + span; k += 128) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (live) {
-                    v = __ldcg(reinterpret_cast<const float4*>(src + k));
-                    const float4 g4 = __ldg(reinterpret_cast<const float4*>(a.gain + k));
-                    v.x = v.x * scale * g4.x; v.y = v.y * scale * g4.y; v.z = v.z * scale * g4.z; v.w = v.w * scale * g4.w;
-                }
-                *reinterpret_cast<float4*>(dst + k) = v;
             }
+            // eight sums over 32 lanes: halved three times, then two plain exchanges; lanes 4 r .. 4 r + 3 hold row r's
+#pragma unroll
+            for (int o = 16, h = ROWS / 2; o >= 4; o >>= 1, h >>= 1) {
+                const bool upper = (lane & o) != 0;
+#pragma unroll
+                for (int j = 0; j < h; j++) {
+                    const float send = upper ? ss[j] : ss[j + h], keep = upper ? ss[j + h] : ss[j];
+                    ss[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 2);
+            ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], 1);
+            if ((lane & 3) == 0) ss_part[warp][lane >> 2] = ss[0];
         } else {
-            for (int k = lo_k + lane * 4; k < lo_k + span; k += 128)
-                *reinterpret_cast<float4*>(dst + k) =
-                    live ? __ldcg(reinterpret_cast<const float4*>(src + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < ROWS; c++) {
+                float* dst = xs + (size_t)c * K + k0;
+                if (c < n) {
+                    const float* src = a.x + (int64_t)c * a.x_stride + k0;
+                    for (int i = 4 * lane; i < len; i += 128) cp_async16(dst + i, src + i);
+                } else {
+                    for (int i = 4 * lane; i < len; i += 128) *reinterpret_cast<float4*>(dst + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
         }
+        __syncwarp();
     }
-    __syncthreads();
 
     // ---- tiles ----
-    float acc[WR][ROWS];
+    unsigned long long acc[2][ROWS];
 #pragma unroll
-    for (int r = 0; r < WR; r++)
+    for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int c = 0; c < ROWS; c++) acc[r][c] = 0.f;
+        for (int c = 0; c < ROWS; c++) acc[r][c] = 0;
+    float scale = 1.f;                                     // the norm's, of row threadIdx.x % ROWS
+    bool have_scale = PRO != X_NORM;
+
+    // The partial sums of `held` tiles, the last of them last_tile, added in warp order and stored.
+    auto finish = [&](int last_tile, int held) {
+        __syncthreads();
+        const int c = threadIdx.x % ROWS;
+        if (!have_scale) {
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) t += ss_part[w][c];
+            scale = rsqrtf(t / (float)K + a.eps);
+            have_scale = true;
+        }
+        constexpr int OUTS = EPI == SWIGLU ? PARTS / 2 : PARTS;
+        for (int e = threadIdx.x; e < held * OUTS; e += THREADS) {
+            const int sl = e / OUTS, rc = e - sl * OUTS, tile = last_tile - (held - 1 - sl) * (int)gridDim.x;
+            const float* part = red + (size_t)sl * WARPS * PARTS + rc;
+            float v = 0.f, up = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; w++) v += part[w * PARTS];
+            if (EPI == SWIGLU) {
+#pragma unroll
+                for (int w = 0; w < WARPS; w++) up += part[w * PARTS + PARTS / 2];
+            }
+            const int col = tile * OUT_PER_TILE + rc / ROWS;
+            if (c >= n || col >= N) continue;
+            float* dst = a.y + (int64_t)c * a.y_stride + col;
+            if (PRO == X_NORM) { v *= scale; up *= scale; }
+#ifdef KLLM_BIAS
+            if (EPI != STORE && a.bias) v += a.bias[col];
+            if (EPI == SWIGLU && a.bias_up) up += a.bias_up[col];
+            if (EPI == STORE && a.act == 3) {
+                v = fmaxf(v, 0.f);
+                v *= v;
+            }
+            if (EPI == SWIGLU && a.act == 2) {
+                v = fminf(v, a.limit);
+                up = fminf(fmaxf(up, -a.limit), a.limit);
+                *dst = v / (1.f + expf(-a.alpha * v)) * (up + 1.f);
+            } else if (EPI == SWIGLU && a.act == 1)
+                *dst = 0.5f * v * (1.f + tanhf(0.79788456080286536f * (v + 0.044715f * v * v * v))) * up;
+            else
+#endif
+            if (EPI == SWIGLU) *dst = (v / (1.f + expf(-v))) * up;
+            else if (EPI == ADD) *dst += v;
+            else *dst = v;
+        }
+    };
 
     // multiply the batch (cur_tile, cur_b) held in `cur` while the following batch loads into `nxt`
-    auto phase = [&](float4 (&cur)[UNROLL][WR], float4 (&nxt)[UNROLL][WR]) {
+    auto phase = [&](ulonglong2 (&cur)[UNROLL][2], ulonglong2 (&nxt)[UNROLL][2]) {
         int nxt_tile = cur_tile, nxt_b = cur_b + 1;
         if (nxt_b == nb) { nxt_b = 0; nxt_tile += gridDim.x; }
         if (nxt_tile < n_tiles) load_batch(nxt, nxt_tile, nxt_b);
+        const float* xk = xs + k0 + cur_b * UNROLL * STEP + 4 * kl;
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++) {
-            const int i = cur_b * UNROLL + u;
-            if (i < my_steps) {
-                const int k = (ks + i * KSLICES) * 128 + 4 * lane;
+        for (int u = 0; u < UNROLL; u++)
+            if (EXACT || cur_b * UNROLL + u < my_steps) {
 #pragma unroll
                 for (int c = 0; c < ROWS; c++) {
-                    const float4 xv = *reinterpret_cast<const float4*>(xs + (size_t)c * K + k);
-#pragma unroll
-                    for (int r = 0; r < WR; r++) {
-                        acc[r][c] = fmaf(cur[u][r].x, xv.x, acc[r][c]);
-                        acc[r][c] = fmaf(cur[u][r].y, xv.y, acc[r][c]);
-                        acc[r][c] = fmaf(cur[u][r].z, xv.z, acc[r][c]);
-                        acc[r][c] = fmaf(cur[u][r].w, xv.w, acc[r][c]);
-                    }
+                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(xk + (size_t)c * K + u * STEP);
+                    fma2(acc[0][c], cur[u][0].x, xv.x);
+                    fma2(acc[1][c], cur[u][1].x, xv.x);
+                    fma2(acc[0][c], cur[u][0].y, xv.y);
+                    fma2(acc[1][c], cur[u][1].y, xv.y);
                 }
             }
-        }
         if (cur_b == nb - 1) {
-            // The lanes' partial sums: 32 values on 32 lanes are summed by halving (each step a
-            // lane hands half of its values to the partner lane and adds what it is handed), so
-            // that lane r * 8 + c ends with the warp's sum of (row r, token c): 31 shuffles instead
-            // of 160, in a fixed order.
-            float v[WR * ROWS];
+            // 16 sums over the 8 lanes of a row: each exchange halves what a lane holds
+            float v[2 * ROWS];
 #pragma unroll
-            for (int r = 0; r < WR; r++)
+            for (int r = 0; r < 2; r++)
 #pragma unroll
-                for (int c = 0; c < ROWS; c++) { v[r * ROWS + c] = acc[r][c]; acc[r][c] = 0.f; }
+                for (int c = 0; c < ROWS; c++) { v[r * ROWS + c] = sum2(acc[r][c]); acc[r][c] = 0; }
 #pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) {
-                const bool upper = (lane & o) != 0;
+            for (int o = 4, h = ROWS; o >= 1; o >>= 1, h >>= 1) {
+                const bool upper = (kl & o) != 0;
 #pragma unroll
-                for (int j = 0; j < o; j++) {
-                    const float send = upper ? v[j] : v[j + o];
-                    const float keep = upper ? v[j + o] : v[j];
+                for (int j = 0; j < h; j++) {
+                    const float send = upper ? v[j] : v[j + h], keep = upper ? v[j + h] : v[j];
                     v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
                 }
             }
-            const float mine = v[0];
-            red[warp * 32 + lane] = mine;              // warp = ks * GROUPS + grp
-            __syncthreads();
-            const int tile = cur_tile;
-            if (threadIdx.x < (EPI == SWIGLU ? 32 : 64)) {
-                const int e = threadIdx.x, g2 = e >> 5, rc = e & 31, r = rc / ROWS, c = rc % ROWS;
-                float v = 0.f, up = 0.f;
-#pragma unroll
-                for (int q = 0; q < KSLICES; q++) v += red[(q * GROUPS + g2) * 32 + rc];      // the slices, in order
-                if (EPI == SWIGLU) {
-#pragma unroll
-                    for (int q = 0; q < KSLICES; q++) up += red[(q * GROUPS + 1) * 32 + rc];
-                }
-                const int col = EPI == SWIGLU ? tile * WR + r : tile * GROUPS * WR + g2 * WR + r;
-                if (c < n && col < N) {
-                    float* dst = a.y + (int64_t)c * a.y_stride + col;
-#ifdef KLLM_BIAS
-                    if (EPI != STORE && a.bias) v += a.bias[col];
-                    if (EPI == SWIGLU && a.bias_up) up += a.bias_up[col];
-                    if (EPI == STORE && a.act == 3) {
-                        v = fmaxf(v, 0.f);
-                        v *= v;
-                    }
-                    if (EPI == SWIGLU && a.act == 2) {
-                        v = fminf(v, a.limit);
-                        up = fminf(fmaxf(up, -a.limit), a.limit);
-                        *dst = v / (1.f + expf(-a.alpha * v)) * (up + 1.f);
-                    } else if (EPI == SWIGLU && a.act == 1)
-                        *dst = 0.5f * v * (1.f + tanhf(0.79788456080286536f * (v + 0.044715f * v * v * v))) * up;
-                    else
-#endif
-                    if (EPI == SWIGLU) *dst = (v / (1.f + expf(-v))) * up;
-                    else if (EPI == ADD) *dst += v;
-                    else *dst = v;
-                }
+            // lane kl: row kl >> 2 of the two, tokens 2 (kl & 3) and the next
+            *reinterpret_cast<float2*>(red + ((size_t)slot * WARPS + warp) * PARTS + ((kl >> 2) * 4 + sub) * ROWS + 2 * (kl & 3)) =
+                make_float2(v[0], v[1]);
+            if (++slot == slots || nxt_tile >= n_tiles) {
+                finish(cur_tile, slot);
+                slot = 0;
+                if (nxt_tile < n_tiles) __syncthreads();
             }
-            __syncthreads();
         }
         cur_tile = nxt_tile;
         cur_b = nxt_b;
@@ -234,11 +279,22 @@ skinny_f32_kernel(const Args a) {
     }
 }
 
-template <int PRO, int EPI>
-int launch(const Args& a, cudaStream_t s) {
+template <int PRO, int EPI, bool EXACT>
+int launch_exact(const Args& a, cudaStream_t s) {
     static size_t attr_smem = 0;
-    const size_t smem = (size_t)ROWS * a.K * sizeof(float);
-    auto kern = skinny_f32_kernel<PRO, EPI>;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int out_per_tile = EPI == SWIGLU ? TILE / 2 : TILE;
+    const int n_tiles = (a.N + out_per_tile - 1) / out_per_tile;
+    const int grid = max(1, min(n_tiles, max(1, sms)));
+    // as many tiles between two summings as shared memory holds beside X, spread evenly
+    const size_t x_bytes = (size_t)ROWS * a.K * 4, slot_bytes = (size_t)WARPS * PARTS * 4;
+    const int most = (int)min((size_t)MAX_SLOTS, (SMEM_MOST - 1024 - x_bytes) / slot_bytes);
+    const int per_cta = (n_tiles + grid - 1) / grid, rounds = (per_cta + most - 1) / most;
+    const int slots = (per_cta + rounds - 1) / rounds;
+    const size_t smem = x_bytes + slots * slot_bytes;
+    auto kern = skinny_f32_kernel<PRO, EPI, EXACT>;
     if (smem > attr_smem) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) {
@@ -248,14 +304,13 @@ int launch(const Args& a, cudaStream_t s) {
         }
         attr_smem = smem;
     }
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int out_per_tile = EPI == SWIGLU ? WR : GROUPS * WR;
-    const int n_tiles = (a.N + out_per_tile - 1) / out_per_tile;
-    const int grid = max(1, min(n_tiles, max(1, sms)));
-    kllm_launch_dep(n_tiles <= 3 * grid, (kern), dim3(grid), dim3(THREADS), smem, s, a);
+    kllm_launch_dep(n_tiles <= 3 * grid, (kern), dim3(grid), dim3(THREADS), smem, s, a, slots);
     KLLM_LAUNCH_STATUS();
+}
+
+template <int PRO, int EPI>
+int launch(const Args& a, cudaStream_t s) {
+    return a.K % (WARPS * STEP * UNROLL) == 0 ? launch_exact<PRO, EPI, true>(a, s) : launch_exact<PRO, EPI, false>(a, s);
 }
 
 }  // namespace
