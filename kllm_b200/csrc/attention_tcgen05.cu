@@ -178,7 +178,7 @@ attn_prefill_tc5_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, int6
     __shared__ int s_req, s_tok0, s_abort;
     const int g = blockIdx.x % n_kv;          // CTAs start in the order of blockIdx.x: all kv heads' longest tiles first
     const int gs = n_heads / n_kv;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         int tile = (gridDim.x - 1 - blockIdx.x) / n_kv, req = -1, tok0 = 0;       // longest key ranges first
         for (int s = 0; s < n_requests; s++) {
@@ -207,7 +207,7 @@ attn_prefill_tc5_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, int6
     tc_fence_after();
     griddep_wait();
     griddep_launch();
-    const unsigned tmem = s_tmem;
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const int tok0 = s_tok0;
     const int n_tok = min(tokens_per_tile, q_start[req + 1] - tok0);
     const int pos0 = start_pos[req] + (tok0 - q_start[req]);
@@ -246,15 +246,15 @@ attn_prefill_tc5_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, int6
       } else if (warp == 4) {
         // ---- issuer of the scores ---------------------------------------------------
         constexpr uint32_t IDESC_S = make_idesc(ROWS, TILE, false);
-        bool ok = mbar_wait(&bar_q_full, 0, abort_flag, status, 2);
+        bool ok = mbar_wait_warp(&bar_q_full, 0, abort_flag, status, 2);
         for (int j = 0; ok && j < ntiles; j++) {            // scores of tile j into buffer j & 1, up to two tiles ahead
             const int s = j % STAGES, b = j & 1;
-            ok = mbar_wait(&bar_kv_full[s], ((unsigned)(j / STAGES)) & 1u, abort_flag, status, 3) &&
-                 mbar_wait(&bar_s_free[b], (((unsigned)(j >> 1)) & 1u) ^ 1u, abort_flag, status, 4);
+            ok = mbar_wait_warp(&bar_kv_full[s], ((unsigned)(j / STAGES)) & 1u, abort_flag, status, 3) &&
+                 mbar_wait_warp(&bar_s_free[b], (((unsigned)(j >> 1)) & 1u) ^ 1u, abort_flag, status, 4);
             if (!ok) break;
             fence_async_smem();                // the copies landed through the generic proxy
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 const unsigned st = sKV + (unsigned)s * 2u * KV_BYTES;
 #pragma unroll
                 for (int kk = 0; kk < HD / 16; kk++) {
@@ -273,12 +273,12 @@ attn_prefill_tc5_kernel(bf16* __restrict__ out, const bf16* __restrict__ q, int6
         for (int j = 0; ok && j < ntiles; j++) {
             const int s = j % STAGES;
             // the stage's arrival was seen by the other issuer; this warp has to see it too
-            ok = mbar_wait(&bar_kv_full[s], ((unsigned)(j / STAGES)) & 1u, abort_flag, status, 5) &&
-                 mbar_wait(&bar_p_full, (unsigned)j & 1u, abort_flag, status, 5);
+            ok = mbar_wait_warp(&bar_kv_full[s], ((unsigned)(j / STAGES)) & 1u, abort_flag, status, 5) &&
+                 mbar_wait_warp(&bar_p_full, (unsigned)j & 1u, abort_flag, status, 5);
             if (!ok) break;
             fence_async_smem();
             tc_fence_after();
-            if (lane == 0) {                   // output += P . V
+            if (elect_one()) {                   // output += P . V
                 const unsigned st = sKV + (unsigned)s * 2u * KV_BYTES;
 #pragma unroll
                 for (int kk = 0; kk < TILE / 16; kk++) {

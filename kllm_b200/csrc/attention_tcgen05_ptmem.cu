@@ -204,7 +204,7 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
     __shared__ int s_req, s_tok0, s_abort;
     const int g = blockIdx.x % n_kv;          // CTAs start in the order of blockIdx.x: all kv heads' longest tiles first
     const int gs = n_heads / n_kv;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         int tile = (gridDim.x - 1 - blockIdx.x) / n_kv, req = -1, tok0 = 0;       // longest key ranges first
         for (int s = 0; s < n_requests; s++) {
@@ -233,7 +233,7 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
     tc_fence_after();
     griddep_wait();
     griddep_launch();
-    const unsigned tmem = s_tmem;
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const int tok0 = s_tok0;
     const int n_tok = min(tokens_per_tile, q_start[req + 1] - tok0);
     const int pos0 = start_pos[req] + (tok0 - q_start[req]);
@@ -279,21 +279,21 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
                            k_lo + (uint32_t)(((kk >> 2) * (TILE * 128) + (kk & 3) * 32) >> 4), IDESC_S, kk > 0);
             umma_commit(&bar_s_full);
         };
-        bool ok = mbar_wait(&bar_q_full, 0, abort_flag, status, 2) &&
-                  mbar_wait(&bar_kv_full[0], 0, abort_flag, status, 3);
+        bool ok = mbar_wait_warp(&bar_q_full, 0, abort_flag, status, 2) &&
+                  mbar_wait_warp(&bar_kv_full[0], 0, abort_flag, status, 3);
         if (ok) {
             fence_async_smem();                // the copies landed through the generic proxy
             tc_fence_after();
-            if (lane == 0) issue_scores(0);
+            if (elect_one()) issue_scores(0);
             __syncwarp();
         }
         for (int j = 0; ok && j < ntiles; j++) {
             const int s = j % STAGES;
             // the probabilities of tile j are in tensor memory and the output is rescaled
-            ok = mbar_wait(&bar_p_full, (unsigned)j & 1u, abort_flag, status, 4);
+            ok = mbar_wait_warp(&bar_p_full, (unsigned)j & 1u, abort_flag, status, 4);
             if (!ok) break;
             tc_fence_after();
-            if (lane == 0) {                   // output += P . V
+            if (elect_one()) {                   // output += P . V
                 const uint32_t v_lo = v_lo0 + (uint32_t)s * (2u * KV_BYTES >> 4);
 #pragma unroll
                 for (int kk = 0; kk < TILE / 16; kk++)
@@ -304,12 +304,12 @@ attn_prefill_tc5_ptmem_kernel(bf16* __restrict__ out, const bf16* __restrict__ q
             __syncwarp();
             if (j + 1 < ntiles) {
                 const int s2 = (j + 1) % STAGES;
-                ok = mbar_wait(&bar_kv_full[s2], ((unsigned)((j + 1) / STAGES)) & 1u, abort_flag, status, 5);
+                ok = mbar_wait_warp(&bar_kv_full[s2], ((unsigned)((j + 1) / STAGES)) & 1u, abort_flag, status, 5);
                 if (!ok) break;
                 fence_async_smem();
                 tc_fence_after();
                 // in issue order behind P.V(j), which reads the columns that these scores overwrite
-                if (lane == 0) issue_scores(s2);
+                if (elect_one()) issue_scores(s2);
                 __syncwarp();
             }
         }

@@ -118,7 +118,7 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __shared__ unsigned s_tmem;
     __shared__ int s_abort;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int nout = (is_gated(EPI)) ? bn / 2 : bn;            // output columns of a tile
     const int b_bytes = bn * 128, stage_bytes = A_BYTES + b_bytes;
@@ -141,12 +141,12 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = s_tmem;
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     griddep_launch();
 
     if (warp == 0) {
         // ---- producer ----------------------------------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_map(&map_a);
             prefetch_map(&map_b);
             if (is_gated(EPI)) prefetch_map(&map_b2);
@@ -159,9 +159,9 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
             const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * nout;
             for (int kb = 0; kb < kblocks; kb++) {
-                ok = mbar_wait(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
                 if (!ok) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     const unsigned a = base + (unsigned)(s * stage_bytes), b = a + A_BYTES;
                     mbar_expect_tx(&bar_full[s], (unsigned)stage_bytes);
                     tma_load_2d(a, &map_a, kb * BK, m0, &bar_full[s]);
@@ -193,15 +193,15 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         unsigned ph = 0, acc_ph = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-            ok = mbar_wait(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, status, 2);
+            ok = mbar_wait_warp(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, status, 2);
             if (!ok) break;
             tc_fence_after();
             const unsigned d = tmem + (unsigned)(acc * MAX_BN);
             for (int kb = 0; kb < kblocks; kb++) {
-                ok = mbar_wait(&bar_full[s], ph, abort_flag, status, 3);
+                ok = mbar_wait_warp(&bar_full[s], ph, abort_flag, status, 3);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     const unsigned a = base + (unsigned)(s * stage_bytes), b = a + A_BYTES;
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++)
@@ -212,7 +212,7 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 if (++s == stages) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
-            if (lane == 0) umma_commit(&bar_acc_full[acc]);
+            if (elect_one()) umma_commit(&bar_acc_full[acc]);
             __syncwarp();
             acc ^= 1;
             if (acc == 0) acc_ph ^= 1u;

@@ -91,7 +91,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __shared__ int s_abort;
     __shared__ int s_first[MAX_EXPERTS + 1], s_off[MAX_EXPERTS + 1];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int nout = GATED ? bn / 2 : bn;                  // output columns of a tile
     const int w_rows = GATED ? 2 * N : N;                  // rows of one expert's matrix
@@ -125,14 +125,14 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem = s_tmem;
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     const int m_tiles = s_first[E];
     const int tiles = m_tiles * n_tiles;
     griddep_launch();
 
     if (warp == 0) {
         // ---- producer ----------------------------------------------------------
-        if (lane == 0) {
+        if (elect_one()) {
             prefetch_map(&map_a);
             prefetch_map(&map_b);
         }
@@ -146,9 +146,9 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             const int row0 = s_off[e] + (gm - s_first[e]) * BM;
             const int wrow = e * w_rows + n0;
             for (int kb = 0; kb < kblocks; kb++) {
-                ok = mbar_wait(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
                 if (!ok) break;
-                if (lane == 0) {
+                if (elect_one()) {
                     const unsigned a = base + (unsigned)(s * stage_bytes), b = a + A_BYTES;
                     mbar_expect_tx(&bar_full[s], (unsigned)stage_bytes);
                     tma_load_2d(a, &map_a, kb * BK, row0, &bar_full[s]);
@@ -178,15 +178,15 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         unsigned ph = 0, acc_ph = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
-            ok = mbar_wait(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, status, 2);
+            ok = mbar_wait_warp(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, status, 2);
             if (!ok) break;
             tc_fence_after();
             const unsigned d = tmem + (unsigned)(acc * MAX_BN);
             for (int kb = 0; kb < kblocks; kb++) {
-                ok = mbar_wait(&bar_full[s], ph, abort_flag, status, 3);
+                ok = mbar_wait_warp(&bar_full[s], ph, abort_flag, status, 3);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     const unsigned a = base + (unsigned)(s * stage_bytes), b = a + A_BYTES;
 #pragma unroll
                     for (int kk = 0; kk < BK / 16; kk++)
@@ -197,7 +197,7 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 if (++s == stages) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
-            if (lane == 0) umma_commit(&bar_acc_full[acc]);
+            if (elect_one()) umma_commit(&bar_acc_full[acc]);
             __syncwarp();
             acc ^= 1;
             if (acc == 0) acc_ph ^= 1u;

@@ -54,6 +54,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, volati
     return true;
 }
 
+// One thread of a converged warp, chosen by the hardware, always the same.  tcgen05 and TMA instructions take their operands from
+// uniform registers: behind `lane == 0`, or behind a branch on one thread's wait, the compiler has to carry them there value by
+// value for whichever threads are active, which measured 75 cycles an MMA and 130 a copy.  Behind elect_one() in warp-uniform code
+// (mbar_wait_warp, warp_index) it sees one thread and uniform values.
+__device__ __forceinline__ bool elect_one() {
+    unsigned one;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
+}
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// mbar_wait of a whole warp: true if every lane's was
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, unsigned parity, volatile int* abort_flag, int* status, int where) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, where));
+}
+
 // one 2-D tile by TMA: box (64 elements of k) x (rows), landing 128-byte swizzled
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
