@@ -14,9 +14,9 @@
 //   4  the same with g = min(acc_gate, limit), u = clamp(acc_up, -limit, limit): g sigmoid(alpha g) (u + 1)
 //   5  y[M, N] bfloat16 = relu(acc)^2
 //
-// A persistent CTA per SM walks output tiles of 128 x BN.  BN, the accumulator's width,
-// is a multiple of 16 up to 256 (the gated epilogue spends half of the columns on
-// `up`).  Measured on this GPU, an M = 128 instruction takes the same time whatever its
+// The gated epilogues (3 and 4) run on pairs of CTAs, further down.  For the others a
+// persistent CTA per SM walks output tiles of 128 x BN.  BN, the accumulator's width,
+// is a multiple of 16 up to 256.  Measured on this GPU, an M = 128 instruction takes the same time whatever its
 // N, so anything narrower than 256 leaves the tensor core partly idle: 256 is the
 // default and narrower tiles are for matrices with fewer columns.  Ten warps, three roles:
 //   warp 0   producer: one lane issues TMA loads (cp.async.bulk.tensor, 128-byte
@@ -111,8 +111,8 @@ __device__ __forceinline__ void load_residual(const void* y, int64_t ldy, int ro
 template <int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                const __grid_constant__ CUtensorMap map_b2, void* __restrict__ y, int64_t ldy, int M, int N, int K,
-                int bn, int stages, float act_limit, float act_alpha, int* status) {
+                void* __restrict__ y, int64_t ldy, int M, int N, int K,
+                int bn, int stages, int* status) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_acc_full[2], bar_acc_empty[2];
     __shared__ unsigned s_tmem;
@@ -120,7 +120,7 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int nout = (is_gated(EPI)) ? bn / 2 : bn;            // output columns of a tile
+    const int nout = bn;                                       // output columns of a tile
     const int b_bytes = bn * 128, stage_bytes = A_BYTES + b_bytes;
     const int m_tiles = (M + BM - 1) / BM;
     const int n_tiles = (N + nout - 1) / nout;
@@ -149,7 +149,6 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         if (elect_one()) {
             prefetch_map(&map_a);
             prefetch_map(&map_b);
-            if (is_gated(EPI)) prefetch_map(&map_b2);
         }
         griddep_wait();
         int s = 0;
@@ -166,7 +165,6 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     mbar_expect_tx(&bar_full[s], (unsigned)stage_bytes);
                     tma_load_2d(a, &map_a, kb * BK, m0, &bar_full[s]);
                     tma_load_2d(b, &map_b, kb * BK, n0, &bar_full[s]);
-                    if (is_gated(EPI)) tma_load_2d(b + (unsigned)(b_bytes / 2), &map_b2, kb * BK, n0, &bar_full[s]);
                 }
                 __syncwarp();
                 issued++;
@@ -242,26 +240,11 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 float v[32];
                 float4 res_next[8];
                 tmem_ld32(t + c * 32, v);
-                if (is_gated(EPI)) {
-                    float u[32];
-                    tmem_ld32(t + bn / 2 + c * 32, u);
-                    tmem_ld_wait();
+                if (EPI == EPI_ADD_F32 && c + 1 < c_hi) load_residual(y, ldy, row, n0 + (c + 1) * 32, limit, row_ok, res_next);
+                tmem_ld_wait();
+                if (EPI == EPI_RELU2) {
 #pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        if (EPI == EPI_CLAMPED) {
-                            const float g = fminf(v[j], act_limit), w = fminf(fmaxf(u[j], -act_limit), act_limit);
-                            v[j] = g / (1.f + expf(-act_alpha * g)) * (w + 1.f);
-                        } else {
-                            v[j] = silu_mul(v[j], u[j]);
-                        }
-                    }
-                } else {
-                    if (EPI == EPI_ADD_F32 && c + 1 < c_hi) load_residual(y, ldy, row, n0 + (c + 1) * 32, limit, row_ok, res_next);
-                    tmem_ld_wait();
-                    if (EPI == EPI_RELU2) {
-#pragma unroll
-                        for (int j = 0; j < 32; j++) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
-                    }
+                    for (int j = 0; j < 32; j++) { v[j] = fmaxf(v[j], 0.f); v[j] *= v[j]; }
                 }
                 const int col = n0 + c * 32;
                 if (row_ok && col < limit) store_chunk<EPI>(y, ldy, row, col, limit, v, res);
@@ -282,19 +265,243 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
+// ---- the gated epilogues on pairs of CTAs ----------------------------------------
+// A gated product's tile is PAIR_F output columns (as many gate and up rows of W) by bn rows of x, bn a multiple of 16 up to 256.
+// W is the 256-row operand of a cta_group::2 instruction and x the one of bn rows, so that the tile's second size follows the
+// number of rows of a step: 845 rows run as five tiles of 176, three even waves, where tiles of 128 x rows had 308 tiles for
+// 148 SMs.  A CTA holds 64 gate rows, the 64 up rows behind them and half of x's rows: 64 bytes a cycle of operands from shared
+// memory at the full rate, where a CTA alone needs 96 and reached 77 % of it.  Roles as above; the leader's warp 1 issues for
+// both, either CTA's producer loads its own operands and announces them on the leader's barriers.  A column's gate and up values
+// lie 64 lanes apart: the two warps that read them exchange half of each through shared memory and finish half of the rows each.
+// (Interleaved by 16 rows they would be a shuffle apart, but eight copies of 16 rows a stage instead of two took longer than
+// the products.)  The results meet in shared memory and leave as whole 128-byte rows.
+//
+// A tile's rows are the fastest in the order of tiles, so that neighbouring pairs share W's rows; x stays in L2.  The last tile of
+// rows is moved back to end with x and leaves what it shares with the tile before to that one: rows behind x's end, which the copy
+// fills with zeros, took longer than rows that are there (64 rows in a tile of 256: 27 us, in one of 64: 14).
+constexpr int PAIR_F = 128;
+constexpr int PAIR_STAGE_ROW = 144;                                  // bytes of a row of results in shared memory, 128 in use
+constexpr int PAIR_SWAP_BYTES = 4 * 2 * 16 * 32 * 4;                 // what the four pairs of epilogue warps exchange
+constexpr int PAIR_OUT_BYTES = MAX_BN * PAIR_STAGE_ROW + PAIR_SWAP_BYTES;
+constexpr int PAIR_SMEM = 1024 + PAIR_OUT_BYTES + 5 * (A_BYTES + MAX_BN / 2 * 128);
+constexpr int PAIR_EPI_WARPS = 8;
+
+template <int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                 const __grid_constant__ CUtensorMap map_up, bf16* __restrict__ y, int64_t ldy, int M, int N, int K, int bn, int stages,
+                 float act_limit, float act_alpha, int* status) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_acc_full[2], bar_acc_empty[2];
+    __shared__ unsigned s_tmem;
+    __shared__ int s_abort;
+
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int b_rows = bn / 2;
+    const unsigned stage_bytes = (unsigned)(A_BYTES + b_rows * 128);         // a multiple of the swizzle's 1024, as bn is of 16
+    unsigned char* results = smem_raw + (base - smem_u32(smem_raw)) + stages * stage_bytes;
+    const int t_tiles = (M + bn - 1) / bn, f_tiles = (N + PAIR_F - 1) / PAIR_F;
+    const int tiles = t_tiles * f_tiles, pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
+    const int kblocks = (K + BK - 1) / BK;
+    volatile int* abort_flag = &s_abort;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        for (int a = 0; a < 2; a++) { mbar_init(&bar_acc_full[a], 1); mbar_init(&bar_acc_empty[a], 2 * PAIR_EPI_WARPS); }
+        s_abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+    griddep_launch();
+
+    if (warp == 0) {
+        // ---- producer: this CTA's rows of W and of x ----
+        int s = 0, issued = 0;
+        unsigned ph = 0;
+        bool ok = true;
+        const unsigned full0 = leader_addr(&bar_full[0]);             // the leader's barriers, 8 bytes apart
+        auto load_w = [&](int s, int f0, int kb) {
+            const unsigned a = base + s * stage_bytes, bar = full0 + 8u * s;
+            if (rank == 0) mbar_expect_tx(&bar_full[s], 2u * stage_bytes);
+            tma_load_2d_pair(a, &map_w, kb * BK, f0, bar);
+            tma_load_2d_pair(a + A_BYTES / 2, &map_up, kb * BK, f0, bar);
+        };
+        auto load_x = [&](int s, int t0, int kb) {
+            tma_load_2d_pair(base + s * stage_bytes + A_BYTES, &map_x, kb * BK, t0, full0 + 8u * s);
+        };
+        auto col0 = [&](int tile) { return tile / t_tiles * PAIR_F + (int)rank * 64; };
+        auto row0 = [&](int tile) { return min(tile % t_tiles * bn, max(0, M - bn)) + (int)rank * b_rows; };
+        // the first stages' weights do not depend on the kernel before
+        const int early = first < tiles ? min(stages, kblocks) : 0;
+        if (elect_one()) {
+            prefetch_map(&map_x);
+            prefetch_map(&map_w);
+            prefetch_map(&map_up);
+            for (int kb = 0; kb < early; kb++) load_w(kb, col0(first), kb);
+        }
+        griddep_wait();
+        if (elect_one())
+            for (int kb = 0; kb < early; kb++) load_x(kb, row0(first), kb);
+        __syncwarp();
+        issued = early;
+        s = early % stages;
+        ph = early == stages ? 1u : 0u;
+        for (int tile = first; ok && tile < tiles; tile += pairs) {
+            const int f0 = col0(tile), t0 = row0(tile);
+            for (int kb = tile == first ? early : 0; kb < kblocks; kb++) {
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
+                if (!ok) break;
+                if (elect_one()) {
+                    load_w(s, f0, kb);
+                    load_x(s, t0, kb);
+                }
+                __syncwarp();
+                issued++;
+                if (++s == stages) { s = 0; ph ^= 1u; }
+            }
+        }
+        if (ok && !*abort_flag) {
+            // the other CTA's products arrive at these barriers: stay until the last has
+            for (int j = 0; ok && j < stages; j++) {
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, status, 1);
+                if (++s == stages) { s = 0; ph ^= 1u; }
+            }
+        } else if (rank == 0) {
+            // copies still in flight must land before the shared memory goes away: wait, with the same bound, for the
+            // stages armed last (the leader for both CTAs; the other one is held by the cluster's barrier)
+            const int back = issued < stages ? issued : stages;
+            for (int j = 0; j < back; j++) {
+                int sj = s - 1 - j;
+                unsigned pj = ph;
+                if (sj < 0) { sj += stages; pj ^= 1u; }
+                const long long t0 = clock64();
+                while (!mbar_try_wait(&bar_full[sj], pj) && clock64() - t0 < kCycleLimit) {}
+            }
+        }
+    } else if (warp == 1) {
+        // ---- tensor-core issuer ----
+        if (rank == 0) {
+            const uint32_t idesc = make_idesc(256, bn);
+            int s = 0, acc = 0;
+            unsigned ph = 0, acc_ph = 0;
+            bool ok = true;
+            for (int tile = first; ok && tile < tiles; tile += pairs) {
+                ok = mbar_wait_warp(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, status, 2);
+                if (!ok) break;
+                tc_fence_after();
+                const unsigned d = tmem + (unsigned)(acc * MAX_BN);
+                for (int kb = 0; kb < kblocks; kb++) {
+                    ok = mbar_wait_warp(&bar_full[s], ph, abort_flag, status, 3);
+                    if (!ok) break;
+                    if (elect_one()) {
+                        const unsigned a = base + s * stage_bytes, b = a + A_BYTES;
+#pragma unroll
+                        for (int kk = 0; kk < BK / 16; kk++)
+                            umma_pair(d, make_desc(a + kk * 32), make_desc(b + kk * 32), idesc, kb > 0 || kk > 0);
+                        umma_commit_pair(&bar_empty[s]);
+                    }
+                    __syncwarp();
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                }
+                if (!ok) break;
+                if (elect_one()) umma_commit_pair(&bar_acc_full[acc]);
+                __syncwarp();
+                acc ^= 1;
+                if (acc == 0) acc_ph ^= 1u;
+            }
+        }
+    } else {
+        // ---- epilogue ----
+        griddep_wait();
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const unsigned lane_base = (unsigned)(quarter * 32) << 16;
+        const int chunks = (bn + 31) / 32, c_lo = half == 0 ? 0 : (chunks + 1) / 2, c_hi = half == 0 ? (chunks + 1) / 2 : chunks;
+        // quarters 0 and 1 hold the gate values of columns 0-31 and 32-63, quarters 2 and 3 the up values
+        const bool up = quarter >= 2;
+        const int group = quarter & 1, swap_id = 3 + half * 2 + group, in_half = threadIdx.x - 64 - half * 128;
+        float* swap = reinterpret_cast<float*>(results + MAX_BN * PAIR_STAGE_ROW) + (half * 2 + group) * 2 * 16 * 32 + lane;
+        int acc = 0;
+        unsigned acc_ph = 0;
+        for (int tile = first; tile < tiles; tile += pairs) {
+            const int t_own = tile % t_tiles * bn, t0 = min(t_own, max(0, M - bn)), f0 = tile / t_tiles * PAIR_F + (int)rank * 64;
+            // all threads of the half go on or none; its results of the tile before have left shared memory
+            if (!half_all(1 + half, mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, status, 4))) break;
+            tc_fence_after();
+            const unsigned t = tmem + lane_base + (unsigned)(acc * MAX_BN);
+#pragma unroll 1
+            for (int c = c_lo; c < c_hi; c++) {
+                float v[32];
+                tmem_ld32(t + c * 32, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; i++) swap[(up * 16 + i) * 32] = up ? v[i] : v[16 + i];
+                named_sync(swap_id, 64);
+                bf16* o = reinterpret_cast<bf16*>(results + (c * 32 + up * 16) * PAIR_STAGE_ROW) + group * 32 + lane;
+#pragma unroll
+                for (int i = 0; i < 16; i++) {             // the gate warp finishes the chunk's first 16 rows of x, the up warp the others
+                    const float got = swap[(!up * 16 + i) * 32];
+                    float g = up ? got : v[i], u = up ? v[16 + i] : got;
+                    if (EPI == EPI_CLAMPED) {
+                        g = fminf(g, act_limit);
+                        u = fminf(fmaxf(u, -act_limit), act_limit);
+                        g = g / (1.f + expf(-act_alpha * g)) * (u + 1.f);
+                    } else {
+                        g = silu_mul(g, u);
+                    }
+                    o[i * (PAIR_STAGE_ROW / 2)] = __float2bfloat16_rn(g);
+                }
+                named_sync(swap_id, 64);                   // both have read before either writes again
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_addr(&bar_acc_empty[acc]));
+            named_sync(1 + half, 128);
+            const int r_hi = min(min(c_hi * 32, bn), M - t0);
+            for (int i = in_half + max(c_lo * 32, t_own - t0) * 8; i < r_hi * 8; i += 128) {
+                const int r = i >> 3, f = f0 + (i & 7) * 8;
+                const uint4 w = *reinterpret_cast<const uint4*>(results + r * PAIR_STAGE_ROW + (i & 7) * 16);
+                bf16* o = y + (int64_t)(t0 + r) * ldy + f;
+                if (f + 8 <= N) {
+                    *reinterpret_cast<uint4*>(o) = w;
+                } else {
+                    const bf16* e = reinterpret_cast<const bf16*>(&w);
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+                        if (f + j < N) o[j] = e[j];
+                }
+            }
+            acc ^= 1;
+            if (acc == 0) acc_ph ^= 1u;
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                        // nothing of the pair's is under way in either CTA any more
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+}
+
 // ---- host side -----------------------------------------------------------------
 
 // Accumulator width: a tile's time does not shrink with its width (see the top of the
 // file), so the widest one with the fewest waves of tiles wins.
-int pick_bn(int M, int N, int epilogue) {
+int pick_bn(int M, int N) {
     const int sms = sm_count();
     const int m_tiles = (M + BM - 1) / BM;
-    const int step = is_gated(epilogue) ? 64 : 16;       // the up half starts on a 32-column chunk
     long long best = -1;
     int best_bn = MAX_BN;
-    for (int bn = MAX_BN; bn >= 64; bn -= step) {
-        const int nout = is_gated(epilogue) ? bn / 2 : bn;
-        const long long tiles = (long long)m_tiles * ((N + nout - 1) / nout);
+    for (int bn = MAX_BN; bn >= 64; bn -= 16) {
+        const long long tiles = (long long)m_tiles * ((N + bn - 1) / bn);
         const long long waves = (tiles + sms - 1) / sms;
         if (best < 0 || waves < best) { best = waves; best_bn = bn; }
     }
@@ -302,8 +509,8 @@ int pick_bn(int M, int N, int epilogue) {
 }
 
 template <int EPI>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb2, void* y, int64_t ldy, int M, int N, int K,
-           int bn, float act_limit, float act_alpha, int* status, cudaStream_t stream) {
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, void* y, int64_t ldy, int M, int N, int K, int bn, int* status,
+           cudaStream_t stream) {
     static bool attr_set = false;
     if (!attr_set) {
         cudaError_t e = cudaFuncSetAttribute(gemm_tc5_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -314,26 +521,62 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb2,
         }
         attr_set = true;
     }
-    const int nout = (is_gated(EPI)) ? bn / 2 : bn;
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + nout - 1) / nout);
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     int stages = (SMEM_BYTES - 1024) / (A_BYTES + bn * 128);
     if (stages > MAX_STAGES) stages = MAX_STAGES;
-    kllm_launch((gemm_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, stream, ma, mb, mb2, y, ldy, M, N, K, bn, stages,
+    kllm_launch((gemm_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, stream, ma, mb, y, ldy, M, N, K, bn, stages, status);
+    KLLM_LAUNCH_STATUS();
+}
+
+// Rows of x in a tile of a pair, and the product's time in units of a wave's row of x: the least waves x (bn + 100).  A wave of
+// K = 2048 takes 4.0 us + 0.040 us a row (64 rows 6.6 us, 128 8.5, 256 14.2): issue and hand-over of a k block beside
+// its products.
+struct PairPlan {
+    int bn;
+    long long cost;
+};
+PairPlan pair_plan(int M, int N) {
+    const long long pairs = sm_count() / 2, f_tiles = (N + PAIR_F - 1) / PAIR_F;
+    PairPlan best{MAX_BN, -1};
+    for (int bn = M < MAX_BN ? (M + 15) / 16 * 16 : MAX_BN; bn >= 16; bn -= 16) {
+        const long long tiles = f_tiles * ((M + bn - 1) / bn), cost = (tiles + pairs - 1) / pairs * (bn + 100);
+        if (best.cost < 0 || cost < best.cost) best = PairPlan{bn, cost};
+    }
+    return best;
+}
+
+template <int EPI>
+int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mu, void* y, int64_t ldy, int M, int N, int K, int bn,
+                float act_limit, float act_alpha, int* status, cudaStream_t stream) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM);
+        if (e != cudaSuccess) {
+            snprintf(g_kllm_err, sizeof(g_kllm_err), "gemm (tcgen05): %d bytes of shared memory refused: %s", PAIR_SMEM,
+                     cudaGetErrorString(e));
+            return (int)e;
+        }
+        attr_set = true;
+    }
+    const long long tiles = (long long)((M + bn - 1) / bn) * ((N + PAIR_F - 1) / PAIR_F), pairs = sm_count() / 2;
+    const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
+    int stages = (PAIR_SMEM - 1024 - PAIR_OUT_BYTES) / (A_BYTES + bn * 64);
+    if (stages > MAX_STAGES) stages = MAX_STAGES;
+    kllm_launch((gemm_pair_kernel<EPI>), dim3(grid), dim3(THREADS), PAIR_SMEM, stream, mx, mw, mu, (bf16*)y, ldy, M, N, K, bn, stages,
                 act_limit, act_alpha, status);
     KLLM_LAUNCH_STATUS();
 }
 
 }  // namespace
 
-// Share of the tensor-core time that tiles of the widest accumulator would use for an
-// M x N product, in percent: full tiles / (waves x CTAs).  Callers use it to choose
-// between this kernel and the library product.
+// Share of its time that a product keeps the tensor cores busy, in percent: full tiles / (waves x CTAs), for the gated epilogues
+// rows x column tiles / (pairs x what pair_plan counts).  Callers use it to choose between this kernel and the library product.
 extern "C" int kllm_gemm_tcgen05_efficiency(int M, int N, int epilogue) {
     if (M <= 0 || N <= 0) return 0;
-    const int nout = is_gated(epilogue) ? MAX_BN / 2 : MAX_BN;
-    const double full = ((double)M / BM) * ((double)N / nout);
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + nout - 1) / nout);
+    if (is_gated(epilogue)) return (int)(100.0 * M * ((double)N / PAIR_F) / ((double)(sm_count() / 2) * pair_plan(M, N).cost));
+    const double full = ((double)M / BM) * ((double)N / MAX_BN);
+    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + MAX_BN - 1) / MAX_BN);
     const long long waves = (tiles + sm_count() - 1) / sm_count();
     return (int)(100.0 * full / (double)(waves * sm_count()));
 }
@@ -352,8 +595,8 @@ extern "C" int kllm_gemm_tcgen05_fits(const void* x, int64_t ldx, const void* w,
     return 1;
 }
 
-// bn: accumulator width of a tile, 0 = chosen here, else a multiple of 16 (64 for the
-// gated epilogues) from 64 to 256.  act_limit, act_alpha: of epilogue 4.  status: device int that a wait which ran out sets
+// bn: accumulator width of a tile, 0 = chosen here, else a multiple of 16 from 64 (for the
+// gated epilogues, whose accumulators are as wide as a tile has rows of x, from 16) to 256.  act_limit, act_alpha: of epilogue 4.  status: device int that a wait which ran out sets
 // (1: producer, 2: accumulator, 3: stage, 4: epilogue).
 extern "C" int kllm_gemm_tcgen05(const void* x, int64_t ldx, const void* w, int64_t ldw, const void* w_up, int M, int N,
                                  int K, void* y, int64_t ldy, int epilogue, int bn, float act_limit, float act_alpha, int* status,
@@ -363,28 +606,29 @@ extern "C" int kllm_gemm_tcgen05(const void* x, int64_t ldx, const void* w, int6
         KLLM_FAIL("gemm (tcgen05): sizes %d x %d x %d, strides %lld/%lld/%lld or an address not taken (k and strides "
                   "multiples of 8, 16-byte aligned addresses)", M, N, K, (long long)ldx, (long long)ldw, (long long)ldy);
     if (epilogue == EPI_CLAMPED && !(act_limit > 0.f)) KLLM_FAIL("gemm (tcgen05): the clamped epilogue needs a positive limit");
-    if (bn == 0) bn = pick_bn(M, N, epilogue);
-    if (bn < 64 || bn > MAX_BN || bn % (is_gated(epilogue) ? 64 : 16))
-        KLLM_FAIL("gemm (tcgen05): accumulator width %d, a multiple of %d from 64 to %d", bn, is_gated(epilogue) ? 64 : 16, MAX_BN);
-    CUtensorMap ma, mb, mb2;
-    const int b_rows = is_gated(epilogue) ? bn / 2 : bn;
-    int r = tensor_map(&ma, x, ldx, M, K, BM);
-    if (r) return r;
-    r = tensor_map(&mb, w, ldw, N, K, b_rows);
-    if (r) return r;
     if (is_gated(epilogue)) {
-        r = tensor_map(&mb2, w_up, ldw, N, K, b_rows);
+        if (bn == 0) bn = pair_plan(M, N).bn;
+        if (bn < 16 || bn > MAX_BN || bn % 16) KLLM_FAIL("gemm (tcgen05): accumulator width %d, a multiple of 16 from 16 to %d", bn, MAX_BN);
+        CUtensorMap mx, mw, mu;
+        int r = tensor_map(&mx, x, ldx, M, K, bn / 2);
+        if (!r) r = tensor_map(&mw, w, ldw, N, K, PAIR_F / 2);
+        if (!r) r = tensor_map(&mu, w_up, ldw, N, K, PAIR_F / 2);
         if (r) return r;
-    } else {
-        mb2 = mb;
+        return epilogue == EPI_CLAMPED
+                   ? launch_pair<EPI_CLAMPED>(mx, mw, mu, y, ldy, M, N, K, bn, act_limit, act_alpha, status, (cudaStream_t)stream)
+                   : launch_pair<EPI_SWIGLU>(mx, mw, mu, y, ldy, M, N, K, bn, 0.f, 0.f, status, (cudaStream_t)stream);
     }
+    if (bn == 0) bn = pick_bn(M, N);
+    if (bn < 64 || bn > MAX_BN || bn % 16) KLLM_FAIL("gemm (tcgen05): accumulator width %d, a multiple of 16 from 64 to %d", bn, MAX_BN);
+    CUtensorMap ma, mb;
+    int r = tensor_map(&ma, x, ldx, M, K, BM);
+    if (!r) r = tensor_map(&mb, w, ldw, N, K, bn);
+    if (r) return r;
     cudaStream_t s = (cudaStream_t)stream;
     switch (epilogue) {
-        case EPI_BF16: return launch<EPI_BF16>(ma, mb, mb2, y, ldy, M, N, K, bn, 0.f, 0.f, status, s);
-        case EPI_F32: return launch<EPI_F32>(ma, mb, mb2, y, ldy, M, N, K, bn, 0.f, 0.f, status, s);
-        case EPI_ADD_F32: return launch<EPI_ADD_F32>(ma, mb, mb2, y, ldy, M, N, K, bn, 0.f, 0.f, status, s);
-        case EPI_CLAMPED: return launch<EPI_CLAMPED>(ma, mb, mb2, y, ldy, M, N, K, bn, act_limit, act_alpha, status, s);
-        case EPI_RELU2: return launch<EPI_RELU2>(ma, mb, mb2, y, ldy, M, N, K, bn, 0.f, 0.f, status, s);
-        default: return launch<EPI_SWIGLU>(ma, mb, mb2, y, ldy, M, N, K, bn, 0.f, 0.f, status, s);
+        case EPI_BF16: return launch<EPI_BF16>(ma, mb, y, ldy, M, N, K, bn, status, s);
+        case EPI_F32: return launch<EPI_F32>(ma, mb, y, ldy, M, N, K, bn, status, s);
+        case EPI_ADD_F32: return launch<EPI_ADD_F32>(ma, mb, y, ldy, M, N, K, bn, status, s);
+        default: return launch<EPI_RELU2>(ma, mb, y, ldy, M, N, K, bn, status, s);
     }
 }

@@ -69,6 +69,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, unsigned parity, v
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, where));
 }
 
+// Named barriers of some of a CTA's warps: `ok` of all 128 threads of barrier `id`; a plain meeting of `threads`.
+__device__ __forceinline__ bool half_all(int id, bool ok) {
+    unsigned r;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.and.pred q, %2, 128, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+                 : "=r"(r) : "r"((unsigned)ok), "r"(id) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory"); }
+
 // one 2-D tile by TMA: box (64 elements of k) x (rows), landing 128-byte swizzled
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
@@ -100,6 +109,42 @@ __device__ __forceinline__ void umma(unsigned d_tmem, uint64_t a_desc, uint64_t 
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+// ---- pairs of CTAs (clusters of two, cta_group::2) ----
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
+    return r;
+}
+// every thread of the cluster; what was written before it is seen after it
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// the address of the leader's (rank 0) copy of a shared variable
+__device__ __forceinline__ unsigned leader_addr(const void* p) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;\n" : "=r"(r) : "r"(smem_u32(p)));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(unsigned addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(addr) : "memory");
+}
+// a tile into this CTA's shared memory that is announced on the barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
+                 ::"r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+// M = 256: this CTA's 128 rows of A and half of B's rows, and the same of the other CTA at the same shared addresses; every CTA's
+// rows of the result in its own tensor memory.  Issued by the leader.
+__device__ __forceinline__ void umma_pair(unsigned d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((unsigned)accumulate) : "memory");
+}
+// arrives at this barrier in both CTAs when the products issued so far are through
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(unsigned taddr, float (&v)[32]) {
     uint32_t* r = reinterpret_cast<uint32_t*>(v);

@@ -10,6 +10,7 @@ its own count).
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -1478,17 +1479,29 @@ def gemm_fits(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue
 
 
 def gemm_pays(n: int, N: int, epilogue: str = "bf16", least: int = 75) -> bool:
-    """Whether ``gemm``'s tiles of 128 rows x 256 accumulator columns would keep the
-    tensor cores of all SMs busy for at least ``least`` percent of the product's time
-    (full tiles over waves x SMs); below that the library product adapts its tiling
-    better.  Same arithmetic as kllm_gemm_tcgen05_efficiency, without loading the library."""
+    """Whether ``gemm`` is the faster route.  Its tiles of 128 rows x 256 accumulator columns have to keep the tensor cores
+    of all SMs busy for at least ``least`` percent of the product's time (full tiles over waves x SMs); below that the
+    library product adapts its tiling better.  The gated epilogues run on pairs of CTAs in tiles that follow the rows, and
+    take the library's activation kernel in: there the line lies at 43 percent of what the kernel's own count of its time
+    allows.  (width 2048, 5632 columns: 200 rows 39 percent, 20.0 us against 16.3, 300: 42, 20.9 and 19.5, 400: 49, 22.9 and
+    23.6, 845: 34.2 and 40.7; 4096 x 14336: 128 rows 42 percent, 49 us against 55; 4096 x 11008: 128 rows 33 percent, 46
+    and 41, 300: 45, 58 and 61.)  Same arithmetic as kllm_gemm_tcgen05_efficiency, without loading the library."""
     if not USE_TCGEN05 or n <= 0 or N <= 0:
         return False
+    if epilogue in _GATED_EPI:
+        return _pair_efficiency(n, N, sm_count() // 2) >= 0.43
     sms = sm_count()
-    nout = 128 if epilogue in _GATED_EPI else 256
-    tiles = -(-n // 128) * -(-N // nout)
+    tiles = -(-n // 128) * -(-N // 256)
     waves = -(-tiles // sms)
-    return 100.0 * (n / 128.0) * (N / float(nout)) / (waves * sms) >= least
+    return 100.0 * (n / 128.0) * (N / 256.0) / (waves * sms) >= least
+
+
+@functools.lru_cache(maxsize=4096)
+def _pair_efficiency(n: int, N: int, pairs: int) -> float:
+    """The share that pair_plan of csrc/gemm_tcgen05.cu leaves the tensor cores busy."""
+    f_tiles = -(-N // 128)
+    cost = min(-(-(f_tiles * -(-n // bn)) // pairs) * (bn + 100) for bn in range(min(256, -(-n // 16) * 16), 15, -16))
+    return n * (N / 128.0) / (pairs * cost)
 
 
 def gemm(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "bf16", out: Optional[torch.Tensor] = None,

@@ -761,6 +761,25 @@ def test_tcgen05_gemm_epilogues(M, N, K, bn):
     kernels.check_status("cuda")
 
 
+@pytest.mark.parametrize("M,N,K,bn", [(1, 8, 8, 0), (17, 8, 72, 16), (300, 264, 136, 128), (513, 1544, 200, 240), (257, 136, 64, 256),
+                                      (1300, 9480, 72, 0)])
+def test_tcgen05_gated_tiles_of_rows(M, N, K, bn):
+    """The gated product's tiles: fewer rows than a tile, a last tile that is moved back over the one before, columns that
+    end inside a CTA's 64 and inside its eight, tiles for more than one wave of the pairs."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(M + N)
+    w, w2 = ((rng.standard_normal((N, K)) * 0.2).astype(np.float32) for _ in range(2))
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    ws, w2s, xs = (as_stored(t, "bfloat16") for t in (w, w2, x))
+    wt, w2t, xt = (dev(t, torch.bfloat16) for t in (w, w2, x))
+    g, u = xs @ ws.T, xs @ w2s.T
+    close(kernels.gemm(xt, wt, weight_up=w2t, epilogue="swiglu", bn=bn), plain.silu(g) * u, "bfloat16", "swiglu")
+    gc, uc = np.minimum(g, 2.0), np.clip(u, -2.0, 2.0)
+    close(kernels.gemm(xt, wt, weight_up=w2t, epilogue="clamped", limit=2.0, alpha=1.5, bn=bn),
+          gc / (1 + np.exp(-1.5 * gc)) * (uc + 1), "bfloat16", "clamped")
+    kernels.check_status("cuda")
+
+
 def test_tcgen05_gemm_rows_do_not_depend_on_the_batch():
     """A row's result is the same bits alone in a small batch and among many rows."""
     from kllm_b200 import kernels
