@@ -14,23 +14,24 @@
 // cores, to a sum in registers, so that the tensor core's own accumulation, which cuts digits
 // off, cannot drift over a long K.
 //
-// Two kernels.  `split_kernel` writes the three parts of a matrix as three bfloat16 planes;
-// `gemm_f32_tc5_kernel` multiplies planes.  W is taken in pieces of rows whose planes (6 bytes a
-// number) stay in L2 between the two (PLANE_LIMIT).  A kernel that split inside the product, in
-// registers, was measured at 392 us for 1003 x 11264 x 2048 (the splitting warps' loads were
-// exposed, and every tile of x split the same weights again).
+// Two kernels.  `split_kernel` writes the three parts of a matrix as three bfloat16 planes; `gemm_f32_tc5_kernel` multiplies
+// planes.  W is taken in pieces of rows whose planes (6 bytes a number, PLANE_LIMIT at most) have two buffers that take turns: a
+// piece is split while the piece before it is being multiplied, beside the product's CTA on every SM (the product is bound by
+// the tensor cores and leaves HBM idle).  A kernel that split inside the product, in registers, was measured at 392 us for
+// 1003 x 11264 x 2048 (the splitting warps' loads were exposed, and every tile of x split the same weights again).
 //
-// The product: one persistent CTA per SM, tiles of 128 rows x 256 columns (gated: 128 gate rows
-// of W and the 128 up rows beside them), ten warps:
-//   warp 0     one lane loads the planes of a k block by TMA (64-byte rows, 64-byte swizzle; 72 KB
-//              a stage, three stages),
-//   warp 1     one lane issues the 12 tcgen05.mma (2 k steps x 6 terms) of a block into one of two
-//              accumulators,
-//   warps 2-9  fetch each finished accumulator (tcgen05.ld) and add it to their sums: a thread
-//              owns one row of half of the tile's columns, and stores it at the end of the tile.
-// Where the tiles leave SMs idle (few rows, narrow matrices) the k range is cut into splits
-// of whole blocks, each a unit of work of its own that leaves its sums in a workspace;
-// a third kernel adds them in split order.
+// The product: persistent pairs of CTAs (clusters of two, cta_group::2), tiles of 256 rows of W (gated: 128 gate and 128 up rows,
+// interleaved by 16 in the planes, so that a column's two values lie 16 lanes apart) x bn rows of x, bn a multiple of 16 up to 256
+// that follows the number of rows: 1003 rows against 8 tiles of W run as 72 tiles of 112 rows, one wave of the 74 pairs.  A CTA
+// holds 128 rows of W and half of the tile's rows of x: 8 KB of operands an instruction of 128 cycles where a CTA alone needs 12.
+// Ten warps a CTA:
+//   warp 0     one thread loads the planes of a k block by TMA (64-byte rows, 64-byte swizzle; 48 KB a stage at bn = 256, four
+//              stages) and announces them on the leader's barriers,
+//   warp 1     of the leader: one thread issues the 12 tcgen05.mma (2 k steps x 6 terms) of a block into one of two accumulators,
+//   warps 2-9  fetch each finished accumulator (tcgen05.ld) and add it to their sums: a thread owns one column of the result for
+//              half of the tile's rows, and stores them at the end of the tile, 32 neighbouring columns a warp.
+// Where whole-K tiles leave pairs idle (few rows, narrow matrices) the k range is cut into splits of whole blocks, each a unit
+// of work of its own that leaves its sums in a workspace; a third kernel adds them in split order.
 //
 // The numbers are split after a multiplication by 2^24, an accumulator is multiplied by 2^-48 where it is added to the sum: bfloat16 ends at 2^-133 as float32 does
 // at 2^-149, so that without it numbers below 2^-110 would lose digits.  With it every float32 below 2^104 is split exactly.
@@ -45,14 +46,14 @@ KLLM_EXPORT_LAST_ERROR(gemm_f32_tcgen05)
 
 namespace {
 
-constexpr int BM = 128, BN = 256;
+constexpr int BM = 128;                         // rows of W a CTA holds; a pair's tile has twice as many
+constexpr int BN = 256;                         // most rows of x in a tile; accumulators lie this many columns apart
 constexpr int BK = 32;                          // a row of a plane is 64 bytes
 constexpr int THREADS = 320;
-constexpr int FETCHERS = 256;
-constexpr int STAGES = 3;
-constexpr int A_PLANE = BM * 64, B_PLANE = BN * 64;
-constexpr int STAGE_BYTES = 3 * (A_PLANE + B_PLANE);
-constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES;
+constexpr int FETCH_WARPS = 8;
+constexpr int MAX_STAGES = 8;
+constexpr int A_PLANE = BM * 64;
+constexpr int SMEM_BYTES = 1024 + 4 * 3 * (A_PLANE + BN / 2 * 64);
 constexpr int TMEM_COLS = 512;
 // Bytes of the planes of one piece of W: with x's planes and the result they stay in the 126 MB of L2.
 constexpr long long PLANE_LIMIT = 72LL << 20;
@@ -82,29 +83,56 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& p0, uint32_t&
     p2 = pack_bf16(ra - __uint_as_float(p1 << 16), rb - __uint_as_float(p1 & 0xffff0000u));
 }
 
-// planes [3][plane_rows][kp] of the rows of src [rows, K] at ld, from plane row `row0` on; a second matrix (src2) may
-// follow after the first one's rows.  Memory bound: 4 bytes read and 6 written a number.
-__global__ void split_kernel(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld, int rows, int K,
-                             bf16* __restrict__ planes, int64_t plane_rows, int kp) {
-    griddep_launch();
-    griddep_wait();
+// planes [3][plane_rows][kp] of the rows of src [rows, K] at ld.  With src2 (gated) the two matrices' rows take turns by 16:
+// row r of src is plane row 32 (r / 16) + r % 16, row r of src2 is 16 behind it.  Memory bound: 4 bytes read and 6 written
+// a number.  BESIDE: launched behind a product that does not read these planes, to run beside it (one CTA on every
+// SM beside the product's, more as that one's end): it waits for the kernel before it at its end instead of its beginning, so that what follows it follows that one too.
+template <bool BESIDE>
+__global__ void __launch_bounds__(256)
+split_kernel(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld, int rows, int K,
+             bf16* __restrict__ planes, int64_t plane_rows, int kp) {
+    if (!BESIDE) {
+        griddep_launch();
+        griddep_wait();
+    }
     const int pieces = kp / 8;
     const int64_t plane = plane_rows * kp, total = (int64_t)rows * (src2 ? 2 : 1) * pieces;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = i / pieces;
-        const int k = (int)(i - r * pieces) * 8;
-        const float* p = (r < rows ? src + r * ld : src2 + (r - rows) * ld) + k;
-        const float4 u = __ldg(reinterpret_cast<const float4*>(p));                     // K is a multiple of 4
-        const float4 v = k + 4 < K ? __ldg(reinterpret_cast<const float4*>(p + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        uint4 q0, q1, q2;
-        split2(u.x, u.y, q0.x, q1.x, q2.x);
-        split2(u.z, u.w, q0.y, q1.y, q2.y);
-        split2(v.x, v.y, q0.z, q1.z, q2.z);
-        split2(v.z, v.w, q0.w, q1.w, q2.w);
-        bf16* o = planes + r * kp + k;
-        *reinterpret_cast<uint4*>(o) = q0;
-        *reinterpret_cast<uint4*>(o + plane) = q1;
-        *reinterpret_cast<uint4*>(o + 2 * plane) = q2;
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 2 * step) {
+        float4 u[2], v[2];                                  // two pieces of eight numbers at a time, their loads ahead of the rest
+        bf16* o[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int64_t i = min(i0 + e * step, total - 1);
+            int64_t r = i / pieces;
+            const int k = (int)(i - r * pieces) * 8;
+            int64_t to = r;
+            const float* from = src;
+            if (src2) {
+                if (r >= rows) { from = src2; r -= rows; }
+                to = (r >> 4) * 32 + (r & 15) + (from == src2 ? 16 : 0);
+            }
+            const float* p = from + r * ld + k;
+            u[e] = __ldg(reinterpret_cast<const float4*>(p));                           // K is a multiple of 4
+            v[e] = k + 4 < K ? __ldg(reinterpret_cast<const float4*>(p + 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            o[e] = planes + to * kp + k;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            if (i0 + e * step >= total) break;
+            uint4 q0, q1, q2;
+            split2(u[e].x, u[e].y, q0.x, q1.x, q2.x);
+            split2(u[e].z, u[e].w, q0.y, q1.y, q2.y);
+            split2(v[e].x, v[e].y, q0.z, q1.z, q2.z);
+            split2(v[e].z, v[e].w, q0.w, q1.w, q2.w);
+            *reinterpret_cast<uint4*>(o[e]) = q0;
+            *reinterpret_cast<uint4*>(o[e] + plane) = q1;
+            *reinterpret_cast<uint4*>(o[e] + 2 * plane) = q2;
+        }
+    }
+    if (BESIDE) {
+        griddep_launch();
+        griddep_wait();
     }
 }
 
@@ -140,128 +168,139 @@ struct Args {
     int64_t ldx, ldw;
     float* y;
     int64_t ldy, split_stride;              // split_stride: elements between the workspace's splits
-    int M, N, K, splits, blocks_per_split;
-    int a_rows, b_rows;                     // rows of a plane of x and of W (gated: gate rows, then up rows)
+    int M, N, K, bn, stages, splits, blocks_per_split;      // N: columns of the result (EPI_PARTIAL: of the workspace)
+    int x_rows, w_rows;                     // rows of a plane of x and of W
     int* status;
 };
 
 template <int EPI>
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Args a) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
+    __shared__ __align__(8) uint64_t bar_full[MAX_STAGES], bar_empty[MAX_STAGES], bar_acc_full[2], bar_acc_empty[2];
     __shared__ unsigned s_tmem;
     __shared__ int s_abort;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
     const unsigned base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    constexpr int NOUT = EPI == EPI_SWIGLU ? BN / 2 : BN;
-    const int m_tiles = (a.M + BM - 1) / BM, n_tiles = (a.N + NOUT - 1) / NOUT;
-    const int units = m_tiles * n_tiles * a.splits;
+    const int bn = a.bn, stages = a.stages;
+    const unsigned b_plane = (unsigned)bn * 32, stage_bytes = 3 * (A_PLANE + b_plane);           // bn / 2 rows of 64 bytes
+    const int t_tiles = (a.M + bn - 1) / bn, tiles = t_tiles * ((a.w_rows + 2 * BM - 1) / (2 * BM));
+    const int units = tiles * a.splits, pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
     const int kblocks = (a.K + BK - 1) / BK;
     volatile int* abort_flag = &s_abort;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
-        for (int i = 0; i < 2; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], FETCHERS); }
+        for (int s = 0; s < stages; s++) { mbar_init(&bar_full[s], 1); mbar_init(&bar_empty[s], 1); }
+        for (int i = 0; i < 2; i++) { mbar_init(&bar_acc_full[i], 1); mbar_init(&bar_acc_empty[i], 2 * FETCH_WARPS); }
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::);
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
-    const unsigned tmem = s_tmem;
-    griddep_launch();
+    const unsigned tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
     griddep_wait();
+    griddep_launch();                       // not before the wait: what starts now may write planes that the kernels before this one read
 
     if (warp == 0) {
-        // ---- producer ----
+        // ---- producer: this CTA's rows of W's planes and of x's ----
         int s = 0, issued = 0;
         unsigned ph = 0;
         bool ok = true;
-        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
-            const int split = unit / (m_tiles * n_tiles), tile = unit - split * (m_tiles * n_tiles);
-            const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * NOUT;
+        const unsigned full0 = leader_addr(&bar_full[0]);             // the leader's barriers, 8 bytes apart
+        for (int unit = first; ok && unit < units; unit += pairs) {
+            const int split = unit / tiles, tile = unit - split * tiles;
+            const int t0 = tile % t_tiles * bn + (int)rank * (bn / 2), w0 = (tile / t_tiles * 2 + (int)rank) * BM;
             const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
             for (int kb = kb0; kb < kb1; kb++) {
-                ok = mbar_wait(&bar_empty[s], ph ^ 1u, abort_flag, a.status, 1);
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, a.status, 1);
                 if (!ok) break;
-                if (lane == 0) {
-                    const unsigned pa = base + (unsigned)(s * STAGE_BYTES), pb = pa + 3 * A_PLANE;
-                    mbar_expect_tx(&bar_full[s], (unsigned)STAGE_BYTES);
+                if (elect_one()) {
+                    const unsigned pa = base + s * stage_bytes, pb = pa + 3 * A_PLANE, bar = full0 + 8u * s;
+                    if (rank == 0) mbar_expect_tx(&bar_full[s], 2 * stage_bytes);
 #pragma unroll
                     for (int p = 0; p < 3; p++) {
-                        tma_load_2d(pa + p * A_PLANE, &map_a, kb * BK, p * a.a_rows + m0, &bar_full[s]);
-                        if (EPI == EPI_SWIGLU) {
-                            tma_load_2d(pb + p * B_PLANE, &map_b, kb * BK, p * a.b_rows + n0, &bar_full[s]);
-                            tma_load_2d(pb + p * B_PLANE + B_PLANE / 2, &map_b, kb * BK, p * a.b_rows + a.N + n0, &bar_full[s]);
-                        } else {
-                            tma_load_2d(pb + p * B_PLANE, &map_b, kb * BK, p * a.b_rows + n0, &bar_full[s]);
-                        }
+                        tma_load_2d_pair(pa + p * A_PLANE, &map_w, kb * BK, p * a.w_rows + w0, bar);
+                        tma_load_2d_pair(pb + p * b_plane, &map_x, kb * BK, p * a.x_rows + t0, bar);
                     }
                 }
                 __syncwarp();
                 issued++;
-                if (++s == STAGES) { s = 0; ph ^= 1u; }
+                if (++s == stages) { s = 0; ph ^= 1u; }
             }
         }
-        if (!ok || *abort_flag) {
-            // copies still in flight must land before the shared memory goes away
-            const int back = issued < STAGES ? issued : STAGES;
+        if (ok && !*abort_flag) {
+            // the other CTA's products arrive at these barriers: stay until the last has
+            for (int j = 0; ok && j < stages; j++) {
+                ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, a.status, 1);
+                if (++s == stages) { s = 0; ph ^= 1u; }
+            }
+        } else if (rank == 0) {
+            // copies still in flight must land before the shared memory goes away (the leader waits for both CTAs', the other
+            // one is held by the cluster's barrier)
+            const int back = issued < stages ? issued : stages;
             for (int j = 0; j < back; j++) {
                 int sj = s - 1 - j;
                 unsigned pj = ph;
-                if (sj < 0) { sj += STAGES; pj ^= 1u; }
+                if (sj < 0) { sj += stages; pj ^= 1u; }
                 const long long t0 = clock64();
                 while (!mbar_try_wait(&bar_full[sj], pj) && clock64() - t0 < kCycleLimit) {}
             }
         }
     } else if (warp == 1) {
         // ---- tensor-core issuer ----
-        const uint32_t idesc = make_idesc(BM, BN);
-        int s = 0, acc = 0;
-        unsigned ph = 0, acc_ph = 0;
-        bool ok = true;
-        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
-            const int split = unit / (m_tiles * n_tiles);
-            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
-            for (int kb = kb0; kb < kb1; kb++) {
-                ok = mbar_wait(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, a.status, 2) &&
-                     mbar_wait(&bar_full[s], ph, abort_flag, a.status, 3);
-                if (!ok) break;
-                tc_fence_after();
-                if (lane == 0) {
-                    const unsigned d = tmem + (unsigned)(acc * BN);
-                    const unsigned pa = base + (unsigned)(s * STAGE_BYTES), pb = pa + 3 * A_PLANE;
-                    constexpr int TA[6] = {0, 2, 1, 0, 1, 0}, TB[6] = {2, 0, 1, 1, 0, 0};
+        if (rank == 0) {
+            const uint32_t idesc = make_idesc(2 * BM, bn);
+            int s = 0, acc = 0;
+            unsigned ph = 0, acc_ph = 0;
+            bool ok = true;
+            for (int unit = first; ok && unit < units; unit += pairs) {
+                const int split = unit / tiles;
+                const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+                for (int kb = kb0; kb < kb1; kb++) {
+                    ok = mbar_wait_warp(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, a.status, 2) &&
+                         mbar_wait_warp(&bar_full[s], ph, abort_flag, a.status, 3);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const unsigned d = tmem + (unsigned)(acc * BN);
+                        const unsigned pa = base + s * stage_bytes, pb = pa + 3 * A_PLANE;
+                        constexpr int TW[6] = {2, 0, 1, 1, 0, 0}, TX[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-                    for (int t = 0; t < 6; t++)
+                        for (int t = 0; t < 6; t++)
 #pragma unroll
-                        for (int kk = 0; kk < BK / 16; kk++)
-                            umma(d, make_desc64(pa + TA[t] * A_PLANE + kk * 32), make_desc64(pb + TB[t] * B_PLANE + kk * 32),
-                                 idesc, kk > 0 || t > 0);
-                    umma_commit(&bar_empty[s]);
-                    umma_commit(&bar_acc_full[acc]);
+                            for (int kk = 0; kk < BK / 16; kk++)
+                                umma_pair(d, make_desc64(pa + TW[t] * A_PLANE + kk * 32), make_desc64(pb + TX[t] * b_plane + kk * 32),
+                                          idesc, kk > 0 || t > 0);
+                        umma_commit_pair(&bar_empty[s]);
+                        umma_commit_pair(&bar_acc_full[acc]);
+                    }
+                    __syncwarp();
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                    acc ^= 1;
+                    if (acc == 0) acc_ph ^= 1u;
                 }
-                __syncwarp();
-                if (++s == STAGES) { s = 0; ph ^= 1u; }
-                acc ^= 1;
-                if (acc == 0) acc_ph ^= 1u;
             }
         }
     } else {
         // ---- sums and epilogue ----
         const int quarter = warp & 3, half = (warp - 2) >> 2;
         const unsigned lane_base = (unsigned)(quarter * 32) << 16;
+        const int chunks = (bn + 31) / 32, c_lo = half == 0 ? 0 : (chunks + 1) / 2, mine = half == 0 ? (chunks + 1) / 2 : chunks / 2;
+        const bool upper = lane >= 16;
         int acc = 0;
         unsigned acc_ph = 0;
         bool ok = true;
-        for (int unit = blockIdx.x; ok && unit < units; unit += gridDim.x) {
-            const int split = unit / (m_tiles * n_tiles), tile = unit - split * (m_tiles * n_tiles);
-            const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * NOUT;
+        for (int unit = first; ok && unit < units; unit += pairs) {
+            const int split = unit / tiles, tile = unit - split * tiles;
+            const int t0 = tile % t_tiles * bn + c_lo * 32, w0 = (tile / t_tiles * 2 + (int)rank) * BM + quarter * 32;
+            const int t_hi = min(tile % t_tiles * bn + bn, a.M);     // rows of x from t0 on that are this tile's
             const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
             float sum[4][32];
 #pragma unroll
@@ -272,85 +311,89 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 ok = mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, a.status, 4);
                 if (!ok) break;
                 tc_fence_after();
-                const unsigned t = tmem + lane_base + (unsigned)(acc * BN);
+                const unsigned t = tmem + lane_base + (unsigned)(acc * BN + c_lo * 32);
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
+                    if (c >= mine) break;
                     float v[32];
-                    // gated: two pieces of gate columns, then the two of the same up columns
-                    tmem_ld32(t + (EPI == EPI_SWIGLU ? (c >> 1) * 128 + half * 64 + (c & 1) * 32 : half * 128 + c * 32), v);
+                    tmem_ld32(t + c * 32, v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int j = 0; j < 32; j++) sum[c][j] = fmaf(v[j], UNSCALE, sum[c][j]);      // one rounding, as the add
                 }
                 tc_fence_before();
-                mbar_arrive(&bar_acc_empty[acc]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(leader_addr(&bar_acc_empty[acc]));
                 acc ^= 1;
                 if (acc == 0) acc_ph ^= 1u;
             }
             ok = __all_sync(0xffffffffu, ok);                       // the warp leaves together or stays for its votes below
             if (!ok) break;
-            const int r = m0 + quarter * 32 + lane;
-            constexpr int CH = EPI == EPI_SWIGLU ? 2 : 4;
-            unsigned odd[CH] = {};                                  // columns whose sum is not finite: taken again below
-            if (r < a.M) {
-                float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (int64_t)r * a.ldy;
-                if constexpr (EPI != EPI_PARTIAL) {
-                    float zero[4] = {};                             // 0 times every sum: NaN where one is not finite
+            // this lane's column; gated: the lower lanes finish the even rows of x, the upper ones the odd rows of the same columns
+            const int col = EPI == EPI_SWIGLU ? w0 / 2 + (lane & 15) : w0 + lane;
+            const bool live = col < a.N;
+            float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (live ? col : 0);
+            constexpr int PER = EPI == EPI_SWIGLU ? 16 : 32;        // values a lane stores of a chunk
 #pragma unroll
-                    for (int c = 0; c < 4; c++)
+            for (int c = 0; c < 4; c++) {
+                if (c >= mine) break;
+                float* s = sum[c];
+                auto row = [&](int j) { return t0 + c * 32 + (EPI == EPI_SWIGLU ? 2 * j + (int)upper : j); };
+                float zero[4] = {};                                 // 0 times every sum: NaN where one is not finite
 #pragma unroll
-                        for (int j = 0; j < 32; j++) zero[j & 3] = fmaf(sum[c][j], 0.f, zero[j & 3]);
-                    // a row of NaN, the common case, needs no second look
-                    if (is_nan((zero[0] + zero[1]) + (zero[2] + zero[3])) && !is_nan(a.x[r * a.ldx])) {
+                for (int j = 0; j < 32; j++) zero[j & 3] = fmaf(s[j], 0.f, zero[j & 3]);
+                const bool look = EPI != EPI_PARTIAL &&
+                                  __any_sync(0xffffffffu, is_nan((zero[0] + zero[1]) + (zero[2] + zero[3])));
+                unsigned odd = 0;                                   // values that are taken again below
+                if constexpr (EPI == EPI_SWIGLU) {
 #pragma unroll
-                        for (int c = 0; c < CH; c++)
-#pragma unroll
-                            for (int j = 0; j < 32; j++) {
-                                const bool good = finite(sum[c][j]) && (EPI != EPI_SWIGLU || finite(sum[(c + 2) & 3][j]));
-                                odd[c] |= (unsigned)!good << j;
-                                if (EPI == EPI_ADD && !good) sum[c][j] = 0.f;
-                            }
+                    for (int j = 0; j < 16; j++) {
+                        const float got = __shfl_xor_sync(0xffffffffu, upper ? s[2 * j] : s[2 * j + 1], 16);
+                        const float g = upper ? got : s[2 * j], u = upper ? s[2 * j + 1] : got;
+                        if (look && !(finite(g) && finite(u))) odd |= 1u << j;
+                        s[j] = silu_mul(g, u);
                     }
-                }
+                } else if (look) {
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        if (col + 4 * q < a.N) {                    // N is a multiple of 4
-                            float4 o;
-                            if constexpr (EPI == EPI_SWIGLU) {
-                                o.x = silu_mul(sum[c][4 * q], sum[c + 2][4 * q]);
-                                o.y = silu_mul(sum[c][4 * q + 1], sum[c + 2][4 * q + 1]);
-                                o.z = silu_mul(sum[c][4 * q + 2], sum[c + 2][4 * q + 2]);
-                                o.w = silu_mul(sum[c][4 * q + 3], sum[c + 2][4 * q + 3]);
-                            } else {
-                                o = make_float4(sum[c][4 * q], sum[c][4 * q + 1], sum[c][4 * q + 2], sum[c][4 * q + 3]);
-                            }
-                            float4* p = reinterpret_cast<float4*>(y + col + 4 * q);
-                            if (EPI == EPI_ADD) {
-                                const float4 h = *p;
-                                o.x += h.x; o.y += h.y; o.z += h.z; o.w += h.w;
-                            }
-                            *p = o;
+                    for (int j = 0; j < 32; j++)
+                        if (!finite(s[j])) {
+                            odd |= 1u << j;
+                            if (EPI == EPI_ADD) s[j] = 0.f;
                         }
-                    }
                 }
-            }
-            if constexpr (EPI != EPI_PARTIAL) {
-                __syncwarp();
+                if (EPI == EPI_ADD) {
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    const int col = n0 + (EPI == EPI_SWIGLU ? half * 64 : half * 128) + c * 32;
-                    for (unsigned rows = __ballot_sync(0xffffffffu, odd[c] != 0); rows != 0; rows &= rows - 1) {
-                        const int of = __ffs(rows) - 1, row = m0 + quarter * 32 + of;
-                        const float* xr = a.x + row * a.ldx;
-                        for (unsigned left = __shfl_sync(0xffffffffu, odd[c], of); left != 0; left &= left - 1) {
-                            const int j = col + __ffs(left) - 1;
-                            if (j >= a.N) break;                    // the tile's columns beyond the matrix
-                            float v = plain_dot(xr, a.w + j * a.ldw, a.K);
-                            if (EPI == EPI_SWIGLU) v = silu_mul(v, plain_dot(xr, a.w_up + j * a.ldw, a.K));
-                            float* e = a.y + row * a.ldy + j;
+                    for (int q = 0; q < 32; q += 16) {              // loads ahead of the stores
+                        float h[16];
+#pragma unroll
+                        for (int j = 0; j < 16; j++) h[j] = live && row(q + j) < t_hi ? y[(int64_t)row(q + j) * a.ldy] : 0.f;
+#pragma unroll
+                        for (int j = 0; j < 16; j++)
+                            if (live && row(q + j) < t_hi) y[(int64_t)row(q + j) * a.ldy] = h[j] + s[q + j];
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < PER; j++)
+                        if (live && row(j) < t_hi) y[(int64_t)row(j) * a.ldy] = s[j];
+                }
+                if (EPI != EPI_PARTIAL && look) {
+                    __syncwarp();
+                    if (!live) odd = 0;
+                    for (unsigned cols = __ballot_sync(0xffffffffu, odd != 0); cols != 0; cols &= cols - 1) {
+                        const int of = __ffs(cols) - 1, at = __shfl_sync(0xffffffffu, col, of), odd_row = of >= 16;
+                        for (unsigned left = __shfl_sync(0xffffffffu, odd, of); left != 0; left &= left - 1) {
+                            const int j = __ffs(left) - 1;
+                            const int r = t0 + c * 32 + (EPI == EPI_SWIGLU ? 2 * j + odd_row : j);
+                            if (r >= t_hi) break;                   // rows behind the tile's, in order
+                            const float* xr = a.x + (int64_t)r * a.ldx;
+                            float* e = a.y + (int64_t)r * a.ldy + at;
+                            // a row of NaN, the common case, needs no second look
+                            if (is_nan(*xr)) {
+                                if (EPI == EPI_ADD && lane == of) *e = *xr;
+                                continue;
+                            }
+                            float v = plain_dot(xr, a.w + (int64_t)at * a.ldw, a.K);
+                            if (EPI == EPI_SWIGLU) v = silu_mul(v, plain_dot(xr, a.w_up + (int64_t)at * a.ldw, a.K));
                             if (lane == of) *e = EPI == EPI_ADD ? *e + v : v;
                         }
                     }
@@ -360,18 +403,19 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();                                                 // nothing of the pair's is under way in either CTA any more
     if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-// The splits' sums, in split order, into the result: stored, added, or (gated: [M, 2 N] sums, the up columns behind the
-// gate columns) silu(gate) * up.  Bound by the workspace's bytes, which lie in L2.
+// The splits' sums, in split order, into the result: stored, added, or (gated: rows of gate and up sums that take turns by 16)
+// silu(gate) * up.  Bound by the workspace's bytes, which lie in L2.
 template <int EPI>
 __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const float* __restrict__ ws, int64_t split_stride,
                                      int M, int N, int splits, const Args a) {
     griddep_launch();
     griddep_wait();
-    const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? 2 * N : N, lane = threadIdx.x & 31;
+    const int n4 = N / 4, ldw = EPI == EPI_SWIGLU ? (N + 15) / 16 * 32 : N, lane = threadIdx.x & 31;
     const int64_t total = (int64_t)M * n4;
     // whole warps walk the elements: a sum that is not finite is taken again by all lanes
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < total; i0 += (int64_t)gridDim.x * blockDim.x) {
@@ -399,11 +443,12 @@ __global__ void reduce_splits_kernel(float* __restrict__ y, int64_t ldy, const f
                     if (lane == of) e[j] = d;
                 }
         };
-        float4 v = mine ? sum(ws + r * ldw + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* part = ws + r * ldw + (EPI == EPI_SWIGLU ? (c >> 4) * 32 + (c & 15) : c);
+        float4 v = mine ? sum(part) : make_float4(0.f, 0.f, 0.f, 0.f);
         again(v, a.w);
         float4 u = v;
         if (EPI == EPI_SWIGLU) {
-            if (mine) u = sum(ws + r * ldw + N + c);
+            if (mine) u = sum(part + 16);
             again(u, a.w_up);
         }
         if (!mine) continue;
@@ -435,7 +480,7 @@ int planes_map(CUtensorMap* out, const bf16* planes, int64_t rows, int K, int kp
 }
 
 template <int EPI>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Args& a, cudaStream_t s) {
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, cudaStream_t s) {
     static bool attr_set = false;
     if (!attr_set) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -446,19 +491,20 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Args& a, cudaStre
         }
         attr_set = true;
     }
-    const int nout = EPI == EPI_SWIGLU ? BN / 2 : BN;
-    const long long units = (long long)((a.M + BM - 1) / BM) * ((a.N + nout - 1) / nout) * a.splits;
-    const int grid = (int)(units < sm_count() ? units : sm_count());
-    kllm_launch((gemm_f32_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, s, ma, mb, a);
+    const long long units = (long long)((a.M + a.bn - 1) / a.bn) * ((a.w_rows + 2 * BM - 1) / (2 * BM)) * a.splits, pairs = sm_count() / 2;
+    const int grid = 2 * (int)(units < pairs ? units : pairs);
+    kllm_launch((gemm_f32_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, s, mw, mx, a);
     KLLM_LAUNCH_STATUS();
 }
 
-int launch_split(const float* src, const float* src2, int64_t ld, int rows, int K, bf16* planes, int64_t plane_rows, int kp,
+// beside: behind a product, to run on the SMs that it occupies
+int launch_split(bool beside, const float* src, const float* src2, int64_t ld, int rows, int K, bf16* planes, int64_t plane_rows, int kp,
                  cudaStream_t s) {
     const int64_t work = (int64_t)rows * (src2 ? 2 : 1) * (kp / 8);
-    const int64_t blocks = (work + 255) / 256, most = 8LL * sm_count();
-    kllm_launch((split_kernel), dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, s, src, src2, ld, rows, K, planes,
-                plane_rows, kp);
+    const int64_t blocks = (work + 511) / 512, most = 8LL * sm_count();
+    const dim3 grid((unsigned)(blocks < most ? blocks : most));
+    if (beside) kllm_launch((split_kernel<true>), grid, dim3(256), 0, s, src, src2, ld, rows, K, planes, plane_rows, kp);
+    else kllm_launch((split_kernel<false>), grid, dim3(256), 0, s, src, src2, ld, rows, K, planes, plane_rows, kp);
     KLLM_LAUNCH_STATUS();
 }
 
@@ -475,9 +521,23 @@ int launch_reduce(float* y, int64_t ldy, const float* ws, int64_t split_stride, 
 // for filling the pipeline and storing; a launch about 3; split sums are written and read at about 4 MB a block's time.
 struct Plan {
     int piece, splits, kp;
-    int64_t a_bytes, b_bytes, ws_bytes;
+    int64_t x_bytes, w_bytes, ws_bytes;
 };
 int64_t up256(int64_t b) { return (b + 255) / 256 * 256; }
+
+// Rows of x in a tile: an instruction's time goes with them (from about 96 on), so the least waves x rows wins, the wider tile
+// at a tie.  w_tiles: tiles of W, each `splits` units of work.
+int pick_bn(int M, int w_tiles, int splits) {
+    const long long pairs = sm_count() / 2;
+    long long best = -1;
+    int best_bn = BN;
+    for (int bn = BN; bn >= 16; bn -= 16) {
+        const long long units = (long long)w_tiles * splits * ((M + bn - 1) / bn), waves = (units + pairs - 1) / pairs;
+        const long long cost = waves * (bn > 96 ? bn : 96);
+        if (best < 0 || cost < best) { best = cost; best_bn = bn; }
+    }
+    return best_bn;
+}
 
 Plan make_plan(int M, int N, int K, int epilogue) {
     Plan p;
@@ -504,9 +564,16 @@ Plan make_plan(int M, int N, int K, int epilogue) {
             if (best < 0 || all < best) { best = all; p.piece = c == n_tiles ? N : (int)c * nout; p.splits = s; }
         }
     }
-    const int64_t cols = (int64_t)p.piece * (gated ? 2 : 1);
-    p.a_bytes = up256(6LL * M * p.kp);
-    p.b_bytes = up256(6LL * cols * p.kp);
+    // Tiles of whole K, their rows of x chosen to fit, save the splits' workspace and the kernel behind where they keep the pairs
+    // busy for most of the time.
+    if (p.splits > 1 && p.piece == N) {
+        const int bn = pick_bn(M, (int)n_tiles, 1);
+        const long long waves = (n_tiles * ((M + bn - 1) / bn) + sms / 2 - 1) / (sms / 2);
+        if (10.0 * n_tiles * M >= 6.0 * (sms / 2) * waves * (bn > 96 ? bn : 96)) p.splits = 1;
+    }
+    const int64_t cols = gated ? (p.piece + 15) / 16 * 32 : p.piece;
+    p.x_bytes = up256(6LL * M * p.kp);
+    p.w_bytes = up256(6LL * cols * p.kp);
     p.ws_bytes = p.splits > 1 ? up256(4LL * p.splits * M * cols) : 0;
     return p;
 }
@@ -517,7 +584,7 @@ Plan make_plan(int M, int N, int K, int epilogue) {
 extern "C" int kllm_gemm_f32_tcgen05_workspace(int M, int N, int K, int epilogue, int64_t* bytes) {
     if (M <= 0 || N <= 0 || K <= 0) { *bytes = 0; return 0; }
     const Plan p = make_plan(M, N, K, epilogue);
-    *bytes = p.a_bytes + p.b_bytes + p.ws_bytes;
+    *bytes = p.x_bytes + (p.piece < N ? 2 : 1) * p.w_bytes + p.ws_bytes;
     return 0;
 }
 
@@ -553,37 +620,41 @@ extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, 
                   "strides multiples of 4, 16-byte aligned addresses)", M, N, K, (long long)ldx, (long long)ldw, (long long)ldy);
     const Plan p = make_plan(M, N, K, epilogue);
     const bool gated = epilogue == EPI_SWIGLU;
-    const int kblocks = (K + BK - 1) / BK;
-    bf16* pa = (bf16*)ws;
-    bf16* pb = (bf16*)((char*)ws + p.a_bytes);
-    float* part = (float*)((char*)ws + p.a_bytes + p.b_bytes);
+    const int kblocks = (K + BK - 1) / BK, pieces = (N + p.piece - 1) / p.piece;
+    bf16* px = (bf16*)ws;
+    bf16* pw[2] = {(bf16*)((char*)ws + p.x_bytes), (bf16*)((char*)ws + p.x_bytes + (pieces > 1 ? p.w_bytes : 0))};
+    float* part = (float*)((char*)pw[1] + p.w_bytes);
     cudaStream_t s = (cudaStream_t)stream;
-    int r = launch_split((const float*)x, nullptr, ldx, M, K, pa, M, p.kp, s);
-    if (r) return r;
-    CUtensorMap ma, mb;
-    r = planes_map(&ma, pa, 3LL * M, K, p.kp, BM);
+    int r = launch_split(false, (const float*)x, nullptr, ldx, M, K, px, M, p.kp, s);
     if (r) return r;
     Args a;
     a.M = M; a.K = K; a.splits = p.splits; a.blocks_per_split = (kblocks + p.splits - 1) / p.splits; a.status = status;
-    a.a_rows = M; a.x = (const float*)x; a.ldx = ldx; a.ldw = ldw;
-    for (int n0 = 0; n0 < N; n0 += p.piece) {
-        const int cols = N - n0 < p.piece ? N - n0 : p.piece;
+    a.x_rows = M; a.x = (const float*)x; a.ldx = ldx; a.ldw = ldw;
+    // The last piece, the shortest, comes first: its splitting is the one that no product hides.
+    for (int i = 0; i < pieces; i++) {
+        const int n0 = (i == 0 ? pieces - 1 : i - 1) * p.piece, cols = N - n0 < p.piece ? N - n0 : p.piece;
         float* yp = (float*)y + n0;
-        a.b_rows = cols * (gated ? 2 : 1);
+        bf16* planes = pw[i & 1];
+        a.w_rows = gated ? (cols + 15) / 16 * 32 : cols;
         a.w = (const float*)w + n0 * ldw; a.w_up = gated ? (const float*)w_up + n0 * ldw : nullptr;
-        r = launch_split(a.w, a.w_up, ldw, cols, K, pb, a.b_rows, p.kp, s);
+        // Beside the product before, which started when its own planes were ready, that is when the product that read this
+        // buffer was over; behind split sums' last kernel as usual.
+        r = launch_split(i > 0 && p.splits == 1, a.w, a.w_up, ldw, cols, K, planes, a.w_rows, p.kp, s);
         if (r) return r;
-        // with splits a gated piece is a plain product with the gate and up columns beside each other
-        const bool pairs = gated && p.splits == 1;
-        r = planes_map(&mb, pb, 3LL * a.b_rows, K, p.kp, pairs ? BN / 2 : BN);
+        a.bn = pick_bn(M, (a.w_rows + 2 * BM - 1) / (2 * BM), p.splits);
+        a.stages = (SMEM_BYTES - 1024) / (3 * (A_PLANE + a.bn * 32));
+        if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
+        CUtensorMap mw, mx;
+        r = planes_map(&mw, planes, 3LL * a.w_rows, K, p.kp, BM);
+        if (!r) r = planes_map(&mx, px, 3LL * M, K, p.kp, a.bn / 2);
         if (r) return r;
         if (p.splits == 1) {
             a.N = cols; a.y = yp; a.ldy = ldy; a.split_stride = 0;
-            r = epilogue == EPI_STORE ? launch<EPI_STORE>(ma, mb, a, s) : epilogue == EPI_ADD ? launch<EPI_ADD>(ma, mb, a, s)
-                                                                                             : launch<EPI_SWIGLU>(ma, mb, a, s);
+            r = epilogue == EPI_STORE ? launch<EPI_STORE>(mw, mx, a, s) : epilogue == EPI_ADD ? launch<EPI_ADD>(mw, mx, a, s)
+                                                                                             : launch<EPI_SWIGLU>(mw, mx, a, s);
         } else {
-            a.N = a.b_rows; a.y = part; a.ldy = a.b_rows; a.split_stride = (int64_t)M * a.b_rows;
-            r = launch<EPI_PARTIAL>(ma, mb, a, s);
+            a.N = a.w_rows; a.y = part; a.ldy = a.w_rows; a.split_stride = (int64_t)M * a.w_rows;
+            r = launch<EPI_PARTIAL>(mw, mx, a, s);
             if (r) return r;
             r = epilogue == EPI_STORE ? launch_reduce<EPI_STORE>(yp, ldy, part, a.split_stride, M, cols, p.splits, a, s)
                 : epilogue == EPI_ADD ? launch_reduce<EPI_ADD>(yp, ldy, part, a.split_stride, M, cols, p.splits, a, s)

@@ -611,9 +611,19 @@ def attention_simt(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vca
     if first < n_req:
         qt = max(1, 64 // group)
         rest = n_tokens - first
-        rc = lib.kllm_attention_simt(_p(out), None, None, _p(q), q.stride(0), _p(kcache), _p(vcache),
-                                     _p(ctx.q_start[first:]), _p(ctx.start_pos[first:]), _p(block_table[first:]),
-                                     block_table.shape[1], n_req - first, rest // qt + (n_req - first), *common, qt, 0, 1,
+        where = (_p(ctx.q_start[first:]), _p(ctx.start_pos[first:]), _p(block_table[first:]), block_table.shape[1], n_req - first,
+                 rest // qt + (n_req - first))
+        if (USE_TCGEN05 and q.dtype == out.dtype == torch.float32 and vd == head_dim and v_row == vd and v_heads == n_kv
+                and head_dim in (64, 128)):
+            # on the tensor cores, every number in three bfloat16 parts
+            tc = load_library("attention_f32_mma")
+            if tc.kllm_attention_f32_mma_fits(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache), n_heads, n_kv, head_dim):
+                rc = tc.kllm_attention_f32_mma(_p(out), _p(q), q.stride(0), _p(kcache), _p(vcache), *where, n_heads, n_kv, head_dim,
+                                               kcache.shape[2], int(window or 0), scale, qt, _p(score_slopes), _p(sinks), segment,
+                                               int(keep or 0), _stream())
+                _check(tc, "attention_f32_mma", rc)
+                return
+        rc = lib.kllm_attention_simt(_p(out), None, None, _p(q), q.stride(0), _p(kcache), _p(vcache), *where, *common, qt, 0, 1,
                                      _p(score_slopes), _p(sinks), segment, v_heads, v_row, out_f32, int(keep or 0),
                                      dtype_code(q.dtype), _stream())
         _check(lib, "attention_simt", rc)
