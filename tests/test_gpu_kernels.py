@@ -276,6 +276,25 @@ def test_cuda_core_attention_portions_and_decoding_tokens(dtype, H, G, hd, page,
         close(got, want, dtype, f"lengths {lengths}")
 
 
+@pytest.mark.parametrize("H,G,hd,page", [(8, 1, 64, 16), (3, 3, 128, 5), (64, 1, 64, 64)])
+@pytest.mark.parametrize("value", [np.inf, 1e35])
+def test_float32_portions_with_values_beyond_the_three_parts(H, G, hd, page, value):
+    """Portions in float32 run on the tensor cores, every number in three bfloat16 parts.  A value that has none (infinite, or
+    larger than 2^104) reaches the rows that see it as arithmetic gives it and leaves the others alone."""
+    def plant(s, q, k, v):
+        if s == 0:
+            v[40, 0, 3] = value
+    lengths, n_new = [130, 65], [130, 64]
+    got, want = attention_case("float32", H, G, hd, page, lengths, n_new, None, seed=H + hd, plant=plant, kernel="simt")
+    got, want = got.cpu().numpy().astype(np.float64), np.asarray(want, dtype=np.float64)
+    odd = ~np.isfinite(want) | (np.abs(want) > 1e20)
+    assert odd.any() and not odd[:40].any()
+    assert np.array_equal(np.isinf(got), np.isinf(want)) and not np.isnan(got).any()
+    close(np.where(odd, 0, got), np.where(odd, 0, want), "float32", "rows and dims without it")
+    fin = odd & np.isfinite(want)
+    assert np.all(np.abs(got[fin] / want[fin] - 1) < 1e-4)
+
+
 @pytest.mark.parametrize("gs", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("window", [None, 300])
