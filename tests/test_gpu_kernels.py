@@ -281,18 +281,18 @@ def test_cuda_core_attention_portions_and_decoding_tokens(dtype, H, G, hd, page,
 def test_float32_portions_with_values_beyond_the_three_parts(H, G, hd, page, value):
     """Portions in float32 run on the tensor cores, every number in three bfloat16 parts.  A value that has none (infinite, or
     larger than 2^104) reaches the rows that see it as arithmetic gives it and leaves the others alone."""
-    def plant(s, q, k, v):
-        if s == 0:
-            v[40, 0, 3] = value
-    lengths, n_new = [130, 65], [130, 64]
-    got, want = attention_case("float32", H, G, hd, page, lengths, n_new, None, seed=H + hd, plant=plant, kernel="simt")
-    got, want = got.cpu().numpy().astype(np.float64), np.asarray(want, dtype=np.float64)
-    odd = ~np.isfinite(want) | (np.abs(want) > 1e20)
-    assert odd.any() and not odd[:40].any()
-    assert np.array_equal(np.isinf(got), np.isinf(want)) and not np.isnan(got).any()
-    close(np.where(odd, 0, got), np.where(odd, 0, want), "float32", "rows and dims without it")
-    fin = odd & np.isfinite(want)
-    assert np.all(np.abs(got[fin] / want[fin] - 1) < 1e-4)
+    def run(value):
+        def plant(s, q, k, v):
+            if s == 0:
+                v[40, 0, 3] = value
+        got, want = attention_case("float32", H, G, hd, page, [130, 65], [130, 64], None, seed=H + hd, plant=plant, kernel="simt")
+        return got.cpu().numpy().astype(np.float64), np.asarray(want, dtype=np.float64)
+    _, want = run(1e35)                                 # finite, so that a weight of 0 times it is 0 in the oracle
+    got, _ = run(value)
+    odd = np.abs(want) > 1e20
+    assert odd[40:130].any() and not odd[:40].any() and not odd[130:].any()
+    close(torch.from_numpy(np.where(odd, 0, got)), np.where(odd, 0, want), "float32", "rows and dims without it")
+    assert np.isposinf(got[odd]).all() if np.isinf(value) else np.all(np.abs(got[odd] / want[odd] - 1) < 1e-4)
 
 
 @pytest.mark.parametrize("gs", [1, 2, 4, 8, 16])
