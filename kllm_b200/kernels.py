@@ -536,7 +536,7 @@ def _kept_room(keep) -> int:
     return -(-int(keep or 0) // 64) * 64
 
 
-SIMT_CHUNK = 256      # keys per CTA when a decoding token's context is cut (attention_simt)
+SIMT_CHUNK = 256      # keys per CTA when a decoding token's context is cut (attention_simt, attention_decode_f32)
 
 
 def attention_simt(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, ctx,
@@ -904,6 +904,44 @@ def attention_decode_fused(out, q, k_new, v_new, cos_sin, kcache, vcache, positi
         head_dim, kcache.shape[2], int(window or 0), scale, int(num_splits),
         *_prefetch_args(prefetch), _stream())
     _check(lib, "attention_tc", rc)
+
+
+def attention_decode_f32_fits(n_heads: int, n_kv: int, head_dim: int) -> bool:
+    """Whether ``attention_decode_f32`` takes heads of this size (64 or 128) in groups of this width (1, 2, 4, 8 or 16)."""
+    return head_dim in (64, 128) and n_heads % max(1, n_kv) == 0 and n_heads // max(1, n_kv) in (1, 2, 4, 8, 16)
+
+
+def attention_decode_f32(out, q, k_new, v_new, cos_sin, kcache, vcache, positions, block_table, counters, n_heads, n_kv, head_dim,
+                         window, scale, ctx_bound: int) -> None:
+    """Decode attention of one float32 token per request (token t is request t) with the rotary encoding, the cache write and
+    the merge of the key ranges inside the kernel (csrc/attention_f32_decode.cu).  q, k_new, v_new are the step's unrotated
+    projections; ``counters`` as in ``attention_decode_fused``; no context is longer than ``ctx_bound``."""
+    _cuda(out, q, k_new, v_new, cos_sin, kcache, vcache, positions, block_table, counters)
+    _i32(block_table, "block_table")
+    if kcache.dtype != torch.float32 or vcache.dtype != torch.float32 or not kcache.is_contiguous() or not vcache.is_contiguous() \
+            or kcache.shape[1] != n_kv or kcache.shape[3] != head_dim or vcache.shape != kcache.shape or out.dtype != torch.float32 \
+            or not out.is_contiguous() or out.shape[1] != n_heads * head_dim:
+        raise KernelError("attention (float32, fused): caches must be [pages, n_kv, page_size, head_dim], out contiguous, all float32")
+    _i32(positions, "positions"); _i32(counters, "counters")
+    n = q.shape[0]
+    if any(t.dtype != torch.float32 or t.stride(1) != 1 for t in (q, k_new, v_new)):
+        raise KernelError("attention (float32, fused): q, k and v must be float32 with dense rows")
+    if cos_sin.dtype != torch.float32 or not cos_sin.is_contiguous() or cos_sin.shape[1] != head_dim:
+        raise KernelError("attention (float32, fused): the cos/sin table must be float32 [positions, head_dim]")
+    if counters.numel() < n * n_kv:
+        raise KernelError("attention (float32, fused): too few counters")
+    bound = min(ctx_bound, int(window)) if window else ctx_bound
+    splits = max(1, -(-bound // SIMT_CHUNK))
+    part_o = part_ml = None
+    if splits > 1:
+        part_o = torch.empty((n, n_heads, splits, head_dim), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((n, n_heads, splits, 2), dtype=torch.float32, device=q.device)
+    lib = load_library("attention_f32_decode")
+    rc = lib.kllm_attention_f32_decode(
+        _p(out), _p(part_o), _p(part_ml), _p(counters), _p(q), q.stride(0), _p(k_new), k_new.stride(0), _p(v_new), v_new.stride(0),
+        _p(cos_sin), _p(kcache), _p(vcache), _p(positions), _p(block_table), block_table.shape[1], n, n_heads, n_kv, head_dim,
+        kcache.shape[2], int(window or 0), scale, SIMT_CHUNK, splits, _stream())
+    _check(lib, "attention_f32_decode", rc)
 
 
 def attention_prefill(out, q, kcache, vcache, q_start, start_pos, block_table, n_requests, n_heads, n_kv,

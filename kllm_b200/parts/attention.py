@@ -271,14 +271,21 @@ class PagedAttention:
         if (self.score_slopes is not None or self.v_head_dim != self.head_dim or self.exact_weights or self.segment
                 or self.keep_first):
             table = None          # ... and has no bias on its scores, one head size, bfloat16 weights, a plain window
-        if (table is not None and cache.writes and ctx.all_single and self.dtype == torch.bfloat16 and group <= 16
-                and self.head_dim in kernels.TC_HEAD_DIMS and self.head_dim % 32 == 0):
+        wide = (table is not None and cache.writes and ctx.all_single and self.dtype == torch.float32
+                and kernels.attention_decode_f32_fits(self.n_heads, self.n_kv, self.head_dim))
+        if wide or (table is not None and cache.writes and ctx.all_single and self.dtype == torch.bfloat16 and group <= 16
+                    and self.head_dim in kernels.TC_HEAD_DIMS and self.head_dim % 32 == 0):
             # decode: rotary encoding, cache write and attention in one kernel
             if self._counters is None or self._counters.numel() < n * self.n_kv:
                 if self._counters is not None:
                     self._counters_kept.append(self._counters)
                 self._counters = torch.zeros(max(256, 2 * n) * self.n_kv, dtype=torch.int32, device=q.device)
             attn = torch.empty((n, self.q_dim), dtype=self.dtype, device=q.device)
+            if wide:
+                kernels.attention_decode_f32(attn, q, k, v, table, cache.k, cache.v, ctx.positions, cache.block_table, self._counters,
+                                             self.n_heads, self.n_kv, self.head_dim, self.window or 0, self.scale,
+                                             ctx.split_bound or ctx.max_ctx)
+                return attn
             kernels.attention_decode_fused(
                 attn, q, k, v, table, cache.k, cache.v, ctx.positions, None, cache.block_table,   # token t is request t
                 self._counters, self.n_heads, self.n_kv, self.head_dim, self.window or 0, self.scale,

@@ -505,6 +505,48 @@ def fused_decode_case(H, G, hd, page, splits, window):
             assert torch.equal(vc[pg, :, slot].float().cpu(), torch.from_numpy(as_stored(vnew[s], "bfloat16").reshape(G, hd)).float())
 
 
+@pytest.mark.parametrize("gs", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("window", [None, 1, 300])
+def test_float32_fused_decode_attention(gs, hd, window):
+    """Rotation, cache write, attention and merge in one kernel: every group width, contexts of one key, at the edges of a batch
+    of keys and of a range, over several ranges; the new token's slot and everything before a window hold NaN; run twice on
+    one counter buffer."""
+    from kllm_b200 import kernels
+    G, page, theta, max_pos = 3, 5, 1e4, 1024
+    H, rng, lengths = G * gs, np.random.default_rng(gs + hd), [1, 8, 9, 256, 257, 700, 33]
+    j = np.arange(hd // 2, dtype=np.float64)
+    ang = np.arange(max_pos, dtype=np.float64)[:, None] * theta ** (-2.0 * j / hd)
+    cos_sin = dev(np.concatenate([np.cos(ang), np.sin(ang)], 1).astype(np.float32))
+    counters = torch.zeros(64, dtype=torch.int32, device="cuda")
+    for rep in range(2):
+        ks, vs, want, qraw, knew, vnew = [], [], [], [], [], []
+        for L in lengths:
+            k, v = ((rng.standard_normal((L, G, hd))).astype(np.float32) for _ in range(2))
+            q = rng.standard_normal((1, H * hd)).astype(np.float32)
+            k_rot = plain.rope(k[-1:].reshape(1, G * hd), [L - 1], G, hd, theta)
+            k_all = np.concatenate([k[:-1].reshape(L - 1, G * hd), k_rot])
+            qs = np.concatenate([np.zeros((L - 1, H * hd)), plain.rope(q, [L - 1], H, hd, theta)])
+            want.append(plain.attention(qs, k_all, v.reshape(L, G * hd), H, G, hd, window=window)[-1:])
+            knew.append(k[-1:].reshape(1, G * hd)); vnew.append(v[-1:].reshape(1, G * hd)); qraw.append(q)
+            hk, hv = k.copy(), v.copy()
+            hk[-1] = hv[-1] = np.nan
+            if window:
+                hk[:max(0, L - window)] = hv[:max(0, L - window)] = np.nan
+            ks.append(hk); vs.append(hv)
+        kc, vc, table = paged(ks, vs, page, sum(-(-L // page) for L in lengths) + 3, rng, "float32", lengths)
+        q_t, k_t, v_t = (dev(np.concatenate(a)) for a in (qraw, knew, vnew))
+        out, pos = torch.empty_like(q_t), dev(np.array([L - 1 for L in lengths], np.int32))
+        kernels.attention_decode_f32(out, q_t, k_t, v_t, cos_sin, kc, vc, pos, table, counters, H, G, hd, window or 0,
+                                     1.0 / math.sqrt(hd), max_pos)
+        close(out, np.concatenate(want), "float32", f"attention, run {rep}")
+        assert int(counters.abs().sum()) == 0, "the counters must be zero again"
+        for s, L in enumerate(lengths):
+            pg, slot = int(table[s, (L - 1) // page]), (L - 1) % page
+            close(kc[pg, :, slot], plain.rope(knew[s], [L - 1], G, hd, theta).reshape(G, hd), "float32", "stored key")
+            assert torch.equal(vc[pg, :, slot].cpu(), torch.from_numpy(vnew[s].reshape(G, hd)))
+
+
 def test_tcgen05_form_follows_the_measurements():
     from kllm_b200 import kernels
     assert kernels.tcgen05_form(128, 4, 8, 2048, 1, 2048) == "tmem"
