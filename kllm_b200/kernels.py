@@ -547,7 +547,8 @@ def attention_simt(out: torch.Tensor, q: torch.Tensor, kcache: torch.Tensor, vca
     (csrc/attention_simt.cu): the attention of the float32 path.  The requests that bring
     one token each at the head of the batch (decoding requests, which the scheduler puts
     first) have their contexts cut into chunks of SIMT_CHUNK keys, one CTA each, merged in
-    chunk order; the portions after them run as tiles of up to 64 (token, head) rows.
+    chunk order; the portions after them run as tiles of up to 64 (token, head) rows, in float32 at
+    head sizes 64 and 128 on the tensor cores at float32 accuracy (csrc/attention_f32_mma.cu).
     ``score_slopes`` (float32 [n_heads]): slope[h] * (key position - query position) is added
     to the scaled scores of head h.  ``v_head_dim``: the size of a head's values and of its
     output where it differs from the keys' (``vcache`` [pages, n_kv, page_size, v_head_dim],
