@@ -74,17 +74,22 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 // The widths that are multiples of 4 up to kThreads * 4 * kVec, 16-byte rows: a thread keeps its V float4 of the row in
 // registers between the sum of squares and the scaling.  One CTA per row and as many threads as the row has float4, up to
 // kThreads, so that all of a row's loads are in flight at once: a row's latency is what a step of few rows waits for, and a
-// step of many is bound by its bytes either way.  In a decode step of 64 rows of 2048 a warp per row took 4.2 us, this takes
-// 2.4; the gains do not depend on the kernel before and are fetched while it ends.  V and the block's size follow from the
-// width alone, so a row is summed in the same order whatever else the step holds.
+// step of many is bound by its bytes either way.  64 rows of 2048: 4.3 us with a warp per row, 2.0 this way (launched back to back); the gains do not depend on the kernel before and are fetched while it ends.
+//
+// Who loads an element does not say who adds it.  LANES (bfloat16 rows of up to kLanesMost): 32 lanes, lane l the squares of the float4
+// l, l + 32, ..., which reach them through shared memory in the time that an exchange of partial sums takes; else thread t those of
+// the float4 that it holds.  This, V and the block's size follow from the width and the element type alone, so a row is summed in
+// the same order whatever else the step holds.
 constexpr int kVec = 8;
+constexpr int kLanesMost = 2048;
 
 __host__ __device__ constexpr int row_threads(int d) { return d / 4 >= kThreads ? kThreads : (d / 4 + 31) / 32 * 32; }
 
-template <typename T, int V>
+template <typename T, int V, bool LANES>
 __global__ void __launch_bounds__(kThreads)
 add_rmsnorm_row_kernel(float* __restrict__ x, const float* __restrict__ res, T* __restrict__ out,
                        const float* __restrict__ gain, const int* __restrict__ rows, int d, float eps) {
+    extern __shared__ float part[];
     __shared__ float red[32];
     const int n4 = d >> 2;
     float4 g[V], v[V];
@@ -116,9 +121,25 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const float* __restrict__ res, T* 
         }
     }
 #pragma unroll
-    for (int k = 0; k < V; k++)
-        if (threadIdx.x + k * blockDim.x < n4) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-    const float scale = rsqrtf(block_sum(ss, red) / (float)d + eps);
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4) {
+            const float q = (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+            if (LANES) part[i] = q;
+            else ss += q;
+        }
+    }
+    if (LANES) {                                           // every warp the same sum
+        const int lane = threadIdx.x & 31;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kLanesMost / 128; k++)
+            if (lane + 32 * k < n4) ss += part[lane + 32 * k];
+        ss = warp_sum(ss);
+    } else {
+        ss = block_sum(ss, red);
+    }
+    const float scale = rsqrtf(ss / (float)d + eps);
     T* orow = out + (int64_t)blockIdx.x * d;
 #pragma unroll
     for (int k = 0; k < V; k++) {
@@ -126,6 +147,50 @@ add_rmsnorm_row_kernel(float* __restrict__ x, const float* __restrict__ res, T* 
         if (i < n4)
             store4(orow + 4 * i, make_float4(v[k].x * scale * g[k].x, v[k].y * scale * g[k].y, v[k].z * scale * g[k].z,
                                              v[k].w * scale * g[k].w));
+    }
+}
+
+// The chosen rows of a bfloat16 result: the sums of add_rmsnorm_kernel (thread t the elements t, t + kThreads, ...) with the row in
+// registers, E elements a thread, for any address and any width up to kThreads * 4 * kVec.  64 rows of 2048: 3.0 us with three
+// passes through memory, 1.5 this way; 2048 rows 7.2 and 5.1.
+template <int E>
+__global__ void __launch_bounds__(kThreads)
+rmsnorm_chosen_kernel(const float* __restrict__ x, const float* __restrict__ res, bf16* __restrict__ out,
+                      const float* __restrict__ gain, const int* __restrict__ rows, int d, float eps) {
+    __shared__ float red[32];
+    float g[E], v[E];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i < d) g[k] = gain[i];
+    }
+    griddep_wait();
+    griddep_launch();
+    const int64_t src = rows[blockIdx.x];
+    const float* xr = x + src * d;
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i < d) v[k] = xr[i];
+    }
+    if (res) {
+        const float* rr = res + src * d;
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+            const int i = threadIdx.x + k * kThreads;
+            if (i < d) v[k] += rr[i];
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < E; k++)
+        if (threadIdx.x + k * kThreads < d) ss += v[k] * v[k];
+    const float scale = rsqrtf(block_sum(ss, red) / (float)d + eps);
+    bf16* orow = out + (int64_t)blockIdx.x * d;
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        const int i = threadIdx.x + k * kThreads;
+        if (i < d) orow[i] = from_f32<bf16>(v[k] * scale * g[k]);
     }
 }
 
@@ -166,13 +231,44 @@ rmsnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
     for (int i = threadIdx.x; i < d; i += blockDim.x) orow[i] = from_f32<T>(xr[i] * scale2 * gain2[i]);
 }
 
-// The same with the row in registers (V float4 a thread; widths, threads and order as in add_rmsnorm_row_kernel).  Two rows
-// of 2048 in a decode step, beside the end of the product before: 9.8 us more with one element a load and three passes
-// through memory, 1.8 this way; 2017 rows 17 us and 8.2.
+// The same with the row in registers (V float4 a thread; widths as in add_rmsnorm_row_kernel), the sums in the order of the kernel
+// above: the elements reach its threads through shared memory.  8 rows of 2048, launched back to back: 10.0 us with one
+// element a load and three passes through memory, 2.0 this way; 2048 rows 14.0 and 9.3.
+__host__ __device__ constexpr int add_threads(int d) { return d <= 512 ? 64 : (d <= 2048 ? 128 : kThreads); }
+__host__ __device__ constexpr int add_block(int d) { return row_threads(d) > add_threads(d) ? row_threads(d) : add_threads(d); }
+
+// The sum of the squares of a row of d = 4 n4 numbers, of which this thread holds the float4 threadIdx.x + k * blockDim.x in v[k], by
+// add_threads(d) threads, thread t the elements t, t + add_threads(d), ...; every thread gets it.  row: shared, 4 V blockDim.x floats.
+template <int V>
+__device__ __forceinline__ float squares_by_element(const float4 (&v)[V], int n4, float* row, float* red) {
+#pragma unroll
+    for (int k = 0; k < V; k++) {                          // zeros behind the row's end add nothing
+        const int i = threadIdx.x + k * blockDim.x;
+        store4(row + 4 * i, i < n4 ? v[k] : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+    __syncthreads();
+    // widths up to 1024 have a block of as many threads as they have float4; wider ones kThreads
+    const int adders = V == 1 ? add_threads(4 * n4) : V == 2 ? add_threads(2048) : kThreads, held = V == 1 ? 4 * blockDim.x : 4 * V * kThreads;
+    constexpr int MOST = V == 1 ? 8 : V == 2 ? 16 : 4 * V;
+    float ss = 0.f;
+    if (threadIdx.x < adders) {
+        float e[MOST];                                     // all loads before the chain of additions
+#pragma unroll
+        for (int k = 0; k < MOST; k++) {
+            const int i = threadIdx.x + k * adders;
+            e[k] = V > 1 || i < held ? row[i] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < MOST; k++) ss += e[k] * e[k];
+    }
+    return block_sum(ss, red);                             // whose barriers also keep the row until all have read it
+}
+
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads)
 rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ gain, float eps,
                        T* __restrict__ out, const float* __restrict__ gain2, float eps2, int d) {
+    extern __shared__ __align__(16) float row[];
     __shared__ float red[32];
     const int n4 = d >> 2;
     float4 g[V], v[V], h[V];
@@ -185,7 +281,6 @@ rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const
     griddep_launch();
     float* xr = x + (int64_t)blockIdx.x * d;
     const float* yr = y + (int64_t)blockIdx.x * d;
-    float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < V; k++) {
         const int i = threadIdx.x + k * blockDim.x;
@@ -194,12 +289,8 @@ rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const
             h[k] = load4(xr + 4 * i);
         }
     }
-#pragma unroll
-    for (int k = 0; k < V; k++)
-        if (threadIdx.x + k * blockDim.x < n4) ss += (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
-    const float scale = rsqrtf(block_sum(ss, red) / (float)d + eps);
+    const float scale = rsqrtf(squares_by_element<V>(v, n4, row, red) / (float)d + eps);
     T* orow = out ? out + (int64_t)blockIdx.x * d : nullptr;
-    float s2 = 0.f;
 #pragma unroll
     for (int k = 0; k < V; k++) {
         const int i = threadIdx.x + k * blockDim.x;
@@ -208,19 +299,21 @@ rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const
             h[k].z += v[k].z * scale * g[k].z; h[k].w += v[k].w * scale * g[k].w;
             store4(xr + 4 * i, h[k]);
             if (orow && !gain2) store4(orow + 4 * i, h[k]);
-            s2 += (h[k].x * h[k].x + h[k].y * h[k].y) + (h[k].z * h[k].z + h[k].w * h[k].w);
         }
     }
     if (!orow || !gain2) return;
-    const float scale2 = rsqrtf(block_sum(s2, red) / (float)d + eps2);
 #pragma unroll
     for (int k = 0; k < V; k++) {
         const int i = threadIdx.x + k * blockDim.x;
-        if (i < n4) {
-            const float4 b = load4(gain2 + 4 * i);
-            store4(orow + 4 * i, make_float4(h[k].x * scale2 * b.x, h[k].y * scale2 * b.y, h[k].z * scale2 * b.z,
-                                             h[k].w * scale2 * b.w));
-        }
+        if (i < n4) g[k] = load4(gain2 + 4 * i);
+    }
+    const float scale2 = rsqrtf(squares_by_element<V>(h, n4, row, red) / (float)d + eps2);
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i < n4)
+            store4(orow + 4 * i, make_float4(h[k].x * scale2 * g[k].x, h[k].y * scale2 * g[k].y, h[k].z * scale2 * g[k].z,
+                                             h[k].w * scale2 * g[k].w));
     }
 }
 
@@ -481,10 +574,10 @@ bool rows_fit(int d, P... p) {
     const uintptr_t addr = ((uintptr_t)p | ...);
     return (d & 3) == 0 && d <= kThreads * 4 * kVec && !(addr & 15);
 }
-// go(integral_constant<int, V>) with the V of a width: 1, 2, 4 or 8 float4 a thread
+// go(integral_constant<int, V>) with the V of a width: 1, 2, 4 or 8 float4 for each of `threads` threads
 template <typename F>
-void by_width(int d, F go) {
-    const int need = (d / 4 + row_threads(d) - 1) / row_threads(d);
+void by_width(int d, int threads, F go) {
+    const int need = (d / 4 + threads - 1) / threads;
     if (need <= 1) go(std::integral_constant<int, 1>());
     else if (need <= 2) go(std::integral_constant<int, 2>());
     else if (need <= 4) go(std::integral_constant<int, 4>());
@@ -500,17 +593,21 @@ extern "C" int kllm_rmsnorm_add(void* x, const void* y, const void* gain, float 
     if (d <= 0) KLLM_FAIL("rmsnorm_add: width %d must be positive", d);
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype != KLLM_F32 && dtype != KLLM_BF16) KLLM_FAIL("rmsnorm_add: unknown element type %d", dtype);
+    const int threads = add_threads(d);
     if (rows_fit(d, x, y, gain, out, gain2)) {
-        auto go = [&](auto element, auto size) {
+        const int block = add_block(d);
+        auto go = [&](auto element) {
             using T = decltype(element);
-            kllm_launch((rmsnorm_add_row_kernel<T, decltype(size)::value>), dim3(n_rows), dim3(row_threads(d)), 0, s, (float*)x,
-                        (const float*)y, (const float*)gain, eps, (T*)out, (const float*)gain2, eps2, d);
+            by_width(d, block, [&](auto size) {
+                constexpr int V = decltype(size)::value;
+                kllm_launch((rmsnorm_add_row_kernel<T, V>), dim3(n_rows), dim3(block), (size_t)16 * V * block, s, (float*)x,
+                            (const float*)y, (const float*)gain, eps, (T*)out, (const float*)gain2, eps2, d);
+            });
         };
-        if (dtype == KLLM_F32) by_width(d, [&](auto size) { go(float(), size); });
-        else by_width(d, [&](auto size) { go(bf16(), size); });
+        if (dtype == KLLM_F32) go(float());
+        else go(bf16());
         KLLM_LAUNCH_STATUS();
     }
-    const int threads = d <= 512 ? 64 : (d <= 2048 ? 128 : kThreads);
     if (dtype == KLLM_F32)
         kllm_launch((rmsnorm_add_kernel<float>), dim3(n_rows), dim3(threads), 0, s, (float*)x, (const float*)y,
                     (const float*)gain, eps, (float*)out, (const float*)gain2, eps2, d);
@@ -527,14 +624,30 @@ extern "C" int kllm_add_rmsnorm(void* x, const void* res, void* out, const void*
     if (n_rows <= 0) return 0;
     if (d <= 0) KLLM_FAIL("rmsnorm: width %d must be positive", d);
     cudaStream_t s = (cudaStream_t)stream;
-    if ((dtype == KLLM_F32 || dtype == KLLM_BF16) && (res == nullptr || res_dtype == KLLM_F32) && rows_fit(d, x, res, gain, out)) {
-        auto go = [&](auto element, auto size) {
-            using T = decltype(element);
-            kllm_launch((add_rmsnorm_row_kernel<T, decltype(size)::value>), dim3(n_rows), dim3(row_threads(d)), 0, s, (float*)x,
-                        (const float*)res, (T*)out, (const float*)gain, rows, d, eps);
+    if (dtype == KLLM_BF16 && rows && (res == nullptr || res_dtype == KLLM_F32) && d <= kThreads * 4 * kVec) {
+        auto go = [&](auto size) {
+            kllm_launch((rmsnorm_chosen_kernel<decltype(size)::value>), dim3(n_rows), dim3(kThreads), 0, s, (const float*)x,
+                        (const float*)res, (bf16*)out, (const float*)gain, rows, d, eps);
         };
-        if (dtype == KLLM_F32) by_width(d, [&](auto size) { go(float(), size); });
-        else by_width(d, [&](auto size) { go(bf16(), size); });
+        const int need = (d + kThreads - 1) / kThreads;
+        if (need <= 2) go(std::integral_constant<int, 2>());
+        else if (need <= 8) go(std::integral_constant<int, 8>());
+        else if (need <= 16) go(std::integral_constant<int, 16>());
+        else go(std::integral_constant<int, 32>());
+        KLLM_LAUNCH_STATUS();
+    }
+    if ((dtype == KLLM_F32 || dtype == KLLM_BF16) && (res == nullptr || res_dtype == KLLM_F32) && rows_fit(d, x, res, gain, out)) {
+        auto go = [&](auto element, auto lanes) {
+            using T = decltype(element);
+            by_width(d, row_threads(d), [&](auto size) {
+                kllm_launch((add_rmsnorm_row_kernel<T, decltype(size)::value, decltype(lanes)::value>), dim3(n_rows),
+                            dim3(row_threads(d)), lanes ? (size_t)d : 0, s, (float*)x, (const float*)res, (T*)out, (const float*)gain,
+                            rows, d, eps);
+            });
+        };
+        if (dtype == KLLM_F32) go(float(), std::false_type());
+        else if (d <= kLanesMost) go(bf16(), std::true_type());
+        else go(bf16(), std::false_type());
         KLLM_LAUNCH_STATUS();
     }
     if (res == nullptr) res_dtype = dtype;

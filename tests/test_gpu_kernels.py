@@ -120,6 +120,76 @@ def test_add_rmsnorm_of_a_row_does_not_depend_on_the_number_of_rows(d):
         assert torch.equal(x_row, outs[0][0]) and torch.equal(out_row, outs[0][1])
 
 
+def _short(rng, *shape):
+    """Numbers of 11 bits over six powers of two: their squares are exact in float32, so that only the order of a sum's
+    additions rounds."""
+    m = rng.integers(1, 2048, size=shape) * rng.choice([-1, 1], size=shape)
+    return (m * 2.0 ** rng.integers(-14, -8, size=shape)).astype(np.float32)
+
+
+@pytest.mark.parametrize("d", [132, 2048, 2047 // 4 * 4])
+def test_the_lanes_of_a_warp_add_a_bfloat16_row(d):
+    """Widths up to 2048, bfloat16 out: lane l adds the squares of the float4 l, l + 32, ..., and the lanes are added in
+    halves, whatever number of threads loads the row.  To the bit, over rows enough for another order to show."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(d)
+    n, eps = 1200, 1e-5
+    x0 = _short(rng, n, d)
+    gain = (1 + 0.2 * rng.standard_normal(d)).astype(np.float32)
+    q = (x0 * x0).reshape(n, d // 4, 4)
+    q = (q[..., 0] + q[..., 1]) + (q[..., 2] + q[..., 3])
+    lanes = np.zeros((n, 32), np.float32)
+    for i in range(0, d // 4, 32):
+        part = q[:, i:i + 32]
+        lanes[:, :part.shape[1]] += part
+    for half in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[:, np.arange(32) ^ half]
+    want = (dev(x0) * _scale_of(lanes[:, :1], d, eps) * dev(gain)).bfloat16()
+    out = torch.empty((n, d), dtype=torch.bfloat16, device="cuda")
+    kernels.add_rmsnorm(dev(x0), None, out, dev(gain), eps)
+    assert torch.equal(out, want)
+
+
+def _add_up(a, threads):
+    """Sums over the last dimension [..., d] of exact squares: thread t adds the elements t, t + threads, ..., the lanes of a
+    warp and then the warps are added in halves."""
+    sums = np.zeros(a.shape[:-1] + (threads,), np.float32)
+    for i in range(0, a.shape[-1], threads):
+        part = a[..., i:i + threads]
+        sums[..., :part.shape[-1]] += part * part
+    lanes = sums.reshape(a.shape[:-1] + (threads // 32, 32))
+    for half in (16, 8, 4, 2, 1):
+        lanes = lanes + lanes[..., np.arange(32) ^ half]
+    warps = np.zeros(a.shape[:-1] + (32,), np.float32)
+    warps[..., :threads // 32] = lanes[..., 0]
+    for half in (16, 8, 4, 2, 1):
+        warps = warps + warps[..., np.arange(32) ^ half]
+    return warps[..., :1]
+
+
+def _scale_of(squares, d, eps):
+    return torch.rsqrt(dev(squares) / torch.tensor(float(d), device="cuda") + torch.tensor(eps, device="cuda"))
+
+
+@pytest.mark.parametrize("d", [7, 132, 512, 513, 2048, 2052, 5120, 8192])
+def test_chosen_rows_and_output_norms_are_added_element_by_element(d):
+    """To the bit: the bfloat16 norm of chosen rows (256 threads) and the norm of a sublayer's output (64, 128 or 256 threads by
+    the width), one element a thread at a time, whatever the address of a row."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(d)
+    n, eps = 1200 if d <= 2052 else 400, 1e-5
+    x0 = _short(rng, n, d)
+    gain = (1 + 0.2 * rng.standard_normal(d)).astype(np.float32)
+    order = rng.permutation(n).astype(np.int32)
+    out = torch.empty((n, d), dtype=torch.bfloat16, device="cuda")
+    kernels.add_rmsnorm(dev(x0), None, out, dev(gain), eps, rows=dev(order))
+    want = (dev(x0) * _scale_of(_add_up(x0, 256), d, eps) * dev(gain)).bfloat16()[dev(order).long()]
+    assert torch.equal(out, want)
+    ones, x = torch.ones(d, device="cuda"), torch.zeros((n, d), device="cuda")
+    kernels.rmsnorm_add(x, dev(x0), ones, eps)
+    assert torch.equal(x, dev(x0) * _scale_of(_add_up(x0, 64 if d <= 512 else 128 if d <= 2048 else 256), d, eps))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("d", [100, 2048 + 16, 7])
 def test_add_rmsnorm(dtype, d):
