@@ -568,11 +568,12 @@ extern "C" int kllm_embed_layernorm(float* x, const void* table, const int* ids,
 }
 
 namespace {
-// Widths and addresses (NULL counts as aligned) that the kernels with the row in registers take.
+// Widths and addresses (NULL counts as aligned) that the kernels with the row in registers take: four elements at a time, of
+// float32 rows and of `out` in its own element type.
 template <typename... P>
-bool rows_fit(int d, P... p) {
+bool rows_fit(int d, int dtype, const void* out, P... p) {
     const uintptr_t addr = ((uintptr_t)p | ...);
-    return (d & 3) == 0 && d <= kThreads * 4 * kVec && !(addr & 15);
+    return (d & 3) == 0 && d <= kThreads * 4 * kVec && !(addr & 15) && !((uintptr_t)out & (dtype == KLLM_BF16 ? 7 : 15));
 }
 // go(integral_constant<int, V>) with the V of a width: 1, 2, 4 or 8 float4 for each of `threads` threads
 template <typename F>
@@ -594,7 +595,7 @@ extern "C" int kllm_rmsnorm_add(void* x, const void* y, const void* gain, float 
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype != KLLM_F32 && dtype != KLLM_BF16) KLLM_FAIL("rmsnorm_add: unknown element type %d", dtype);
     const int threads = add_threads(d);
-    if (rows_fit(d, x, y, gain, out, gain2)) {
+    if (rows_fit(d, dtype, out, x, y, gain, gain2)) {
         const int block = add_block(d);
         auto go = [&](auto element) {
             using T = decltype(element);
@@ -636,7 +637,7 @@ extern "C" int kllm_add_rmsnorm(void* x, const void* res, void* out, const void*
         else go(std::integral_constant<int, 32>());
         KLLM_LAUNCH_STATUS();
     }
-    if ((dtype == KLLM_F32 || dtype == KLLM_BF16) && (res == nullptr || res_dtype == KLLM_F32) && rows_fit(d, x, res, gain, out)) {
+    if ((dtype == KLLM_F32 || dtype == KLLM_BF16) && (res == nullptr || res_dtype == KLLM_F32) && rows_fit(d, dtype, out, x, res, gain)) {
         auto go = [&](auto element, auto lanes) {
             using T = decltype(element);
             by_width(d, row_threads(d), [&](auto size) {
