@@ -124,11 +124,9 @@ __device__ __noinline__ void plain_rows(const Args& a, const Tile& t) {
             for (int i = 0; i < D; i++) sc = fmaf(q[i], a.kcache[at + lane + 32 * i], sc);
             sc = warp_sum(sc) * a.scale + slope * (float)(k - p);
             const float m_new = fmaxf(m, sc);
-            float alpha = 1.f, w = 0.f;
-            if (m_new != -INFINITY) {
-                alpha = expf(m - m_new);
-                w = expf(sc - m_new);
-            }
+            // while the scores seen are all -inf the maximum is no base: such a key weighs 0, and one whose score is NaN stays NaN
+            // (fmaxf passes it over)
+            const float alpha = m_new == -INFINITY ? 1.f : expf(m - m_new), w = expf(sc - (m_new == -INFINITY ? 0.f : m_new));
             l = l * alpha + w;
             m = m_new;
 #pragma unroll

@@ -369,6 +369,71 @@ def test_float32_portions_with_values_beyond_the_three_parts(H, G, hd, page, val
     assert np.isposinf(got[odd]).all() if np.isinf(value) else np.all(np.abs(got[odd] / want[odd] - 1) < 1e-4)
 
 
+def attention_rows(q, k, v, first, window, segment, keep, slopes, sinks):
+    """Attention in 64 bits row by row over the visible keys alone, so that a value that is not finite counts where it is
+    seen and nowhere else.  q [n, H, hd] of positions first, first + 1, ...; k, v [L, G, hd]."""
+    H, G, hd = q.shape[1], k.shape[1], q.shape[2]
+    q, k, v = (a.astype(np.float64) for a in (q, k, v))
+    out = np.zeros(q.shape)
+    with np.errstate(all="ignore"):
+        for i, h in np.ndindex(q.shape[:2]):
+            p, g = first + i, h // (H // G)
+            lo = max(p + 1 - window if window else 0, p - p % segment if segment else 0, 0)
+            at = [j for j in range(p + 1) if j >= lo or j < keep]
+            sc = k[at, g] @ q[i, h] / math.sqrt(hd) + (0.0 if slopes is None else slopes[h] * (np.array(at) - p))
+            m = np.max(sc if sinks is None else np.append(sc, sinks[h]))
+            w = np.exp(sc - m)
+            total = w.sum() + (0.0 if sinks is None else np.exp(sinks[h] - m))
+            out[i, h] = (w[:, None] * v[at, g]).sum(axis=0) / total
+    return out.reshape(len(q), H * hd)
+
+
+def same_as_arithmetic(got, want):
+    got = got.cpu().numpy().astype(np.float64)
+    for kind in (np.isnan, np.isposinf, np.isneginf):
+        assert np.array_equal(kind(got), kind(want)), f"{kind.__name__}: {kind(got).sum()} of {got.size}, {kind(want).sum()} wanted"
+    plain_ones = np.isfinite(want)
+    assert plain_ones.any()
+    close(torch.from_numpy(np.where(plain_ones, got, 0)), np.where(plain_ones, want, 0), "float32")
+
+
+@pytest.mark.parametrize("H,G,hd", [(8, 2, 64), (3, 1, 128)])
+@pytest.mark.parametrize("options", ["none", "window", "segment", "keep", "slopes", "sinks"])
+@pytest.mark.parametrize("where,value", [("k", np.nan), ("k", np.inf), ("k", -np.inf), ("q", np.nan), ("q", np.inf), ("q", 1e33),
+                                         ("v", np.nan), ("v", np.inf)])
+def test_float32_portions_row_by_row(H, G, hd, options, where, value):
+    """Portions in float32 whose rows are computed again key by key because a value has no three bfloat16 parts, under every
+    mask and term of a score.  The value sits in the first key, which is the first that a row sees, and in one in the middle
+    (k and v), or in two queries."""
+    from kllm_b200 import kernels
+    from types import SimpleNamespace
+    rng = np.random.default_rng(hd + len(options))
+    lengths, n_new, page = [150, 70], [131, 70], 16
+    window, segment, keep = 40 if options in ("window", "keep") else 0, 48 if options == "segment" else 0, 5 if options == "keep" else 0
+    slopes = (0.02 * (1 + np.arange(H))).astype(np.float32) if options == "slopes" else None
+    sinks = rng.standard_normal(H).astype(np.float32) if options == "sinks" else None
+    ks, vs, qs = ([rng.standard_normal((L, heads, hd)).astype(np.float32) for L in lengths] for heads in (G, G, H))
+    qs = [0.3 * q for q in qs]
+    for a, n, places in ((ks, "k", (0, 90)), (vs, "v", (0, 90)), (qs, "q", (60, 100))):
+        if n == where:
+            for at in places:
+                a[0][at, 0, 7] = value
+    want = np.concatenate([attention_rows(q[L - nn:], k, v, L - nn, window, segment, keep, slopes, sinks)
+                           for q, k, v, L, nn in zip(qs, ks, vs, lengths, n_new)])
+    kc, vc, table = paged(ks, vs, page, sum(-(-L // page) for L in lengths) + 3, rng, "float32", lengths)
+    q = dev(np.concatenate([q[L - nn:].reshape(nn, H * hd) for q, L, nn in zip(qs, lengths, n_new)]).astype(np.float32))
+    out = torch.empty_like(q)
+    ctx = SimpleNamespace(n_tokens=sum(n_new), n_requests=2, q_start=dev(np.array([0, 131, 201], np.int32)),
+                          start_pos=dev(np.array([19, 0], np.int32)), host_n_new=n_new, all_single=False, max_ctx=150, split_bound=0)
+    kernels.attention_simt(out, q, kc, vc, ctx, table, H, G, hd, window, 1.0 / math.sqrt(hd), segment=segment, keep=keep,
+                           score_slopes=None if slopes is None else dev(slopes), sinks=None if sinks is None else dev(sinks))
+    if where == "q" and value == 1e33:
+        close(out, want, "float32")                        # one key takes it all
+    else:
+        assert not np.isfinite(want).all()
+        same_as_arithmetic(out, want)
+
+
 @pytest.mark.parametrize("gs", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("hd", [64, 128])
 @pytest.mark.parametrize("window", [None, 300])
