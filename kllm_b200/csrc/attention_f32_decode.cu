@@ -126,13 +126,12 @@ attn_f32_decode_kernel(const Args a) {
             sc[u] = v < hi ? d[0] * a.scale : -INFINITY;
             mx = fmaxf(mx, sc[u]);
         }
-        const float m_new = fmaxf(m, mx);
-        float alpha = 1.f, p[UNROLL] = {};
-        if (m_new != -INFINITY) {
-            alpha = expf(m - m_new);                       // 0 while nothing had been seen
+        // 0 while nothing had been seen.  A maximum of -inf is no base: its keys weigh 0, and a score that is NaN, which fmaxf passes
+        // over, stays NaN.
+        const float m_new = fmaxf(m, mx), base = m_new == -INFINITY ? 0.f : m_new, alpha = m_new == -INFINITY ? 1.f : expf(m - m_new);
+        float p[UNROLL];
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++) p[u] = expf(sc[u] - m_new);
-        }
+        for (int u = 0; u < UNROLL; u++) p[u] = expf(sc[u] - base);
         l = l * alpha + ((p[0] + p[1]) + (p[2] + p[3]));
         m = m_new;
 #pragma unroll
@@ -173,7 +172,7 @@ attn_f32_decode_kernel(const Args a) {
         float4 r = zero4;
 #pragma unroll
         for (int i = 0; i < GROUPS; i++) {
-            const float w = sm[i][h] == -INFINITY ? 0.f : expf(sm[i][h] - M);      // a group without a key
+            const float w = sl[i][h] == 0.f ? 0.f : expf(sm[i][h] - M);            // 0: a group without a key, or with weights of 0 alone
             const float4 x = *reinterpret_cast<const float4*>(&so[i][h][c]);
             L += sl[i][h] * w;
             r.x += x.x * w; r.y += x.y * w; r.z += x.z * w; r.w += x.w * w;

@@ -686,6 +686,29 @@ def test_float32_fused_decode_attention(gs, hd, window):
             assert torch.equal(vc[pg, :, slot].cpu(), torch.from_numpy(vnew[s].reshape(G, hd)))
 
 
+@pytest.mark.parametrize("gs,hd", [(1, 64), (8, 64), (16, 64), (4, 128)])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("L,keys", [(10, [8]), (258, [256]), (265, list(range(260, 264))), (300, list(range(256))), (70, [0])])
+def test_float32_fused_decode_attention_with_keys_that_are_not_finite(gs, hd, value, L, keys):
+    """Cached keys that are not finite: the only ones of a group of lanes (in the first range or the last), the whole of a
+    range, the first key.  Every result is what arithmetic gives: NaN is not lost where a maximum passes it over, and a
+    key that weighs 0 leaves the others alone."""
+    from kllm_b200 import kernels
+    G, page, H, rng = 2, 16, 2 * gs, np.random.default_rng(gs + hd + L)
+    k, v = (rng.standard_normal((L, G, hd)).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((1, H, hd)).astype(np.float32)
+    k[keys, 0, 7] = value
+    want = attention_rows(q, k, v, L - 1, 0, 0, 0, None, None)
+    knew, vnew = k[-1:].reshape(1, G * hd), v[-1:].reshape(1, G * hd)
+    kc, vc, table = paged([k], [v], page, -(-L // page) + 3, rng, "float32", [L])
+    cos_sin = dev(np.concatenate([np.ones((512, hd // 2)), np.zeros((512, hd // 2))], 1).astype(np.float32))     # no rotation
+    out = torch.empty((1, H * hd), device="cuda")
+    counters = torch.zeros(64, dtype=torch.int32, device="cuda")
+    kernels.attention_decode_f32(out, dev(q.reshape(1, -1)), dev(knew), dev(vnew), cos_sin, kc, vc, dev(np.array([L - 1], np.int32)),
+                                 table, counters, H, G, hd, 0, 1.0 / math.sqrt(hd), 512)
+    same_as_arithmetic(out, want)
+
+
 def test_tcgen05_form_follows_the_measurements():
     from kllm_b200 import kernels
     assert kernels.tcgen05_form(128, 4, 8, 2048, 1, 2048) == "tmem"
