@@ -912,6 +912,25 @@ def test_skinny_gemm_prologues_and_epilogues(n, N, K):
     close(got, plain.round_act_bf16(plain.rmsnorm(big[:n], gain, 1e-5)) @ ws.T, "bfloat16", "norm prologue, no gather")
 
 
+@pytest.mark.parametrize("K", [128, 2048, 5632])
+def test_float32_skinny_gemm_adds_its_parts_of_k_in_pairs(K):
+    """The 16 warps' sums, one product each here, meet in four rounds of additions: to the bit."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(K)
+    N, steps = 96, K // 32
+    per = -(-steps // 16)
+    firsts = [w * per * 32 for w in range(16)]
+    w = rng.standard_normal((N, K)).astype(np.float32)
+    x = np.zeros((2, K), np.float32)
+    x[0, [k for k in firsts if k < K]] = 1.0               # products are exact, the other values of k add 0
+    v = [w[:, k] if k < K else np.zeros(N, np.float32) for k in firsts]
+    while len(v) > 1:
+        half = len(v) // 2
+        v = [a + b for a, b in zip(v[:half], v[half:])]
+    got = kernels.skinny_gemm(dev(w), x=dev(x), epilogue="f32").cpu().numpy()
+    assert np.array_equal(got[0], v[0]) and not got[1].any()
+
+
 @pytest.mark.parametrize("n", [1, 3, 8])
 @pytest.mark.parametrize("N,K", [(48, 128), (2560, 2048), (101, 384), (2048, 5632), (33, 4096), (2, 256)])
 def test_float32_skinny_gemm_prologues_and_epilogues(n, N, K):
