@@ -274,20 +274,23 @@ gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 // both, either CTA's producer loads its own operands and announces them on the leader's barriers.  A column's gate and up values
 // lie 64 lanes apart: the two warps that read them exchange half of each through shared memory and finish half of the rows each.
 // (Interleaved by 16 rows they would be a shuffle apart, but eight copies of 16 rows a stage instead of two took longer than
-// the products.)  The results meet in shared memory and leave as whole 128-byte rows.
+// the products.)  The results meet in shared memory and leave as whole 128-byte rows.  Sixteen warps finish them: what a warp waits for
+// is its chain of exchange, expf and division, and with eight a tile of 256 rows took 9 us, longer than the products of K up to
+// 1300 that it runs beside (768 x 3072, 4096 rows: 60.9 us with eight warps, 31.6 with sixteen, 38.0 for the kernel of
+// CTAs alone that this one replaced; 1024 x 2816: 45.0, 33.9, 40.5; 2048 x 5632: 124.8, 120.8, 139.8).
 //
 // A tile's rows are the fastest in the order of tiles, so that neighbouring pairs share W's rows; x stays in L2.  The last tile of
 // rows is moved back to end with x and leaves what it shares with the tile before to that one: rows behind x's end, which the copy
 // fills with zeros, took longer than rows that are there (64 rows in a tile of 256: 27 us, in one of 64: 14).
 constexpr int PAIR_F = 128;
 constexpr int PAIR_STAGE_ROW = 144;                                  // bytes of a row of results in shared memory, 128 in use
-constexpr int PAIR_SWAP_BYTES = 4 * 2 * 16 * 32 * 4;                 // what the four pairs of epilogue warps exchange
+constexpr int PAIR_SWAP_BYTES = 8 * 2 * 8 * 32 * 4;                  // what the eight pairs of epilogue warps exchange
 constexpr int PAIR_OUT_BYTES = MAX_BN * PAIR_STAGE_ROW + PAIR_SWAP_BYTES;
 constexpr int PAIR_SMEM = 1024 + PAIR_OUT_BYTES + 5 * (A_BYTES + MAX_BN / 2 * 128);
-constexpr int PAIR_EPI_WARPS = 8;
+constexpr int PAIR_EPI_WARPS = 16, PAIR_THREADS = 64 + 32 * PAIR_EPI_WARPS;
 
 template <int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_up, bf16* __restrict__ y, int64_t ldy, int M, int N, int K, int bn, int stages,
                  float act_limit, float act_alpha, int* status) {
@@ -423,51 +426,59 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     } else {
         // ---- epilogue ----
         griddep_wait();
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        // four warps of each quarter of the lanes; set `part` of them has a quarter of the tile's rows of x, 16 at a time
+        const int quarter = warp & 3, part = (warp - 2) >> 2;
         const unsigned lane_base = (unsigned)(quarter * 32) << 16;
-        const int chunks = (bn + 31) / 32, c_lo = half == 0 ? 0 : (chunks + 1) / 2, c_hi = half == 0 ? (chunks + 1) / 2 : chunks;
+        const int c_lo = bn / 16 * part / 4, c_hi = bn / 16 * (part + 1) / 4;
         // quarters 0 and 1 hold the gate values of columns 0-31 and 32-63, quarters 2 and 3 the up values
         const bool up = quarter >= 2;
-        const int group = quarter & 1, swap_id = 3 + half * 2 + group, in_half = threadIdx.x - 64 - half * 128;
-        float* swap = reinterpret_cast<float*>(results + MAX_BN * PAIR_STAGE_ROW) + (half * 2 + group) * 2 * 16 * 32 + lane;
+        const int group = quarter & 1, swap_id = 5 + part * 2 + group, in_part = threadIdx.x - 64 - part * 128;
+        float* swap = reinterpret_cast<float*>(results + MAX_BN * PAIR_STAGE_ROW) + (part * 2 + group) * 2 * 8 * 32 + lane;
         int acc = 0;
         unsigned acc_ph = 0;
         for (int tile = first; tile < tiles; tile += pairs) {
             const int t_own = tile % t_tiles * bn, t0 = min(t_own, max(0, M - bn)), f0 = tile / t_tiles * PAIR_F + (int)rank * 64;
-            // all threads of the half go on or none; its results of the tile before have left shared memory
-            if (!half_all(1 + half, mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, status, 4))) break;
+            // all threads of the set go on or none; its results of the tile before have left shared memory
+            if (!half_all(1 + part, mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, status, 4))) break;
             tc_fence_after();
             const unsigned t = tmem + lane_base + (unsigned)(acc * MAX_BN);
+            float v[16];
+            if (c_lo < c_hi) tmem_ld16(t + c_lo * 16, v);
 #pragma unroll 1
             for (int c = c_lo; c < c_hi; c++) {
-                float v[32];
-                tmem_ld32(t + c * 32, v);
                 tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; i++) swap[(up * 16 + i) * 32] = up ? v[i] : v[16 + i];
+                for (int i = 0; i < 8; i++) swap[(up * 8 + i) * 32] = up ? v[i] : v[8 + i];
                 named_sync(swap_id, 64);
-                bf16* o = reinterpret_cast<bf16*>(results + (c * 32 + up * 16) * PAIR_STAGE_ROW) + group * 32 + lane;
+                // the gate warp finishes the first 8 of the 16 rows of x, the up warp the others
+                float g[8], u[8], den[8];
 #pragma unroll
-                for (int i = 0; i < 16; i++) {             // the gate warp finishes the chunk's first 16 rows of x, the up warp the others
-                    const float got = swap[(!up * 16 + i) * 32];
-                    float g = up ? got : v[i], u = up ? v[16 + i] : got;
-                    if (EPI == EPI_CLAMPED) {
-                        g = fminf(g, act_limit);
-                        u = fminf(fmaxf(u, -act_limit), act_limit);
-                        g = g / (1.f + expf(-act_alpha * g)) * (u + 1.f);
-                    } else {
-                        g = silu_mul(g, u);
-                    }
-                    o[i * (PAIR_STAGE_ROW / 2)] = __float2bfloat16_rn(g);
+                for (int i = 0; i < 8; i++) {
+                    const float got = swap[(!up * 8 + i) * 32];
+                    g[i] = up ? got : v[i];
+                    u[i] = up ? v[8 + i] : got;
                 }
                 named_sync(swap_id, 64);                   // both have read before either writes again
+                if (c + 1 < c_hi) tmem_ld16(t + (c + 1) * 16, v);
+                // a division checks for what its short form cannot do, one after the other: what leads to it is done for all 8 before
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    if (EPI == EPI_CLAMPED) {
+                        g[i] = fminf(g[i], act_limit);
+                        u[i] = fminf(fmaxf(u[i], -act_limit), act_limit) + 1.f;
+                    }
+                    den[i] = 1.f + expf(EPI == EPI_CLAMPED ? -act_alpha * g[i] : -g[i]);
+                }
+                bf16* o = reinterpret_cast<bf16*>(results + (c * 16 + up * 8) * PAIR_STAGE_ROW) + group * 32 + lane;
+#pragma unroll
+                for (int i = 0; i < 8; i++) o[i * (PAIR_STAGE_ROW / 2)] = __float2bfloat16_rn(g[i] / den[i] * u[i]);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(leader_addr(&bar_acc_empty[acc]));
-            named_sync(1 + half, 128);
-            const int r_hi = min(min(c_hi * 32, bn), M - t0);
-            for (int i = in_half + max(c_lo * 32, t_own - t0) * 8; i < r_hi * 8; i += 128) {
+            named_sync(1 + part, 128);
+            const int r_hi = min(c_hi * 16, M - t0);
+            for (int i = in_part + max(c_lo * 16, t_own - t0) * 8; i < r_hi * 8; i += 128) {
                 const int r = i >> 3, f = f0 + (i & 7) * 8;
                 const uint4 w = *reinterpret_cast<const uint4*>(results + r * PAIR_STAGE_ROW + (i & 7) * 16);
                 bf16* o = y + (int64_t)(t0 + r) * ldy + f;
@@ -563,7 +574,7 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap&
     const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
     int stages = (PAIR_SMEM - 1024 - PAIR_OUT_BYTES) / (A_BYTES + bn * 64);
     if (stages > MAX_STAGES) stages = MAX_STAGES;
-    kllm_launch((gemm_pair_kernel<EPI>), dim3(grid), dim3(THREADS), PAIR_SMEM, stream, mx, mw, mu, (bf16*)y, ldy, M, N, K, bn, stages,
+    kllm_launch((gemm_pair_kernel<EPI>), dim3(grid), dim3(PAIR_THREADS), PAIR_SMEM, stream, mx, mw, mu, (bf16*)y, ldy, M, N, K, bn, stages,
                 act_limit, act_alpha, status);
     KLLM_LAUNCH_STATUS();
 }

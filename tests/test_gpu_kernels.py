@@ -1022,6 +1022,26 @@ def test_tcgen05_gated_tiles_of_rows(M, N, K, bn):
     kernels.check_status("cuda")
 
 
+def test_tcgen05_gated_tiles_of_every_height_give_the_same_bits():
+    """Four sets of warps finish a quarter of a tile's rows each, 16 at a time: tiles of 16 rows, where three of the sets have
+    none, to 256, over several tiles a pair, against the formula and one another."""
+    from kllm_b200 import kernels
+    rng = np.random.default_rng(11)
+    M, N, K = 531, 10000, 72
+    x = rng.standard_normal((M, K)).astype(np.float32)
+    w, w2 = ((rng.standard_normal((N, K)) * 0.1).astype(np.float32) for _ in range(2))
+    xs, ws, w2s = (as_stored(a, "bfloat16") for a in (x, w, w2))
+    xt, wt, w2t = (dev(a, torch.bfloat16) for a in (x, w, w2))
+    want = plain.silu(xs @ ws.T) * (xs @ w2s.T)
+    first = None
+    for bn in range(16, 257, 16):
+        got = kernels.gemm(xt, wt, weight_up=w2t, epilogue="swiglu", bn=bn)
+        close(got, want, "bfloat16", f"tiles of {bn} rows")
+        first = got if first is None else first
+        assert torch.equal(got, first), bn
+    kernels.check_status("cuda")
+
+
 def test_tcgen05_gemm_rows_do_not_depend_on_the_batch():
     """A row's result is the same bits alone in a small batch and among many rows."""
     from kllm_b200 import kernels
