@@ -1539,7 +1539,7 @@ def design_comparison(args):
                         kernels.skinny_gemm(w[:ff], weight_up=w[ff:], x=h, epilogue="swiglu", bias=b, bias_up=b, activation=act)
                         return
                     o = torch.empty((n, ff), dtype=tdt, device=dev)
-                    if b is None and tdt == torch.bfloat16 and kernels.gemm_pays(n, ff, "swiglu"):
+                    if b is None and tdt == torch.bfloat16 and kernels.gemm_pays(n, ff, "swiglu", K=width):
                         kernels.gemm(h, w[:ff], weight_up=w[ff:], epilogue="swiglu", out=o)
                         return
                     gu = kernels.linear(h, w, out_dtype=f32)
@@ -1684,7 +1684,7 @@ def design_comparison(args):
                         return
                     o = torch.empty((n, ff), dtype=tdt, device=dev)
                     epi = "clamped" if clamped else "swiglu"
-                    if tdt == torch.bfloat16 and kernels.gemm_pays(n, ff, epi):
+                    if tdt == torch.bfloat16 and kernels.gemm_pays(n, ff, epi, K=width):
                         kernels.gemm(h, w[:ff], weight_up=w[ff:], epilogue=epi, out=o, **kw)
                         return
                     gu = kernels.linear(h, w, out_dtype=f32)
@@ -1744,7 +1744,7 @@ def design_comparison(args):
                         kernels.skinny_gemm(w[:eff], weight_up=w[eff:], x=h, epilogue="swiglu")
                     else:
                         o = torch.empty((n, eff), dtype=tdt, device=dev)
-                        if tdt == torch.bfloat16 and kernels.gemm_pays(n, eff, "swiglu"):
+                        if tdt == torch.bfloat16 and kernels.gemm_pays(n, eff, "swiglu", K=width):
                             kernels.gemm(h, w[:eff], weight_up=w[eff:], epilogue="swiglu", out=o)
                         else:
                             gu = kernels.linear(h, w, out_dtype=f32)

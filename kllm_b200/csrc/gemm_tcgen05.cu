@@ -581,15 +581,14 @@ int launch_pair(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap&
 
 }  // namespace
 
-// Share of its time that a product keeps the tensor cores busy, in percent: full tiles / (waves x CTAs), for the gated epilogues
-// rows x column tiles / (pairs x what pair_plan counts).  Callers use it to choose between this kernel and the library product.
-extern "C" int kllm_gemm_tcgen05_efficiency(int M, int N, int epilogue) {
+// What a gated product of M rows and N columns runs as: rows of x in a tile, waves of tiles.
+extern "C" int kllm_gemm_tcgen05_pair_plan(int M, int N, int* bn, int* waves) {
+    *bn = *waves = 0;
     if (M <= 0 || N <= 0) return 0;
-    if (is_gated(epilogue)) return (int)(100.0 * M * ((double)N / PAIR_F) / ((double)(sm_count() / 2) * pair_plan(M, N).cost));
-    const double full = ((double)M / BM) * ((double)N / MAX_BN);
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + MAX_BN - 1) / MAX_BN);
-    const long long waves = (tiles + sm_count() - 1) / sm_count();
-    return (int)(100.0 * full / (double)(waves * sm_count()));
+    const PairPlan p = pair_plan(M, N);
+    *bn = p.bn;
+    *waves = (int)(p.cost / (p.bn + 100));
+    return 0;
 }
 
 // 1 if the kernel takes these sizes and addresses, else 0 (the caller then uses the

@@ -1428,7 +1428,7 @@ def prompt_layers(x: torch.Tensor, layers, n_layers: int, ctx, block_table: torc
     form = tcgen05_choice(head_dim, n_heads // n_kv, n_kv, n - singles, ctx.n_requests - singles, ctx.max_ctx)
     xn, qkv, attn, act = new(n, d), new(n, wide), new(n, q_dim), new(n, inter)
     gate_up = None
-    if not (gemm_pays(n, inter, "swiglu") and gemm_fits(xn, first[2][:inter], act, "swiglu", first[2][inter:])):
+    if not (gemm_pays(n, inter, "swiglu", K=d) and gemm_fits(xn, first[2][:inter], act, "swiglu", first[2][inter:])):
         gate_up = new(n, 2 * inter, dtype=torch.float32)
     name = "attention_tcgen05" + ("_ptmem" if form == "tmem" else "")
     used = [("norm", None, "kllm_add_rmsnorm"), ("rope", None, "kllm_rope_append"),
@@ -1527,30 +1527,46 @@ def gemm_fits(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue
     return bool(lib.kllm_gemm_tcgen05_fits(*_gemm_args(x, weight, weight_up, out, epilogue)))
 
 
-def gemm_pays(n: int, N: int, epilogue: str = "bf16", least: int = 75) -> bool:
+def gemm_pays(n: int, N: int, epilogue: str = "bf16", least: int = 75, K: int = 2048) -> bool:
     """Whether ``gemm`` is the faster route.  Its tiles of 128 rows x 256 accumulator columns have to keep the tensor cores
     of all SMs busy for at least ``least`` percent of the product's time (full tiles over waves x SMs); below that the
-    library product adapts its tiling better.  The gated epilogues run on pairs of CTAs in tiles that follow the rows, and
-    take the library's activation kernel in: there the line lies at 43 percent of what the kernel's own count of its time
-    allows.  (width 2048, 5632 columns: 200 rows 39 percent, 20.0 us against 16.3, 300: 42, 20.9 and 19.5, 400: 49, 22.9 and
-    23.6, 845: 34.2 and 40.7; 4096 x 14336: 128 rows 42 percent, 49 us against 55; 4096 x 11008: 128 rows 33 percent, 46
-    and 41, 300: 45, 58 and 61.)  Same arithmetic as kllm_gemm_tcgen05_efficiency, without loading the library."""
+    library product adapts its tiling better.
+
+    The gated epilogues run on pairs of CTAs in tiles that follow the rows, and take the library's activation kernel in: for
+    them (whatever ``least``) the two routes' times are estimated from n, N and the width ``K``, each by a form fitted to 432
+    sizes (K 256 to 14336, N 1024 to 28672, n 24 to 4096; 10 % off what was measured on average), and the shorter one is taken.
+    Over those sizes that costs 0.6 % more than always taking the faster route; 12 % at most where a call takes more than 10 us.
+    us, gemm and library: 2048 x 5632, 128 rows 14.0 and 12.7, 300 rows 19.3 and 19.6, 845 rows 32.5 and 40.3; 4096 x 14336, 64
+    rows 43.0 and 44.9, 128 rows 46.0 and 53.7; 4096 x 11008, 128 rows 42.9 and 40.1; 1024 x 2816, 128 rows 7.9 and 7.3, 512
+    rows 10.2 and 12.2."""
     if not USE_TCGEN05 or n <= 0 or N <= 0:
         return False
     if epilogue in _GATED_EPI:
-        return _pair_efficiency(n, N, sm_count() // 2) >= 0.43
+        return _gated_pays(n, N, K, sm_count() // 2)
     sms = sm_count()
     tiles = -(-n // 128) * -(-N // 256)
     waves = -(-tiles // sms)
     return 100.0 * (n / 128.0) * (N / 256.0) / (waves * sms) >= least
 
 
-@functools.lru_cache(maxsize=4096)
-def _pair_efficiency(n: int, N: int, pairs: int) -> float:
-    """The share that pair_plan of csrc/gemm_tcgen05.cu leaves the tensor cores busy."""
+def pair_plan(n: int, N: int, pairs: int) -> tuple:
+    """(rows of x in a tile, waves of tiles) as pair_plan of csrc/gemm_tcgen05.cu chooses them."""
     f_tiles = -(-N // 128)
-    cost = min(-(-(f_tiles * -(-n // bn)) // pairs) * (bn + 100) for bn in range(min(256, -(-n // 16) * 16), 15, -16))
-    return n * (N / 128.0) / (pairs * cost)
+    waves = lambda bn: -(-(f_tiles * -(-n // bn)) // pairs)
+    bn = min(range(min(256, -(-n // 16) * 16), 15, -16), key=lambda bn: waves(bn) * (bn + 100))
+    return bn, waves(bn)
+
+
+@functools.lru_cache(maxsize=4096)
+def _gated_pays(n: int, N: int, K: int, pairs: int) -> bool:
+    bn, waves = pair_plan(n, N, pairs)
+    weights, kblocks = 1e-6 * K * N, -(-K // 64)          # millions of weights of one of the two matrices
+    # us: launch and end; a wave's k blocks, a fixed part and one that goes with the rows, and what a tile costs beside them; what of the
+    # weights' bytes is not hidden behind that
+    here = 3.84 + waves * (kblocks * (0.117 + 0.00078 * bn) + 1.01) + 0.253 * weights
+    # the library's two launches, the weights, the products (halfway to whole tiles of 256 rows), float32 sums written and read back
+    library = 4.6 + 0.28 * weights + 2.4e-3 * weights * 0.5 * (n + -(-n // 256) * 256) + 2.03e-6 * n * N
+    return here < library
 
 
 def gemm(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "bf16", out: Optional[torch.Tensor] = None,

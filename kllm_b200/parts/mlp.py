@@ -91,7 +91,7 @@ class GatedMLP:
                                        bias=self.b_gate, bias_up=self.b_up, activation=self.activation, limit=self.limit,
                                        alpha=self.alpha)
         epilogue = "clamped" if self.activation == "clamped" else "swiglu" if self.plain else None
-        if (epilogue and self.dtype == torch.bfloat16 and kernels.gemm_pays(n, self.inter, epilogue)
+        if (epilogue and self.dtype == torch.bfloat16 and kernels.gemm_pays(n, self.inter, epilogue, K=self.hidden)
                 and kernels.gemm_fits(xn, w_gate, act, epilogue, w_up)):
             # large portions: both products and the activation in one tcgen05 kernel
             kernels.gemm(xn, w_gate, weight_up=w_up, epilogue=epilogue, out=act, limit=self.limit, alpha=self.alpha)

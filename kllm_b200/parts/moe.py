@@ -162,7 +162,7 @@ class RoutedExperts:
             aligned = xn.data_ptr() % 16 == 0 and w_gate.data_ptr() % 16 == 0 and w_up.data_ptr() % 16 == 0
             if aligned and kernels.skinny_fits(xn.shape[0], self.hidden, self.dtype):
                 return kernels.skinny_gemm(w_gate, weight_up=w_up, x=xn, epilogue="swiglu"), None
-            if self.dtype == torch.bfloat16 and kernels.gemm_pays(xn.shape[0], f, "swiglu"):
+            if self.dtype == torch.bfloat16 and kernels.gemm_pays(xn.shape[0], f, "swiglu", K=self.hidden):
                 act = torch.empty((xn.shape[0], f), dtype=self.dtype, device=xn.device)
                 if kernels.gemm_fits(xn, w_gate, act, "swiglu", w_up):
                     return kernels.gemm(xn, w_gate, weight_up=w_up, epilogue="swiglu", out=act), None
