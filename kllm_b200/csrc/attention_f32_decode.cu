@@ -42,7 +42,7 @@ __global__ void __launch_bounds__(THREADS)
 attn_f32_decode_kernel(const Args a) {
     constexpr int LPK = HD / 4, KPW = 32 / LPK, GROUPS = WARPS * KPW;       // lanes of a key, keys a load, lane groups of the CTA
     constexpr int BATCH = UNROLL * KPW, OWN = LPK / GS;                     // keys of a batch; lanes that hold one head's score
-    static_assert(GS <= LPK, "a lane holds one head's score");
+    static_assert(GS <= LPK && UNROLL == 4, "a lane holds one head's score; four keys a batch");
     __shared__ __align__(16) float so[GROUPS][GS][HD];
     __shared__ float sm[GROUPS][GS], sl[GROUPS][GS];
     __shared__ int s_last;
@@ -138,13 +138,15 @@ attn_f32_decode_kernel(const Args a) {
         for (int h = 0; h < GS; h++) {
             const int from_lane = sub * LPK + h * OWN;
             const float al = __shfl_sync(0xffffffffu, alpha, from_lane);
-            o[h].x *= al; o[h].y *= al; o[h].z *= al; o[h].w *= al;
+            float w[UNROLL];
 #pragma unroll
-            for (int u = 0; u < UNROLL; u++) {
-                const float w = __shfl_sync(0xffffffffu, p[u], from_lane);
-                o[h].x = fmaf(w, vb[u].x, o[h].x); o[h].y = fmaf(w, vb[u].y, o[h].y);
-                o[h].z = fmaf(w, vb[u].z, o[h].z); o[h].w = fmaf(w, vb[u].w, o[h].w);
-            }
+            for (int u = 0; u < UNROLL; u++) w[u] = __shfl_sync(0xffffffffu, p[u], from_lane);
+            // the batch's values first, then one addition to what was there: as many instructions, a chain of roundings a quarter as long
+            auto four = [&](float a0, float a1, float a2, float a3) { return fmaf(w[3], a3, fmaf(w[2], a2, fmaf(w[1], a1, w[0] * a0))); };
+            o[h].x = fmaf(o[h].x, al, four(vb[0].x, vb[1].x, vb[2].x, vb[3].x));
+            o[h].y = fmaf(o[h].y, al, four(vb[0].y, vb[1].y, vb[2].y, vb[3].y));
+            o[h].z = fmaf(o[h].z, al, four(vb[0].z, vb[1].z, vb[2].z, vb[3].z));
+            o[h].w = fmaf(o[h].w, al, four(vb[0].w, vb[1].w, vb[2].w, vb[3].w));
         }
     };
     while (at < hi) {                                      // the same for all lanes of a warp

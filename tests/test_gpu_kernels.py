@@ -686,6 +686,42 @@ def test_float32_fused_decode_attention(gs, hd, window):
             assert torch.equal(vc[pg, :, slot].cpu(), torch.from_numpy(vnew[s].reshape(G, hd)))
 
 
+@pytest.mark.parametrize("H,G,hd,L,n_new", [(32, 4, 64, 700, 1), (8, 2, 128, 1500, 1), (32, 4, 64, 333, 333), (8, 2, 128, 700, 200)])
+@pytest.mark.parametrize("sharp", [0.3, 1.0, 3.0])
+def test_float32_attention_is_no_further_from_64_bits_than_multiply_adds(H, G, hd, L, n_new, sharp, monkeypatch):
+    """Four decoding tokens, or a portion, by the kernels that the float32 path takes and by csrc/attention_simt.cu, from nearly even
+    weights, where the sum over the keys rounds most, to a few that stand out: the relative error over all outputs."""
+    from types import SimpleNamespace
+    from kllm_b200 import kernels
+    g = torch.Generator(device="cuda").manual_seed(L + hd)
+    rnd = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    n_req, pages = (4, -(-L // 64)) if n_new == 1 else (1, -(-L // 64))
+    q, kc, vc = rnd(n_req * n_new, H * hd) * sharp, rnd(n_req * pages, G, 64, hd), rnd(n_req * pages, G, 64, hd)
+    i32 = lambda *a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    table = torch.arange(n_req * pages, dtype=torch.int32, device="cuda").view(n_req, pages)
+    dense = lambda c: c.view(n_req, pages, G, 64, hd).transpose(2, 3).reshape(n_req, pages * 64, G, hd)[:, :L]
+    k, v = (dense(c).double().repeat_interleave(H // G, 2) for c in (kc, vc))
+    sc = torch.einsum("rqhd,rkhd->rhqk", q.view(n_req, n_new, H, hd).double(), k) / math.sqrt(hd)
+    pos = torch.arange(L - n_new, L, device="cuda")
+    sc = sc.masked_fill(torch.arange(L, device="cuda")[None] > pos[:, None], -math.inf)
+    want = torch.einsum("rhqk,rkhd->rqhd", torch.softmax(sc, -1), v).reshape(n_req * n_new, H * hd)
+    ctx = SimpleNamespace(n_tokens=n_req * n_new, n_requests=n_req, q_start=i32(*range(0, n_req * n_new + 1, n_new)),
+                          start_pos=i32(*[L - n_new] * n_req), host_n_new=[n_new] * n_req, all_single=n_new == 1, max_ctx=L, split_bound=0,
+                          positions=pos.int().repeat(n_req), token_req=torch.arange(n_req, device="cuda").repeat_interleave(n_new).int())
+    scale, got, plain_way = 1.0 / math.sqrt(hd), torch.empty_like(q), torch.empty_like(q)
+    if n_new == 1:
+        knew, vnew = (dense(c)[:, L - 1].reshape(n_req, G * hd).contiguous() for c in (kc, vc))
+        still = torch.cat([torch.ones(L, hd // 2), torch.zeros(L, hd // 2)], 1).cuda()
+        kernels.attention_decode_f32(got, q, knew, vnew, still, kc, vc, ctx.positions, table, torch.zeros(n_req * G, dtype=torch.int32,
+                                     device="cuda"), H, G, hd, 0, scale, L)
+    else:
+        kernels.attention_simt(got, q, kc, vc, ctx, table, H, G, hd, 0, scale)
+    monkeypatch.setattr(kernels, "USE_TCGEN05", False)
+    kernels.attention_simt(plain_way, q, kc, vc, ctx, table, H, G, hd, 0, scale)
+    error = [float((o.double() - want).norm() / want.norm()) for o in (got, plain_way)]
+    assert error[0] <= error[1], error
+
+
 @pytest.mark.parametrize("gs,hd", [(1, 64), (8, 64), (16, 64), (4, 128)])
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("L,keys", [(10, [8]), (258, [256]), (265, list(range(260, 264))), (300, list(range(256))), (70, [0])])
