@@ -79,17 +79,17 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 
-// The warps' values, `stride` floats apart, added in pairs: warp 0's and warp 8's, ..., then the halves' halves.  One after the other
-// they rounded 8 to 9 % more over the sums of this file's sizes than the 8 parts of K of an earlier form; in pairs it is less than that.
+// The warps' values, `stride` floats apart, added in pairs: 0 and 1, 2 and 3, ..., then the pairs'.  One after the other they rounded 8 to
+// 9 % more over the sums of this file's sizes than the 8 parts of K of an earlier form; in pairs it is less than that.  (Warp w and
+// w + 8 first, which keeps eight sums at a time, cost the stream of weights its registers: a decode step of 8 tokens 1827 us, 1768 this way.)
 __device__ __forceinline__ float sum_warps(const float* p, int stride) {
-    float v[WARPS];
+    float half[2];
 #pragma unroll
-    for (int w = 0; w < WARPS; w++) v[w] = p[w * stride];
-#pragma unroll
-    for (int h = WARPS / 2; h >= 1; h >>= 1)
-#pragma unroll
-        for (int w = 0; w < h; w++) v[w] += v[w + h];
-    return v[0];
+    for (int h = 0; h < 2; h++) {
+        const float* q = p + h * 8 * stride;
+        half[h] = ((q[0] + q[stride]) + (q[2 * stride] + q[3 * stride])) + ((q[4 * stride] + q[5 * stride]) + (q[6 * stride] + q[7 * stride]));
+    }
+    return half[0] + half[1];
 }
 
 // EXACT: every warp's part of K is a whole number of batches.

@@ -961,8 +961,7 @@ def test_float32_skinny_gemm_adds_its_parts_of_k_in_pairs(K):
     x[0, [k for k in firsts if k < K]] = 1.0               # products are exact, the other values of k add 0
     v = [w[:, k] if k < K else np.zeros(N, np.float32) for k in firsts]
     while len(v) > 1:
-        half = len(v) // 2
-        v = [a + b for a, b in zip(v[:half], v[half:])]
+        v = [a + b for a, b in zip(v[::2], v[1::2])]
     got = kernels.skinny_gemm(dev(w), x=dev(x), epilogue="f32").cpu().numpy()
     assert np.array_equal(got[0], v[0]) and not got[1].any()
 
