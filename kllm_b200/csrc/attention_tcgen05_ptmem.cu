@@ -133,7 +133,6 @@ __device__ __forceinline__ void tmem_st32(unsigned taddr, const uint32_t (&r)[32
                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
 // byte offset of 16-byte piece `ch` (0..7) of row `r` inside a swizzled panel of 128-byte rows
 __device__ __forceinline__ unsigned swz(int r, int ch) {

@@ -30,8 +30,10 @@
 //   warp 1     of the leader: one thread issues the 12 tcgen05.mma (2 k steps x 6 terms) of a block into one of two accumulators,
 //   warps 2-9  fetch each finished accumulator (tcgen05.ld) and add it to their sums: a thread owns one column of the result for
 //              half of the tile's rows, and stores them at the end of the tile, 32 neighbouring columns a warp.
-// Where whole-K tiles leave pairs idle (few rows, narrow matrices) the k range is cut into splits of whole blocks, each a unit
-// of work of its own that leaves its sums in a workspace; a third kernel adds them in split order.
+// The k range is cut into splits of whole blocks (make_plan) that are summed by themselves and then added in split order: that is part of
+// the result, and a long K rounds less this way.  Where whole-K tiles leave pairs idle (few rows, narrow matrices) a split is a
+// unit of work of its own that leaves its sums in a workspace, and a third kernel adds them; else (sums_stay) a unit has all of K and
+// its threads put the sums of the splits before aside in tensor memory.
 //
 // The numbers are split after a multiplication by 2^24, an accumulator is multiplied by 2^-48 where it is added to the sum: bfloat16 ends at 2^-133 as float32 does
 // at 2^-149, so that without it numbers below 2^-110 would lose digits.  With it every float32 below 2^104 is split exactly.
@@ -168,12 +170,14 @@ struct Args {
     int64_t ldx, ldw;
     float* y;
     int64_t ldy, split_stride;              // split_stride: elements between the workspace's splits
-    int M, N, K, bn, stages, splits, blocks_per_split;      // N: columns of the result (EPI_PARTIAL: of the workspace)
+    int M, N, K, bn, stages;                // N: columns of the result (EPI_PARTIAL: of the workspace)
+    int units_of_k, blocks_per_unit, blocks_per_split;      // units a tile's K is cut into; k blocks
     int x_rows, w_rows;                     // rows of a plane of x and of W
     int* status;
 };
 
-template <int EPI>
+// ASIDE: a unit has several splits, bn is at most 128
+template <int EPI, bool ASIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Args a) {
     extern __shared__ unsigned char smem_raw[];
@@ -186,7 +190,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     const int bn = a.bn, stages = a.stages;
     const unsigned b_plane = (unsigned)bn * 32, stage_bytes = 3 * (A_PLANE + b_plane);           // bn / 2 rows of 64 bytes
     const int t_tiles = (a.M + bn - 1) / bn, tiles = t_tiles * ((a.w_rows + 2 * BM - 1) / (2 * BM));
-    const int units = tiles * a.splits, pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
+    const int units = tiles * a.units_of_k, pairs = gridDim.x >> 1, first = blockIdx.x >> 1;
     const int kblocks = (a.K + BK - 1) / BK;
     volatile int* abort_flag = &s_abort;
 
@@ -217,7 +221,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int unit = first; ok && unit < units; unit += pairs) {
             const int split = unit / tiles, tile = unit - split * tiles;
             const int t0 = tile % t_tiles * bn + (int)rank * (bn / 2), w0 = (tile / t_tiles * 2 + (int)rank) * BM;
-            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+            const int kb0 = split * a.blocks_per_unit, kb1 = min(kblocks, kb0 + a.blocks_per_unit);
             for (int kb = kb0; kb < kb1; kb++) {
                 ok = mbar_wait_warp(&bar_empty[s], ph ^ 1u, abort_flag, a.status, 1);
                 if (!ok) break;
@@ -262,7 +266,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             bool ok = true;
             for (int unit = first; ok && unit < units; unit += pairs) {
                 const int split = unit / tiles;
-                const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
+                const int kb0 = split * a.blocks_per_unit, kb1 = min(kblocks, kb0 + a.blocks_per_unit);
                 for (int kb = kb0; kb < kb1; kb++) {
                     ok = mbar_wait_warp(&bar_acc_empty[acc], acc_ph ^ 1u, abort_flag, a.status, 2) &&
                          mbar_wait_warp(&bar_full[s], ph, abort_flag, a.status, 3);
@@ -294,6 +298,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         const unsigned lane_base = (unsigned)(quarter * 32) << 16;
         const int chunks = (bn + 31) / 32, c_lo = half == 0 ? 0 : (chunks + 1) / 2, mine = half == 0 ? (chunks + 1) / 2 : chunks / 2;
         const bool upper = lane >= 16;
+        constexpr int CHUNKS = ASIDE ? 2 : 4;                            // most that a warp has
         int acc = 0;
         unsigned acc_ph = 0;
         bool ok = true;
@@ -301,33 +306,55 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             const int split = unit / tiles, tile = unit - split * tiles;
             const int t0 = tile % t_tiles * bn + c_lo * 32, w0 = (tile / t_tiles * 2 + (int)rank) * BM + quarter * 32;
             const int t_hi = min(tile % t_tiles * bn + bn, a.M);     // rows of x from t0 on that are this tile's
-            const int kb0 = split * a.blocks_per_split, kb1 = min(kblocks, kb0 + a.blocks_per_split);
-            float sum[4][32];
+            const int kb0 = split * a.blocks_per_unit, kb1 = min(kblocks, kb0 + a.blocks_per_unit);
+            float sum[CHUNKS][32];
+            int kb = kb0;
+            do {                                                    // one split (ASIDE), or all there is
+                const int end = ASIDE ? min(kb1, kb + a.blocks_per_split) : kb1;
 #pragma unroll
-            for (int c = 0; c < 4; c++)
+                for (int c = 0; c < CHUNKS; c++)
 #pragma unroll
-                for (int j = 0; j < 32; j++) sum[c][j] = 0.f;
-            for (int kb = kb0; kb < kb1; kb++) {
-                ok = mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, a.status, 4);
-                if (!ok) break;
-                tc_fence_after();
-                const unsigned t = tmem + lane_base + (unsigned)(acc * BN + c_lo * 32);
+                    for (int j = 0; j < 32; j++) sum[c][j] = 0.f;
+                for (; kb < end; kb++) {
+                    ok = mbar_wait(&bar_acc_full[acc], acc_ph, abort_flag, a.status, 4);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const unsigned t = tmem + lane_base + (unsigned)(acc * BN + c_lo * 32);
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    if (c >= mine) break;
-                    float v[32];
-                    tmem_ld32(t + c * 32, v);
-                    tmem_ld_wait();
+                    for (int c = 0; c < CHUNKS; c++) {
+                        if (c >= mine) break;
+                        float v[32];
+                        tmem_ld32(t + c * 32, v);
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; j++) sum[c][j] = fmaf(v[j], UNSCALE, sum[c][j]);      // one rounding, as the add
+                        for (int j = 0; j < 32; j++) sum[c][j] = fmaf(v[j], UNSCALE, sum[c][j]);      // one rounding, as the add
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(leader_addr(&bar_acc_empty[acc]));
+                    acc ^= 1;
+                    if (acc == 0) acc_ph ^= 1u;
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(leader_addr(&bar_acc_empty[acc]));
-                acc ^= 1;
-                if (acc == 0) acc_ph ^= 1u;
-            }
-            ok = __all_sync(0xffffffffu, ok);                       // the warp leaves together or stays for its votes below
+                ok = __all_sync(0xffffffffu, ok);                   // the warp leaves together or stays for what follows
+                if (ASIDE && ok) {
+                    unsigned kept = tmem + (unsigned)(BN / 2);      // columns that accumulators of up to 128 leave free
+                    asm volatile("" : "+r"(kept));                  // not worth a register in the loop above
+                    kept += lane_base + (unsigned)(c_lo * 32);
+#pragma unroll
+                    for (int c = 0; c < CHUNKS; c++) {
+                        if (c >= mine) break;
+                        if (kb > a.blocks_per_split) {
+                            float v[32];
+                            tmem_ld32(kept + c * 32, v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 32; j++) sum[c][j] = v[j] + sum[c][j];
+                        }
+                        if (kb < kb1) tmem_st32(kept + c * 32, sum[c]);
+                    }
+                    tmem_st_wait();
+                }
+            } while (ASIDE && ok && kb < kb1);
             if (!ok) break;
             // this lane's column; gated: the lower lanes finish the even rows of x, the upper ones the odd rows of the same columns
             const int col = EPI == EPI_SWIGLU ? w0 / 2 + (lane & 15) : w0 + lane;
@@ -335,7 +362,7 @@ gemm_f32_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             float* y = a.y + (EPI == EPI_PARTIAL ? split * a.split_stride : 0) + (live ? col : 0);
             constexpr int PER = EPI == EPI_SWIGLU ? 16 : 32;        // values a lane stores of a chunk
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < CHUNKS; c++) {
                 if (c >= mine) break;
                 float* s = sum[c];
                 auto row = [&](int j) { return t0 + c * 32 + (EPI == EPI_SWIGLU ? 2 * j + (int)upper : j); };
@@ -479,11 +506,11 @@ int planes_map(CUtensorMap* out, const bf16* planes, int64_t rows, int K, int kp
     return 0;
 }
 
-template <int EPI>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, cudaStream_t s) {
+template <int EPI, bool ASIDE>
+int launch_kernel(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, cudaStream_t s) {
     static bool attr_set = false;
     if (!attr_set) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tc5_kernel<EPI, ASIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) {
             snprintf(g_kllm_err, sizeof(g_kllm_err), "gemm float32 (tcgen05): %d bytes of shared memory refused: %s", SMEM_BYTES,
                      cudaGetErrorString(e));
@@ -491,10 +518,15 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, cudaStre
         }
         attr_set = true;
     }
-    const long long units = (long long)((a.M + a.bn - 1) / a.bn) * ((a.w_rows + 2 * BM - 1) / (2 * BM)) * a.splits, pairs = sm_count() / 2;
+    const long long units = (long long)((a.M + a.bn - 1) / a.bn) * ((a.w_rows + 2 * BM - 1) / (2 * BM)) * a.units_of_k, pairs = sm_count() / 2;
     const int grid = 2 * (int)(units < pairs ? units : pairs);
-    kllm_launch((gemm_f32_tc5_kernel<EPI>), dim3(grid), dim3(THREADS), SMEM_BYTES, s, mw, mx, a);
+    kllm_launch((gemm_f32_tc5_kernel<EPI, ASIDE>), dim3(grid), dim3(THREADS), SMEM_BYTES, s, mw, mx, a);
     KLLM_LAUNCH_STATUS();
+}
+
+template <int EPI>
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Args& a, cudaStream_t s) {
+    return a.blocks_per_split < a.blocks_per_unit ? launch_kernel<EPI, true>(mw, mx, a, s) : launch_kernel<EPI, false>(mw, mx, a, s);
 }
 
 // beside: behind a product, to run on the SMs that it occupies
@@ -517,10 +549,10 @@ int launch_reduce(float* y, int64_t ldy, const float* ws, int64_t split_stride, 
 }
 
 // How a product is cut: W in pieces of `piece` output columns (whole tiles, the last piece takes the rest), a piece's K
-// in `splits` ranges.  The cost that is made least, in k blocks of one CTA (0.8 us): a unit costs its blocks and about 3
-// for filling the pipeline and storing; a launch about 3; split sums are written and read at about 4 MB a block's time.
+// in `splits` ranges, which one unit sums with the earlier ones put aside (sums_stay) or each a unit of its own.
 struct Plan {
     int piece, splits, kp;
+    bool sums_stay;
     int64_t x_bytes, w_bytes, ws_bytes;
 };
 int64_t up256(int64_t b) { return (b + 255) / 256 * 256; }
@@ -539,6 +571,25 @@ int pick_bn(int M, int w_tiles, int splits) {
     return best_bn;
 }
 
+// Whether tiles of whole K, their rows of x chosen to fit, do better than a unit a split with the splits' workspace and the kernel behind:
+// they keep the pairs busy for most of the time, their splits' sums fit beside the accumulators, and they take no more than 1.1
+// times as long, by a k block's 0.22 + 0.0036 bn us (5632 x 2048, whole K: 700 rows in tiles of 80 0.53, 1003 of 112 0.61, 2048 of 240
+// 1.1), 1.5 for a split's sums to the workspace, and 2.4 and 5 MB a us for the kernel behind.  5632 x 2048, 700 rows: 112 us whole,
+// 93 by splits; 2048 x 2560, 845 rows: 51 and 59.
+bool whole_k_pays(int M, int w_tiles, int kblocks, int splits) {
+    const int pairs = sm_count() / 2, bn = pick_bn(M, w_tiles, 1), bn_split = pick_bn(M, w_tiles, splits);
+    auto waves = [&](int rows, int units) { return ((long long)w_tiles * units * ((M + rows - 1) / rows) + pairs - 1) / pairs; };
+    auto block = [](int rows) { return 0.22 + 0.0036 * (rows > 64 ? rows : 64); };
+    if (bn > BN / 2 || 10.0 * w_tiles * M < 6.0 * pairs * waves(bn, 1) * (bn > 96 ? bn : 96)) return false;
+    const double whole = waves(bn, 1) * kblocks * block(bn);
+    const double split = waves(bn_split, splits) * ((kblocks + splits - 1) / splits * block(bn_split) + 1.5) + 2.4 +
+                         8e-6 * splits * (double)M * w_tiles * (2 * BM) / 5;
+    return whole <= 1.1 * split;
+}
+
+// The splits decide in which order a result is added up, so their number does not follow the way the kernel is built: the count is that
+// of tiles of 128 rows of x, one for every SM at a time.  Least is a sum of k blocks (0.8 us of such a tile) in which a tile costs its
+// blocks and 3, a launch 3, and sums are written and read at 4 MB a block's time.
 Plan make_plan(int M, int N, int K, int epilogue) {
     Plan p;
     const bool gated = epilogue == EPI_SWIGLU;
@@ -564,17 +615,11 @@ Plan make_plan(int M, int N, int K, int epilogue) {
             if (best < 0 || all < best) { best = all; p.piece = c == n_tiles ? N : (int)c * nout; p.splits = s; }
         }
     }
-    // Tiles of whole K, their rows of x chosen to fit, save the splits' workspace and the kernel behind where they keep the pairs
-    // busy for most of the time.
-    if (p.splits > 1 && p.piece == N) {
-        const int bn = pick_bn(M, (int)n_tiles, 1);
-        const long long waves = (n_tiles * ((M + bn - 1) / bn) + sms / 2 - 1) / (sms / 2);
-        if (10.0 * n_tiles * M >= 6.0 * (sms / 2) * waves * (bn > 96 ? bn : 96)) p.splits = 1;
-    }
     const int64_t cols = gated ? (p.piece + 15) / 16 * 32 : p.piece;
     p.x_bytes = up256(6LL * M * p.kp);
     p.w_bytes = up256(6LL * cols * p.kp);
-    p.ws_bytes = p.splits > 1 ? up256(4LL * p.splits * M * cols) : 0;
+    p.sums_stay = p.splits > 1 && p.piece == N && whole_k_pays(M, (int)n_tiles, kblocks, p.splits);
+    p.ws_bytes = p.splits > 1 && !p.sums_stay ? up256(4LL * p.splits * M * cols) : 0;
     return p;
 }
 
@@ -628,7 +673,10 @@ extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, 
     int r = launch_split(false, (const float*)x, nullptr, ldx, M, K, px, M, p.kp, s);
     if (r) return r;
     Args a;
-    a.M = M; a.K = K; a.splits = p.splits; a.blocks_per_split = (kblocks + p.splits - 1) / p.splits; a.status = status;
+    const bool whole = p.splits == 1 || p.sums_stay;
+    a.M = M; a.K = K; a.blocks_per_split = (kblocks + p.splits - 1) / p.splits; a.status = status;
+    a.units_of_k = whole ? 1 : p.splits;
+    a.blocks_per_unit = whole ? kblocks : a.blocks_per_split;
     a.x_rows = M; a.x = (const float*)x; a.ldx = ldx; a.ldw = ldw;
     // The last piece, the shortest, comes first: its splitting is the one that no product hides.
     for (int i = 0; i < pieces; i++) {
@@ -639,16 +687,16 @@ extern "C" int kllm_gemm_f32_tcgen05(const void* x, int64_t ldx, const void* w, 
         a.w = (const float*)w + n0 * ldw; a.w_up = gated ? (const float*)w_up + n0 * ldw : nullptr;
         // Beside the product before, which started when its own planes were ready, that is when the product that read this
         // buffer was over; behind split sums' last kernel as usual.
-        r = launch_split(i > 0 && p.splits == 1, a.w, a.w_up, ldw, cols, K, planes, a.w_rows, p.kp, s);
+        r = launch_split(i > 0 && whole, a.w, a.w_up, ldw, cols, K, planes, a.w_rows, p.kp, s);
         if (r) return r;
-        a.bn = pick_bn(M, (a.w_rows + 2 * BM - 1) / (2 * BM), p.splits);
+        a.bn = pick_bn(M, (a.w_rows + 2 * BM - 1) / (2 * BM), a.units_of_k);
         a.stages = (SMEM_BYTES - 1024) / (3 * (A_PLANE + a.bn * 32));
         if (a.stages > MAX_STAGES) a.stages = MAX_STAGES;
         CUtensorMap mw, mx;
         r = planes_map(&mw, planes, 3LL * a.w_rows, K, p.kp, BM);
         if (!r) r = planes_map(&mx, px, 3LL * M, K, p.kp, a.bn / 2);
         if (r) return r;
-        if (p.splits == 1) {
+        if (whole) {
             a.N = cols; a.y = yp; a.ldy = ldy; a.split_stride = 0;
             r = epilogue == EPI_STORE ? launch<EPI_STORE>(mw, mx, a, s) : epilogue == EPI_ADD ? launch<EPI_ADD>(mw, mx, a, s)
                                                                                              : launch<EPI_SWIGLU>(mw, mx, a, s);

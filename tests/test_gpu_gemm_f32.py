@@ -152,6 +152,33 @@ def test_infinities(rows, cols, k, epilogue):
         assert torch.equal(kind(got), kind(want)), kind.__name__
 
 
+@pytest.mark.parametrize("stay,part,cols,k,epilogue,splits", [(500, 400, 2560, 2048, "f32", 3), (700, 600, 2048, 2048, "add", 3),
+                                                              (250, 190, 2816, 1024, "swiglu", 3), (870, 800, 516, 1500, "swiglu", 4)])
+def test_splits_are_added_in_one_order_whoever_adds_them(stay, part, cols, k, epilogue, splits):
+    """With ``stay`` rows a pair sums all of K, the splits before put aside in tensor memory; with ``part`` rows every split is
+    a unit of work and a kernel behind adds them: rows that both have come out the same to the bit, and as near to 64 bits as
+    sums of K / splits are."""
+    from kllm_b200 import kernels
+    from kllm_b200.csrc.build import load_library
+    lib, epi, up = load_library("gemm_f32_tcgen05"), ("f32", "add", "swiglu").index(epilogue), lambda b: -(-b // 256) * 256
+    kp, w_rows = -(-k // 8) * 8, -(-cols // 16) * 32 if epilogue == "swiglu" else cols
+    for rows, sums in ((stay, 0), (part, up(4 * splits * part * w_rows))):
+        cut, size = (ctypes.c_int * 2)(), ctypes.c_int64(0)
+        lib.kllm_gemm_f32_tcgen05_plan(rows, cols, k, epi, ctypes.addressof(cut), ctypes.addressof(cut) + 4)
+        lib.kllm_gemm_f32_tcgen05_workspace(rows, cols, k, epi, ctypes.byref(size))
+        assert tuple(cut) == (cols, splits) and size.value == up(6 * rows * kp) + up(6 * w_rows * kp) + sums
+    g = torch.Generator(device="cuda").manual_seed(stay + k)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    x, w, w2, y = rnd(stay, k), rnd(cols, k) * 0.05, rnd(cols, k) * 0.05, rnd(stay, cols)
+    got = []
+    for rows in (stay, part):
+        out = y[:rows].clone()
+        kernels.gemm_f32(x[:rows], w, weight_up=w2 if epilogue == "swiglu" else None, epilogue=epilogue, out=out)
+        got.append(out)
+    assert torch.equal(got[0][:part], got[1])
+    _product(stay, cols, k, epilogue)
+
+
 def test_route():
     """Which float32 products run here, and that the general product takes the route and agrees with float64."""
     from kllm_b200 import kernels
