@@ -3,7 +3,8 @@
 // The CUDA cores reach a quarter of their rate on this (csrc/attention_simt.cu: 257 us for 1003 tokens, 32 heads of 64 on
 // 4 kv heads, 17 TFLOP/s).  Here every number of Q, K, V and of the probabilities is the sum of three bfloat16 numbers,
 //     v = v0 + v1 + v2,  v0 = bf16(v), v1 = bf16(v - v0), v2 = bf16(v - v0 - v1),
-// and a product of two is the six products whose parts matter at 24 bits (x2 y0 + x0 y2 + x1 y1 + x1 y0 + x0 y1, then x0 y0).
+// and a product of two is the six products whose parts matter at 24 bits (x2 y0 + x0 y2 + x1 y1 + x1 y0 + x0 y1, then x0 y0); x1 y2,
+// x2 y1 and x2 y2, below 2^-24 of it, are left out.
 // The five small ones and the large one have accumulators of their own that hold one score, or one key tile of one output, and
 // are then added by the rounding adds of the CUDA cores: what the tensor cores cut off in their accumulation cannot drift over a
 // long context.
@@ -13,9 +14,9 @@
 // A CTA of four warps has a tile of up to 64 rows, a row being one (query token, head), 16 rows a warp.  Key tiles of KT keys come
 // as float32 by asynchronous copies while the tile before is being multiplied, all threads split them into three bfloat16 planes
 // (16-byte pieces, exclusive-or swizzled), and the warps read the planes with ldmatrix.  Two CTAs an SM at head size 64 (104 KB
-// each), one at 128.  Measured: 1003 tokens, 32 heads
-// of 64 on 4 kv heads 120 us a layer (the CUDA cores 257); bound by the rate of mma.sync and, between two meetings of the CTA, by the
-// splitting of a key tile.
+// each), one at 128.  Measured: 1003 tokens, 32 heads of 64 on 4 kv heads 121 us a layer (the CUDA cores 257), the tensor cores'
+// pipe busy for 38 % of it, DRAM for 1 %: two CTAs of four warps are all that 222 registers and 104 KB leave an SM, and they
+// split every key tile between two meetings of the CTA.  Relative error of the outputs about half the multiply-add kernel's.
 //
 // Masks, sinks, slopes, window and kept keys as in attention_simt.cu, expf and one division at the end too.  V is split after a
 // multiplication by 2^24, which the division takes back, so that small values keep their digits.  An operand that is not finite,

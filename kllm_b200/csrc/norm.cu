@@ -74,7 +74,8 @@ __device__ __forceinline__ float4 load4(const bf16* p) {
 // The widths that are multiples of 4 up to kThreads * 4 * kVec, 16-byte rows: a thread keeps its V float4 of the row in
 // registers between the sum of squares and the scaling.  One CTA per row and as many threads as the row has float4, up to
 // kThreads, so that all of a row's loads are in flight at once: a row's latency is what a step of few rows waits for, and a
-// step of many is bound by its bytes either way.  64 rows of 2048: 4.3 us with a warp per row, 2.0 this way (launched back to back); the gains do not depend on the kernel before and are fetched while it ends.
+// step of many is bound by its bytes either way.  64 rows of 2048: 4.3 us with a warp per row, 2.0 this way (launched back to
+// back); the gains do not depend on the kernel before and are fetched while it ends.
 //
 // Who loads an element does not say who adds it.  LANES (bfloat16 rows of up to kLanesMost): 32 lanes, lane l the squares of the float4
 // l, l + 32, ..., which reach them through shared memory in the time that an exchange of partial sums takes; else thread t those of

@@ -1602,10 +1602,11 @@ def gemm(x: torch.Tensor, weight: torch.Tensor, *, epilogue: str = "bf16", out: 
 
 
 # From these sizes on a float32 product runs on the tensor cores (csrc/gemm_f32_tcgen05.cu), below them through the
-# library, both timed over 9 to 2048 rows.  The weights' three parts are written and read back by every call: at 16 rows
-# that costs what the tensor cores save (the four products of a TinyLlama layer: 204 us against 218), at 33 rows 216 us
-# against 322.  A matrix whose parts are larger than L2 goes through HBM again: 32000 x 2048 takes 271 us against the
-# library's 178 at 64 rows and 302 against 313 at 128.  Small matrices are latency: 1024 x 512 at 1003 rows 31.8 against 30.8.
+# library.  The weights' three parts are written and read back by every call: the four products of a TinyLlama layer take
+# 163 us here against 185 at 16 rows, 170 against 286 at 33; gate and up alone (2048 x 11264) 80 against 63 at 32 rows and
+# 80 against 94 at 33.  A matrix whose parts are larger than L2 goes through HBM again: 32000 x 2048 takes 233 us against the
+# library's 169 at 64 rows, 234 against 310 at 96 and 254 against 308 at 128.  Small matrices are latency: 1024 x 512
+# 12.0 against 9.5 at 9 rows, 12.8 against 15.1 at 33; the line below a million weights is kept, it decides results' bits.
 GEMM_F32_LEAST_ROWS = 33
 GEMM_F32_LEAST_WEIGHTS = 1 << 20
 GEMM_F32_L2_WEIGHTS = 25 << 20          # 150 MB of parts: about what L2 and the write-back in flight hide

@@ -745,6 +745,16 @@ def test_float32_fused_decode_attention_with_keys_that_are_not_finite(gs, hd, va
     same_as_arithmetic(out, want)
 
 
+def test_the_float32_decode_route_asks_for_what_the_kernel_takes():
+    from kllm_b200 import kernels
+    from kllm_b200.csrc.build import load_library
+    fits = load_library("attention_f32_decode").kllm_attention_f32_decode_fits
+    for heads in (1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 64):
+        for kv in (1, 2, 3, 4, 8, 16):
+            for hd in (16, 32, 48, 64, 96, 128, 256):
+                assert kernels.attention_decode_f32_fits(heads, kv, hd) == bool(fits(heads, kv, hd)), (heads, kv, hd)
+
+
 def test_tcgen05_form_follows_the_measurements():
     from kllm_b200 import kernels
     assert kernels.tcgen05_form(128, 4, 8, 2048, 1, 2048) == "tmem"
