@@ -234,12 +234,13 @@ rmsnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y, const flo
 
 // The same with the row in registers (V float4 a thread; widths as in add_rmsnorm_row_kernel), the sums in the order of the kernel
 // above: the elements reach its threads through shared memory.  8 rows of 2048, launched back to back: 10.0 us with one
-// element a load and three passes through memory, 2.0 this way; 2048 rows 14.0 and 9.3.
+// element a load and three passes through memory, 1.9 this way; 2048 rows 14.0 and 8.6.
 __host__ __device__ constexpr int add_threads(int d) { return d <= 512 ? 64 : (d <= 2048 ? 128 : kThreads); }
 __host__ __device__ constexpr int add_block(int d) { return row_threads(d) > add_threads(d) ? row_threads(d) : add_threads(d); }
 
 // The sum of the squares of a row of d = 4 n4 numbers, of which this thread holds the float4 threadIdx.x + k * blockDim.x in v[k], by
-// add_threads(d) threads, thread t the elements t, t + add_threads(d), ...; every thread gets it.  row: shared, 4 V blockDim.x floats.
+// add_threads(d) threads, thread t the elements t, t + add_threads(d), ...; every thread gets it, in the order of block_sum.
+// row: shared, 4 V blockDim.x floats; red: shared, 8 floats of this call's own.
 template <int V>
 __device__ __forceinline__ float squares_by_element(const float4 (&v)[V], int n4, float* row, float* red) {
 #pragma unroll
@@ -251,9 +252,8 @@ __device__ __forceinline__ float squares_by_element(const float4 (&v)[V], int n4
     // widths up to 1024 have a block of as many threads as they have float4; wider ones kThreads
     const int adders = V == 1 ? add_threads(4 * n4) : V == 2 ? add_threads(2048) : kThreads, held = V == 1 ? 4 * blockDim.x : 4 * V * kThreads;
     constexpr int MOST = V == 1 ? 8 : V == 2 ? 16 : 4 * V;
-    float ss = 0.f;
     if (threadIdx.x < adders) {
-        float e[MOST];                                     // all loads before the chain of additions
+        float e[MOST], ss = 0.f;                           // all loads before the chain of additions
 #pragma unroll
         for (int k = 0; k < MOST; k++) {
             const int i = threadIdx.x + k * adders;
@@ -261,8 +261,16 @@ __device__ __forceinline__ float squares_by_element(const float4 (&v)[V], int n4
         }
 #pragma unroll
         for (int k = 0; k < MOST; k++) ss += e[k] * e[k];
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
     }
-    return block_sum(ss, red);                             // whose barriers also keep the row until all have read it
+    __syncthreads();
+    // two, four or eight warps, in halves
+    const float4 lo = load4(red);
+    if (adders == 64) return lo.x + lo.y;
+    if (adders == 128) return (lo.x + lo.z) + (lo.y + lo.w);
+    const float4 hi = load4(red + 4);
+    return ((lo.x + hi.x) + (lo.z + hi.z)) + ((lo.y + hi.y) + (lo.w + hi.w));
 }
 
 template <typename T, int V>
@@ -270,7 +278,7 @@ __global__ void __launch_bounds__(kThreads)
 rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ gain, float eps,
                        T* __restrict__ out, const float* __restrict__ gain2, float eps2, int d) {
     extern __shared__ __align__(16) float row[];
-    __shared__ float red[32];
+    __shared__ __align__(16) float red[2][8];
     const int n4 = d >> 2;
     float4 g[V], v[V], h[V];
 #pragma unroll
@@ -290,7 +298,7 @@ rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const
             h[k] = load4(xr + 4 * i);
         }
     }
-    const float scale = rsqrtf(squares_by_element<V>(v, n4, row, red) / (float)d + eps);
+    const float scale = rsqrtf(squares_by_element<V>(v, n4, row, red[0]) / (float)d + eps);
     T* orow = out ? out + (int64_t)blockIdx.x * d : nullptr;
 #pragma unroll
     for (int k = 0; k < V; k++) {
@@ -308,7 +316,7 @@ rmsnorm_add_row_kernel(float* __restrict__ x, const float* __restrict__ y, const
         const int i = threadIdx.x + k * blockDim.x;
         if (i < n4) g[k] = load4(gain2 + 4 * i);
     }
-    const float scale2 = rsqrtf(squares_by_element<V>(h, n4, row, red) / (float)d + eps2);
+    const float scale2 = rsqrtf(squares_by_element<V>(h, n4, row, red[1]) / (float)d + eps2);
 #pragma unroll
     for (int k = 0; k < V; k++) {
         const int i = threadIdx.x + k * blockDim.x;
